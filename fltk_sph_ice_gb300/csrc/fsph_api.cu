@@ -650,12 +650,15 @@ int boundary_build(fsph_ctx *c) {
     DevParams p = make_dev(c->P, c->nb, 1.0f); /* n = the boundary count */
     launch_hash(p, c->b_in, c->b_key, c->b_rank, c->b_count, s);
     launch_scan(c->b_count, c->b_cell, c->block_sums, c->ncells, s);
-    launch_scatter_sort(p, c->b_key, c->b_rank, c->b_cell, c->b_id, c->ncells, s); /* b_id: slot -> input */
+    CellOrder o = launch_scatter(p, c->b_key, c->b_rank, c->b_cell, c->b_id, s);
+    o.sorted = c->b_rank; /* free once the scatter has run */
     Gather g{};
     g.n4 = 1;
     g.src4[0] = c->b_in;
     g.dst4[0] = c->b_pos;
-    launch_gather(c->nb, c->b_id, g, nullptr, s);
+    launch_gather(c->nb, o, g, nullptr, s);
+    FSPH_CUDA(c, cudaMemcpyAsync(c->b_id, c->b_rank, (size_t)c->nb * sizeof(unsigned int), cudaMemcpyDeviceToDevice,
+                                 s)); /* b_id: slot -> input */
     attach_boundary(c, p);
     launch_boundary_near(p, c->ncells, c->b_near, s);
     launch_boundary_volume(p, c->b_scale, s);
@@ -669,18 +672,21 @@ int boundary_build(fsph_ctx *c) {
 
 /* ---------------- building blocks of a step ---------------- */
 
-/* perm = the slots in (cell, previous slot) order, from the hashed cells:
+/* the order of the slots by (cell, previous slot), from the hashed cells:
  * the counting sort (grid_sort 0) or the LSD radix sort (grid_sort 1) */
-void sort_cells(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
-    if (c->P.grid_sort == 1) launch_radix_sort_cells(p.n, c->key, c->ncells, c->radix, c->perm, s);
-    else launch_scatter_sort(p, c->key, c->rank, c->cell_start, c->perm, c->ncells, s);
+CellOrder sort_cells(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
+    if (c->P.grid_sort != 1) return launch_scatter(p, c->key, c->rank, c->cell_start, c->perm, s);
+    launch_radix_sort_cells(p.n, c->key, c->ncells, c->radix, c->perm, s);
+    CellOrder o;
+    o.perm = c->perm;
+    return o;
 }
 
-/* sort of the slots of x (device order) by cell: leaves perm */
-void enqueue_sort(fsph_ctx *c, const DevParams &p, const float4 *x, cudaStream_t s) {
+/* the order of the slots of x (device order) by cell */
+CellOrder enqueue_sort(fsph_ctx *c, const DevParams &p, const float4 *x, cudaStream_t s) {
     launch_hash(p, x, c->key, c->rank, c->count, s);
     launch_scan(c->count, c->cell_start, c->block_sums, c->ncells, s);
-    sort_cells(c, p, s);
+    return sort_cells(c, p, s);
 }
 
 /* the grid rebuild used inside the loop and after it (positions = current x*) */
@@ -688,10 +694,10 @@ void enqueue_rebuild(fsph_ctx *c, const DevParams &p, int it, cudaStream_t s) {
     BufSet &I = c->set[it], &O = c->set[1 - it];
     launch_hash_parity(p, c->ppos[0], c->ppos[1], c->ctl, c->key, c->rank, c->count, s);
     launch_scan(c->count, c->cell_start, c->block_sums, c->ncells, s);
-    sort_cells(c, p, s);
+    const CellOrder o = sort_cells(c, p, s);
     const bool ws = c->P.warm_start != 0 || c->P.collect_features != 0;
     float *t_lam = reinterpret_cast<float *>(c->rank); /* free once the scatter has run */
-    launch_rebuild_gather(p.n, c->perm, c->ctl, I.pos, c->ppos[0], c->ppos[1], I.id, I.attr, c->dens, O.pos, O.vel,
+    launch_rebuild_gather(p.n, o, c->ctl, I.pos, c->ppos[0], c->ppos[1], I.id, I.attr, c->dens, O.pos, O.vel,
                           O.id, O.attr, c->pres, c->key, c->nl.cellb, ws ? c->xpred : nullptr, c->tmp4, t_lam, s);
     launch_rebuild_copy(p.n, c->ctl, O.pos, O.vel, O.id, O.attr, c->pres, I.pos, c->ppos[0], c->ppos[1], c->xb, I.id,
                         I.attr, c->dens, c->tmp4, ws ? c->xpred : nullptr, t_lam, s);
@@ -723,7 +729,7 @@ int enqueue_pbf_pre(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
     int src = 0, it = 1;
     const float4 *acc = nullptr;
     if (pbf_prepass(c)) {
-        enqueue_sort(c, p, c->set[0].pos, s);
+        const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
         Gather g{};
         g.n4 = dw ? 3 : 2; g.n1 = 2;
         g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
@@ -731,7 +737,7 @@ int enqueue_pbf_pre(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
         g.src4[2] = dw; g.dst4[2] = c->vort; /* vort is rewritten at the end of the step */
         g.src1[0] = c->set[0].id; g.dst1[0] = c->set[1].id;
         g.src1[1] = c->set[0].attr; g.dst1[1] = c->set[1].attr;
-        launch_gather(p.n, c->perm, g, nullptr, s);
+        launch_gather(p.n, o, g, nullptr, s);
         launch_pbf_density(p, c->cell_start, c->set[1].pos, c->dens, s);
         launch_pbf_visc(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->dens, c->acc, s);
         acc = c->acc;
@@ -741,7 +747,7 @@ int enqueue_pbf_pre(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
     launch_predict_hash(p, c->set[src].pos, c->set[src].vel, acc, c->ppos[1], c->key, c->rank, c->count, dw,
                         ws ? c->tmp4 : nullptr, s);
     launch_scan(c->count, c->cell_start, c->block_sums, c->ncells, s);
-    sort_cells(c, p, s);
+    const CellOrder o = sort_cells(c, p, s);
     Gather g{};
     g.n4 = ws ? 4 : 3; g.n1 = 3;
     g.src4[0] = c->set[src].pos; g.dst4[0] = c->set[it].pos;
@@ -751,7 +757,7 @@ int enqueue_pbf_pre(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
     g.src1[0] = c->set[src].id; g.dst1[0] = c->set[it].id;
     g.src1[1] = c->set[src].attr; g.dst1[1] = c->set[it].attr;
     g.src1[2] = c->key; g.dst1[2] = c->nl.cellb;
-    launch_gather(p.n, c->perm, g, c->ctl, s);
+    launch_gather(p.n, o, g, c->ctl, s);
     launch_build_list(p, c->cell_start, c->xb, c->nl, s);
     return it;
 }
@@ -900,14 +906,14 @@ int build_pbf_graph(fsph_ctx *c, const DevParams &p) {
 int sph_step(fsph_ctx *c, const DevParams &p) {
     cudaStream_t s = c->stream;
     FSPH_CUDA(c, cudaMemsetAsync(c->ctl, 0, sizeof(DevCtl), s));
-    enqueue_sort(c, p, c->set[0].pos, s);
+    const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
     Gather g{};
     g.n4 = 2; g.n1 = 2;
     g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
     g.src4[1] = c->set[0].vel; g.dst4[1] = c->set[1].vel;
     g.src1[0] = c->set[0].id; g.dst1[0] = c->set[1].id;
     g.src1[1] = c->set[0].attr; g.dst1[1] = c->set[1].attr;
-    launch_gather(p.n, c->perm, g, c->ctl, s);
+    launch_gather(p.n, o, g, c->ctl, s);
     launch_sph_density(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->dens, c->pres, c->nl, s);
     launch_sph_force(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->acc, c->nl, s);
     launch_sph_integrate(p, c->set[1].pos, c->set[1].vel, c->acc, c->set[1].id, c->set[1].attr, c->set[0].pos,
@@ -1029,6 +1035,8 @@ int repartition(fsph_ctx *c) {
         launch_mark_active(n, c->set[0].attr, c->key, s);
         launch_scan(c->key, c->part_scan, c->part_bsum, (unsigned int)n, s);
         launch_partition_perm(n, c->part_scan, c->perm, s);
+        CellOrder o;
+        o.perm = c->perm;
         Gather g{};
         g.n4 = 3; g.n1 = 2;
         g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
@@ -1036,7 +1044,7 @@ int repartition(fsph_ctx *c) {
         g.src4[2] = c->dstep; g.dst4[2] = c->tmp4;
         g.src1[0] = c->set[0].id; g.dst1[0] = c->set[1].id;
         g.src1[1] = c->set[0].attr; g.dst1[1] = c->set[1].attr;
-        launch_gather(n, c->perm, g, nullptr, s);
+        launch_gather(n, o, g, nullptr, s);
         float4 *tf = reinterpret_cast<float4 *>(c->nl.list);
         launch_gather_rows(n, c->perm, reinterpret_cast<const float4 *>(c->feat), tf, kFeatures / 4, s);
         FSPH_CUDA(c, cudaMemcpyAsync(c->set[0].pos, c->set[1].pos, (size_t)n * 16, cudaMemcpyDeviceToDevice, s));
@@ -1062,7 +1070,7 @@ int repartition(fsph_ctx *c) {
  * gather x (and w) into set[1].pos / ppos[0] / xb, ids into set[1].id. */
 int build_on(fsph_ctx *c, const DevParams &p, const float4 *x) {
     cudaStream_t s = c->stream;
-    enqueue_sort(c, p, x, s);
+    const CellOrder o = enqueue_sort(c, p, x, s);
     Gather g{};
     g.n4 = 3; g.n1 = 3;
     g.src4[0] = x; g.dst4[0] = c->set[1].pos;
@@ -1071,7 +1079,7 @@ int build_on(fsph_ctx *c, const DevParams &p, const float4 *x) {
     g.src1[0] = c->set[0].id; g.dst1[0] = c->set[1].id;
     g.src1[1] = c->set[0].attr; g.dst1[1] = c->set[1].attr;
     g.src1[2] = c->key; g.dst1[2] = c->nl.cellb;
-    launch_gather(p.n, c->perm, g, nullptr, s);
+    launch_gather(p.n, o, g, nullptr, s);
     launch_build_list(p, c->cell_start, c->xb, c->nl, s);
     return check_launch(c);
 }
@@ -1625,12 +1633,12 @@ int fsph_neighbors_ex(fsph_ctx *c, const float *pos4, int n, float radius, int w
         x = c->tmp4;
         ids = c->set[1].attr;
     }
-    enqueue_sort(c, p, x, s);
+    const CellOrder o = enqueue_sort(c, p, x, s);
     Gather g{};
     g.n4 = 1; g.n1 = 1;
     g.src4[0] = x; g.dst4[0] = c->set[1].pos;
     g.src1[0] = ids; g.dst1[0] = c->set[1].id;
-    launch_gather(n, c->perm, g, nullptr, s);
+    launch_gather(n, o, g, nullptr, s);
     unsigned int *cnt = c->rank; /* free once the scatter has run */
     launch_nb_count(p, c->cell_start, c->set[1].pos, cnt, s);
     std::vector<unsigned int> hc((size_t)n), ho((size_t)n + 1);
@@ -1769,13 +1777,13 @@ int fsph_step_fields(fsph_ctx *c, float dt, void *stream) {
     FSPH_CUDA(c, cudaStreamSynchronize(s));
     /* results keep the sorted order of this evaluation (res_id); the
      * particles themselves stay where they are */
-    enqueue_sort(c, p, c->set[0].pos, s);
+    const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
     Gather g{};
     g.n4 = 2; g.n1 = 1;
     g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
     g.src4[1] = c->set[0].vel; g.dst4[1] = c->set[1].vel;
     g.src1[0] = c->set[0].id; g.dst1[0] = c->res_id;
-    launch_gather(p.n, c->perm, g, nullptr, s);
+    launch_gather(p.n, o, g, nullptr, s);
     if (c->P.solver == FSPH_SOLVER_WCSPH) {
         launch_sph_density(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->dens, c->pres, c->nl, s);
         launch_sph_force(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->acc, c->nl, s);
@@ -2306,12 +2314,12 @@ int fsph_time_pass(fsph_ctx *c, int pass, int reps, float *avg_ms) {
     cudaStream_t s = c->stream;
     if (sph_pass) {
         /* the state of a WCSPH step before its passes: grid on x, sorted x, v */
-        enqueue_sort(c, p, c->set[0].pos, s);
+        const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
         Gather g{};
         g.n4 = 2;
         g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
         g.src4[1] = c->set[0].vel; g.dst4[1] = c->set[1].vel;
-        launch_gather(p.n, c->perm, g, nullptr, s);
+        launch_gather(p.n, o, g, nullptr, s);
         launch_sph_density(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->dens, c->pres, c->nl, s);
         cudaEvent_t e0, e1;
         FSPH_CUDA(c, cudaEventCreate(&e0));
@@ -2349,14 +2357,14 @@ int fsph_time_pass(fsph_ctx *c, int pass, int reps, float *avg_ms) {
             launch_correction(p, c->cell_start, c->ppos[0], c->ppos[1], c->xb, c->ctl, c->dpart, 0ull, 0ull, 0,
                               nullptr, c->nl, s);
         } else if (pass == FSPH_PASS_GRID) {
-            enqueue_sort(c, p, c->set[1].pos, s);
+            const CellOrder o = enqueue_sort(c, p, c->set[1].pos, s);
             Gather g{};
             g.n4 = 3; g.n1 = 1;
             g.src4[0] = c->set[1].pos; g.dst4[0] = c->set[1].vel;
             g.src4[1] = c->set[1].pos; g.dst4[1] = c->ppos[1];
             g.src4[2] = c->set[1].pos; g.dst4[2] = c->acc;
             g.src1[0] = c->set[1].id; g.dst1[0] = c->set[1].attr;
-            launch_gather(p.n, c->perm, g, nullptr, s);
+            launch_gather(p.n, o, g, nullptr, s);
         } else if (pass == FSPH_PASS_LIST) {
             launch_build_list(p, c->cell_start, c->xb, c->nl, s);
         } else {
@@ -2429,7 +2437,7 @@ int fsph_pbf_eval_xsph_vorticity(fsph_ctx *c, const float *pos4, const float *ve
     unsigned int *dh = reinterpret_cast<unsigned int *>(c->pres);
     float *ds = reinterpret_cast<float *>(c->dens);
     FSPH_CUDA(c, cudaMemcpyAsync(dh, dens, (size_t)n * 4, cudaMemcpyHostToDevice, s));
-    enqueue_sort(c, p, c->set[0].pos, s);
+    const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
     Gather g{};
     g.n4 = 3; g.n1 = 3;
     g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
@@ -2438,7 +2446,7 @@ int fsph_pbf_eval_xsph_vorticity(fsph_ctx *c, const float *pos4, const float *ve
     g.src1[0] = c->set[0].id; g.dst1[0] = c->set[1].id;
     g.src1[1] = c->key; g.dst1[1] = c->nl.cellb;
     g.src1[2] = dh; g.dst1[2] = reinterpret_cast<unsigned int *>(ds);
-    launch_gather(n, c->perm, g, nullptr, s);
+    launch_gather(n, o, g, nullptr, s);
     launch_build_list(p, c->cell_start, c->xb, c->nl, s);
     /* the end-of-step passes of a PBF step, on these inputs */
     launch_xsph_vort(p, c->cell_start, c->set[1].pos, c->set[1].vel, ds, c->acc, c->vort, FeatureOut{}, c->nl, s);
@@ -2463,13 +2471,13 @@ int fsph_sph_eval_forces(fsph_ctx *c, const float *pos4, const float *vel4, int 
     if (n == 0) return FSPH_OK;
     DevParams p = dev_for(c, n, 1.0f);
     cudaStream_t s = c->stream;
-    enqueue_sort(c, p, c->set[0].pos, s);
+    const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
     Gather g{};
     g.n4 = 2; g.n1 = 1;
     g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
     g.src4[1] = c->set[0].vel; g.dst4[1] = c->set[1].vel;
     g.src1[0] = c->set[0].id; g.dst1[0] = c->set[1].id;
-    launch_gather(n, c->perm, g, nullptr, s);
+    launch_gather(n, o, g, nullptr, s);
     launch_sph_density(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->dens, c->pres, c->nl, s);
     launch_sph_force(p, c->cell_start, c->set[1].pos, c->set[1].vel, c->acc, c->nl, s);
     FSPH_TRY(check_launch(c));

@@ -544,19 +544,19 @@ DevParams loop_params(const fsph_batch *b, float dt) {
     return lp;
 }
 
-void benqueue_sort_tail(fsph_batch *b, cudaStream_t s) {
+CellOrder benqueue_sort_tail(fsph_batch *b, cudaStream_t s) {
     launch_scan(b->count, b->cell_start, b->block_sums, b->ncells, s);
     DevParams q{};
     q.n = b->n;
-    launch_scatter_sort(q, b->key, b->rank, b->cell_start, b->perm, b->ncells, s);
+    return launch_scatter(q, b->key, b->rank, b->cell_start, b->perm, s);
 }
 
 /* in-loop / post-loop rebuild: re-sort every scene on the current x* */
 void benqueue_rebuild(fsph_batch *b, const BLaunch &L, cudaStream_t s) {
     blaunch_hash_parity(L, b->ppos[0], b->ppos[1], b->ctl, b->key, b->rank, b->count, s);
-    benqueue_sort_tail(b, s);
+    const CellOrder o = benqueue_sort_tail(b, s);
     float *t_lam = reinterpret_cast<float *>(b->rank); /* free once the scatter has run */
-    launch_rebuild_gather(b->n, b->perm, b->ctl, b->pos[1], b->ppos[0], b->ppos[1], b->id[1], b->attr[1], b->dens,
+    launch_rebuild_gather(b->n, o, b->ctl, b->pos[1], b->ppos[0], b->ppos[1], b->id[1], b->attr[1], b->dens,
                           b->pos[0], b->vel[0], b->id[0], b->attr[0], b->tdens, b->key, b->nl.cellb, nullptr, nullptr,
                           t_lam, s);
     launch_rebuild_copy(b->n, b->ctl, b->pos[0], b->vel[0], b->id[0], b->attr[0], b->tdens, b->pos[1], b->ppos[0],
@@ -567,7 +567,7 @@ void benqueue_rebuild(fsph_batch *b, const BLaunch &L, cudaStream_t s) {
 void benqueue_pre(fsph_batch *b, const BLaunch &L, cudaStream_t s) {
     cudaMemsetAsync(b->ctl, 0, sizeof(DevCtl), s);
     blaunch_predict_hash(L, b->pos[0], b->vel[0], b->ppos[1], b->key, b->rank, b->count, s);
-    benqueue_sort_tail(b, s);
+    const CellOrder o = benqueue_sort_tail(b, s);
     Gather g{};
     g.n4 = 3; g.n1 = 3;
     g.src4[0] = b->pos[0]; g.dst4[0] = b->pos[1];
@@ -576,7 +576,7 @@ void benqueue_pre(fsph_batch *b, const BLaunch &L, cudaStream_t s) {
     g.src1[0] = b->id[0]; g.dst1[0] = b->id[1];
     g.src1[1] = b->attr[0]; g.dst1[1] = b->attr[1];
     g.src1[2] = b->key; g.dst1[2] = b->nl.cellb;
-    launch_gather(b->n, b->perm, g, b->ctl, s);
+    launch_gather(b->n, o, g, b->ctl, s);
     blaunch_build_list(L, b->cell_start, b->xb, b->nl, s);
 }
 

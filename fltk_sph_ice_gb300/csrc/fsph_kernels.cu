@@ -142,31 +142,34 @@ __global__ void k_scatter(int n, const unsigned int *__restrict__ key, const uns
     perm[cell_start[key[i]] + rank[i]] = (unsigned int)i;
 }
 
-/* The atomic ranks order a cell's slots arbitrarily; sorting each cell's
- * (few) previous-slot indices makes the permutation the stable order of the
- * 64-bit key (cell << 32 | previous slot), identical on every run. */
-__global__ void k_cell_sort(const unsigned int *__restrict__ cell_start, unsigned int *__restrict__ perm,
-                            unsigned int ncells) {
-    unsigned int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncells) return;
-    unsigned int s = cell_start[c], e = cell_start[c + 1];
-    if (e - s < 2) return;
-    for (unsigned int a = s + 1; a < e; ++a) {
-        unsigned int v = perm[a];
-        unsigned int b = a;
-        while (b > s && perm[b - 1] > v) {
-            perm[b] = perm[b - 1];
-            --b;
-        }
-        perm[b] = v;
-    }
+/* The atomic ranks order a cell's slots arbitrarily.  Counting, for each
+ * scattered entry, the smaller previous slots of its cell gives its place in
+ * the stable order of the 64-bit key (cell << 32 | previous slot), identical
+ * on every run.  Every entry counts for itself (about 10 independent loads,
+ * one or two lines), so the kernel that moves the particles does it on the
+ * way and no kernel sorts the cells.  One thread per cell, an insertion
+ * sort in global memory (a serial chain of dependent loads and stores) had
+ * taken 27 us at 4,096 particles, 37 us at 1 M and 110 us for the 4.7 M of a
+ * batch; whole calls went from 102.6 to 83.7 us (lambda pass, 4,096), 568 to
+ * 548 us (PBF step, 262 k) and 5,755 to 5,658 us (batch step).
+ * s: the previous slot of scattered entry u; returns its slot in the order. */
+__device__ __forceinline__ unsigned int ranked_slot(unsigned int u, const CellOrder &o, unsigned int &s) {
+    s = o.perm[u];
+    if (!o.key) return u; /* perm is the order itself (radix sort, partition) */
+    const unsigned int c = o.key[s];
+    const unsigned int a = o.cell_start[c], e = o.cell_start[c + 1];
+    unsigned int d = a;
+    for (unsigned int v = a; v < e; ++v) d += o.perm[v] < s ? 1u : 0u;
+    return d;
 }
 
-__global__ void k_gather(int n, const unsigned int *__restrict__ perm, Gather g, DevCtl *count_build) {
-    int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d == 0 && count_build) count_build->builds += 1u;
-    if (d >= n) return;
-    unsigned int s = perm ? perm[d] : (unsigned int)d;
+__global__ void k_gather(int n, CellOrder o, Gather g, DevCtl *count_build) {
+    int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u == 0 && count_build) count_build->builds += 1u;
+    if (u >= n) return;
+    unsigned int s;
+    const unsigned int d = ranked_slot((unsigned int)u, o, s);
+    if (o.sorted) o.sorted[d] = s;
 #pragma unroll
     for (int k = 0; k < 6; ++k)
         if (k < g.n4) g.dst4[k][d] = g.src4[k][s];
@@ -187,7 +190,7 @@ __global__ void k_hash_parity(DevParams p, const float4 *ppos0, const float4 *pp
 }
 
 /* Gather every array carried through the iterations into temporaries. */
-__global__ void k_rebuild_gather(int n, const unsigned int *__restrict__ perm, const DevCtl *ctl,
+__global__ void k_rebuild_gather(int n, CellOrder o, const DevCtl *ctl,
                                  const float4 *__restrict__ pos, const float4 *ppos0, const float4 *ppos1,
                                  const unsigned int *__restrict__ id, const unsigned int *__restrict__ attr,
                                  const float *__restrict__ dens, float4 *__restrict__ t_pos,
@@ -196,10 +199,11 @@ __global__ void k_rebuild_gather(int n, const unsigned int *__restrict__ perm, c
                                  const unsigned int *__restrict__ key, unsigned int *__restrict__ cellb,
                                  const float4 *__restrict__ xpred, float4 *__restrict__ t_xpred,
                                  float *__restrict__ t_lam) {
-    int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= n) return;
+    int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= n) return;
     const float4 *x4 = ctl->parity ? ppos1 : ppos0;
-    unsigned int s = perm[d];
+    unsigned int s;
+    const unsigned int d = ranked_slot((unsigned int)u, o, s);
     if (cellb) cellb[d] = key[s];
     if (xpred) t_xpred[d] = xpred[s];
     /* lambda of the last pass lives in the .w of the other buffer */
@@ -1022,24 +1026,28 @@ void launch_scan(unsigned int *count, unsigned int *cell_start, unsigned int *bl
     k_scan_top<<<1, 1024, 0, s>>>(block_sums, nb, cell_start, ncells);
     k_scan_add<<<blocks_for(ncells, 1024), 1024, 0, s>>>(cell_start, block_sums, ncells);
 }
-void launch_scatter_sort(const DevParams &p, const unsigned int *key, const unsigned int *rank,
-                         const unsigned int *cell_start, unsigned int *perm, unsigned int ncells, cudaStream_t s) {
+CellOrder launch_scatter(const DevParams &p, const unsigned int *key, const unsigned int *rank,
+                         const unsigned int *cell_start, unsigned int *perm, cudaStream_t s) {
     k_scatter<<<blocks_for(p.n), kBlock, 0, s>>>(p.n, key, rank, cell_start, perm);
-    k_cell_sort<<<blocks_for(ncells), kBlock, 0, s>>>(cell_start, perm, ncells);
+    CellOrder o;
+    o.perm = perm;
+    o.key = key;
+    o.cell_start = cell_start;
+    return o;
 }
-void launch_gather(int n, const unsigned int *perm, const Gather &g, DevCtl *count_build, cudaStream_t s) {
-    k_gather<<<blocks_for(n), kBlock, 0, s>>>(n, perm, g, count_build);
+void launch_gather(int n, const CellOrder &o, const Gather &g, DevCtl *count_build, cudaStream_t s) {
+    k_gather<<<blocks_for(n), kBlock, 0, s>>>(n, o, g, count_build);
 }
 void launch_hash_parity(const DevParams &p, const float4 *ppos0, const float4 *ppos1, const DevCtl *ctl,
                         unsigned int *key, unsigned int *rank, unsigned int *count, cudaStream_t s) {
     k_hash_parity<<<blocks_for(p.n), kBlock, 0, s>>>(p, ppos0, ppos1, ctl, key, rank, count);
 }
-void launch_rebuild_gather(int n, const unsigned int *perm, const DevCtl *ctl, const float4 *pos, const float4 *ppos0,
+void launch_rebuild_gather(int n, const CellOrder &o, const DevCtl *ctl, const float4 *pos, const float4 *ppos0,
                            const float4 *ppos1, const unsigned int *id, const unsigned int *attr, const float *dens,
                            float4 *t_pos, float4 *t_x, unsigned int *t_id, unsigned int *t_attr, float *t_dens,
                            const unsigned int *key, unsigned int *cellb, const float4 *xpred, float4 *t_xpred,
                            float *t_lam, cudaStream_t s) {
-    k_rebuild_gather<<<blocks_for(n), kBlock, 0, s>>>(n, perm, ctl, pos, ppos0, ppos1, id, attr, dens, t_pos, t_x,
+    k_rebuild_gather<<<blocks_for(n), kBlock, 0, s>>>(n, o, ctl, pos, ppos0, ppos1, id, attr, dens, t_pos, t_x,
                                                       t_id, t_attr, t_dens, key, cellb, xpred, t_xpred, t_lam);
 }
 void launch_rebuild_copy(int n, DevCtl *ctl, const float4 *t_pos, const float4 *t_x, const unsigned int *t_id,

@@ -34,11 +34,20 @@ void launch_hash(const DevParams &p, const float4 *x, unsigned int *key, unsigne
 /* exclusive scan of count[C] into cell_start[C+1]; zeroes count for the next build */
 void launch_scan(unsigned int *count, unsigned int *cell_start, unsigned int *block_sums, unsigned int ncells,
                  cudaStream_t s);
-/* perm[cell_start[key] + rank] = slot, then each cell's slots sorted ascending */
-void launch_scatter_sort(const DevParams &p, const unsigned int *key, const unsigned int *rank,
-                         const unsigned int *cell_start, unsigned int *perm, unsigned int ncells, cudaStream_t s);
+/* The order of a grid build.  key == NULL: perm[d] = the previous slot of slot
+ * d.  Else perm holds each cell's previous slots in the arbitrary order of the
+ * atomic ranks, and the kernel that moves the particles ranks them on the way
+ * (ranked_slot in fsph_kernels.cu); sorted (optional) then receives the order
+ * itself, for callers that need it afterwards. */
+struct CellOrder {
+    const unsigned int *perm = nullptr, *key = nullptr, *cell_start = nullptr;
+    unsigned int *sorted = nullptr;
+};
+/* perm[cell_start[key] + rank] = slot; returns the order it stands for */
+CellOrder launch_scatter(const DevParams &p, const unsigned int *key, const unsigned int *rank,
+                         const unsigned int *cell_start, unsigned int *perm, cudaStream_t s);
 
-/* dst[d] = src[perm[d]] for up to 6 float4 and 4 u32 streams (perm == NULL: plain copy) */
+/* dst[d] = src[previous slot of d] for up to 6 float4 and 4 u32 streams */
 struct Gather {
     const float4 *src4[6];
     float4 *dst4[6];
@@ -46,12 +55,12 @@ struct Gather {
     unsigned int *dst1[4];
     int n4, n1;
 };
-void launch_gather(int n, const unsigned int *perm, const Gather &g, DevCtl *count_build, cudaStream_t s);
+void launch_gather(int n, const CellOrder &o, const Gather &g, DevCtl *count_build, cudaStream_t s);
 
 /* in-loop rebuild (the current x* buffer is chosen on the device by ctl->parity) */
 void launch_hash_parity(const DevParams &p, const float4 *ppos0, const float4 *ppos1, const DevCtl *ctl,
                         unsigned int *key, unsigned int *rank, unsigned int *count, cudaStream_t s);
-void launch_rebuild_gather(int n, const unsigned int *perm, const DevCtl *ctl, const float4 *pos, const float4 *ppos0,
+void launch_rebuild_gather(int n, const CellOrder &o, const DevCtl *ctl, const float4 *pos, const float4 *ppos0,
                            const float4 *ppos1, const unsigned int *id, const unsigned int *attr, const float *dens,
                            float4 *t_pos, float4 *t_x, unsigned int *t_id, unsigned int *t_attr, float *t_dens,
                            const unsigned int *key, unsigned int *cellb, const float4 *xpred, float4 *t_xpred,

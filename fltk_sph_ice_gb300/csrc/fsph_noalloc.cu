@@ -115,16 +115,17 @@ extern "C" int fsph_pbf_eval_lambda_noalloc(const fsph_params *params, const flo
     if (cudaMemsetAsync(ctl, 0, sizeof(DevCtl), s) != cudaSuccess) return FSPH_CUDA_ERROR;
     launch_hash(p, reinterpret_cast<const float4 *>(pos4), key, rank, count, s);
     launch_scan(count, cell_start, bsum, nc, s);
-    launch_scatter_sort(p, key, rank, cell_start, perm, nc, s);
+    CellOrder o = launch_scatter(p, key, rank, cell_start, perm, s);
+    o.sorted = rank; /* free once the scatter has run */
     Gather g{};
     g.n4 = 1;
     g.n1 = 0;
     g.src4[0] = reinterpret_cast<const float4 *>(pos4);
     g.dst4[0] = x;
-    launch_gather(n, perm, g, nullptr, s);
+    launch_gather(n, o, g, nullptr, s);
     launch_lambda(p, cell_start, x, x, d_sorted, ctl, part, 0ull, 0, NbrLists{}, s);
-    launch_unsort1(n, perm, reinterpret_cast<const unsigned int *>(d_sorted), reinterpret_cast<unsigned int *>(dens), s);
-    launch_unsort_w(n, perm, x, lambda, s);
+    launch_unsort1(n, o.sorted, reinterpret_cast<const unsigned int *>(d_sorted), reinterpret_cast<unsigned int *>(dens), s);
+    launch_unsort_w(n, o.sorted, x, lambda, s);
     if (cudaGetLastError() != cudaSuccess) return FSPH_CUDA_ERROR;
     return FSPH_OK;
 }
