@@ -50,22 +50,12 @@ __global__ void k_hash(DevParams p, const float4 *__restrict__ x4, unsigned int 
     hash_body(p, i, f3(x4[i]), key, rank, count);
 }
 
-/* Scan phase 1: each 1024-thread block scans kScanTile = 4096 counts. */
-__global__ void __launch_bounds__(1024) k_scan_local(unsigned int *__restrict__ count,
-                                                     unsigned int *__restrict__ out,
-                                                     unsigned int *__restrict__ block_sums, unsigned int ncells) {
+/* exclusive prefix of v over the 1024 threads of a block; total: the block's sum */
+__device__ __forceinline__ unsigned int block_scan(unsigned int v, unsigned int &total) {
     __shared__ unsigned int warp_tot[32];
-    const unsigned int base = blockIdx.x * kScanTile + threadIdx.x * 4;
-    unsigned int v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        unsigned int idx = base + k;
-        v[k] = idx < ncells ? count[idx] : 0u;
-        if (idx < ncells) count[idx] = 0u;
-    }
-    unsigned int t = v[0] + v[1] + v[2] + v[3];
+    __shared__ unsigned int s_total;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned int incl = t;
+    unsigned int incl = v;
     for (int o = 1; o < 32; o <<= 1) {
         unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
@@ -80,47 +70,62 @@ __global__ void __launch_bounds__(1024) k_scan_local(unsigned int *__restrict__ 
             if (lane >= o) wi += y;
         }
         warp_tot[lane] = wi - w; /* exclusive prefix of the warps */
-        if (lane == 31) block_sums[blockIdx.x] = wi;
+        if (lane == 31) s_total = wi;
     }
     __syncthreads();
-    unsigned int run = warp_tot[warp] + incl - t;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        unsigned int idx = base + k;
-        if (idx < ncells) out[idx] = run;
-        run += v[k];
+    total = s_total;
+    return warp_tot[warp] + incl - v;
+}
+
+/* Scan phase 1: each 1024-thread block scans kScanTile = 4096 counts, four a
+ * thread in one 16-byte load (count and out are 16-byte aligned arrays), and
+ * zeroes them.  A table of one tile ends here: the block also writes the
+ * grand total to out[ncells]. */
+__global__ void __launch_bounds__(1024) k_scan_local(unsigned int *__restrict__ count,
+                                                     unsigned int *__restrict__ out,
+                                                     unsigned int *__restrict__ block_sums, unsigned int ncells) {
+    const unsigned int base = blockIdx.x * kScanTile + threadIdx.x * 4;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    const bool whole = base + 4 <= ncells;
+    if (whole) {
+        v = *reinterpret_cast<const uint4 *>(count + base);
+        *reinterpret_cast<uint4 *>(count + base) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+        unsigned int t[4] = {0u, 0u, 0u, 0u};
+        for (int k = 0; k < 4; ++k)
+            if (base + k < ncells) {
+                t[k] = count[base + k];
+                count[base + k] = 0u;
+            }
+        v = make_uint4(t[0], t[1], t[2], t[3]);
+    }
+    unsigned int total;
+    const unsigned int run = block_scan(v.x + v.y + v.z + v.w, total);
+    const uint4 r = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+    if (whole) {
+        *reinterpret_cast<uint4 *>(out + base) = r;
+    } else {
+        const unsigned int t[4] = {r.x, r.y, r.z, r.w};
+        for (int k = 0; k < 4; ++k)
+            if (base + k < ncells) out[base + k] = t[k];
+    }
+    if (threadIdx.x == 0) {
+        block_sums[blockIdx.x] = total;
+        if (gridDim.x == 1) out[ncells] = total;
     }
 }
 
 /* Scan phase 2: one block scans the block totals; writes the grand total to out[ncells]. */
 __global__ void __launch_bounds__(1024) k_scan_top(unsigned int *__restrict__ block_sums, unsigned int nblocks,
                                                    unsigned int *__restrict__ out, unsigned int ncells) {
-    __shared__ unsigned int warp_tot[32];
     const int per = (nblocks + 1023) / 1024;
     const unsigned int start = threadIdx.x * per;
     unsigned int t = 0;
     for (int k = 0; k < per; ++k)
         if (start + k < nblocks) t += block_sums[start + k];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned int incl = t;
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned int w = warp_tot[lane];
-        unsigned int wi = w;
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned int y = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += y;
-        }
-        warp_tot[lane] = wi - w;
-        if (lane == 31) out[ncells] = wi;
-    }
-    __syncthreads();
-    unsigned int run = warp_tot[warp] + incl - t;
+    unsigned int total;
+    unsigned int run = block_scan(t, total);
+    if (threadIdx.x == 0) out[ncells] = total;
     for (int k = 0; k < per; ++k)
         if (start + k < nblocks) {
             unsigned int b = block_sums[start + k];
@@ -129,10 +134,30 @@ __global__ void __launch_bounds__(1024) k_scan_top(unsigned int *__restrict__ bl
         }
 }
 
-__global__ void k_scan_add(unsigned int *__restrict__ out, const unsigned int *__restrict__ block_sums,
-                           unsigned int ncells) {
-    unsigned int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < ncells) out[i] += block_sums[i / kScanTile];
+/* Scan phase 3: block b adds the total before its tile.  SUM: the totals are
+ * still the tiles' own (no phase 2 has run), so the block sums the b totals
+ * before it; the last block writes the grand total. */
+template <bool SUM>
+__global__ void __launch_bounds__(1024) k_scan_add(unsigned int *__restrict__ out,
+                                                   const unsigned int *__restrict__ block_sums, unsigned int ncells) {
+    unsigned int add;
+    if (SUM) {
+        unsigned int t = 0;
+        for (unsigned int k = threadIdx.x; k < blockIdx.x; k += 1024u) t += block_sums[k];
+        block_scan(t, add);
+        if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) out[ncells] = add + block_sums[blockIdx.x];
+    } else {
+        add = block_sums[blockIdx.x];
+    }
+    const unsigned int base = blockIdx.x * kScanTile + threadIdx.x * 4;
+    if (base + 4 <= ncells) {
+        uint4 v = *reinterpret_cast<const uint4 *>(out + base);
+        v.x += add; v.y += add; v.z += add; v.w += add;
+        *reinterpret_cast<uint4 *>(out + base) = v;
+    } else {
+        for (int k = 0; k < 4; ++k)
+            if (base + k < ncells) out[base + k] += add;
+    }
 }
 
 __global__ void k_scatter(int n, const unsigned int *__restrict__ key, const unsigned int *__restrict__ rank,
@@ -1021,10 +1046,19 @@ void launch_hash(const DevParams &p, const float4 *x, unsigned int *key, unsigne
 }
 void launch_scan(unsigned int *count, unsigned int *cell_start, unsigned int *block_sums, unsigned int ncells,
                  cudaStream_t s) {
-    unsigned int nb = scan_blocks(ncells);
+    const unsigned int nb = scan_blocks(ncells);
     k_scan_local<<<nb, 1024, 0, s>>>(count, cell_start, block_sums, ncells);
-    k_scan_top<<<1, 1024, 0, s>>>(block_sums, nb, cell_start, ncells);
-    k_scan_add<<<blocks_for(ncells, 1024), 1024, 0, s>>>(cell_start, block_sums, ncells);
+    if (nb == 1) return;
+    /* Up to kScanSum tiles every block of the last phase sums the totals before
+     * it itself (at most kScanSum / 1024 loads a thread) instead of a phase of
+     * one block between the two: a launch less, about 4 us of each grid build.
+     * Past it those loads (nb^2 / 2 words in all) cost more than the launch. */
+    if (nb <= kScanSum) {
+        k_scan_add<true><<<nb, 1024, 0, s>>>(cell_start, block_sums, ncells);
+    } else {
+        k_scan_top<<<1, 1024, 0, s>>>(block_sums, nb, cell_start, ncells);
+        k_scan_add<false><<<nb, 1024, 0, s>>>(cell_start, block_sums, ncells);
+    }
 }
 CellOrder launch_scatter(const DevParams &p, const unsigned int *key, const unsigned int *rank,
                          const unsigned int *cell_start, unsigned int *perm, cudaStream_t s) {

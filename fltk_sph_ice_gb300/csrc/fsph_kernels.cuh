@@ -18,6 +18,7 @@ constexpr int kBlock = 256;
 constexpr int kPassBlock = FSPH_PASS_BLOCK;
 constexpr int kBlockMax = 512;  /* largest block of the batched persistent kernels */
 constexpr int kScanTile = 4096; /* cells per block of the first scan phase */
+constexpr unsigned int kScanSum = 2048; /* tiles up to which the scan runs in two phases */
 
 inline unsigned int blocks_for(long long n, int b = kBlock) { return (unsigned int)((n + b - 1) / b); }
 inline unsigned int scan_blocks(unsigned int ncells) { return (ncells + kScanTile - 1) / kScanTile; }

@@ -7,7 +7,7 @@ same order, so a step from the same state is the same bit for bit."""
 import numpy as np
 import pytest
 
-from fltk_sph_ice_gb300 import abi, rxSPH, scenes
+from fltk_sph_ice_gb300 import abi, rxPBDSPH, rxSPH, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +48,30 @@ def test_ranked_and_radix_orders_step_identically(gpu, kind, n):
         ps.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("side", [3, 16, 17, 203, 204])
+def test_cell_table_scan_at_tile_edges(gpu, side):
+    """The scan over the cell table takes one phase up to 4,096 cells, two up
+    to 2,048 tiles of those and three past that: the neighbour sets of a few
+    particles spread over the whole grid against brute force (whole numbers)."""
+    h = 1.0
+    p = scenes.pbf_params(h, [0.0] * 3, [1.0] * 3, 600)
+    p.cell_skin = 0.0  # a cell is h (1 + 1e-3) wide, plus one cell of padding on each side
+    for a in range(3):
+        p.box_max[a] = (side - 2) * 1.001 * h * 0.9999
+    p.particle_radius = 0.25
+    rng = np.random.default_rng(side)
+    n, top = 600, float(p.box_max[0])
+    pos = np.zeros((n, 4), np.float32)
+    c = rng.uniform(0, top, (60, 3))
+    pos[:, :3] = np.clip(c[rng.integers(0, 60, n)] + rng.uniform(-1, 1, (n, 3)), 0, top)
+    ps = rxPBDSPH(p)
+    ps.Set(pos)
+    off, idx = ps.GetNeights()
+    ps.close()
+    x = pos[:, :3].astype(np.float64)
+    d2 = ((x[:, None] - x[None]) ** 2)
+    near = (d2[..., 0] + d2[..., 1] + d2[..., 2]).astype(np.float32) <= np.float32(h * h)
+    assert np.array_equal(np.diff(off), near.sum(1))
+    assert np.array_equal(idx, np.nonzero(near)[1])
