@@ -112,10 +112,8 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK)
                                                    float4 *ppos0, float4 *ppos1, float *__restrict__ dens, DevCtl *ctl,
                                                    ErrPartial *part, cudaGraphConditionalHandle hwhile, int use_graph,
                                                    const ListEntry *__restrict__ list,
-                                                   const unsigned char *__restrict__ cnt,
-                                                   const unsigned int *__restrict__ cellb) {
+                                                   const unsigned char *__restrict__ cnt) {
     __shared__ DevParams s_p;
-    __shared__ unsigned int s_rs[9 * BLOCK];
     const unsigned int par = *((volatile unsigned int *)&ctl->parity);
     float4 *pp = par ? ppos1 : ppos0;
     float e1 = 0.f, e2 = 0.f, em = 0.f;
@@ -125,7 +123,7 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK)
         const DevParams p = s_p;
         const bool valid = li < tl.count;
         const int i = tl.start + (valid ? li : 0);
-        const float C = lambda_body<LPP>(p, cell_start, pp, dens, ctl, list, cnt, cellb, s_rs + threadIdx.x, i, sub,
+        const float C = lambda_body<LPP>(p, cell_start, pp, dens, ctl, list, cnt, i, sub,
                                          valid);
         if (valid && sub == 0) {
             e1 += C > 0.0f ? C : 0.0f;
@@ -145,10 +143,8 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK) kb_correctio
                                                        float *part, cudaGraphConditionalHandle hif,
                                                        cudaGraphConditionalHandle hif2, int use_graph,
                                                        const ListEntry *__restrict__ list,
-                                                       const unsigned char *__restrict__ cnt,
-                                                       const unsigned int *__restrict__ cellb) {
+                                                       const unsigned char *__restrict__ cnt) {
     __shared__ DevParams s_p;
-    __shared__ unsigned int s_rs[9 * BLOCK];
     const unsigned int par = *((volatile unsigned int *)&ctl->parity);
     const float4 *__restrict__ src = par ? ppos1 : ppos0;
     float4 *__restrict__ dst = par ? ppos0 : ppos1;
@@ -159,8 +155,7 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK) kb_correctio
         const DevParams p = s_p;
         const bool valid = li < tl.count;
         const int i = tl.start + (valid ? li : 0);
-        const float d2 = correction_body<LPP>(p, cell_start, src, dst, xb, ctl, nullptr, list, cnt, cellb,
-                                              s_rs + threadIdx.x, i, sub, valid);
+        const float d2 = correction_body<LPP>(p, cell_start, src, dst, xb, ctl, nullptr, list, cnt, i, sub, valid);
         worst = fmaxf(worst, d2 / p.skin2);
     }
     correction_tail(lp, ctl, part, worst, par, hif, hif2, use_graph);
@@ -185,17 +180,15 @@ __global__ void __launch_bounds__(BLOCK) kb_xsph_vort(BatchArgs b, const unsigne
                                                       float4 *__restrict__ vort,
                                                       const ListEntry *__restrict__ list,
                                                       const unsigned char *__restrict__ cnt,
-                                                      const unsigned int *__restrict__ cellb,
                                                       const float *__restrict__ mrho, float2 *__restrict__ wm) {
     __shared__ DevParams s_p;
-    __shared__ unsigned int s_rs[9 * BLOCK];
     const FeatureOut fo{};
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const BTile tl = tile_begin(b, t, s_p);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
             xsph_vort_body<false, FSPH_POST_PRE != 0>(p, tl.start + threadIdx.x, cell_start, pos, vel, dens, vel_out,
-                                                      vort, fo, list, cnt, cellb, s_rs + threadIdx.x, mrho, wm);
+                                                      vort, fo, list, cnt, mrho, wm);
     }
 }
 
@@ -206,16 +199,14 @@ __global__ void __launch_bounds__(BLOCK) kb_vort_apply(BatchArgs b, const unsign
                                                        const float4 *__restrict__ vel_in, float4 *__restrict__ vel_out,
                                                        const ListEntry *__restrict__ list,
                                                        const unsigned char *__restrict__ cnt,
-                                                       const unsigned int *__restrict__ cellb,
-                                                       const float2 *__restrict__ wm) {
+                                                      const float2 *__restrict__ wm) {
     __shared__ DevParams s_p;
-    __shared__ unsigned int s_rs[9 * BLOCK];
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const BTile tl = tile_begin(b, t, s_p);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
             vort_apply_body<FSPH_POST_PRE != 0>(p, tl.start + threadIdx.x, cell_start, pos, vort, dens, vel_in,
-                                                vel_out, list, cnt, cellb, s_rs + threadIdx.x, wm);
+                                                vel_out, list, cnt, wm);
     }
 }
 
@@ -314,7 +305,7 @@ unsigned int blaunch_lambda(const BLaunch &L, const DevParams &lp, const unsigne
     FSPH_BLOCK_SWITCH(L.block, FSPH_LANES_SWITCH(L.lanes, {
         auto k = kb_lambda<B_, L_>;
         g = persistent_grid(k, B_, L.cons.ntiles, L.sms);
-        k<<<g, B_, 0, s>>>(L.cons, lp, cell_start, p0, p1, dens, ctl, part, hw, use_graph, nl.list, nl.cnt, nl.cellb);
+        k<<<g, B_, 0, s>>>(L.cons, lp, cell_start, p0, p1, dens, ctl, part, hw, use_graph, nl.list, nl.cnt);
     }))
     return g;
 }
@@ -325,8 +316,7 @@ unsigned int blaunch_correction(const BLaunch &L, const DevParams &lp, const uns
     FSPH_BLOCK_SWITCH(L.block, FSPH_LANES_SWITCH(L.lanes, {
         auto k = kb_correction<B_, L_>;
         g = persistent_grid(k, B_, L.cons.ntiles, L.sms);
-        k<<<g, B_, 0, s>>>(L.cons, lp, cell_start, p0, p1, xb, ctl, part, hif, hif2, use_graph, nl.list, nl.cnt,
-                           nl.cellb);
+        k<<<g, B_, 0, s>>>(L.cons, lp, cell_start, p0, p1, xb, ctl, part, hif, hif2, use_graph, nl.list, nl.cnt);
     }))
     return g;
 }
@@ -340,7 +330,7 @@ void blaunch_xsph_vort(const BLaunch &L, const unsigned int *cell_start, const f
         }
         auto k = kb_xsph_vort<B_>;
         k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, cell_start, pos, vel, dens, vel_out, vort,
-                                                                       nl.list, nl.cnt, nl.cellb, mrho, wm);
+                                                                       nl.list, nl.cnt, mrho, wm);
     })
 }
 void blaunch_vort_apply(const BLaunch &L, const unsigned int *cell_start, const float4 *pos, const float4 *vort,
@@ -349,7 +339,7 @@ void blaunch_vort_apply(const BLaunch &L, const unsigned int *cell_start, const 
     FSPH_BLOCK_SWITCH(L.block, {
         auto k = kb_vort_apply<B_>;
         k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, cell_start, pos, vort, dens, vel_in,
-                                                                       vel_out, nl.list, nl.cnt, nl.cellb, wm);
+                                                                       vel_out, nl.list, nl.cnt, wm);
     })
 }
 

@@ -133,36 +133,18 @@ __device__ __forceinline__ bool cell_row_ok(const DevParams &p, unsigned int bas
 
 /* Neighbour lists: up to kListMax entries per particle, transposed (entry
  * k of slot i at list_at(k, i, n)) so a warp's lanes read consecutive
- * words.  An entry is the candidate's slot (32 bits).  Built with
- * FSPH_LIST16 it is (row << 12) | (j - row_start) in 16 bits, row = the
- * (dz, dy) index 0..8 of the 27-cell neighbourhood of the particle's build
- * cell: half the list bytes, but every candidate then pays a shared-memory
- * row-start lookup, and the passes are bound by instruction issue (the
- * 32-bit form measured 14 % faster per step).  A count of kListOverflow
- * sends the particle to the cell walk. */
+ * words.  An entry is the candidate's slot (32 bits; 16-bit row / offset
+ * entries halve the list bytes, but every candidate then pays a row-start
+ * lookup: 14 % slower per step).  A count of kListOverflow sends the particle
+ * to the cell walk.  Entries are stored in groups of four: group g of slot i
+ * is the 16-byte word [g * n + i], so a warp reads four entries of its 32
+ * slots with one coalesced 512-byte load; a list's last group is padded with
+ * its last entry. */
 constexpr int kListMax = 64;
 constexpr unsigned char kListOverflow = 255;
-#ifndef FSPH_LIST16
-#define FSPH_LIST32
-#endif
-#ifdef FSPH_LIST32
-typedef unsigned int ListEntry;   /* the candidate's slot itself */
-#else
-typedef unsigned short ListEntry; /* (row << 12) | (slot - row start) */
-#endif
-/* 32-bit entries are stored in groups of four: group g of slot i is the
- * 16-byte word [g * n + i], so a warp reads four entries of its 32 slots
- * with one coalesced 512-byte load; a list's last group is padded with its
- * last entry.  FSPH_LIST_SCALAR keeps one entry per word ([t * n + i]). */
-#if defined(FSPH_LIST32) && !defined(FSPH_LIST_SCALAR)
-#define FSPH_LIST_GROUPED 1
-#endif
+typedef unsigned int ListEntry;
 __host__ __device__ inline size_t list_at(int t, int i, int n) {
-#ifdef FSPH_LIST_GROUPED
     return ((size_t)(t >> 2) * (size_t)n + (size_t)i) * 4 + (size_t)(t & 3);
-#else
-    return (size_t)t * (size_t)n + (size_t)i;
-#endif
 }
 
 /* Warm-start features of a particle at the end of a step, all dimensionless:

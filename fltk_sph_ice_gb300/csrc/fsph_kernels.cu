@@ -272,7 +272,7 @@ __global__ void k_rebuild_copy(int n, DevCtl *ctl, const float4 *__restrict__ t_
 /* ======================================================================== */
 
 /* Every slot j within the list radius (= the cell width) of slot i at the
- * build positions xb, self included, as (row << 12) | (j - row_start). */
+ * build positions xb, self included. */
 __global__ void k_build_list(DevParams p, const unsigned int *__restrict__ cell_start,
                              const float4 *__restrict__ xb, const unsigned int *__restrict__ cellb,
                              ListEntry *__restrict__ list, unsigned char *__restrict__ cnt) {
@@ -358,9 +358,7 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_lambda(DevParams
                                                    DevCtl *ctl, ErrPartial *part,
                                                    cudaGraphConditionalHandle hwhile, int use_graph,
                                                    const ListEntry *__restrict__ list,
-                                                   const unsigned char *__restrict__ cnt,
-                                                   const unsigned int *__restrict__ cellb) {
-    __shared__ unsigned int s_rs[9 * kPassBlock];
+                                                   const unsigned char *__restrict__ cnt) {
     const unsigned int par = *((volatile unsigned int *)&ctl->parity);
     float4 *pp = par ? ppos1 : ppos0;
     float e1 = 0.f, e2 = 0.f, em = 0.f;
@@ -375,8 +373,7 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_lambda(DevParams
          c = next_chunk(c, nw, stat, &ctl->grab, lane)) {
         const int i = c * 32 + lane;
         if (i < p.n) {
-            const float C = lambda_body<1, KAHAN>(p, cell_start, pp, dens, ctl, list, cnt, cellb, s_rs + threadIdx.x,
-                                                  i, 0, true);
+            const float C = lambda_body<1, KAHAN>(p, cell_start, pp, dens, ctl, list, cnt, i, 0, true);
             q1 += err_fix(C > 0.0f ? C : 0.0f);
             q2 += err_fix(fabsf(C));
             em = fmaxf(em, fabsf(C));
@@ -398,8 +395,7 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_lambda(DevParams
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
 #endif
         if (i < p.n) {
-            const float C = lambda_body<1, KAHAN>(p, cell_start, pp, dens, ctl, list, cnt, cellb, s_rs + threadIdx.x,
-                                                  i, 0, true);
+            const float C = lambda_body<1, KAHAN>(p, cell_start, pp, dens, ctl, list, cnt, i, 0, true);
             e1 += C > 0.0f ? C : 0.0f;
             e2 += fabsf(C);
             em = fmaxf(em, fabsf(C));
@@ -420,9 +416,7 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_correction(DevPa
                                                        cudaGraphConditionalHandle hif2, int use_graph,
                                                        float4 *__restrict__ dp_out,
                                                        const ListEntry *__restrict__ list,
-                                                       const unsigned char *__restrict__ cnt,
-                                                       const unsigned int *__restrict__ cellb) {
-    __shared__ unsigned int s_rs[9 * kPassBlock];
+                                                       const unsigned char *__restrict__ cnt) {
     const unsigned int par = *((volatile unsigned int *)&ctl->parity);
     const float4 *__restrict__ src = par ? ppos1 : ppos0;
     float4 *__restrict__ dst = par ? ppos0 : ppos1;
@@ -443,8 +437,7 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_correction(DevPa
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
 #endif
         if (i < p.n)
-            disp2 = fmaxf(disp2, correction_body<1>(p, cell_start, src, dst, xb, ctl, dp_out, list, cnt, cellb,
-                                                    s_rs + threadIdx.x, i, 0, true));
+            disp2 = fmaxf(disp2, correction_body<1>(p, cell_start, src, dst, xb, ctl, dp_out, list, cnt, i, 0, true));
     }
     correction_tail(p, ctl, part, disp2, par, hif, hif2, use_graph);
 }
@@ -484,13 +477,10 @@ __global__ void __launch_bounds__(kBlock) k_xsph_vort(DevParams p, const unsigne
                                                       float4 *__restrict__ vort, FeatureOut fo,
                                                       const ListEntry *__restrict__ list,
                                                       const unsigned char *__restrict__ cnt,
-                                                      const unsigned int *__restrict__ cellb,
                                                       const float *__restrict__ mrho, float2 *__restrict__ wm) {
-    __shared__ unsigned int s_rs[9 * kBlock];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    xsph_vort_body<NBR, PRE>(p, i, cell_start, pos, vel, dens, vel_out, vort, fo, list, cnt, cellb,
-                             s_rs + threadIdx.x, mrho, wm);
+    xsph_vort_body<NBR, PRE>(p, i, cell_start, pos, vel, dens, vel_out, vort, fo, list, cnt, mrho, wm);
 }
 
 /* eta_i = sum_j (m / rho_j)(|w_j| - |w_i|) grad_i W_ij; f = eps (eta/|eta|) x w_i;
@@ -504,13 +494,10 @@ __global__ void __launch_bounds__(kBlock) k_vort_apply(DevParams p, const unsign
                                                        float4 *__restrict__ vel_out,
                                                        const ListEntry *__restrict__ list,
                                                        const unsigned char *__restrict__ cnt,
-                                                       const unsigned int *__restrict__ cellb,
-                                                       const float2 *__restrict__ wm) {
-    __shared__ unsigned int s_rs[9 * kBlock];
+                                                      const float2 *__restrict__ wm) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    vort_apply_body<PRE>(p, i, cell_start, pos, vort, dens, vel_in, vel_out, list, cnt, cellb, s_rs + threadIdx.x,
-                         wm);
+    vort_apply_body<PRE>(p, i, cell_start, pos, vort, dens, vel_in, vel_out, list, cnt, wm);
 }
 
 /* ======================================================================== */
@@ -583,7 +570,7 @@ __global__ void __launch_bounds__(kBlock) k_boundary_lambda(DevParams p, const u
     const float agr = p.ag * p.inv_rest_dens;
     float wsum = 0.f, sd = 0.f;
     for_each_candidate<1>(
-        p, cell_start, nullptr, nullptr, nullptr, 0, xb, nullptr, 0, [&](unsigned int j) { return pp[j]; },
+        p, cell_start, nullptr, nullptr, 0, xb, 0, [&](unsigned int j) { return pp[j]; },
         [&](unsigned int, const float4 &xj4) {
             const float3 d = xb - f3(xj4);
             const float r2 = dot3(d, d);
@@ -668,10 +655,8 @@ __global__ void __launch_bounds__(kBlock) k_sph_density(DevParams p, const unsig
         }
     if (list) {
         ovf = k > kListMax;
-#ifdef FSPH_LIST_GROUPED
         if (!ovf) /* pad the last group (k >= 1: the slot itself is always listed) */
             for (int t = k; (t & 3) != 0; ++t) list[list_at(t, i, p.n)] = last;
-#endif
         cnt[i] = ovf ? kListOverflow : (unsigned char)k;
     }
     const float rho = p.mass * p.aw * acc;
@@ -736,10 +721,8 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
     if (!valid || sub != 0) return;
     if (list) {
         const bool ovf = k > kListMax;
-#ifdef FSPH_LIST_GROUPED
         if (!ovf) /* pad the last group (k >= 1: the slot itself is always listed) */
             for (int u = k; (u & 3) != 0; ++u) list[list_at(u, i, p.n)] = (ListEntry)last;
-#endif
         cnt[i] = ovf ? kListOverflow : (unsigned char)k;
     }
     const float rho = p.mass * p.aw * acc;
@@ -774,7 +757,7 @@ __global__ void __launch_bounds__(kBlock) k_sph_force(DevParams p, const unsigne
     const float prsi = xi4.w;
     float3 fp = make_float3(0.f, 0.f, 0.f), fv = make_float3(0.f, 0.f, 0.f);
     for_each_candidate<LPP>(
-        p, cell_start, list, cnt, nullptr, i, xi, nullptr, sub,
+        p, cell_start, list, cnt, i, xi, sub,
         [&](unsigned int j) { return PosVel{__ldg(pos + j), __ldg(vel + j)}; },
         [&](unsigned int, const PosVel &b) {
             const float3 d = xi - f3(b.x);
@@ -1132,7 +1115,7 @@ void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *p
     auto k = p.compensated ? k_lambda<true> : k_lambda<false>;
     k<<<pass_blocks(p.n, (const void *)k, FSPH_PERSIST_LAMBDA != 0), kPassBlock, 0, s>>>(p, cell_start, ppos0, ppos1, dens, ctl, part,
                                          (cudaGraphConditionalHandle)while_handle, use_graph,
-                                         p.use_lists ? nl.list : nullptr, nl.cnt, nl.cellb);
+                                         p.use_lists ? nl.list : nullptr, nl.cnt);
 }
 void launch_build_list(const DevParams &p, const unsigned int *cell_start, const float4 *xb, const NbrLists &nl,
                        cudaStream_t s) {
@@ -1147,7 +1130,7 @@ void launch_correction(const DevParams &p, const unsigned int *cell_start, float
                                                                                     ctl, part,
                                                     (cudaGraphConditionalHandle)if_handle,
                                                     (cudaGraphConditionalHandle)if_handle2, use_graph, dp_out,
-                                                    p.use_lists ? nl.list : nullptr, nl.cnt, nl.cellb);
+                                                    p.use_lists ? nl.list : nullptr, nl.cnt);
 }
 void launch_finalize(const DevParams &p, const float4 *pos_b, const float4 *ppos0, const float4 *ppos1,
                      const DevCtl *ctl, const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a,
@@ -1164,14 +1147,14 @@ void launch_xsph_vort(const DevParams &p, const unsigned int *cell_start, const 
     auto k = nbr ? (pre ? k_xsph_vort<true, true> : k_xsph_vort<true, false>)
                  : (pre ? k_xsph_vort<false, true> : k_xsph_vort<false, false>);
     k<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, vel, dens, vel_out, vort, fo,
-                                         p.use_lists ? nl.list : nullptr, nl.cnt, nl.cellb, mrho, wm);
+                                         p.use_lists ? nl.list : nullptr, nl.cnt, mrho, wm);
 }
 void launch_vort_apply(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vort,
                        const float *dens, const float4 *vel_in, float4 *vel_out, const NbrLists &nl, cudaStream_t s,
                        const float2 *wm) {
     auto k = wm ? k_vort_apply<true> : k_vort_apply<false>;
     k<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, vort, dens, vel_in, vel_out,
-                                         p.use_lists ? nl.list : nullptr, nl.cnt, nl.cellb, wm);
+                                         p.use_lists ? nl.list : nullptr, nl.cnt, wm);
 }
 int sph_force_lanes(int n);
 void launch_sph_density(const DevParams &p, const unsigned int *cell_start, float4 *pos, float4 *vel, float *dens,

@@ -23,9 +23,8 @@ namespace fsph {
  * cells around the current position.  List entries are taken kBatch at a
  * time: their indices are decoded and their positions loaded before any is
  * used, so each thread keeps kBatch independent loads in flight (the passes
- * are bound by load latency, not by arithmetic).  rs: this thread's 9 row
- * starts in shared memory, strided by the block size.  Load selects the
- * load flavour for x. */
+ * are bound by load latency, not by arithmetic).  Load selects the load
+ * flavour for x. */
 #ifndef FSPH_KBATCH
 #define FSPH_KBATCH 4
 #endif
@@ -129,9 +128,7 @@ __device__ __forceinline__ void prefetch_list_group(const uint4 *a) {
 template <int LPP, class Load, class F>
 __device__ __forceinline__ void for_each_candidate(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                                    const ListEntry *__restrict__ list,
-                                                   const unsigned char *__restrict__ cnt,
-                                                   const unsigned int *__restrict__ cellb, int i, float3 xi,
-                                                   unsigned int *rs, int sub, Load &&load, F &&f) {
+                                                   const unsigned char *__restrict__ cnt, int i, float3 xi, int sub, Load &&load, F &&f) {
     int k = list ? (int)cnt[i] : (int)kListOverflow;
 #if FSPH_DEBUG_BOUNDS
     if (k > kListMax && k != (int)kListOverflow) { /* a count the build never writes: walk the cells */
@@ -139,7 +136,6 @@ __device__ __forceinline__ void for_each_candidate(const DevParams &p, const uns
         k = (int)kListOverflow;
     }
 #endif
-#ifdef FSPH_LIST_GROUPED
     if (LPP == 1 && kBatch == 4 && k != (int)kListOverflow) {
         /* one 16-byte load brings the next four entries (the tail group is
          * padded with a valid slot, so every load stays in bounds) */
@@ -161,29 +157,14 @@ __device__ __forceinline__ void for_each_candidate(const DevParams &p, const uns
             for (int u = 0; u < 4; ++u)
                 if (t0 + u < k) f(j[u], xj[u]);
         }
-    } else
-#endif
-    if (k != (int)kListOverflow) {
-#ifndef FSPH_LIST32
-        const int cb = (int)cellb[i];
-#pragma unroll
-        for (int r = 0; r < 9; ++r) {
-            const int base = cb + ((r / 3 - 1) * p.gy + (r % 3 - 1)) * p.gx;
-            rs[r * blockDim.x] = cell_row_ok(p, (unsigned int)base) ? __ldg(cell_start + base - 1) : 0u;
-        }
-#endif
+    } else if (k != (int)kListOverflow) {
         for (int t0 = sub; t0 < k; t0 += kBatch * LPP) {
             unsigned int j[kBatch];
             decltype(load(0u)) xj[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
                 const int t = t0 + u * LPP < k ? t0 + u * LPP : k - 1;
-#ifdef FSPH_LIST32
                 j[u] = bounded(p, __ldg(list + list_at(t, i, p.n)), (unsigned int)p.n, kBoundSlot);
-#else
-                const unsigned int e = __ldg(list + list_at(t, i, p.n));
-                j[u] = bounded(p, rs[((e >> 12) % 9u) * blockDim.x] + (e & 0xfffu), (unsigned int)p.n, kBoundSlot);
-#endif
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) xj[u] = load(j[u]);
@@ -264,14 +245,13 @@ __device__ __forceinline__ void hash_body(const DevParams &p, int i, float3 x, u
 }
 
 /* Every slot j within the list radius (= the cell width) of slot i at the
- * build positions xb, self included, as (row << 12) | (j - row_start). */
+ * build positions xb, self included, in ascending order. */
 __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const unsigned int *__restrict__ cell_start,
                                                 const float4 *__restrict__ xb, const unsigned int *__restrict__ cellb,
                                                 ListEntry *__restrict__ list, unsigned char *__restrict__ cnt) {
     const float3 xi = f3(xb[i]);
     const int cb = (int)cellb[i];
     int k = 0;
-    bool ovf = false;
     ListEntry last = 0;
 #pragma unroll 1
     for (int r = 0; r < 9; ++r) {
@@ -279,7 +259,6 @@ __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const
         if (!cell_row_ok(p, (unsigned int)base)) continue;
         const unsigned int s = __ldg(cell_start + base - 1);
         const unsigned int e = bounded(p, __ldg(cell_start + base + 2), (unsigned int)p.n + 1u, kBoundSlot);
-        if (e - s > 4095u) ovf = true;
         /* four candidates' loads in flight before their tests */
         for (unsigned int j0 = s; j0 < e; j0 += 4) {
             float4 xc[4];
@@ -289,22 +268,16 @@ __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const
             for (int u = 0; u < 4; ++u) {
                 const float3 d = xi - f3(xc[u]);
                 if (j0 + u < e && dot3(d, d) < p.rl2) {
-#ifdef FSPH_LIST32
                     last = j0 + u;
-#else
-                    last = (ListEntry)((r << 12) | (j0 + u - s));
-#endif
                     if (k < kListMax) list[list_at(k, i, p.n)] = last;
                     ++k;
                 }
             }
         }
     }
-    const bool overflow = ovf || k > kListMax;
-#ifdef FSPH_LIST_GROUPED
+    const bool overflow = k > kListMax;
     if (!overflow) /* pad the last group (k >= 1: the slot itself is always listed) */
         for (int t = k; (t & 3) != 0; ++t) list[list_at(t, i, p.n)] = last;
-#endif
     cnt[i] = overflow ? kListOverflow : (unsigned char)k;
 }
 
@@ -317,8 +290,7 @@ template <int LPP, bool KAHAN = false>
 __device__ __forceinline__ float lambda_body(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                              float4 *pp, float *__restrict__ dens, DevCtl *ctl,
                                              const ListEntry *__restrict__ list,
-                                             const unsigned char *__restrict__ cnt,
-                                             const unsigned int *__restrict__ cellb, unsigned int *rs, int i, int sub,
+                                             const unsigned char *__restrict__ cnt, int i, int sub,
                                              bool valid) {
     const float3 xi = f3(pp[i]);
     float wsum = 0.f, wc = 0.f, sd = 0.f;
@@ -334,7 +306,7 @@ __device__ __forceinline__ float lambda_body(const DevParams &p, const unsigned 
     /* plain (L1-cached) loads: only the .w words of pp are written by this
      * pass, and the neighbour loop reads x, y, z */
     for_each_candidate<LPP>(
-        p, cell_start, list, cnt, cellb, i, xi, rs, sub, [&](unsigned int j) { return pp[j]; },
+        p, cell_start, list, cnt, i, xi, sub, [&](unsigned int j) { return pp[j]; },
         [&](unsigned int, const float4 &xj4) {
             /* branch-free: outside h both q and t clamp to zero; the self
              * pair (d = 0) adds W(0) to the density and nothing else */
@@ -553,8 +525,7 @@ __device__ __forceinline__ float correction_body(const DevParams &p, const unsig
                                                  const float4 *__restrict__ src, float4 *__restrict__ dst,
                                                  const float4 *__restrict__ xb, DevCtl *ctl,
                                                  float4 *__restrict__ dp_out, const ListEntry *__restrict__ list,
-                                                 const unsigned char *__restrict__ cnt,
-                                                 const unsigned int *__restrict__ cellb, unsigned int *rs, int i,
+                                                 const unsigned char *__restrict__ cnt, int i,
                                                  int sub, bool valid) {
     const float4 xi4 = src[i];
     const float3 xi = f3(xi4);
@@ -574,7 +545,7 @@ __device__ __forceinline__ float correction_body(const DevParams &p, const unsig
     const float agl = agr;
 #endif
     for_each_candidate<LPP>(
-        p, cell_start, list, cnt, cellb, i, xi, rs, sub, [&](unsigned int j) { return __ldg(src + j); },
+        p, cell_start, list, cnt, i, xi, sub, [&](unsigned int j) { return __ldg(src + j); },
         [&](unsigned int, const float4 &xj4) {
             /* branch-free: t = 0 outside h and d = 0 for the self pair */
             const float3 d = xi - f3(xj4);
@@ -705,7 +676,6 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
                                                float4 *__restrict__ vort, const FeatureOut &fo,
                                                const ListEntry *__restrict__ list,
                                                const unsigned char *__restrict__ cnt,
-                                               const unsigned int *__restrict__ cellb, unsigned int *rs,
                                                const float *__restrict__ mrho_in = nullptr,
                                                float2 *__restrict__ wm = nullptr) {
     const float3 xi = f3(pos[i]), vi = f3(vel[i]);
@@ -720,7 +690,7 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
     /* branch-free pair terms: q and t clamp to zero outside h, and the self
      * pair (d = 0, v_ij = 0) adds only to the neighbour count */
     for_each_candidate<1>(
-        p, cell_start, list, cnt, cellb, i, xi, rs, 0, [&](unsigned int j) { return __ldg(pos + j); },
+        p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return __ldg(pos + j); },
         [&](unsigned int j, const float4 &xj4) {
             const float3 d = xi - f3(xj4);
             const float r2 = dot3(d, d);
@@ -803,8 +773,7 @@ __device__ __forceinline__ void vort_apply_body(const DevParams &p, int i, const
                                                 const float *__restrict__ dens, const float4 *__restrict__ vel_in,
                                                 float4 *__restrict__ vel_out, const ListEntry *__restrict__ list,
                                                 const unsigned char *__restrict__ cnt,
-                                                const unsigned int *__restrict__ cellb, unsigned int *rs,
-                                                const float2 *__restrict__ wm = nullptr) {
+                                               const float2 *__restrict__ wm = nullptr) {
     float4 v4 = vel_in[i];
     if (p.vort_eps != 0.0f) {
         const float3 xi = f3(pos[i]);
@@ -812,7 +781,7 @@ __device__ __forceinline__ void vort_apply_body(const DevParams &p, int i, const
         const float wmi = sqrtf(dot3(wi, wi));
         float3 eta = make_float3(0.f, 0.f, 0.f);
         for_each_candidate<1>(
-            p, cell_start, list, cnt, cellb, i, xi, rs, 0, [&](unsigned int j) { return __ldg(pos + j); },
+            p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return __ldg(pos + j); },
             [&](unsigned int j, const float4 &xj4) {
                 const float3 d = xi - f3(xj4);
                 const float r2 = dot3(d, d);
