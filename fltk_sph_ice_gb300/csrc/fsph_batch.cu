@@ -90,17 +90,23 @@ __global__ void __launch_bounds__(BLOCK) kb_hash_parity(BatchArgs b, const float
     }
 }
 
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) kb_build_list(BatchArgs b, const unsigned int *__restrict__ cell_start,
-                                                       const float4 *__restrict__ xb,
-                                                       const unsigned int *__restrict__ cellb,
-                                                       ListEntry *__restrict__ list,
-                                                       unsigned char *__restrict__ cnt) {
+/* the blocks are kListBlock threads whatever the tiles' size: each walks its
+ * tile kListBlock slots at a time */
+__global__ void __launch_bounds__(kListBlock) kb_build_list(BatchArgs b, const unsigned int *__restrict__ cell_start,
+                                                            const float4 *__restrict__ xb,
+                                                            const unsigned int *__restrict__ cellb,
+                                                            ListEntry *__restrict__ list,
+                                                            unsigned char *__restrict__ cnt) {
     __shared__ DevParams s_p;
+    __shared__ PairTile s_tile[kListBlock / 32];
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const BTile tl = tile_begin(b, t, s_p);
         const DevParams p = s_p;
-        if ((int)threadIdx.x < tl.count) build_list_body(p, tl.start + threadIdx.x, cell_start, xb, cellb, list, cnt);
+        for (int o = 0; o < tl.count; o += kListBlock) {
+            const int at = o + (int)threadIdx.x;
+            build_list_warp(p, tl.start + at, at < tl.count, cell_start, xb, cellb, list, cnt,
+                            s_tile[threadIdx.x >> 5]);
+        }
     }
 }
 
@@ -292,11 +298,8 @@ void blaunch_hash_parity(const BLaunch &L, const float4 *p0, const float4 *p1, c
 }
 void blaunch_build_list(const BLaunch &L, const unsigned int *cell_start, const float4 *xb, const NbrLists &nl,
                         cudaStream_t s) {
-    FSPH_BLOCK_SWITCH(L.block, {
-        auto k = kb_build_list<B_>;
-        k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, cell_start, xb, nl.cellb, nl.list,
-                                                                       nl.cnt);
-    })
+    kb_build_list<<<persistent_grid(kb_build_list, kListBlock, L.full.ntiles, L.sms), kListBlock, 0, s>>>(
+        L.full, cell_start, xb, nl.cellb, nl.list, nl.cnt);
 }
 unsigned int blaunch_lambda(const BLaunch &L, const DevParams &lp, const unsigned int *cell_start, float4 *p0,
                             float4 *p1, float *dens, DevCtl *ctl, ErrPartial *part, unsigned long long hw,

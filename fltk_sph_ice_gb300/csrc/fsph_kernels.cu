@@ -271,14 +271,15 @@ __global__ void k_rebuild_copy(int n, DevCtl *ctl, const float4 *__restrict__ t_
 /* neighbour lists                                                          */
 /* ======================================================================== */
 
-/* Every slot j within the list radius (= the cell width) of slot i at the
- * build positions xb, self included. */
-__global__ void k_build_list(DevParams p, const unsigned int *__restrict__ cell_start,
-                             const float4 *__restrict__ xb, const unsigned int *__restrict__ cellb,
-                             ListEntry *__restrict__ list, unsigned char *__restrict__ cnt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    build_list_body(p, i, cell_start, xb, cellb, list, cnt);
+/* The lists of every slot, a warp for 32 consecutive ones (build_list_warp). */
+__global__ void __launch_bounds__(kListBlock) k_build_list(DevParams p, const unsigned int *__restrict__ cell_start,
+                                                           const float4 *__restrict__ xb,
+                                                           const unsigned int *__restrict__ cellb,
+                                                           ListEntry *__restrict__ list,
+                                                           unsigned char *__restrict__ cnt) {
+    __shared__ PairTile s_tile[kListBlock / 32];
+    const int i = blockIdx.x * kListBlock + threadIdx.x;
+    build_list_warp(p, i, i < p.n, cell_start, xb, cellb, list, cnt, s_tile[threadIdx.x >> 5]);
 }
 
 /* ======================================================================== */
@@ -1120,7 +1121,7 @@ void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *p
 void launch_build_list(const DevParams &p, const unsigned int *cell_start, const float4 *xb, const NbrLists &nl,
                        cudaStream_t s) {
     if (!p.use_lists) return;
-    k_build_list<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, xb, nl.cellb, nl.list, nl.cnt);
+    k_build_list<<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, xb, nl.cellb, nl.list, nl.cnt);
 }
 void launch_correction(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                        const float4 *xb, DevCtl *ctl, float *part, unsigned long long if_handle,
