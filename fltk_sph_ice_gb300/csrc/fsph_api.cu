@@ -18,6 +18,7 @@
  *     caller's particle order through the device slot -> particle index map;
  *   - no GL buffers and no CPU neighbour mirror (rx_sph_pbd_gpu.cpp:962-1011).
  */
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -86,8 +87,7 @@ struct fsph_ctx {
     int gdim[3] = {0, 0, 0};
     DevCtl *ctl = nullptr;
     DevCtl *ctl_host = nullptr;
-    unsigned int *flag = nullptr;      /* input-validation flag */
-    unsigned int *flag_host = nullptr;
+    unsigned int *flag = nullptr;      /* input-validation flag, pinned host memory */
     /* warm start */
     float4 *xpred = nullptr;           /* x* before the iterations, iteration order */
     float4 *dstep = nullptr;           /* x*_final - x*_pred of the last step, home order */
@@ -1214,8 +1214,7 @@ int fsph_create(const fsph_params *params, fsph_ctx **out) {
     if (cudaMalloc((void **)&c->ctl, sizeof(DevCtl)) != cudaSuccess) return bail(FSPH_OOM);
     if (cudaMallocHost((void **)&c->ctl_host, sizeof(DevCtl)) != cudaSuccess) return bail(FSPH_OOM);
     std::memset(c->ctl_host, 0, sizeof(DevCtl));
-    if (cudaMalloc((void **)&c->flag, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
-    if (cudaMallocHost((void **)&c->flag_host, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
+    if (cudaMallocHost((void **)&c->flag, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
     if (cudaMalloc((void **)&c->warm_valid, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
     if (cudaMalloc((void **)&c->mlp_dev, sizeof(MlpDev)) != cudaSuccess) return bail(FSPH_OOM);
     cudaMemsetAsync(c->warm_valid, 0, sizeof(unsigned int), c->stream);
@@ -1237,8 +1236,7 @@ int fsph_destroy(fsph_ctx *c) {
     free_boundary(c);
     cudaFree(c->ctl);
     if (c->ctl_host) cudaFreeHost(c->ctl_host);
-    cudaFree(c->flag);
-    if (c->flag_host) cudaFreeHost(c->flag_host);
+    if (c->flag) cudaFreeHost(c->flag);
     cudaFree(c->warm_valid);
     cudaFree(c->mlp_dev);
     cudaFree(c->obs_dev);
@@ -1317,12 +1315,11 @@ int fsph_set_particles(fsph_ctx *c, const float *pos4, const float *vel4, int n,
     if (where != FSPH_HOST && where != FSPH_DEVICE) return fail(c, FSPH_INVALID_ARG, "where");
     FSPH_TRY(load_particles(c, pos4, vel4, n, where));
     /* finiteness is checked on the device, where the data now is */
-    FSPH_CUDA(c, cudaMemsetAsync(c->flag, 0, sizeof(unsigned int), c->stream));
+    *c->flag = 0u;
     if (n > 0) launch_check_finite(n, c->set[0].pos, c->set[0].vel, c->flag, c->stream);
-    FSPH_CUDA(c, cudaMemcpyAsync(c->flag_host, c->flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream));
     FSPH_CUDA(c, cudaStreamSynchronize(c->stream));
     FSPH_TRY(check_launch(c));
-    if (*c->flag_host) {
+    if (*c->flag) {
         c->n = 0;
         return fail(c, FSPH_NAN_DETECTED, "non-finite input position or velocity");
     }
@@ -1358,13 +1355,16 @@ int fsph_set_array(fsph_ctx *c, int type, const void *data, int start, int count
         /* staged and checked before it replaces anything: a range with a
          * non-finite value is rejected and the state stays as it was (the
          * same rule as fsph_set_particles) */
-        FSPH_CUDA(c, cudaMemcpyAsync(c->tmp4, data, (size_t)count * 16, k, s));
-        FSPH_CUDA(c, cudaMemsetAsync(c->flag, 0, sizeof(unsigned int), s));
-        launch_check_finite(count, c->tmp4, nullptr, c->flag, s);
-        FSPH_CUDA(c, cudaMemcpyAsync(c->flag_host, c->flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-        FSPH_TRY(check_launch(c));
+        *c->flag = 0u;
+        if (where == FSPH_DEVICE && device_span(data, (size_t)count * 16, 16)) {
+            launch_check_finite(count, (const float4 *)data, nullptr, c->flag, s, c->tmp4);
+        } else {
+            FSPH_CUDA(c, cudaMemcpyAsync(c->tmp4, data, (size_t)count * 16, k, s));
+            launch_check_finite(count, c->tmp4, nullptr, c->flag, s);
+        }
+            FSPH_TRY(check_launch(c));
         FSPH_CUDA(c, cudaStreamSynchronize(s));
-        if (*c->flag_host) return fail(c, FSPH_NAN_DETECTED, "non-finite position or velocity");
+        if (*c->flag) return fail(c, FSPH_NAN_DETECTED, "non-finite position or velocity");
         float4 *dst = type == FSPH_POSITION ? c->set[0].pos : c->set[0].vel;
         if (c->home_identity)
             FSPH_CUDA(c, cudaMemcpyAsync(dst + start, c->tmp4, (size_t)count * 16, cudaMemcpyDeviceToDevice, s));
@@ -1494,6 +1494,19 @@ int fsph_sync(fsph_ctx *c) {
     return FSPH_OK;
 }
 
+namespace {
+/* p points into an array of the context (fsph_device_ptr hands some out):
+ * reordering one of them into another goes through the staging */
+bool own_buffer(const fsph_ctx *c, const void *p) {
+    const char *q = (const char *)p;
+    const size_t n = (size_t)std::max(c->cap, 1);
+    auto in = [&](const void *b, size_t elem) { return b && q >= (const char *)b && q < (const char *)b + n * elem; };
+    return in(c->set[0].pos, 16) || in(c->set[1].pos, 16) || in(c->set[0].vel, 16) || in(c->set[1].vel, 16) ||
+           in(c->set[0].id, 4) || in(c->set[1].id, 4) || in(c->set[0].attr, 4) || in(c->set[1].attr, 4) ||
+           in(c->acc, 16) || in(c->vort, 16) || in(c->dens, 4) || in(c->pres, 4);
+}
+}  // namespace
+
 int fsph_get_array(fsph_ctx *c, int type, void *dst, int where, void *stream) {
     if (!c || !dst) return FSPH_INVALID_ARG;
     FSPH_USABLE(c);
@@ -1513,8 +1526,15 @@ int fsph_get_array(fsph_ctx *c, int type, void *dst, int where, void *stream) {
                         type == FSPH_CORRECTION || type == FSPH_DENSITY || type == FSPH_PRESSURE ||
                         type == FSPH_SCALING_FACTOR;
     if (result && c->res_in_res_id) id = c->res_id;
-    /* staging in device memory: the rank / key arrays are free between steps */
-    float4 *t4 = c->set[1].pos;
+    /* a caller's device buffer is written by the reordering kernel itself;
+     * else staging in device memory, free between steps */
+    const bool words = type == FSPH_DENSITY || type == FSPH_PRESSURE || type == FSPH_ATTRIBUTE ||
+                       type == FSPH_SCALING_FACTOR || type == FSPH_SORTED_ID;
+    const bool direct = where == FSPH_DEVICE && type != FSPH_SORTED_ID && type != FSPH_CORRECTION &&
+                        type != FSPH_FEATURES && !own_buffer(c, dst) &&
+                        device_span(dst, (size_t)n * (words ? 4 : 16), words ? 4 : 16);
+    float4 *t4 = direct && !words ? (float4 *)dst : c->set[1].pos;
+    unsigned int *t1 = direct && words ? (unsigned int *)dst : c->set[1].id;
     bool vec = true;
     switch (type) {
     case FSPH_POSITION: launch_unsort4(n, id, c->set[0].pos, t4, 1, s); break;
@@ -1554,12 +1574,12 @@ int fsph_get_array(fsph_ctx *c, int type, void *dst, int where, void *stream) {
         const unsigned int *src = type == FSPH_DENSITY ? reinterpret_cast<const unsigned int *>(c->dens)
                                   : type == FSPH_PRESSURE ? reinterpret_cast<const unsigned int *>(c->pres)
                                                           : c->set[0].attr;
-        launch_unsort1(n, id, src, c->set[1].id, s); /* id = set[0].id for the attribute */
+        launch_unsort1(n, id, src, t1, s); /* id = set[0].id for the attribute */
         break;
     }
     case FSPH_SCALING_FACTOR:
         vec = false;
-        launch_unsort_w(n, id, c->ppos[1 - (c->ctl_host->parity & 1)], reinterpret_cast<float *>(c->set[1].id), s);
+        launch_unsort_w(n, id, c->ppos[1 - (c->ctl_host->parity & 1)], reinterpret_cast<float *>(t1), s);
         break;
     case FSPH_SORTED_ID:
         vec = false;
@@ -1571,7 +1591,9 @@ int fsph_get_array(fsph_ctx *c, int type, void *dst, int where, void *stream) {
     FSPH_TRY(check_launch(c));
     const void *src = vec ? (const void *)t4 : (const void *)c->set[1].id;
     size_t bytes = (size_t)n * (vec ? 16 : 4);
-    FSPH_CUDA(c, cudaMemcpyAsync(dst, src, bytes, where == FSPH_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, s));
+    if (!direct)
+        FSPH_CUDA(c, cudaMemcpyAsync(dst, src, bytes,
+                                     where == FSPH_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, s));
     FSPH_CUDA(c, cudaStreamSynchronize(s));
     return FSPH_OK;
 }
@@ -1624,11 +1646,10 @@ int fsph_neighbors_ex(fsph_ctx *c, const float *pos4, int n, float radius, int w
         /* the given positions stand in for the particles: scratch copy, ids 0..n-1 */
         FSPH_CUDA(c, cudaMemcpyAsync(c->tmp4, pos4, (size_t)n * 16,
                                      where == FSPH_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
-        FSPH_CUDA(c, cudaMemsetAsync(c->flag, 0, sizeof(unsigned int), s));
+        *c->flag = 0u;
         launch_check_finite(n, c->tmp4, nullptr, c->flag, s);
-        FSPH_CUDA(c, cudaMemcpyAsync(c->flag_host, c->flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-        FSPH_CUDA(c, cudaStreamSynchronize(s));
-        if (*c->flag_host) return fail(c, FSPH_NAN_DETECTED, "non-finite position");
+            FSPH_CUDA(c, cudaStreamSynchronize(s));
+        if (*c->flag) return fail(c, FSPH_NAN_DETECTED, "non-finite position");
         launch_iota(n, c->set[1].attr, s);
         x = c->tmp4;
         ids = c->set[1].attr;
@@ -2004,11 +2025,10 @@ int fsph_set_boundary(fsph_ctx *c, const float *bpos4, int nb, int where) {
     FSPH_TRY(dalloc(c, &c->b_id, n)); FSPH_TRY(dalloc(c, &c->b_key, n)); FSPH_TRY(dalloc(c, &c->b_rank, n));
     cudaMemcpyKind k = where == FSPH_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     FSPH_CUDA(c, cudaMemcpyAsync(c->b_in, bpos4, n * sizeof(float4), k, c->stream));
-    FSPH_CUDA(c, cudaMemsetAsync(c->flag, 0, sizeof(unsigned int), c->stream));
+    *c->flag = 0u;
     launch_check_finite(nb, c->b_in, nullptr, c->flag, c->stream);
-    FSPH_CUDA(c, cudaMemcpyAsync(c->flag_host, c->flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream));
     FSPH_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (*c->flag_host) {
+    if (*c->flag) {
         free_boundary(c);
         return fail(c, FSPH_NAN_DETECTED, "non-finite boundary position");
     }
@@ -2492,6 +2512,42 @@ int fsph_sph_eval_forces(fsph_ctx *c, const float *pos4, const float *vel4, int 
 }
 
 }  // extern "C"
+
+namespace fsph {
+namespace {
+typedef CUresult (*PointerAttributes)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr);
+PointerAttributes pointer_attributes() { /* the driver's cuPointerGetAttributes, looked up once, thread-safely */
+    static const PointerAttributes get = []() -> PointerAttributes {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<PointerAttributes>(fn);
+        return nullptr;
+    }();
+    return get;
+}
+}  // namespace
+bool device_span(const void *p, size_t bytes, size_t align) {
+    const PointerAttributes get = pointer_attributes();
+    int dev = -1;
+    if (!get || !p || (reinterpret_cast<uintptr_t>(p) & (align - 1)) || cudaGetDevice(&dev) != cudaSuccess)
+        return false;
+    unsigned int type = 0, managed = 1;
+    int ordinal = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[5] = {&type, &managed, &ordinal, &start, &size};
+    const CUdeviceptr at = (CUdeviceptr) reinterpret_cast<uintptr_t>(p);
+    if (get(5, what, to, at) != CUDA_SUCCESS) return false;
+    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == dev && start != 0 && at >= start &&
+           bytes <= size && at - start <= size - bytes;
+}
+}  // namespace fsph
 
 /* Parameter builders shared with the allocation-free entry point
  * (fsph_noalloc.cu) and the batched scenes (fsph_batch.cu). */

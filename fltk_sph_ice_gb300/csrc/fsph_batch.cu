@@ -379,6 +379,7 @@ struct fsph_batch {
     BTile *d_tiles_full = nullptr, *d_tiles_cons = nullptr;
     int nt_full = 0, nt_cons = 0, cap_tiles_full = 0, cap_tiles_cons = 0;
     DevCtl *ctl = nullptr, *ctl_host = nullptr;
+    unsigned int *flag = nullptr; /* input-validation flag, pinned host memory */
     ErrPartial *epart = nullptr;
     float *dpart = nullptr;
     int cap_part = 0;
@@ -440,6 +441,7 @@ void bfree(fsph_batch *b) {
     cudaFree(b->d_scenes); cudaFree(b->d_offs); cudaFree(b->d_tiles_full); cudaFree(b->d_tiles_cons);
     cudaFree(b->ctl); cudaFree(b->epart); cudaFree(b->dpart); cudaFree(b->d_err);
     if (b->ctl_host) cudaFreeHost(b->ctl_host);
+    if (b->flag) cudaFreeHost(b->flag);
     if (b->h_err) cudaFreeHost(b->h_err);
 }
 
@@ -783,6 +785,7 @@ int fsph_batch_create(const fsph_params *params, const int *counts, int nscenes,
     A(&b->ctl, 1);
     if (st != FSPH_OK) return bail(st);
     if (cudaMallocHost((void **)&b->ctl_host, sizeof(DevCtl)) != cudaSuccess) return bail(FSPH_OOM);
+    if (cudaMallocHost((void **)&b->flag, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
     if (cudaMallocHost((void **)&b->h_err, 3 * sizeof(float) * nscenes) != cudaSuccess) return bail(FSPH_OOM);
     std::memset(b->ctl_host, 0, sizeof(DevCtl));
     std::memset(b->h_err, 0, 3 * sizeof(float) * nscenes);
@@ -827,19 +830,21 @@ int fsph_batch_set_particles(fsph_batch *b, const float *pos4, const float *vel4
     cudaMemcpyKind k = where == FSPH_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const size_t bytes = (size_t)b->n * sizeof(float4);
     cudaStream_t s = b->stream;
-    FB_CUDA(b, cudaMemcpyAsync(b->pos[0], pos4, bytes, k, s));
-    if (vel4) FB_CUDA(b, cudaMemcpyAsync(b->vel[0], vel4, bytes, k, s));
-    else FB_CUDA(b, cudaMemsetAsync(b->vel[0], 0, bytes, s));
+    *b->flag = 0u;
+    const bool direct = where == FSPH_DEVICE && device_span(pos4, bytes, 16) && (!vel4 || device_span(vel4, bytes, 16));
+    if (direct) {
+        launch_check_finite(b->n, (const float4 *)pos4, (const float4 *)vel4, b->flag, s, b->pos[0], b->vel[0]);
+    } else {
+        FB_CUDA(b, cudaMemcpyAsync(b->pos[0], pos4, bytes, k, s));
+        if (vel4) FB_CUDA(b, cudaMemcpyAsync(b->vel[0], vel4, bytes, k, s));
+        launch_check_finite(b->n, b->pos[0], vel4 ? b->vel[0] : nullptr, b->flag, s);
+    }
+    if (!vel4) FB_CUDA(b, cudaMemsetAsync(b->vel[0], 0, bytes, s));
     FB_CUDA(b, cudaMemsetAsync(b->attr[0], 0, (size_t)b->n * 4, s));
     launch_iota(b->n, b->id[0], s);
-    unsigned int *flag = b->rank; /* scratch between steps */
-    FB_CUDA(b, cudaMemsetAsync(flag, 0, sizeof(unsigned int), s));
-    launch_check_finite(b->n, b->pos[0], b->vel[0], flag, s);
-    unsigned int hflag = 0;
-    FB_CUDA(b, cudaMemcpyAsync(&hflag, flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     FB_CUDA(b, cudaStreamSynchronize(s));
     FB_CUDA(b, cudaGetLastError());
-    if (hflag) return bfail(b, FSPH_NAN_DETECTED, "non-finite input position or velocity");
+    if (*b->flag) return bfail(b, FSPH_NAN_DETECTED, "non-finite input position or velocity");
     b->loaded = true;
     return FSPH_OK;
 }
@@ -871,12 +876,15 @@ int fsph_batch_get_array(fsph_batch *b, int type, void *dst, int where) {
     const int n = b->n;
     cudaMemcpyKind k = where == FSPH_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     if (type == FSPH_POSITION || type == FSPH_VELOCITY) {
-        launch_unsort4(n, b->id[0], type == FSPH_POSITION ? b->pos[0] : b->vel[0], b->tmp4, 1, s);
-        FB_CUDA(b, cudaMemcpyAsync(dst, b->tmp4, (size_t)n * 16, k, s));
+        const bool direct = where == FSPH_DEVICE && device_span(dst, (size_t)n * 16, 16);
+        launch_unsort4(n, b->id[0], type == FSPH_POSITION ? b->pos[0] : b->vel[0],
+                       direct ? (float4 *)dst : b->tmp4, 1, s);
+        if (!direct) FB_CUDA(b, cudaMemcpyAsync(dst, b->tmp4, (size_t)n * 16, k, s));
     } else if (type == FSPH_DENSITY) {
-        float *t = reinterpret_cast<float *>(b->key);
+        const bool direct = where == FSPH_DEVICE && device_span(dst, (size_t)n * 4, 4);
+        float *t = direct ? (float *)dst : reinterpret_cast<float *>(b->key);
         launch_unsort1(n, b->id[0], reinterpret_cast<const unsigned int *>(b->dens), reinterpret_cast<unsigned int *>(t), s);
-        FB_CUDA(b, cudaMemcpyAsync(dst, t, (size_t)n * 4, k, s));
+        if (!direct) FB_CUDA(b, cudaMemcpyAsync(dst, t, (size_t)n * 4, k, s));
     } else {
         return bfail(b, FSPH_INVALID_ARG, "batched arrays: POSITION, VELOCITY, DENSITY");
     }

@@ -184,6 +184,14 @@ void launch_iota(int n, unsigned int *dst, cudaStream_t s);
 void launch_unsort_rows(int n, const unsigned int *id, const float4 *src, float4 *dst, int k4, cudaStream_t s);
 void launch_pack_w(int n, float4 *dst, const float *w, cudaStream_t s);
 /* *flag |= 1 when any x/y/z of a (or b, if given) is not finite */
-void launch_check_finite(int n, const float4 *a, const float4 *b, unsigned int *flag, cudaStream_t s);
+/* *bad = 1 (pinned host memory) when a component of a or b (optional) is not
+ * finite; dst_a / dst_b (optional) receive copies */
+void launch_check_finite(int n, const float4 *a, const float4 *b, unsigned int *bad, cudaStream_t s,
+                         float4 *dst_a = nullptr, float4 *dst_b = nullptr);
+/* [p, p + bytes) lies in one allocation of the current device and p is aligned
+ * to `align`: a kernel may then read or write the caller's memory itself.
+ * Anything else (host or managed memory, another device, a range that leaves
+ * its allocation) takes a copy call, which reports what is wrong with it. */
+bool device_span(const void *p, size_t bytes, size_t align);
 
 }  // namespace fsph
