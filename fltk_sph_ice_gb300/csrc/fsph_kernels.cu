@@ -811,21 +811,50 @@ __device__ inline bool ref_neighbor(float3 xi, float3 xj, float h2) {
     return __double2float_rn(dd) <= h2;
 }
 
-__global__ void k_nb_count(DevParams p, const unsigned int *__restrict__ cell_start, const float4 *__restrict__ pos,
-                           unsigned int *__restrict__ cnt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    float3 xi = f3(pos[i]);
-    int3 c = cell_of(xi, p);
+/* Neighbour counts of a warp's 32 consecutive slots, in particle order
+ * (cnt_p[id]), and the neighbours themselves in the list storage (up to
+ * kListMax a slot; cnt = kListOverflow past that) for k_nb_rows: the search,
+ * from the warp's tile (tile_masks, a hair wider than the radius), is done
+ * once.  total: the sum over all slots. */
+__global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsigned int *__restrict__ cell_start,
+                                                         const float4 *__restrict__ pos,
+                                                         const unsigned int *__restrict__ id,
+                                                         unsigned int *__restrict__ cnt_p,
+                                                         unsigned long long *__restrict__ total,
+                                                         ListEntry *__restrict__ list,
+                                                         unsigned char *__restrict__ cnt) {
+    __shared__ PairTile s_tile[kListBlock / 32];
+    PairTile &t = s_tile[threadIdx.x >> 5];
+    const int i = blockIdx.x * kListBlock + threadIdx.x;
+    const bool valid = i < p.n;
+    const float3 xi = valid ? f3(__ldg(pos + i)) : make_float3(0.f, 0.f, 0.f);
+    const int3 c = cell_of(xi, p);
+    const int words = tile_masks(p, cell_start, pos, xi, cell_index(c, p), valid, p.h2 * (1.0f + 1e-4f), t);
     unsigned int k = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy) {
-            unsigned int s, e;
-            row_range(cell_start, c, dy, dz, p, s, e);
-            for (unsigned int j = s; j < e; ++j)
-                if (ref_neighbor(xi, f3(pos[j]), p.h2)) ++k;
+    if (valid) {
+        auto meet = [&](unsigned int j) {
+            if (ref_neighbor(xi, f3(__ldg(pos + j)), p.h2)) {
+                if (k < (unsigned int)kListMax) list[list_at((int)k, i, p.n)] = j;
+                ++k;
+            }
+        };
+        if (words < 0) {
+            for (int dz = -1; dz <= 1; ++dz)
+                for (int dy = -1; dy <= 1; ++dy) {
+                    unsigned int s, e;
+                    row_range(cell_start, c, dy, dz, p, s, e);
+                    for (unsigned int j = s; j < e; ++j) meet(j);
+                }
+        } else {
+            TileWalk walk(t, words);
+            for (unsigned int j; walk.next(j);) meet(j);
         }
-    cnt[i] = k;
+        cnt_p[id[i]] = k;
+        cnt[i] = k > (unsigned int)kListMax ? kListOverflow : (unsigned char)k;
+    }
+    unsigned long long sum = k;
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total, sum);
 }
 
 /* squared distance as the reference's rxNeigh::Dist2: the difference of the
@@ -836,26 +865,82 @@ __device__ inline float ref_dist2(float3 xi, float3 xj) {
     return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez)));
 }
 
-__global__ void k_nb_fill(DevParams p, const unsigned int *__restrict__ cell_start, const float4 *__restrict__ pos,
-                          const unsigned int *__restrict__ id, const unsigned int *__restrict__ offsets,
-                          int *__restrict__ out, float *__restrict__ d2out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+/* Rows of the neighbour sets, one warp per slot: the particle indices of its
+ * neighbours in ascending order at out[offsets[particle] ...] (and each pair's
+ * squared distance).  A row of up to kListMax entries is in the list storage:
+ * each lane holds one or two and counts the smaller ones.  Longer rows are
+ * found again by walking the cells and sorted in place by one lane. */
+__global__ void __launch_bounds__(kBlock) k_nb_rows(DevParams p, const unsigned int *__restrict__ cell_start,
+                                                    const float4 *__restrict__ pos,
+                                                    const unsigned int *__restrict__ id,
+                                                    const unsigned int *__restrict__ offsets,
+                                                    const ListEntry *__restrict__ list,
+                                                    const unsigned char *__restrict__ cnt, int *__restrict__ out,
+                                                    float *__restrict__ d2out) {
+    const int lane = threadIdx.x & 31;
+    const int i = (int)(((long long)blockIdx.x * kBlock + threadIdx.x) >> 5);
     if (i >= p.n) return;
-    float3 xi = f3(pos[i]);
-    int3 c = cell_of(xi, p);
-    unsigned int k = offsets[i];
+    const int k = (int)cnt[i];
+    const size_t at = offsets[id[i]];
+    const float3 xi = f3(__ldg(pos + i));
+    if (k != (int)kListOverflow) {
+        unsigned int j[2] = {0u, 0u};
+        int v[2] = {0, 0}, r[2] = {0, 0};
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (lane + 32 * u < k) {
+                j[u] = __ldg(list + list_at(lane + 32 * u, i, p.n));
+                v[u] = (int)__ldg(id + j[u]);
+            }
+        for (int t = 0; t < k; ++t) {
+            const int w = __shfl_sync(0xffffffffu, t < 32 ? v[0] : v[1], t & 31);
+            r[0] += w < v[0] ? 1 : 0;
+            r[1] += w < v[1] ? 1 : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (lane + 32 * u < k) {
+                out[at + r[u]] = v[u];
+                if (d2out) d2out[at + r[u]] = ref_dist2(xi, f3(__ldg(pos + j[u])));
+            }
+        return;
+    }
+    if (lane != 0) return;
+    const int3 c = cell_of(xi, p);
+    int m = 0; /* a heap of the entries met so far, the largest index first */
+    auto swap = [&](int a, int b) {
+        const int w = out[at + a];
+        out[at + a] = out[at + b];
+        out[at + b] = w;
+        if (d2out) {
+            const float f = d2out[at + a];
+            d2out[at + a] = d2out[at + b];
+            d2out[at + b] = f;
+        }
+    };
     for (int dz = -1; dz <= 1; ++dz)
         for (int dy = -1; dy <= 1; ++dy) {
             unsigned int s, e;
             row_range(cell_start, c, dy, dz, p, s, e);
             for (unsigned int j = s; j < e; ++j) {
-                const float3 xj = f3(pos[j]);
-                if (ref_neighbor(xi, xj, p.h2)) {
-                    if (d2out) d2out[k] = ref_dist2(xi, xj);
-                    out[k++] = (int)id[j];
-                }
+                const float3 xj = f3(__ldg(pos + j));
+                if (!ref_neighbor(xi, xj, p.h2)) continue;
+                out[at + m] = (int)__ldg(id + j);
+                if (d2out) d2out[at + m] = ref_dist2(xi, xj);
+                for (int q = m++; q > 0 && out[at + (q - 1) / 2] < out[at + q]; q = (q - 1) / 2) swap(q, (q - 1) / 2);
             }
         }
+    for (int end = m - 1; end > 0; --end) {
+        swap(0, end);
+        for (int q = 0;;) {
+            int l = 2 * q + 1;
+            if (l >= end) break;
+            if (l + 1 < end && out[at + l + 1] > out[at + l]) ++l;
+            if (out[at + q] >= out[at + l]) break;
+            swap(q, l);
+            q = l;
+        }
+    }
 }
 
 /* ======================================================================== */
@@ -1215,13 +1300,15 @@ void launch_sph_integrate(const DevParams &p, const float4 *pos_b, const float4 
     k_sph_integrate<<<blocks_for(p.n), kBlock, 0, s>>>(p, pos_b, vel_b, acc, id_b, attr_b, pos_a, vel_a, id_a,
                                                        attr_a);
 }
-void launch_nb_count(const DevParams &p, const unsigned int *cell_start, const float4 *pos, unsigned int *cnt,
-                     cudaStream_t s) {
-    k_nb_count<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, cnt);
+void launch_nb_count(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const unsigned int *id,
+                     unsigned int *cnt_p, unsigned long long *total, const NbrLists &nl, cudaStream_t s) {
+    k_nb_count<<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, pos, id, cnt_p, total, nl.list,
+                                                                  nl.cnt);
 }
-void launch_nb_fill(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const unsigned int *id,
-                    const unsigned int *offsets, int *out, float *d2out, cudaStream_t s) {
-    k_nb_fill<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, id, offsets, out, d2out);
+void launch_nb_rows(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const unsigned int *id,
+                    const unsigned int *offsets, const NbrLists &nl, int *out, float *d2out, cudaStream_t s) {
+    k_nb_rows<<<blocks_for((long long)p.n * 32), kBlock, 0, s>>>(p, cell_start, pos, id, offsets, nl.list, nl.cnt, out,
+                                                                 d2out);
 }
 void launch_delete_regions(int n, float4 *pos, float4 *vel, unsigned int *attr, const float4 *reg, int nreg,
                            cudaStream_t s) {

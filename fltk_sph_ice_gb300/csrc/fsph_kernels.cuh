@@ -136,12 +136,10 @@ void launch_sph_integrate(const DevParams &p, const float4 *pos_b, const float4 
                           unsigned int *id_a, unsigned int *attr_a, cudaStream_t s);
 
 /* ---- neighbour sets under the reference criterion ---- */
-void launch_nb_count(const DevParams &p, const unsigned int *cell_start, const float4 *pos, unsigned int *cnt,
-                     cudaStream_t s);
-/* CSR rows from offsets: neighbour slots mapped through id, and (d2out,
- * when given) each pair's squared distance as the reference's Dist2 */
-void launch_nb_fill(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const unsigned int *id,
-                    const unsigned int *offsets, int *out, float *d2out, cudaStream_t s);
+void launch_nb_count(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const unsigned int *id,
+                     unsigned int *cnt_p, unsigned long long *total, const NbrLists &nl, cudaStream_t s);
+void launch_nb_rows(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const unsigned int *id,
+                    const unsigned int *offsets, const NbrLists &nl, int *out, float *d2out, cudaStream_t s);
 
 /* ---- deletion regions and the active / parked partition ---- */
 /* reg: nreg pairs (lo, hi) of float4 */

@@ -68,3 +68,26 @@ def test_batched_lists_do_not_depend_on_the_tiles(gpu):
         got.append(b.get(abi.RX_POSITION))
         b.close()
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("kind", ["sparse", "thin", "clumped", "dense"])
+@pytest.mark.parametrize("n", [1, 33, 900])
+def test_neighbour_rows_against_brute_force(gpu, kind, n):
+    """Rows of no, one, up to 64 (one or two a lane) and more neighbours (the
+    clumps), of the context's particles and of given positions, whole numbers
+    and squared distances equal to the reference criterion's."""
+    p, x = _scene(kind, n, 7 * n)
+    ps = rxPBDSPH(p)
+    ps.Set(x)
+    ps.Update(0.0016) if kind == "sparse" else None  # a slot order that is not the particles'
+    for prts, h in ((None, -1.0), (x[::-1].copy(), 0.8 * H)):
+        off, idx, d2 = ps.SetParticlesToCell(prts, h)
+        q = (ps.GetArrayVBO(abi.RX_POSITION) if prts is None else prts)[:, :3].astype(np.float64)
+        r = np.float32(p.h if h < 0 else h)
+        e = (q[:, None] - q[None]) ** 2
+        want = (e[..., 0] + e[..., 1] + e[..., 2]).astype(np.float32)
+        near = want <= np.float32(r * r)
+        assert np.array_equal(np.diff(off), near.sum(1))
+        assert np.array_equal(idx, np.nonzero(near)[1])
+        assert np.array_equal(d2, want[near])
+    ps.close()
