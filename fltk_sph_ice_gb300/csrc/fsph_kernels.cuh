@@ -90,6 +90,9 @@ void launch_pbf_visc(const DevParams &p, const unsigned int *cell_start, const f
 void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1, float *dens,
                    DevCtl *ctl, ErrPartial *part, unsigned long long while_handle, int use_graph,
                    const NbrLists &nl, cudaStream_t s);
+/* density and lambda of x (slot order) at order[slot], walking the cells */
+void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,
+                        float *dens, float *lambda, cudaStream_t s);
 void launch_correction(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                        const float4 *xb, DevCtl *ctl, float *part, unsigned long long if_handle,
                        unsigned long long if_handle2, int use_graph, float4 *dp_out, const NbrLists &nl,

@@ -6,8 +6,10 @@
  * the grid tables and sorted copies the pass needs.  Host code only ever
  * holds that array's device address, looked up with cudaGetSymbolAddress
  * once per device; the array's name in host code is a host-side stand-in,
- * not a device address, and is never passed to a kernel.  The kernels are
- * the ones the context-based path launches, so the results are the same.
+ * not a device address, and is never passed to a kernel.  The grid kernels
+ * are the ones the context-based path launches and the pair terms are its
+ * own (lambda_terms), summed by several lanes a particle, so the results are
+ * the same to rounding.
  */
 #include <cuda_runtime.h>
 
@@ -38,17 +40,13 @@ constexpr size_t kOffKey = align256(kOffBsum + ((kMaxC + kScanTile - 1) / kScanT
 constexpr size_t kOffRank = align256(kOffKey + kMaxP * 4);
 constexpr size_t kOffPerm = align256(kOffRank + kMaxP * 4);
 constexpr size_t kOffX = align256(kOffPerm + kMaxP * 4);                    /* float4[kMaxP] */
-constexpr size_t kOffDens = align256(kOffX + kMaxP * 16);
-constexpr size_t kOffCtl = align256(kOffDens + kMaxP * 4);
-constexpr size_t kOffPart = align256(kOffCtl + sizeof(DevCtl));
-/* two ErrPartial slots per block: room for the fixed-point partials (ErrPartialFix) */
-constexpr size_t kScratchBytes = align256(kOffPart + 2 * ((kMaxP + kPassBlock - 1) / kPassBlock) * sizeof(ErrPartial));
+constexpr size_t kScratchBytes = align256(kOffX + kMaxP * 16);
 
 constexpr int kMaxDevices = 64;
 
 }  // namespace
 
-/* The fixed working memory (about 10.3 MB per device). */
+/* The fixed working memory (about 10.2 MB per device). */
 static __device__ __align__(256) unsigned char g_fsph_noalloc_scratch[kScratchBytes];
 
 namespace {
@@ -104,15 +102,11 @@ extern "C" int fsph_pbf_eval_lambda_noalloc(const fsph_params *params, const flo
     unsigned int *rank = reinterpret_cast<unsigned int *>(base + kOffRank);
     unsigned int *perm = reinterpret_cast<unsigned int *>(base + kOffPerm);
     float4 *x = reinterpret_cast<float4 *>(base + kOffX);
-    float *d_sorted = reinterpret_cast<float *>(base + kOffDens);
-    DevCtl *ctl = reinterpret_cast<DevCtl *>(base + kOffCtl);
-    ErrPartial *part = reinterpret_cast<ErrPartial *>(base + kOffPart);
 
     const DevParams p = dev_params_for(P, n, 1.0f);
     const unsigned int nc = (unsigned int)cells;
     /* the array keeps the previous call's contents: clear what must start at zero */
     if (cudaMemsetAsync(count, 0, (size_t)nc * sizeof(unsigned int), s) != cudaSuccess) return FSPH_CUDA_ERROR;
-    if (cudaMemsetAsync(ctl, 0, sizeof(DevCtl), s) != cudaSuccess) return FSPH_CUDA_ERROR;
     launch_hash(p, reinterpret_cast<const float4 *>(pos4), key, rank, count, s);
     launch_scan(count, cell_start, bsum, nc, s);
     CellOrder o = launch_scatter(p, key, rank, cell_start, perm, s);
@@ -123,9 +117,7 @@ extern "C" int fsph_pbf_eval_lambda_noalloc(const fsph_params *params, const flo
     g.src4[0] = reinterpret_cast<const float4 *>(pos4);
     g.dst4[0] = x;
     launch_gather(n, o, g, nullptr, s);
-    launch_lambda(p, cell_start, x, x, d_sorted, ctl, part, 0ull, 0, NbrLists{}, s);
-    launch_unsort1(n, o.sorted, reinterpret_cast<const unsigned int *>(d_sorted), reinterpret_cast<unsigned int *>(dens), s);
-    launch_unsort_w(n, o.sorted, x, lambda, s);
+    launch_lambda_walk(p, cell_start, x, o.sorted, dens, lambda, s);
     if (cudaGetLastError() != cudaSuccess) return FSPH_CUDA_ERROR;
     return FSPH_OK;
 }

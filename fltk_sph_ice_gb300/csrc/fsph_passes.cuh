@@ -445,15 +445,13 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
 
 /* ---------------- constraint iterations ---------------- */
 
-/* lambda pass of one particle: density, C, sum |grad C|^2 (with the k = i
- * term), lambda into x*.w and rho into dens (lane 0 of a valid group).
- * Returns C (the caller turns it into the error terms). */
-template <int LPP, bool KAHAN = false>
-__device__ __forceinline__ float lambda_body(const DevParams &p, const unsigned int *__restrict__ cell_start,
-                                             float4 *pp, float *__restrict__ dens, DevCtl *ctl,
-                                             const ListEntry *__restrict__ list,
-                                             const unsigned char *__restrict__ cnt, int i, int sub,
-                                             bool valid) {
+/* Density, C, sum |grad C|^2 (with the k = i term) and lambda of one particle;
+ * returns C (every lane of a group gets the same values). */
+template <int LPP, bool KAHAN>
+__device__ __forceinline__ float lambda_terms(const DevParams &p, const unsigned int *__restrict__ cell_start,
+                                              const float4 *pp, const ListEntry *__restrict__ list,
+                                              const unsigned char *__restrict__ cnt, int i, int sub, float &rho_out,
+                                              float &lam_out) {
     const float3 xi = f3(pp[i]);
     float wsum = 0.f, wc = 0.f, sd = 0.f;
     float3 gs = make_float3(0.f, 0.f, 0.f);
@@ -521,7 +519,20 @@ __device__ __forceinline__ float lambda_body(const DevParams &p, const unsigned 
     }
     float C = rho * p.inv_rest_dens - 1.0f;
     float Cc = (p.clamp_constraint && C < 0.0f) ? 0.0f : C;
-    float lam = -Cc / (sd + p.epsilon);
+    rho_out = rho;
+    lam_out = -Cc / (sd + p.epsilon);
+    return C;
+}
+
+/* lambda pass of one particle: lambda into x*.w and rho into dens (lane 0 of a
+ * valid group).  Returns C (the caller turns it into the error terms). */
+template <int LPP, bool KAHAN = false>
+__device__ __forceinline__ float lambda_body(const DevParams &p, const unsigned int *__restrict__ cell_start,
+                                             float4 *pp, float *__restrict__ dens, DevCtl *ctl,
+                                             const ListEntry *__restrict__ list,
+                                             const unsigned char *__restrict__ cnt, int i, int sub, bool valid) {
+    float rho, lam;
+    const float C = lambda_terms<LPP, KAHAN>(p, cell_start, pp, list, cnt, i, sub, rho, lam);
     if (valid && sub == 0) {
         reinterpret_cast<float *>(pp + i)[3] = lam;
         dens[i] = rho;

@@ -342,7 +342,7 @@ int fsph_sph_eval_forces(fsph_ctx *ctx, const float *pos4, const float *vel4, in
 
 /* ---- allocation-free variant ---- */
 /* Largest inputs of fsph_pbf_eval_lambda_noalloc: its scratch is a fixed
- * device array of about 10.3 MB inside the library. */
+ * device array of about 10.2 MB inside the library. */
 #define FSPH_NOALLOC_MAX_PARTICLES 65536
 #define FSPH_NOALLOC_MAX_CELLS (1 << 20)
 /* The lambda pass of fsph_pbf_eval_lambda (density and scaling factor of n

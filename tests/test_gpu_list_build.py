@@ -4,6 +4,8 @@ tanks), clumps whose candidates overflow a list or a warp's tile.  A pass over
 the lists and a walk over the 27 cells meet the same neighbours in the same
 ascending order, and what else either meets adds exact zeros, so a step with
 lists equals the same step walking the cells bit for bit."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -91,3 +93,43 @@ def test_neighbour_rows_against_brute_force(gpu, kind, n):
         assert np.array_equal(idx, np.nonzero(near)[1])
         assert np.array_equal(d2, want[near])
     ps.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 700, 8000, 20000, 40000, 65536])
+def test_allocation_free_lambda_at_every_lane_count(gpu, n):
+    """The allocation-free pass takes 32 to 4 lanes a particle by size; density
+    and lambda against 64 bits.  The bars: a sum of about 30 terms of one sign,
+    each rounded a few times (1e-6 of the density); lambda has that error
+    divided by |C| >= 0.1 here and the error of its denominator (2e-5)."""
+    import torch
+    rng = np.random.default_rng(n)
+    s = 0.5 * H * 0.9  # compressed: C is far from zero
+    m = int(np.ceil(n ** (1 / 3)))
+    x = np.zeros((n, 4), np.float32)
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    x[:, :3] = 0.3 * H + g * s + rng.uniform(-0.05, 0.05, (n, 3)) * s
+    p = scenes.pbf_params(H, [0.0] * 3, [m * s + 0.6 * H] * 3, n)
+    t = torch.from_numpy(x).cuda()
+    d, lam = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+    ptr = lambda a: ctypes.c_void_p(a.data_ptr())  # noqa: E731
+    L = abi.lib()
+    L.fsph_pbf_eval_lambda_noalloc.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_int] + [ctypes.c_void_p] * 3
+    torch.cuda.synchronize()
+    assert L.fsph_pbf_eval_lambda_noalloc(ctypes.byref(p), ptr(t), n, ptr(d), ptr(lam), None) == abi.OK
+    torch.cuda.synchronize()
+    at = rng.choice(n, min(n, 300), replace=False)  # rows checked against every particle
+    h = float(np.float32(p.h))
+    q = t[:, :3].double()
+    dv = q[torch.from_numpy(at).cuda()][:, None] - q[None]
+    r = dv.square().sum(-1).sqrt()
+    rho = float(p.mass) * 315 / (64 * np.pi * h ** 9) * (h * h - r * r).clamp(min=0).pow(3).sum(1)
+    gr = torch.where(r > 0, 45 / (np.pi * h ** 6) * (h - r).clamp(min=0).square() / r.clamp(min=1e-12),
+                     torch.zeros_like(r)) / p.rest_dens
+    gd = gr[..., None] * dv
+    sd = gd.square().sum((1, 2)) + gd.sum(1).square().sum(1)
+    want = -(rho / p.rest_dens - 1) / (sd + p.epsilon)
+    at = torch.from_numpy(at).cuda()
+    assert ((d[at] - rho).abs() <= 1e-6 * rho).all()
+    keep = (rho / p.rest_dens - 1).abs() >= 0.1
+    assert keep.any() or n < 700
+    assert ((lam[at] - want).abs() <= 2e-5 * want.abs())[keep].all()
