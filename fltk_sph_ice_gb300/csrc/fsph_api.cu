@@ -1756,7 +1756,12 @@ int fsph_density_grid(fsph_ctx *c, const int *nn, const double *minp, const doub
         hi[a] = lo[a] + size * (1.0 + 0.01);
     }
     DevParams p = dev_for(c, c->n_active, 1.0f); /* the deleted particles are parked far away */
-    FSPH_TRY(build_on(c, p, c->set[0].pos));
+    /* the positions in cell order are all that the nodes read: no lists */
+    const CellOrder o = enqueue_sort(c, p, c->set[0].pos, s);
+    Gather g{};
+    g.n4 = 1;
+    g.src4[0] = c->set[0].pos; g.dst4[0] = c->set[1].pos;
+    launch_gather(p.n, o, g, nullptr, s);
     if (!dout) FSPH_CUDA(c, cudaMallocAsync((void **)&dout, (size_t)tot * sizeof(float), s));
     launch_density_grid(p, c->cell_start, c->set[1].pos, nn, minp, d, lo, hi, dout, s);
     cudaError_t e = cudaGetLastError();

@@ -22,6 +22,7 @@
  *   k_sph_*            rxSPH::calDensity / calForce / integrate (rx_sph_cpu.cpp:495-1077)
  */
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "fsph_kernels.cuh"
@@ -1018,51 +1019,134 @@ __global__ void k_gather_rows(int n, const unsigned int *__restrict__ perm, cons
 /* density on a lattice (for meshing)                                       */
 /* ======================================================================== */
 
+/* Sums and products of two floats without their rounding errors: the result
+ * and its error (Knuth; Dekker; the product's error from one fused operation),
+ * with no contraction by the compiler. */
+struct Split {
+    float h, l; /* the value is h + l */
+};
+__device__ __forceinline__ Split two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    return Split{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
+__device__ __forceinline__ Split two_diff(float a, float b) { return two_sum(a, -b); }
+__device__ __forceinline__ Split two_prod(float a, float b) {
+    const float q = __fmul_rn(a, b);
+    return Split{q, __fmaf_rn(a, b, -q)};
+}
+/* h + l with the error of the sum kept (|h| >= |l| or h = 0) */
+__device__ __forceinline__ Split renorm(float h, float l) {
+    const float s = __fadd_rn(h, l);
+    return Split{s, __fsub_rn(l, __fsub_rn(s, h))};
+}
+__device__ __forceinline__ Split split_of(double v) {
+    const float h = (float)v;
+    return Split{h, (float)(v - (double)h)};
+}
+
 /* The density field at the nodes of an nx x ny x nz lattice (i fastest),
  * node (i, j, k) at minp + (i, j, k) d: 0 outside [lo, hi], else
- * sum_j m W(r_j) over the particles with fl32(|x - x_j|^2 in double) <=
- * fl32(h h), r_j = fl32(sqrt(Dist2)), W in double and the sum in float, as
- * rxPBDSPH::CalColorField (rx_sph_pbd.cpp:2075-2108, the CPU form of
- * pbdsphCalDensityInGrid, rx_pbdsph_kernel.cu:1220-1299).  A float
- * distance test in a 1e-4 band around h^2 skips the double evaluation for
- * the candidates far outside. */
-__global__ void __launch_bounds__(kBlock) k_density_grid(DevParams p, const unsigned int *__restrict__ cell_start,
-                                                         const float4 *__restrict__ pos, int nx, int ny, int nz,
-                                                         double3 minp, double3 dd, double3 lo, double3 hi,
-                                                         float *__restrict__ out) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)nx * ny * nz) return;
-    const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / ((long long)nx * ny));
+ * sum_j m W(r_j) over the particles with fl32(|x - x_j|^2) <= fl32(h h),
+ * r_j = fl32(sqrt(Dist2)), the terms W in more than single precision and the
+ * sum in float, as rxPBDSPH::CalColorField (rx_sph_pbd.cpp:2075-2108, the CPU
+ * form of pbdsphCalDensityInGrid, rx_pbdsph_kernel.cu:1220-1299).
+ *
+ * The reference's terms are doubles.  This GPU runs 2 FP64 lanes a clock and
+ * SM, and a warp whose nodes meet their neighbours at different steps of the
+ * walk ran the 22 FP64 instructions of a term at nearly every one of its 290
+ * steps: 1,492 us for 0.31 M nodes.  The whole call went from 1,662 to 255 us,
+ * and to 185 without building neighbour lists that the nodes never read.  Here
+ *  - a thread first collects its candidates by the single-precision test (a
+ *    1e-4 band around h^2), then evaluates them together with the others of
+ *    its warp (about 35 terms, all lanes busy); a warp is a brick of nodes, so
+ *    its lanes walk the same cells;
+ *  - the terms are sums and products of split floats (48 bits: relative errors
+ *    of 1e-14 where the sum that takes them is rounded to 6e-8), about 105
+ *    single-precision instructions;
+ *  - lengths are scaled by a power of two (len.sc, exact) so that h lies in
+ *    [1, 2): no step leaves the range of floats for any h. */
+struct LatticeLen {
+    float sc;        /* the power of two */
+    float h2;        /* fl32(h h) sc^2 */
+    Split hh;        /* h^2 sc^2 */
+    Split c;         /* m aw / sc^6 */
+};
+constexpr int kLatBlock = 128, kLatMax = 48; /* threads a block; candidates collected before they are evaluated */
+__global__ void __launch_bounds__(kLatBlock) k_density_grid(DevParams p, const unsigned int *__restrict__ cell_start,
+                                                            const float4 *__restrict__ pos, int nx, int ny, int nz,
+                                                            int3 lb, LatticeLen len, double3 minp, double3 dd,
+                                                            double3 lo, double3 hi, float *__restrict__ out) {
+    __shared__ unsigned int s_j[kLatMax][kLatBlock];
+    /* a warp's brick of 2^lb.x x 2^lb.y x 2^lb.z nodes */
+    const int lane = threadIdx.x & 31;
+    const int bx = (nx + (1 << lb.x) - 1) >> lb.x, by = (ny + (1 << lb.y) - 1) >> lb.y;
+    const long long brick = (long long)blockIdx.x * (kLatBlock / 32) + (threadIdx.x >> 5);
+    const long long i = ((brick % bx) << lb.x) + (lane & ((1 << lb.x) - 1));
+    const long long j = (((brick / bx) % by) << lb.y) + ((lane >> lb.x) & ((1 << lb.y) - 1));
+    const long long k = ((brick / ((long long)bx * by)) << lb.z) + (lane >> (lb.x + lb.y));
+    if (i >= nx || j >= ny || k >= nz) return;
     /* minp + Vec3(i, j, k) * d, each product and sum rounded in double */
     const double X = __dadd_rn(minp.x, __dmul_rn((double)i, dd.x));
     const double Y = __dadd_rn(minp.y, __dmul_rn((double)j, dd.y));
     const double Z = __dadd_rn(minp.z, __dmul_rn((double)k, dd.z));
     float acc = 0.0f;
     if (X >= lo.x && X <= hi.x && Y >= lo.y && Y <= hi.y && Z >= lo.z && Z <= hi.z) {
-        const float3 xf = make_float3((float)X, (float)Y, (float)Z);
+        const Split sx = split_of(X), sy = split_of(Y), sz = split_of(Z);
+        const float3 xf = make_float3(sx.h, sy.h, sz.h);
         const int3 c = cell_of(xf, p);
         const float band = p.h2 * (1.0f + 1e-4f);
-        const double hd = (double)p.h, aw = (double)p.aw_d, m = (double)p.mass;
+        int m = 0;
+        auto square = [&](Split a, float x) { /* ((a - x) sc)^2 */
+            const Split e = two_diff(a.h, x);
+            const Split t = renorm(e.h, __fadd_rn(e.l, a.l));
+            const float h = __fmul_rn(t.h, len.sc), l = __fmul_rn(t.l, len.sc);
+            Split q = two_prod(h, h);
+            q.l = __fmaf_rn(__fadd_rn(h, h), l, q.l);
+            return q;
+        };
+        auto evaluate = [&]() {
+            for (int t = 0; t < m; ++t) {
+                const float4 xq = __ldg(pos + s_j[t][threadIdx.x]);
+                const Split a = square(sx, xq.x), b = square(sy, xq.y), d = square(sz, xq.z);
+                const Split ab = two_sum(a.h, b.h), abd = two_sum(ab.h, d.h);
+                const float d2 = __fadd_rn(
+                    abd.h, __fadd_rn(__fadd_rn(__fadd_rn(a.l, b.l), d.l), __fadd_rn(ab.l, abd.l)));
+                if (!(d2 <= len.h2)) continue;
+                const float r = __fsqrt_rn(d2);
+                const Split rr = two_prod(r, r);
+                const Split dq = two_diff(len.hh.h, rr.h);
+                const Split q = renorm(dq.h, __fsub_rn(__fadd_rn(dq.l, len.hh.l), rr.l)); /* h^2 - r^2 */
+                Split q2 = two_prod(q.h, q.h);
+                q2.l = __fmaf_rn(__fadd_rn(q.h, q.h), q.l, q2.l);
+                Split q3 = two_prod(q2.h, q.h);
+                q3.l = __fmaf_rn(q2.l, q.h, __fmaf_rn(q2.h, q.l, q3.l));
+                Split w = two_prod(len.c.h, q3.h);
+                w.l = __fmaf_rn(len.c.l, q3.h, __fmaf_rn(len.c.h, q3.l, w.l));
+                const Split sum = two_sum(acc, w.h);
+                acc = __fadd_rn(sum.h, __fadd_rn(sum.l, w.l));
+            }
+            m = 0;
+        };
         for (int dz = -1; dz <= 1; ++dz)
             for (int dy = -1; dy <= 1; ++dy) {
                 unsigned int s, e;
                 row_range(cell_start, c, dy, dz, p, s, e);
-                for (unsigned int q = s; q < e; ++q) {
-                    const float4 xq = __ldg(pos + q);
-                    const float3 df = xf - f3(xq);
-                    if (dot3(df, df) > band) continue;
-                    const double ex = X - (double)xq.x, ey = Y - (double)xq.y, ez = Z - (double)xq.z;
-                    const float d2 =
-                        __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez)));
-                    if (d2 <= p.h2) {
-                        const double r = (double)sqrtf(d2);
-                        const double qq = __dsub_rn(__dmul_rn(hd, hd), __dmul_rn(r, r));
-                        acc = __double2float_rn(__dadd_rn((double)acc, __dmul_rn(m, __dmul_rn(__dmul_rn(__dmul_rn(aw, qq), qq), qq))));
+                for (unsigned int q0 = s; q0 < e; q0 += 4) { /* four loads in flight */
+                    float4 xq[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) xq[u] = __ldg(pos + min(q0 + u, e - 1));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float3 df = xf - f3(xq[u]);
+                        if (q0 + u >= e || dot3(df, df) > band) continue;
+                        if (m == kLatMax) evaluate();
+                        s_j[m++][threadIdx.x] = q0 + u;
                     }
                 }
             }
+        evaluate();
     }
-    out[t] = acc;
+    out[(k * ny + j) * nx + i] = acc;
 }
 
 /* ======================================================================== */
@@ -1355,11 +1439,34 @@ void launch_gather_rows(int n, const unsigned int *perm, const float4 *src, floa
 void launch_density_grid(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const int nn[3],
                          const double minp[3], const double d[3], const double lo[3], const double hi[3], float *out,
                          cudaStream_t s) {
-    const long long tot = (long long)nn[0] * nn[1] * nn[2];
-    k_density_grid<<<blocks_for(tot), kBlock, 0, s>>>(p, cell_start, pos, nn[0], nn[1], nn[2],
-                                                      make_double3(minp[0], minp[1], minp[2]),
-                                                      make_double3(d[0], d[1], d[2]), make_double3(lo[0], lo[1], lo[2]),
-                                                      make_double3(hi[0], hi[1], hi[2]), out);
+    /* bricks of 4 x 4 x 2 nodes; an axis with fewer nodes gives its share to the others */
+    int most[3], lb[3] = {2, 2, 1};
+    for (int a = 0; a < 3; ++a) {
+        most[a] = 0;
+        while (most[a] < 5 && (1ll << most[a]) < nn[a]) ++most[a];
+        lb[a] = std::min(lb[a], most[a]);
+    }
+    for (int a = 0; a < 3; ++a)
+        while (lb[0] + lb[1] + lb[2] < 5 && lb[a] < most[a]) ++lb[a];
+    lb[0] += 5 - (lb[0] + lb[1] + lb[2]); /* fewer than 32 nodes in all */
+    long long bricks = 1;
+    for (int a = 0; a < 3; ++a) bricks *= ((long long)nn[a] + (1 << lb[a]) - 1) >> lb[a];
+    auto split = [](double v) {
+        const float h = (float)v;
+        return Split{h, (float)(v - (double)h)};
+    };
+    int ex = 0;
+    std::frexp((double)p.h, &ex); /* h = f 2^ex, f in [1/2, 1) */
+    const double sc = std::ldexp(1.0, 1 - ex), hs = (double)p.h * sc;
+    LatticeLen len;
+    len.sc = (float)sc;
+    len.h2 = (float)((double)p.h2 * sc * sc);
+    len.hh = split(hs * hs);
+    len.c = split((double)p.mass * p.aw_d * std::ldexp(1.0, 6 * (ex - 1)));
+    k_density_grid<<<blocks_for(bricks, kLatBlock / 32), kLatBlock, 0, s>>>(
+        p, cell_start, pos, nn[0], nn[1], nn[2], make_int3(lb[0], lb[1], lb[2]), len,
+        make_double3(minp[0], minp[1], minp[2]), make_double3(d[0], d[1], d[2]), make_double3(lo[0], lo[1], lo[2]),
+        make_double3(hi[0], hi[1], hi[2]), out);
 }
 /* The reference's cell hash of each position (z Gy Gx + y Gx + x):
  * rule 0 = its CPU grid (rxNNGrid::CalGridHash(Vec3), rx_nnsearch.h:590-599:
