@@ -49,6 +49,12 @@ struct CellOrder {
 CellOrder launch_scatter(const DevParams &p, const unsigned int *key, const unsigned int *rank,
                          const unsigned int *cell_start, unsigned int *perm, cudaStream_t s);
 
+/* the whole build of a small cloud (hash, scan, order, x4 into x_out, order[slot]
+ * = particle) in one launch; false (nothing launched) when it is too large */
+constexpr int kSmallGrid = 8192;
+bool launch_small_grid(const DevParams &p, unsigned int ncells, const float4 *x4, float4 *x_out, unsigned int *order,
+                       unsigned int *cell_start, cudaStream_t s);
+
 /* dst[d] = src[previous slot of d] for up to 6 float4 and 4 u32 streams */
 struct Gather {
     const float4 *src4[6];

@@ -105,19 +105,22 @@ extern "C" int fsph_pbf_eval_lambda_noalloc(const fsph_params *params, const flo
 
     const DevParams p = dev_params_for(P, n, 1.0f);
     const unsigned int nc = (unsigned int)cells;
-    /* the array keeps the previous call's contents: clear what must start at zero */
-    if (cudaMemsetAsync(count, 0, (size_t)nc * sizeof(unsigned int), s) != cudaSuccess) return FSPH_CUDA_ERROR;
-    launch_hash(p, reinterpret_cast<const float4 *>(pos4), key, rank, count, s);
-    launch_scan(count, cell_start, bsum, nc, s);
-    CellOrder o = launch_scatter(p, key, rank, cell_start, perm, s);
-    o.sorted = rank; /* free once the scatter has run */
-    Gather g{};
-    g.n4 = 1;
-    g.n1 = 0;
-    g.src4[0] = reinterpret_cast<const float4 *>(pos4);
-    g.dst4[0] = x;
-    launch_gather(n, o, g, nullptr, s);
-    launch_lambda_walk(p, cell_start, x, o.sorted, dens, lambda, s);
+    const float4 *in = reinterpret_cast<const float4 *>(pos4);
+    if (!launch_small_grid(p, nc, in, x, rank, cell_start, s)) {
+        /* the array keeps the previous call's contents: clear what must start at zero */
+        if (cudaMemsetAsync(count, 0, (size_t)nc * sizeof(unsigned int), s) != cudaSuccess) return FSPH_CUDA_ERROR;
+        launch_hash(p, in, key, rank, count, s);
+        launch_scan(count, cell_start, bsum, nc, s);
+        CellOrder o = launch_scatter(p, key, rank, cell_start, perm, s);
+        o.sorted = rank; /* free once the scatter has run */
+        Gather g{};
+        g.n4 = 1;
+        g.n1 = 0;
+        g.src4[0] = in;
+        g.dst4[0] = x;
+        launch_gather(n, o, g, nullptr, s);
+    }
+    launch_lambda_walk(p, cell_start, x, rank, dens, lambda, s);
     if (cudaGetLastError() != cudaSuccess) return FSPH_CUDA_ERROR;
     return FSPH_OK;
 }

@@ -95,7 +95,7 @@ def test_neighbour_rows_against_brute_force(gpu, kind, n):
     ps.close()
 
 
-@pytest.mark.parametrize("n", [1, 31, 700, 8000, 20000, 40000, 65536])
+@pytest.mark.parametrize("n", [1, 31, 700, 1024, 1025, 8192, 8193, 20000, 40000, 65536])
 def test_allocation_free_lambda_at_every_lane_count(gpu, n):
     """The allocation-free pass takes 32 to 4 lanes a particle by size; density
     and lambda against 64 bits.  The bars: a sum of about 30 terms of one sign,
