@@ -906,7 +906,10 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
     const bool valid = i < p.n;
     const float3 xi = valid ? f3(__ldg(pos + i)) : make_float3(0.f, 0.f, 0.f);
     const int3 c = cell_of(xi, p);
-    const int words = tile_masks(p, cell_start, pos, xi, cell_index(c, p), valid, p.h2 * (1.0f + 1e-4f), t);
+    int found;
+    unsigned int some;
+    const bool ok = tile_masks(p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
+                               found, some);
     unsigned int k = 0;
     if (valid) {
         auto meet = [&](unsigned int j) {
@@ -915,7 +918,7 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
                 ++k;
             }
         };
-        if (words < 0) {
+        if (!ok) {
             for (int dz = -1; dz <= 1; ++dz)
                 for (int dy = -1; dy <= 1; ++dy) {
                     unsigned int s, e;
@@ -923,8 +926,8 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
                     for (unsigned int j = s; j < e; ++j) meet(j);
                 }
         } else {
-            TileWalk walk(t, words);
-            for (unsigned int j; walk.next(j);) meet(j);
+            TileWalk walk(t, some);
+            for (int f = 0; f < found; ++f) meet(walk.next());
         }
         cnt_p[id[i]] = k;
         cnt[i] = k > (unsigned int)kListMax ? kListOverflow : (unsigned char)k;

@@ -16,7 +16,7 @@ constexpr int kBlock = 256;
 #define FSPH_PASS_BLOCK 512
 #endif
 constexpr int kPassBlock = FSPH_PASS_BLOCK;
-constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 4.6 KB each */
+constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 9.2 KB each */
 constexpr int kBlockMax = 512;  /* largest block of the batched persistent kernels */
 constexpr int kScanTile = 4096; /* cells per block of the first scan phase */
 constexpr unsigned int kScanSum = 2048; /* tiles up to which the scan runs in two phases */

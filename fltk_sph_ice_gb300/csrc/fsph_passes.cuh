@@ -11,6 +11,8 @@
  * sums are combined with shuffles, and lane 0 of the group writes.
  */
 #pragma once
+#include <cuda_fp16.h>
+
 #include "fsph_kernels.cuh"
 
 namespace fsph {
@@ -259,12 +261,18 @@ __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const
         if (!cell_row_ok(p, base)) continue;
         const unsigned int s = __ldg(cell_start + base - 1);
         const unsigned int e = bounded(p, __ldg(cell_start + base + 2), (unsigned int)p.n + 1u, kBoundSlot);
-        for (unsigned int j = s; j < e; ++j) {
-            const float3 d = xi - f3(__ldg(xb + j));
-            if (dot3(d, d) < p.rl2) {
-                last = j;
-                if (k < kListMax) list[list_at(k, i, p.n)] = last;
-                ++k;
+        for (unsigned int j0 = s; j0 < e; j0 += 4) { /* four loads in flight */
+            float4 xc[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xc[u] = __ldg(xb + min(j0 + u, e - 1));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float3 d = xi - f3(xc[u]);
+                if (j0 + u < e && dot3(d, d) < p.rl2) {
+                    last = j0 + u;
+                    if (k < kListMax) list[list_at(k, i, p.n)] = last;
+                    ++k;
+                }
             }
         }
     }
@@ -274,137 +282,210 @@ __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const
     cnt[i] = overflow ? kListOverflow : (unsigned char)k;
 }
 
-/* The candidates of the 32 consecutive slots of a warp, searched together.
- * The slots lie in a run of three or four cells along x, so in each of the
- * nine rows of cells their candidates are one range of slots, about 1.7 times
- * what a lane's own three cells hold.  The warp stages 32 of them at a time in
- * shared memory and every lane tests all 32 from there: the loads are
- * broadcasts, four candidates an LDS.128 and axis, the differences and squares
- * are packed two to an instruction (add / fma.rn.f32x2), and the sign of
- * r^2 - rr^2 shifts into a mask, 19 instructions per four candidates.  A
- * thread that walks its own cells needs one gathered load, about 12
- * instructions and, since some lane hits at almost every candidate, the ten of
- * the store path for each: it was bound by issue (76 % active).  Measured:
- * 291 -> 266 us at 1,048,576 particles, whole steps 548 -> 533 us (262 k, 4
- * iterations) and 5,658 -> 5,527 us (batch of 256). */
+/* The candidates of the 32 consecutive slots of a warp, searched together on
+ * the tensor cores.  The slots lie in a run of three or four cells along x, so
+ * in each of the nine rows of cells their candidates are one range of slots,
+ * about 1.9 times what a lane's own three cells hold.  The warp takes 32 of
+ * them at a time and computes all 32 x 32 values r^2 / rr^2 - 1 as products of
+ * 16 terms (mma.m16n8k16): with coordinates relative to the warp, in units of
+ * the radius and split into two halves of 11 bits each, r^2 = |xi|^2 + |xj|^2 -
+ * 2 xi.xj needs the three products of the halves (their last, 2^-22, left out),
+ * the two norms (split too) and the constant.  The error of a value is below
+ * 1e-4 (coordinates of at most 5 in a run of six cells, sums of 16 terms below
+ * 50), and the constant is 1 + 2^-12: every slot within the radius is found,
+ * and one in some thousands that lies a hair beyond it, which a pass evaluates
+ * to zero.  The signs shift into masks, eight candidates of four slots a lane,
+ * which two shuffles turn into 32 candidates of one slot.
+ * About 95 instructions for 32 x 32 tests.  Tested two at a time in packed
+ * single precision they took 170 and the build 266 us at 1 M particles, a
+ * thread walking its own cells 291 us, both bound by instruction issue; this
+ * form takes 184 us, 18 instead of 33 us at 6,912 particles, and a batch step
+ * went from 5,397 to 5,117 us. */
 constexpr int kTileWords = 32; /* masks of a warp's candidates: 32 x 32 slots */
 struct __align__(16) PairTile {
-    float x[32], y[32], z[32];
-    unsigned int mask[kTileWords][32]; /* [w][lane], bit 31 - k: slot base[w] + k is within the radius */
-    unsigned int base[kTileWords];
+    uint4 k0[32], k1[32];               /* operand rows: the first and last eight of the 16 terms */
+    unsigned int mask[kTileWords][32];  /* [w][lane], bit 31 - k: candidate k of word w is within the radius */
+    unsigned int slot[kTileWords][32];  /* [w][k]: the candidates' slots */
 };
 
-__device__ __forceinline__ unsigned long long pack_f2(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
+__device__ __forceinline__ unsigned int half_pair(float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const unsigned int *>(&v);
 }
-__device__ __forceinline__ unsigned long long add_f2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
+__device__ __forceinline__ float half_round(float v) { return __half2float(__float2half_rn(v)); }
+__device__ __forceinline__ void load_matrices(unsigned int (&r)[4], const uint4 *row) {
+    const unsigned int at = (unsigned int)__cvta_generic_to_shared(row);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(at)
+                 : "memory");
 }
-__device__ __forceinline__ unsigned long long fma_f2(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
+/* m << 1 with the sign of v shifted in */
+__device__ __forceinline__ unsigned int sign_in(unsigned int m, float v) {
+    return __funnelshift_l(__float_as_uint(v), m, 1);
 }
-/* m << 1 with the sign bit of a half of v shifted in */
-__device__ __forceinline__ unsigned int sign_in(unsigned int m, unsigned long long v, int half) {
-    return __funnelshift_l((unsigned int)(v >> (32 * half)), m, 1);
+/* the four signs' masks of a 16 x 8 tile of tests: rows g and g + 8, columns
+ * 2c and 2c + 1 (lane = 4g + c) */
+__device__ __forceinline__ void test_tile(unsigned int &m0, unsigned int &m1, unsigned int a0, unsigned int a1,
+                                          unsigned int a2, unsigned int a3, unsigned int b0, unsigned int b1) {
+    float d0, d1, d2, d3;
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%10, %10, %10, %10};"
+        : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3)
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+    m0 = sign_in(sign_in(m0, d0), d1);
+    m1 = sign_in(sign_in(m1, d2), d3);
 }
 
 /* Fills t with the masks of the warp's slots (position xi, build cell `cell`,
  * cells ascending over the lanes; valid = false for padding lanes, after the
- * valid ones) against x4, within sqrt(r2max).  The words of one lane are in
- * ascending slot order.  Returns the number of words, or -1 when they do not
- * fit; every lane of the warp calls it and gets the same answer.  Lanes in
- * different rows of cells (a run that wraps, sparse fluid) take turns, row by
- * row: a row's range then never reaches the next row, and no slot is met twice. */
-__device__ __forceinline__ int tile_masks(const DevParams &p, const unsigned int *__restrict__ cell_start,
-                                          const float4 *__restrict__ x4, float3 xi, unsigned int cell, bool valid,
-                                          float r2max, PairTile &t) {
+ * valid ones) against x4, within sqrt(r2max).  The candidates of one lane are
+ * in ascending slot order.  count: how many this lane's slot has, some: bit
+ * 31 - w set when word w holds any.  Returns false, for every lane of the
+ * warp, when the candidates do not fit or a coordinate is out of the operands'
+ * range (a particle far outside the box, or not a number).  Lanes in different
+ * rows of cells, or more than six cells apart (a run that wraps, sparse fluid),
+ * take turns: a row's range then never reaches the next row, and no slot is met
+ * twice. */
+__device__ __forceinline__ bool tile_masks(const DevParams &p, const unsigned int *__restrict__ cell_start,
+                                           const float4 *__restrict__ x4, float3 xi, unsigned int cell, bool valid,
+                                           float r2max, PairTile &t, int &count, unsigned int &some) {
     const int lane = threadIdx.x & 31;
     const unsigned int row = (cell - p.cell_off) / (unsigned int)p.gx;
-    const unsigned long long nx = pack_f2(-xi.x, -xi.x), ny = pack_f2(-xi.y, -xi.y), nz = pack_f2(-xi.z, -xi.z);
-    const unsigned long long nr = pack_f2(-r2max, -r2max);
+    const float inv = rsqrtf(r2max);
+    /* operand B: candidate 8 q + 2 s + b is column 2 q + b of step s; the rows are
+     * stored so that neither the stores nor the loads of eight rows collide */
+    uint4 *const st0 = t.k0 + 8 * (lane >> 3) + 2 * ((lane >> 3) ^ ((lane >> 1) & 3)) + (lane & 1);
+    uint4 *const st1 = t.k1 + (st0 - t.k0);
+    const int lrow = 8 * ((lane & 7) >> 1) + 2 * (((lane & 7) >> 1) ^ (lane >> 3)) + (lane & 1);
+    const unsigned int pick1 = (lane & 2) ? 0x3726u : 0x5140u, pick2 = (lane & 1) ? 0x6273u : 0x0415u;
+    const int own = (lane >> 2) + 8 * (lane & 3); /* the slot whose 32 candidates this lane ends up with */
+    int cnt = 0;
+    unsigned int any = 0u;
+    bool bad = false;
     unsigned int todo = __ballot_sync(0xffffffffu, valid);
     int w = 0;
     while (todo) {
         const int lead = __ffs((int)todo) - 1;
         const unsigned int lead_row = __shfl_sync(0xffffffffu, row, lead);
-        const bool mine = valid && row == lead_row;
-        const unsigned int grp = __ballot_sync(0xffffffffu, mine);
         const unsigned int first = __shfl_sync(0xffffffffu, cell, lead);
-        const unsigned int last = __shfl_sync(0xffffffffu, cell, 31 - __clz((int)grp));
+        const bool mine = (todo >> lane & 1u) && row == lead_row && cell - first <= 5u;
+        const unsigned int grp = __ballot_sync(0xffffffffu, mine);
+        const int tail = 31 - __clz((int)grp);
+        const unsigned int last = __shfl_sync(0xffffffffu, cell, tail);
         todo &= ~grp;
-        unsigned int s = 0u, e = 0u; /* lane r < 9: the slots of row r's cells first - 1 .. last + 1 */
+        const float ox = 0.5f * (__shfl_sync(0xffffffffu, xi.x, lead) + __shfl_sync(0xffffffffu, xi.x, tail));
+        const float oy = __shfl_sync(0xffffffffu, xi.y, lead), oz = __shfl_sync(0xffffffffu, xi.z, lead);
+        /* lane r < 9: row r's cells first - 1 .. last + 1 hold the slots from s on; the
+         * rows' candidates are numbered through, row r's from `from` on */
+        unsigned int s = 0u, len = 0u;
         if (lane < 9) {
             const int o = ((lane / 3 - 1) * p.gy + (lane % 3 - 1)) * p.gx;
             const unsigned int a = (unsigned int)((int)first + o), b = (unsigned int)((int)last + o);
             if (cell_row_ok(p, a) && cell_row_ok(p, b)) {
                 s = __ldg(cell_start + (a - 1u));
-                e = bounded(p, __ldg(cell_start + (b + 2u)), (unsigned int)p.n + 1u, kBoundSlot);
+                len = bounded(p, __ldg(cell_start + (b + 2u)), (unsigned int)p.n + 1u, kBoundSlot) - s;
             }
         }
-#pragma unroll 1
-        for (int r = 0; r < 9; ++r) {
-            const unsigned int s0 = __shfl_sync(0xffffffffu, s, r), e0 = __shfl_sync(0xffffffffu, e, r);
-#pragma unroll 1
-            for (unsigned int j0 = s0; j0 < e0; j0 += 32) {
-                if (w == kTileWords) return -1;
-                const unsigned int j = j0 + (unsigned int)lane;
-                /* past the row's end: so far away that the test fails (r^2 = inf) */
-                const float4 q = j < e0 ? __ldg(x4 + j) : make_float4(1e30f, 1e30f, 1e30f, 0.0f);
-                __syncwarp(); /* the last word's tests have read the stage */
-                t.x[lane] = q.x;
-                t.y[lane] = q.y;
-                t.z[lane] = q.z;
-                __syncwarp();
-                unsigned int m = 0u;
+        unsigned int from = len;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const ulonglong2 X = reinterpret_cast<const ulonglong2 *>(t.x)[k];
-                    const ulonglong2 Y = reinterpret_cast<const ulonglong2 *>(t.y)[k];
-                    const ulonglong2 Z = reinterpret_cast<const ulonglong2 *>(t.z)[k];
-                    const unsigned long long x0 = add_f2(X.x, nx), x1 = add_f2(X.y, nx);
-                    const unsigned long long y0 = add_f2(Y.x, ny), y1 = add_f2(Y.y, ny);
-                    const unsigned long long z0 = add_f2(Z.x, nz), z1 = add_f2(Z.y, nz);
-                    const unsigned long long a = fma_f2(z0, z0, fma_f2(y0, y0, fma_f2(x0, x0, nr)));
-                    const unsigned long long b = fma_f2(z1, z1, fma_f2(y1, y1, fma_f2(x1, x1, nr)));
-                    m = sign_in(m, a, 0);
-                    m = sign_in(m, a, 1);
-                    m = sign_in(m, b, 0);
-                    m = sign_in(m, b, 1);
-                }
-                t.mask[w][lane] = mine ? m : 0u;
-                if (lane == 0) t.base[w] = j0;
-                ++w;
+        for (int o = 1; o < 16; o <<= 1) {
+            const unsigned int v = __shfl_up_sync(0xffffffffu, from, o);
+            if (lane >= o) from += v;
+        }
+        const unsigned int total = __shfl_sync(0xffffffffu, from, 8);
+        from -= len; /* lane 9 and on: the total */
+        const unsigned int shift = s - from;
+        if (total > (unsigned int)(kTileWords - w) * 32u) return false;
+        /* operand A: the warp's own slots */
+        __syncwarp(); /* the last operands of the group before have been read */
+        {
+            const float x = mine ? (xi.x - ox) * inv : 0.0f, y = mine ? (xi.y - oy) * inv : 0.0f,
+                        z = mine ? (xi.z - oz) * inv : 0.0f;
+            bad |= !(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= 8.0f) || !(x + y + z == x + y + z);
+            const float xh = half_round(x), yh = half_round(y), zh = half_round(z);
+            const float xl = half_round(x - xh), yl = half_round(y - yh), zl = half_round(z - zh);
+            const float nn = x * x + y * y + z * z, nh = half_round(nn);
+            t.k0[lane] = make_uint4(half_pair(-2.f * xh, -2.f * yh), half_pair(-2.f * zh, -2.f * xh),
+                                    half_pair(-2.f * yh, -2.f * zh), half_pair(-2.f * xl, -2.f * yl));
+            t.k1[lane] = make_uint4(half_pair(-2.f * zl, nh), half_pair(nn - nh, 1.0f), half_pair(1.0f, -1.0f),
+                                    half_pair(-0x1p-12f, 0.0f));
+        }
+        __syncwarp();
+        unsigned int a0[4], a1[4]; /* rows 0-7, 8-15, 16-23, 24-31; terms 0-7 and 8-15 */
+        load_matrices(a0, t.k0 + lane);
+        load_matrices(a1, t.k1 + lane);
+        int r = 0;
+#pragma unroll 1
+        for (unsigned int q0 = 0u; q0 < total; q0 += 32u, ++w) {
+            const unsigned int q = q0 + (unsigned int)lane;
+            unsigned int j = q + __shfl_sync(0xffffffffu, shift, r);
+            for (;;) { /* the rows that these 32 candidates reach into */
+                const unsigned int next = __shfl_sync(0xffffffffu, from, r + 1);
+                if (next >= q0 + 32u || r == 8) break;
+                ++r;
+                const unsigned int sh = __shfl_sync(0xffffffffu, shift, r);
+                if (q >= next) j = q + sh;
             }
+            float x = 30.0f, y = 30.0f, z = 30.0f; /* past the last candidate: far away */
+            if (q < total) {
+                const float4 c = __ldg(x4 + j);
+                x = (c.x - ox) * inv;
+                y = (c.y - oy) * inv;
+                z = (c.z - oz) * inv;
+                bad |= !(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= 8.0f) || !(x + y + z == x + y + z);
+            }
+            const float xh = half_round(x), yh = half_round(y), zh = half_round(z);
+            const float nn = x * x + y * y + z * z, nh = half_round(nn);
+            const unsigned int xy = half_pair(xh, yh);
+            __syncwarp(); /* the operands of the last word have been read */
+            *st0 = make_uint4(xy, half_pair(zh, x - xh), half_pair(y - yh, z - zh), xy);
+            *st1 = make_uint4(half_pair(zh, 1.0f), half_pair(1.0f, nh), half_pair(nn - nh, 1.0f),
+                              half_pair(1.0f, 0.0f));
+            t.slot[w][lane] = j;
+            __syncwarp();
+            unsigned int b0[4], b1[4];
+            load_matrices(b0, t.k0 + lrow);
+            load_matrices(b1, t.k1 + lrow);
+            unsigned int m0 = 0u, m1 = 0u, m2 = 0u, m3 = 0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                test_tile(m0, m1, a0[0], a0[1], a1[0], a1[1], b0[k], b1[k]);
+                test_tile(m2, m3, a0[2], a0[3], a1[2], a1[3], b0[k], b1[k]);
+            }
+            /* byte k of lane c: candidates 8c .. 8c + 7 of slot g + 8k; the quad's four
+             * lanes exchange bytes until lane c has all of slot g + 8c */
+            unsigned int m = __byte_perm(__byte_perm(m0, m1, 0x0040), __byte_perm(m2, m3, 0x0040), 0x5410);
+            m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 2), pick1);
+            m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 1), pick2);
+            if (!(grp >> own & 1u)) m = 0u;
+            t.mask[w][own] = m;
+            cnt += __popc(m);
+            if (m) any |= 0x80000000u >> w;
         }
     }
     __syncwarp();
-    return w;
+    const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
+    count = __shfl_sync(0xffffffffu, cnt, holder);
+    some = __shfl_sync(0xffffffffu, any, holder);
+    return !__any_sync(0xffffffffu, bad);
 }
 
-/* One lane's slots of a tile, ascending. */
+/* One lane's candidates of a tile, ascending: next() is called `count` times. */
 struct TileWalk {
     const PairTile &t;
-    int words, w = 0;
-    unsigned int m = 0u, base = 0u;
-    __device__ __forceinline__ TileWalk(const PairTile &tile, int nwords) : t(tile), words(nwords) {}
-    __device__ __forceinline__ bool next(unsigned int &j) {
-        while (m == 0u) {
-            if (w == words) return false;
+    unsigned int some, m = 0u;
+    int w = 0;
+    __device__ __forceinline__ TileWalk(const PairTile &tile, unsigned int words) : t(tile), some(words) {}
+    __device__ __forceinline__ unsigned int next() {
+        if (m == 0u) {
+            w = __clz((int)some);
+            some ^= 0x80000000u >> w;
             m = t.mask[w][threadIdx.x & 31];
-            base = t.base[w];
-            ++w;
         }
         const int b = __clz((int)m);
         m ^= 0x80000000u >> b;
-        j = base + (unsigned int)b;
-        return true;
+        return t.slot[w][b];
     }
 };
 
@@ -418,29 +499,28 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
                                                 unsigned char *__restrict__ cnt, PairTile &t) {
     const float3 xi = valid ? f3(__ldg(xb + i)) : make_float3(0.f, 0.f, 0.f);
     const unsigned int cell = valid ? __ldg(cellb + i) : 0u;
-    const int words = tile_masks(p, cell_start, xb, xi, cell, valid, p.rl2, t);
+    int count;
+    unsigned int some;
+    const bool ok = tile_masks(p, cell_start, xb, xi, cell, valid, p.rl2, t, count, some);
     if (!valid) return;
-    if (words < 0) {
+    if (!ok) {
         build_list_body(p, i, cell_start, xb, cell, list, cnt);
         return;
     }
-    TileWalk walk(t, words);
+    TileWalk walk(t, some);
     unsigned int last = 0u;
-    int k = 0;
-    for (int got = 4; got == 4;) {
+    const int most = min(count, kListMax);
+    for (int k = 0; k < most; k += 4) {
         unsigned int v[4];
-        got = 0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) { /* the last group is padded with its last entry */
-            if (got == u && walk.next(last)) ++got;
+            if (k + u < most) last = walk.next();
             v[u] = last;
         }
-        if (got && k < kListMax)
-            reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
-                make_uint4(v[0], v[1], v[2], v[3]);
-        k += got;
+        reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
+            make_uint4(v[0], v[1], v[2], v[3]);
     }
-    cnt[i] = k > kListMax ? kListOverflow : (unsigned char)k;
+    cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
 }
 
 /* ---------------- constraint iterations ---------------- */
