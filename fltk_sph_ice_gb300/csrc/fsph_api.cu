@@ -87,6 +87,8 @@ struct fsph_ctx {
     int gdim[3] = {0, 0, 0};
     DevCtl *ctl = nullptr;
     DevCtl *ctl_host = nullptr;
+    LoopCtl *loop = nullptr;           /* the one-kernel constraint loop's counters */
+    bool loop_kernel = false;          /* the step graph runs it */
     unsigned int *flag = nullptr;      /* input-validation flag, pinned host memory */
     /* warm start */
     float4 *xpred = nullptr;           /* x* before the iterations, iteration order */
@@ -596,8 +598,10 @@ int alloc_particles(fsph_ctx *c, int cap) {
         FSPH_TRY(dalloc(c, &c->radix.hist, nh)); FSPH_TRY(dalloc(c, &c->radix.offs, nh + 1)); /* + the total */
         FSPH_TRY(dalloc(c, &c->radix.bsum, scan_blocks((unsigned int)nh)));
     }
-    FSPH_TRY(dalloc(c, &c->epart, 2 * blocks_for((long long)n, kPassBlock))); /* room for ErrPartialFix */
-    FSPH_TRY(dalloc(c, &c->dpart, blocks_for((long long)n, kPassBlock)));
+    const size_t parts = std::max(blocks_for((long long)n, kPassBlock),
+                                  blocks_for(std::min((long long)n, (long long)kDeepMax), kDeepBlock));
+    FSPH_TRY(dalloc(c, &c->epart, 2 * parts)); /* room for ErrPartialFix */
+    FSPH_TRY(dalloc(c, &c->dpart, parts));
     for (int k = 0; k < 2; ++k) {
         FSPH_CUDA(c, cudaMemsetAsync(c->set[k].pos, 0, n * sizeof(float4), c->stream));
         FSPH_CUDA(c, cudaMemsetAsync(c->set[k].vel, 0, n * sizeof(float4), c->stream));
@@ -875,11 +879,19 @@ int build_pbf_graph(fsph_ctx *c, const DevParams &p) {
     hrb2 = 0;
     if (ext) FSPH_CUDA(c, cudaGraphConditionalHandleCreate(&hrb2, capg, 0, cudaGraphCondAssignDefault));
     FSPH_CUDA(c, cudaStreamBeginCaptureToGraph(c->s2, wbody, &inode, nullptr, 1, cudaStreamCaptureModeRelaxed));
-    launch_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->ctl, c->epart, hw, 1, c->nl, c->s2);
-    launch_boundary_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->ctl, c->b_stat, c->b_lam, c->s2);
-    launch_correction(p, c->cell_start, c->ppos[0], c->ppos[1], c->xb, c->ctl, c->dpart, hrb, hrb2, ext ? 3 : 1,
-                      nullptr, c->nl, c->s2);
+    c->loop_kernel = loop_fits(p);
+    cudaError_t le = cudaSuccess;
+    if (c->loop_kernel) {
+        le = launch_pbf_loop(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->xb, c->ctl, c->loop, hw, hrb, hrb2,
+                             ext ? 1 : 0, c->nl, c->s2);
+    } else {
+        launch_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->ctl, c->epart, hw, 1, c->nl, c->s2);
+        launch_boundary_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->ctl, c->b_stat, c->b_lam, c->s2);
+        launch_correction(p, c->cell_start, c->ppos[0], c->ppos[1], c->xb, c->ctl, c->dpart, hrb, hrb2, ext ? 3 : 1,
+                          nullptr, c->nl, c->s2);
+    }
     FSPH_CUDA(c, cudaStreamEndCapture(c->s2, &wbody));
+    FSPH_CUDA(c, le);
     FSPH_CUDA(c, cudaStreamUpdateCaptureDependencies(s, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies));
 
     if (ext) {
@@ -925,6 +937,7 @@ int sph_step(fsph_ctx *c, const DevParams &p) {
  * into a graph: the step is launch-bound at the configured 32k particles. */
 int build_sph_graph(fsph_ctx *c, const DevParams &p) {
     drop_graph(c);
+    c->loop_kernel = false;
     cudaGraph_t g;
     FSPH_CUDA(c, cudaGraphCreate(&g, 0));
     c->graph = g;
@@ -957,10 +970,11 @@ void fill_stats(fsph_ctx *c, fsph_step_stats *st) {
     st->status = FSPH_OK;
     st->bounds_bits = (int)h.bounds_bits;
     if (c->last_step_graph) /* every grid build after the first is one run of the rebuild body */
-        st->kernels = c->k_top + (int)h.iter * c->k_iter + ((int)h.builds - 1) * c->k_rebuild;
+        st->kernels = c->k_top + (int)(c->loop_kernel ? h.loops : h.iter) * c->k_iter +
+                      ((int)h.builds - 1) * c->k_rebuild;
     if (c->P.solver == FSPH_SOLVER_PBF) {
         if (h.nan_flag) st->status = FSPH_NAN_DETECTED;
-        else if (h.mlp_err) st->status = FSPH_TIMEOUT; /* the tcgen05 inference gave up on an MMA */
+        else if (h.mlp_err || h.wait_err) st->status = FSPH_TIMEOUT; /* the inference or the loop gave up a wait */
         else if (st->density_error > c->P.eta) st->status = FSPH_NOT_CONVERGED;
     }
     if (h.bounds_bits && st->status != FSPH_NAN_DETECTED)
@@ -1211,14 +1225,16 @@ int fsph_create(const fsph_params *params, fsph_ctx **out) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(FSPH_CUDA_ERROR);
     if (cudaStreamCreateWithFlags(&c->s2, cudaStreamNonBlocking) != cudaSuccess) return bail(FSPH_CUDA_ERROR);
     if (cudaStreamCreateWithFlags(&c->s3, cudaStreamNonBlocking) != cudaSuccess) return bail(FSPH_CUDA_ERROR);
-    if (cudaMalloc((void **)&c->ctl, sizeof(DevCtl)) != cudaSuccess) return bail(FSPH_OOM);
+    static_assert(sizeof(DevCtl) <= 256, "the loop's counters follow the control block");
+    if (cudaMalloc((void **)&c->ctl, 256 + sizeof(LoopCtl)) != cudaSuccess) return bail(FSPH_OOM);
+    c->loop = reinterpret_cast<LoopCtl *>(reinterpret_cast<unsigned char *>(c->ctl) + 256);
     if (cudaMallocHost((void **)&c->ctl_host, sizeof(DevCtl)) != cudaSuccess) return bail(FSPH_OOM);
     std::memset(c->ctl_host, 0, sizeof(DevCtl));
     if (cudaMallocHost((void **)&c->flag, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
     if (cudaMalloc((void **)&c->warm_valid, sizeof(unsigned int)) != cudaSuccess) return bail(FSPH_OOM);
     if (cudaMalloc((void **)&c->mlp_dev, sizeof(MlpDev)) != cudaSuccess) return bail(FSPH_OOM);
     cudaMemsetAsync(c->warm_valid, 0, sizeof(unsigned int), c->stream);
-    cudaMemsetAsync(c->ctl, 0, sizeof(DevCtl), c->stream);
+    cudaMemsetAsync(c->ctl, 0, 256 + sizeof(LoopCtl), c->stream);
     if ((st = alloc_particles(c, params->max_particles)) != FSPH_OK) return bail(st);
     if ((st = alloc_grid(c)) != FSPH_OK) return bail(st);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return bail(FSPH_CUDA_ERROR);
@@ -1457,7 +1473,8 @@ int fsph_step(fsph_ctx *c, float dt, void *stream, fsph_step_stats *stats) {
             std::fflush(c->log);
         }
         if (stats->status == FSPH_NAN_DETECTED) return fail(c, FSPH_NAN_DETECTED, "NaN in density or position");
-        if (stats->status == FSPH_TIMEOUT) return fail(c, FSPH_TIMEOUT, "warm-start inference: an MMA wait ran out");
+        if (stats->status == FSPH_TIMEOUT) return fail(c, FSPH_TIMEOUT, c->ctl_host->wait_err ? "constraint loop: a grid barrier's wait ran out"
+                                                               : "warm-start inference: an MMA wait ran out");
         if (stats->bounds_bits)
             return fail(c, FSPH_CUDA_ERROR, "debug bounds check: an index out of range (bits " +
                                                 std::to_string(stats->bounds_bits) + ")");

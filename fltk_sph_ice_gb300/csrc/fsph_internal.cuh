@@ -186,6 +186,17 @@ struct DevCtl {
     float err1, err2, errmax;   /* errors of the last lambda pass */
     unsigned int bounds_bits;   /* FSPH_DEBUG_BOUNDS builds: the index checks that failed (kBound*) */
     unsigned int grab, grab2;   /* FSPH_DYN_CHUNKS: chunks handed out on demand (lambda, correction pass) */
+    unsigned int loops;         /* launches of the one-kernel constraint loop in this step */
+    unsigned int wait_err;      /* 1 when that loop gave up waiting for its blocks */
+};
+
+/* State of the one-kernel constraint loop (fsph_loop.cu) between its blocks;
+ * all zero outside a launch.  Iteration t of a launch uses the sums t % 3. */
+struct LoopCtl {
+    unsigned long long e1[3], e2[3]; /* error sums in units of 2^-32 */
+    unsigned int em[3], disp[3];     /* largest |C| and |x* - xb|^2 (float bits) */
+    unsigned int nan[3];             /* a density (of this iteration) or a position (of the one before) is not a number */
+    unsigned int arrived, left;      /* the grid barrier's and the last block's counters */
 };
 
 /* Per-block partial sums of the lambda pass (one-sided, two-sided, max). */

@@ -406,8 +406,8 @@ __global__ void k_pbf_visc(DevParams p, const unsigned int *__restrict__ cell_st
  * into x*.w, block partial errors; the last block reduces the errors in a
  * fixed order, advances the iteration counter and decides whether the
  * device-side loop continues. */
-template <bool KAHAN>
-__global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_lambda(DevParams p, const unsigned int *__restrict__ cell_start,
+template <bool KAHAN, bool DEEP>
+__global__ void __launch_bounds__(DEEP ? kDeepBlock : kPassBlock, DEEP ? kDeepMinB : FSPH_PASS_MINB) k_lambda(DevParams p, const unsigned int *__restrict__ cell_start,
                                                    float4 *ppos0, float4 *ppos1, float *__restrict__ dens,
                                                    DevCtl *ctl, ErrPartial *part,
                                                    cudaGraphConditionalHandle hwhile, int use_graph,
@@ -415,49 +415,26 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_lambda(DevParams
                                                    const unsigned char *__restrict__ cnt) {
     const unsigned int par = *((volatile unsigned int *)&ctl->parity);
     float4 *pp = par ? ppos1 : ppos0;
-    float e1 = 0.f, e2 = 0.f, em = 0.f;
-#if FSPH_PERSIST_LAMBDA && FSPH_DYN_CHUNKS
     /* persistent warps: whole round-robin rounds, then the leftover chunks
-     * on demand; the error sums are fixed point, exact in any order */
+     * on demand (DEEP: one chunk a warp, in order); the error sums are fixed
+     * point, exact in any order */
     unsigned long long q1 = 0ull, q2 = 0ull;
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5, nchunks = (p.n + 31) >> 5;
-    const int stat = max(nchunks / nw - FSPH_DYN_EXTRA, 0) * nw;
-    for (int c = first_chunk((blockIdx.x * blockDim.x + threadIdx.x) >> 5, stat, &ctl->grab, lane); c < nchunks;
-         c = next_chunk(c, nw, stat, &ctl->grab, lane)) {
+    float em = 0.f;
+    const int lane = threadIdx.x & 31, warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int nw = (int)((gridDim.x * blockDim.x) >> 5), nchunks = (p.n + 31) >> 5;
+    const int stat = DEEP ? nchunks : max(nchunks / nw - FSPH_DYN_EXTRA, 0) * nw;
+    for (int c = DEEP ? warp : first_chunk(warp, stat, &ctl->grab, lane); c < nchunks;
+         c = DEEP ? nchunks : next_chunk(c, nw, stat, &ctl->grab, lane)) {
         const int i = c * 32 + lane;
         if (i < p.n) {
-            const float C = lambda_body<1, KAHAN>(p, cell_start, pp, dens, ctl, list, cnt, i, 0, true);
+            const float C = lambda_body<1, KAHAN, DEEP>(p, cell_start, pp, dens, ctl, list, cnt, i, 0, true);
             q1 += err_fix(C > 0.0f ? C : 0.0f);
             q2 += err_fix(fabsf(C));
             em = fmaxf(em, fabsf(C));
         }
     }
-    (void)e1; (void)e2;
     lambda_tail_fix(p, ctl, part, q1, q2, em, hwhile, use_graph);
 }
-#else
-#if FSPH_PERSIST_LAMBDA
-    /* persistent warps: warp w takes the 32-slot chunks w, w + W, ... in a
-     * fixed order (the error sums stay deterministic) */
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 32 < p.n; c += nw) {
-        const int i = c * 32 + lane;
-#else
-    {
-        const int i = blockIdx.x * blockDim.x + threadIdx.x;
-#endif
-        if (i < p.n) {
-            const float C = lambda_body<1, KAHAN>(p, cell_start, pp, dens, ctl, list, cnt, i, 0, true);
-            e1 += C > 0.0f ? C : 0.0f;
-            e2 += fabsf(C);
-            em = fmaxf(em, fabsf(C));
-        }
-    }
-    lambda_tail(p, ctl, part, e1, e2, em, hwhile, use_graph);
-}
-#endif
 
 /* Density and lambda of every slot by walking the cells, LPP lanes a particle,
  * written to the particle's place (order[slot]): the whole pass of the
@@ -475,8 +452,14 @@ __global__ void __launch_bounds__(kBlock) k_lambda_walk(DevParams p, const unsig
     const int sub = t % LPP;
     const bool valid = t / LPP < p.n;
     const int i = valid ? t / LPP : p.n - 1; /* padding lanes run a real slot and write nothing */
+    const float3 xi = f3(__ldg(x + i));
     float rho, lam;
-    lambda_terms<LPP, false>(p, cell_start, x, nullptr, nullptr, i, sub, rho, lam);
+    lambda_terms<LPP, false>(
+        p, x, xi,
+        [&](auto &&load, auto &&f) {
+            for_each_candidate<LPP>(p, cell_start, nullptr, nullptr, i, xi, sub, load, f);
+        },
+        rho, lam);
     if (!valid || sub != 0) return;
     const unsigned int o = order[i];
     dens[o] = rho;
@@ -487,7 +470,8 @@ __global__ void __launch_bounds__(kBlock) k_lambda_walk(DevParams p, const unsig
  * x*_i <- walls(x*_i + dp_i) into the other ping-pong buffer; the largest
  * displacement since the last grid build decides whether the grid must be
  * rebuilt before the next pass. */
-__global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_correction(DevParams p, const unsigned int *__restrict__ cell_start,
+template <bool DEEP>
+__global__ void __launch_bounds__(DEEP ? kDeepBlock : kPassBlock, DEEP ? kDeepMinB : FSPH_PASS_MINB) k_correction(DevParams p, const unsigned int *__restrict__ cell_start,
                                                        float4 *ppos0, float4 *ppos1,
                                                        const float4 *__restrict__ xb, DevCtl *ctl, float *part,
                                                        cudaGraphConditionalHandle hif,
@@ -499,24 +483,9 @@ __global__ void __launch_bounds__(kPassBlock, FSPH_PASS_MINB) k_correction(DevPa
     const float4 *__restrict__ src = par ? ppos1 : ppos0;
     float4 *__restrict__ dst = par ? ppos0 : ppos1;
     float disp2 = 0.f;
-#if FSPH_PERSIST_CORRECTION && FSPH_DYN_CHUNKS
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5, nchunks = (p.n + 31) >> 5, stat = (nchunks / nw) * nw;
-    for (int c = first_chunk((blockIdx.x * blockDim.x + threadIdx.x) >> 5, stat, &ctl->grab2, lane); c < nchunks;
-         c = next_chunk(c, nw, stat, &ctl->grab2, lane)) {
-        const int i = c * 32 + lane;
-#elif FSPH_PERSIST_CORRECTION
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 32 < p.n; c += nw) {
-        const int i = c * 32 + lane;
-#else
-    {
-        const int i = blockIdx.x * blockDim.x + threadIdx.x;
-#endif
-        if (i < p.n)
-            disp2 = fmaxf(disp2, correction_body<1>(p, cell_start, src, dst, xb, ctl, dp_out, list, cnt, i, 0, true));
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < p.n)
+        disp2 = correction_body<1, DEEP>(p, cell_start, src, dst, xb, ctl, dp_out, list, cnt, i, 0, true);
     correction_tail(p, ctl, part, disp2, par, hif, hif2, use_graph);
 }
 
@@ -548,8 +517,8 @@ __global__ void k_finalize(DevParams p, const float4 *__restrict__ pos_b, const 
 
 /* omega_i = sum_j (v_j - v_i) x grad_j W_ij (grad_j = -grad_i), and the
  * XSPH update v_i + c sum_j (m / rho_j)(v_j - v_i) W_ij. */
-template <bool NBR, bool PRE>
-__global__ void __launch_bounds__(kBlock) k_xsph_vort(DevParams p, const unsigned int *__restrict__ cell_start,
+template <bool NBR, bool PRE, bool DEEP>
+__global__ void __launch_bounds__(DEEP ? kDeepBlock : kBlock) k_xsph_vort(DevParams p, const unsigned int *__restrict__ cell_start,
                                                       const float4 *__restrict__ pos, const float4 *__restrict__ vel,
                                                       const float *__restrict__ dens, float4 *__restrict__ vel_out,
                                                       float4 *__restrict__ vort, FeatureOut fo,
@@ -558,13 +527,13 @@ __global__ void __launch_bounds__(kBlock) k_xsph_vort(DevParams p, const unsigne
                                                       const float *__restrict__ mrho, float2 *__restrict__ wm) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    xsph_vort_body<NBR, PRE>(p, i, cell_start, pos, vel, dens, vel_out, vort, fo, list, cnt, mrho, wm);
+    xsph_vort_body<NBR, PRE, DEEP>(p, i, cell_start, pos, vel, dens, vel_out, vort, fo, list, cnt, mrho, wm);
 }
 
 /* eta_i = sum_j (m / rho_j)(|w_j| - |w_i|) grad_i W_ij; f = eps (eta/|eta|) x w_i;
  * v_i <- v_i + dt f. */
-template <bool PRE>
-__global__ void __launch_bounds__(kBlock) k_vort_apply(DevParams p, const unsigned int *__restrict__ cell_start,
+template <bool PRE, bool DEEP>
+__global__ void __launch_bounds__(DEEP ? kDeepBlock : kBlock) k_vort_apply(DevParams p, const unsigned int *__restrict__ cell_start,
                                                        const float4 *__restrict__ pos,
                                                        const float4 *__restrict__ vort,
                                                        const float *__restrict__ dens,
@@ -575,7 +544,7 @@ __global__ void __launch_bounds__(kBlock) k_vort_apply(DevParams p, const unsign
                                                       const float2 *__restrict__ wm) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    vort_apply_body<PRE>(p, i, cell_start, pos, vort, dens, vel_in, vel_out, list, cnt, wm);
+    vort_apply_body<PRE, DEEP>(p, i, cell_start, pos, vort, dens, vel_in, vel_out, list, cnt, wm);
 }
 
 /* ======================================================================== */
@@ -1357,40 +1326,39 @@ void launch_pbf_visc(const DevParams &p, const unsigned int *cell_start, const f
                      const float *dens, float4 *acc, cudaStream_t s) {
     k_pbf_visc<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, vel, dens, acc);
 }
-/* blocks of a constraint-pass launch: one per kPassBlock slots, or (with
- * persistent warps) the resident blocks of the whole GPU, at most that */
-static unsigned int pass_blocks(int n, const void *kernel, bool persistent) {
-    unsigned int b = blocks_for(n, kPassBlock);
-    if (persistent) {
-        /* resident blocks of each pass kernel, looked up once (contexts may
-         * step from several host threads) */
-        static std::mutex mu;
-        static const void *known[4] = {nullptr, nullptr, nullptr, nullptr};
-        static int resident[4] = {0, 0, 0, 0};
-        std::lock_guard<std::mutex> lock(mu);
-        int k = 0;
-        while (k < 4 && known[k] && known[k] != kernel) ++k;
-        if (k == 4) k = 3;
-        if (known[k] != kernel) {
-            int dev = 0, sms = 0, per = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kPassBlock, 0);
-            resident[k] = std::max(1, sms * std::max(per, 1));
-            known[k] = kernel;
-        }
-        b = std::min(b, (unsigned int)resident[k]);
+/* resident blocks of the persistent lambda pass, looked up once per kernel
+ * (contexts may step from several host threads) */
+static unsigned int resident_blocks(const void *kernel) {
+    static std::mutex mu;
+    static const void *known[2] = {nullptr, nullptr};
+    static int resident[2] = {0, 0};
+    std::lock_guard<std::mutex> lock(mu);
+    const int k = !known[0] || known[0] == kernel ? 0 : 1;
+    if (known[k] != kernel) {
+        int dev = 0, sms = 0, per = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kPassBlock, 0);
+        resident[k] = std::max(1, sms * std::max(per, 1));
+        known[k] = kernel;
     }
-    return b;
+    return (unsigned int)resident[k];
 }
+
+/* the passes' shape by size (kDeepMax in fsph_kernels.cuh) */
+static bool deep_pass(const DevParams &p) { return p.n <= kDeepMax && p.use_lists; }
 
 void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1, float *dens,
                    DevCtl *ctl, ErrPartial *part, unsigned long long while_handle, int use_graph,
                    const NbrLists &nl, cudaStream_t s) {
-    auto k = p.compensated ? k_lambda<true> : k_lambda<false>;
-    k<<<pass_blocks(p.n, (const void *)k, FSPH_PERSIST_LAMBDA != 0), kPassBlock, 0, s>>>(p, cell_start, ppos0, ppos1, dens, ctl, part,
-                                         (cudaGraphConditionalHandle)while_handle, use_graph,
-                                         p.use_lists ? nl.list : nullptr, nl.cnt);
+    const bool deep = deep_pass(p);
+    auto k = deep ? (p.compensated ? k_lambda<true, true> : k_lambda<false, true>)
+                  : (p.compensated ? k_lambda<true, false> : k_lambda<false, false>);
+    const unsigned int blocks = deep ? blocks_for(p.n, kDeepBlock)
+                                     : std::min(blocks_for(p.n, kPassBlock), resident_blocks((const void *)k));
+    k<<<blocks, deep ? kDeepBlock : kPassBlock, 0, s>>>(p, cell_start, ppos0, ppos1, dens, ctl, part,
+                                                        (cudaGraphConditionalHandle)while_handle, use_graph,
+                                                        p.use_lists ? nl.list : nullptr, nl.cnt);
 }
 void launch_build_list(const DevParams &p, const unsigned int *cell_start, const float4 *xb, const NbrLists &nl,
                        cudaStream_t s) {
@@ -1401,11 +1369,13 @@ void launch_correction(const DevParams &p, const unsigned int *cell_start, float
                        const float4 *xb, DevCtl *ctl, float *part, unsigned long long if_handle,
                        unsigned long long if_handle2, int use_graph, float4 *dp_out, const NbrLists &nl,
                        cudaStream_t s) {
-    k_correction<<<pass_blocks(p.n, (const void *)k_correction, FSPH_PERSIST_CORRECTION != 0), kPassBlock, 0, s>>>(p, cell_start, ppos0, ppos1, xb,
-                                                                                    ctl, part,
-                                                    (cudaGraphConditionalHandle)if_handle,
-                                                    (cudaGraphConditionalHandle)if_handle2, use_graph, dp_out,
-                                                    p.use_lists ? nl.list : nullptr, nl.cnt);
+    const bool deep = deep_pass(p);
+    auto k = deep ? k_correction<true> : k_correction<false>;
+    const int block = deep ? kDeepBlock : kPassBlock;
+    k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, ppos0, ppos1, xb, ctl, part,
+                                               (cudaGraphConditionalHandle)if_handle,
+                                               (cudaGraphConditionalHandle)if_handle2, use_graph, dp_out,
+                                               p.use_lists ? nl.list : nullptr, nl.cnt);
 }
 void launch_finalize(const DevParams &p, const float4 *pos_b, const float4 *ppos0, const float4 *ppos1,
                      const DevCtl *ctl, const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a,
@@ -1418,18 +1388,23 @@ void launch_xsph_vort(const DevParams &p, const unsigned int *cell_start, const 
                       const float *dens, float4 *vel_out, float4 *vort, const FeatureOut &fo, const NbrLists &nl,
                       cudaStream_t s, const float *mrho, float2 *wm) {
     /* the neighbour means cost a gather per pair: only when they are used */
-    const bool nbr = fo.feat && fo.nbr, pre = mrho && wm;
-    auto k = nbr ? (pre ? k_xsph_vort<true, true> : k_xsph_vort<true, false>)
-                 : (pre ? k_xsph_vort<false, true> : k_xsph_vort<false, false>);
-    k<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, vel, dens, vel_out, vort, fo,
-                                         p.use_lists ? nl.list : nullptr, nl.cnt, mrho, wm);
+    const bool nbr = fo.feat && fo.nbr, pre = mrho && wm, deep = deep_pass(p);
+    auto k = nbr ? (pre ? (deep ? k_xsph_vort<true, true, true> : k_xsph_vort<true, true, false>)
+                        : k_xsph_vort<true, false, false>)
+                 : (pre ? (deep ? k_xsph_vort<false, true, true> : k_xsph_vort<false, true, false>)
+                        : k_xsph_vort<false, false, false>);
+    const int block = deep && pre ? kDeepBlock : kBlock;
+    k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, pos, vel, dens, vel_out, vort, fo,
+                                               p.use_lists ? nl.list : nullptr, nl.cnt, mrho, wm);
 }
 void launch_vort_apply(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vort,
                        const float *dens, const float4 *vel_in, float4 *vel_out, const NbrLists &nl, cudaStream_t s,
                        const float2 *wm) {
-    auto k = wm ? k_vort_apply<true> : k_vort_apply<false>;
-    k<<<blocks_for(p.n), kBlock, 0, s>>>(p, cell_start, pos, vort, dens, vel_in, vel_out,
-                                         p.use_lists ? nl.list : nullptr, nl.cnt, wm);
+    const bool deep = wm && deep_pass(p);
+    auto k = deep ? k_vort_apply<true, true> : wm ? k_vort_apply<true, false> : k_vort_apply<false, false>;
+    const int block = deep ? kDeepBlock : kBlock;
+    k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, pos, vort, dens, vel_in, vel_out,
+                                               p.use_lists ? nl.list : nullptr, nl.cnt, wm);
 }
 static int lanes_to_fill(int n, int most);
 int sph_force_lanes(int n) { return lanes_to_fill(n, 8); }

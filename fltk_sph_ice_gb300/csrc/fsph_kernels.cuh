@@ -16,6 +16,12 @@ constexpr int kBlock = 256;
 #define FSPH_PASS_BLOCK 512
 #endif
 constexpr int kPassBlock = FSPH_PASS_BLOCK;
+/* up to kDeepMax particles the list passes run in blocks of 64 with eight
+ * candidates in flight (for_each_candidate's DEEP; 12 blocks an SM, 72
+ * registers): 14 blocks of 512 left 138 SMs idle at 6,912 particles.  A lambda
+ * and a correction pass together: 31.0 -> 22.6 us at 6,912, 33.0 -> 27.7 at
+ * 32,000, 43.1 -> 42.0 at 131,072, 71.4 -> 81.6 at 294,912 */
+constexpr int kDeepBlock = 64, kDeepMinB = 12, kDeepMax = 65536;
 constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 9.2 KB each */
 constexpr int kBlockMax = 512;  /* largest block of the batched persistent kernels */
 constexpr int kScanTile = 4096; /* cells per block of the first scan phase */
@@ -96,6 +102,17 @@ void launch_pbf_visc(const DevParams &p, const unsigned int *cell_start, const f
 void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1, float *dens,
                    DevCtl *ctl, ErrPartial *part, unsigned long long while_handle, int use_graph,
                    const NbrLists &nl, cudaStream_t s);
+/* The whole constraint loop of a small scene in one cooperative kernel
+ * (fsph_loop.cu): iterations until the loop ends or a grid rebuild is due, then
+ * the three conditions are set (post: the third exists).  loop_fits: p.n is at
+ * most kLoopMax, lists are on, there is no boundary (its lambda is a kernel of
+ * its own between the passes) and every block is resident at once. */
+constexpr int kLoopMax = 65536;
+bool loop_fits(const DevParams &p);
+cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
+                            float *dens, const float4 *xb, DevCtl *ctl, LoopCtl *lc, unsigned long long while_handle,
+                            unsigned long long if_handle, unsigned long long if_handle2, int post, const NbrLists &nl,
+                            cudaStream_t s);
 /* density and lambda of x (slot order) at order[slot], walking the cells */
 void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,
                         float *dens, float *lambda, cudaStream_t s);

@@ -127,10 +127,16 @@ __device__ __forceinline__ void prefetch_list_group(const uint4 *a) {
 #endif
 }
 
-template <int LPP, class Load, class F>
+/* DEEP: for launches that leave the GPU's warps few (kDeepMax): eight
+ * candidates and the next two list groups in flight instead of four
+ * candidates, so that a particle's chain of dependent loads is half as long;
+ * it takes the registers that so few warps leave unused.  The order in which
+ * f meets the candidates, and so the result, is the same. */
+template <int LPP, bool DEEP = false, class Load, class F>
 __device__ __forceinline__ void for_each_candidate(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                                    const ListEntry *__restrict__ list,
-                                                   const unsigned char *__restrict__ cnt, int i, float3 xi, int sub, Load &&load, F &&f) {
+                                                   const unsigned char *__restrict__ cnt, int i, float3 xi, int sub,
+                                                   Load &&load, F &&f) {
     int k = list ? (int)cnt[i] : (int)kListOverflow;
 #if FSPH_DEBUG_BOUNDS
     if (k > kListMax && k != (int)kListOverflow) { /* a count the build never writes: walk the cells */
@@ -138,7 +144,28 @@ __device__ __forceinline__ void for_each_candidate(const DevParams &p, const uns
         k = (int)kListOverflow;
     }
 #endif
-    if (LPP == 1 && kBatch == 4 && k != (int)kListOverflow) {
+    if (DEEP && k != (int)kListOverflow) {
+        const uint4 *lg = reinterpret_cast<const uint4 *>(list) + i;
+        const size_t n = (size_t)p.n;
+        uint4 e[2];
+        e[0] = load_list_group(lg);
+        e[1] = load_list_group(k > 4 ? lg + n : lg);
+        for (int t0 = 0; t0 < k; t0 += 8) {
+            const uint4 *nx = lg + (size_t)((t0 >> 2) + 2) * n;
+            uint4 g[2] = {e[0], e[0]};
+            if (t0 + 8 < k) g[0] = load_list_group(nx);
+            if (t0 + 12 < k) g[1] = load_list_group(nx + n);
+            const unsigned int j[8] = {e[0].x, e[0].y, e[0].z, e[0].w, e[1].x, e[1].y, e[1].z, e[1].w};
+            decltype(load(0u)) xj[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) xj[u] = load(bounded(p, j[u], (unsigned int)p.n, kBoundSlot));
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (t0 + u < k) f(bounded(p, j[u], (unsigned int)p.n, kBoundSlot), xj[u]);
+            e[0] = g[0];
+            e[1] = g[1];
+        }
+    } else if (LPP == 1 && kBatch == 4 && k != (int)kListOverflow) {
         /* one 16-byte load brings the next four entries (the tail group is
          * padded with a valid slot, so every load stays in bounds) */
         const uint4 *lg = reinterpret_cast<const uint4 *>(list) + i;
@@ -525,14 +552,12 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
 
 /* ---------------- constraint iterations ---------------- */
 
-/* Density, C, sum |grad C|^2 (with the k = i term) and lambda of one particle;
- * returns C (every lane of a group gets the same values). */
-template <int LPP, bool KAHAN>
-__device__ __forceinline__ float lambda_terms(const DevParams &p, const unsigned int *__restrict__ cell_start,
-                                              const float4 *pp, const ListEntry *__restrict__ list,
-                                              const unsigned char *__restrict__ cnt, int i, int sub, float &rho_out,
-                                              float &lam_out) {
-    const float3 xi = f3(pp[i]);
+/* Density, C, sum |grad C|^2 (with the k = i term) and lambda of one particle
+ * at xi; returns C (every lane of a group gets the same values).
+ * each(load, f) calls f(j, load(j)) for the lane's candidates. */
+template <int LPP, bool KAHAN, class Each>
+__device__ __forceinline__ float lambda_terms(const DevParams &p, const float4 *pp, float3 xi, Each &&each,
+                                              float &rho_out, float &lam_out) {
     float wsum = 0.f, wc = 0.f, sd = 0.f;
     float3 gs = make_float3(0.f, 0.f, 0.f);
     const float agr = p.ag * p.inv_rest_dens;
@@ -545,8 +570,8 @@ __device__ __forceinline__ float lambda_terms(const DevParams &p, const unsigned
 #endif
     /* plain (L1-cached) loads: only the .w words of pp are written by this
      * pass, and the neighbour loop reads x, y, z */
-    for_each_candidate<LPP>(
-        p, cell_start, list, cnt, i, xi, sub, [&](unsigned int j) { return pp[j]; },
+    each(
+        [&](unsigned int j) { return pp[j]; },
         [&](unsigned int, const float4 &xj4) {
             /* branch-free: outside h both q and t clamp to zero; the self
              * pair (d = 0) adds W(0) to the density and nothing else */
@@ -575,9 +600,11 @@ __device__ __forceinline__ float lambda_terms(const DevParams &p, const unsigned
         gs.z = group_sum<LPP>(gs.z);
     }
     float rho = p.mass * p.aw * wsum;
-    sd += dot3(gs, gs);
+    /* the roundings spelt out: a compiler may fuse either product of x x + y y, or
+     * this scaling with what is added below, and every kernel has to agree */
+    sd = __fadd_rn(sd, __fmaf_rn(gs.z, gs.z, __fmaf_rn(gs.y, gs.y, __fmul_rn(gs.x, gs.x))));
 #if FSPH_FOLD
-    sd *= agr * agr;
+    sd = __fmul_rn(sd, agr * agr);
 #endif
     if (p.nb) {
         /* boundary particles (rx_sph_pbd.cpp:728-748, 795-818): density
@@ -606,13 +633,17 @@ __device__ __forceinline__ float lambda_terms(const DevParams &p, const unsigned
 
 /* lambda pass of one particle: lambda into x*.w and rho into dens (lane 0 of a
  * valid group).  Returns C (the caller turns it into the error terms). */
-template <int LPP, bool KAHAN = false>
+template <int LPP, bool KAHAN = false, bool DEEP = false>
 __device__ __forceinline__ float lambda_body(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                              float4 *pp, float *__restrict__ dens, DevCtl *ctl,
                                              const ListEntry *__restrict__ list,
                                              const unsigned char *__restrict__ cnt, int i, int sub, bool valid) {
+    const float3 xi = f3(pp[i]);
     float rho, lam;
-    const float C = lambda_terms<LPP, KAHAN>(p, cell_start, pp, list, cnt, i, sub, rho, lam);
+    const float C = lambda_terms<LPP, KAHAN>(
+        p, pp, xi,
+        [&](auto &&load, auto &&f) { for_each_candidate<LPP, DEEP>(p, cell_start, list, cnt, i, xi, sub, load, f); },
+        rho, lam);
     if (valid && sub == 0) {
         reinterpret_cast<float *>(pp + i)[3] = lam;
         dens[i] = rho;
@@ -770,19 +801,11 @@ __device__ __forceinline__ void lambda_tail_fix(const DevParams &lp, DevCtl *ctl
     }
 }
 
-/* correction pass of one particle: dp_i = sum_j (lambda_i + lambda_j + s_corr)
- * grad W_ij / rho0, x*_i <- walls(x*_i + dp_i) into dst (lane 0 of a valid
- * group).  Returns |x*_i - xb_i|^2 (0 for the other lanes). */
-template <int LPP>
-__device__ __forceinline__ float correction_body(const DevParams &p, const unsigned int *__restrict__ cell_start,
-                                                 const float4 *__restrict__ src, float4 *__restrict__ dst,
-                                                 const float4 *__restrict__ xb, DevCtl *ctl,
-                                                 float4 *__restrict__ dp_out, const ListEntry *__restrict__ list,
-                                                 const unsigned char *__restrict__ cnt, int i,
-                                                 int sub, bool valid) {
-    const float4 xi4 = src[i];
-    const float3 xi = f3(xi4);
-    const float li = xi4.w;
+/* dp_i = sum_j (lambda_i + lambda_j + s_corr) grad W_ij / rho0 of one particle
+ * at xi with lambda li (every lane of a group gets it). */
+template <int LPP, class Each>
+__device__ __forceinline__ float3 correction_terms(const DevParams &p, const float4 *src, float3 xi, float li,
+                                                   Each &&each) {
     float3 acc = make_float3(0.f, 0.f, 0.f);
     const float k_dt2 = -p.ap_k * p.dt * p.dt;
     const float agr = p.ag * p.inv_rest_dens;
@@ -797,8 +820,8 @@ __device__ __forceinline__ float correction_body(const DevParams &p, const unsig
 #else
     const float agl = agr;
 #endif
-    for_each_candidate<LPP>(
-        p, cell_start, list, cnt, i, xi, sub, [&](unsigned int j) { return __ldg(src + j); },
+    each(
+        [&](unsigned int j) { return src[j]; },
         [&](unsigned int, const float4 &xj4) {
             /* branch-free: t = 0 outside h and d = 0 for the self pair */
             const float3 d = xi - f3(xj4);
@@ -830,7 +853,7 @@ __device__ __forceinline__ float correction_body(const DevParams &p, const unsig
         acc.z = group_sum<LPP>(acc.z);
     }
 #if FSPH_FOLD
-    acc = agr * acc;
+    acc = make_float3(__fmul_rn(agr, acc.x), __fmul_rn(agr, acc.y), __fmul_rn(agr, acc.z)); /* as in lambda_terms */
 #endif
     if (p.nb) {
         /* boundary terms (rx_sph_pbd.cpp:977-1019): lambda_b, and s_corr of
@@ -853,6 +876,24 @@ __device__ __forceinline__ float correction_body(const DevParams &p, const unsig
         });
         acc = acc + accb;
     }
+    return acc;
+}
+
+/* correction pass of one particle: x*_i <- walls(x*_i + dp_i) into dst (lane 0
+ * of a valid group).  Returns |x*_i - xb_i|^2 (0 for the other lanes). */
+template <int LPP, bool DEEP = false>
+__device__ __forceinline__ float correction_body(const DevParams &p, const unsigned int *__restrict__ cell_start,
+                                                 const float4 *__restrict__ src, float4 *__restrict__ dst,
+                                                 const float4 *__restrict__ xb, DevCtl *ctl,
+                                                 float4 *__restrict__ dp_out, const ListEntry *__restrict__ list,
+                                                 const unsigned char *__restrict__ cnt, int i, int sub, bool valid) {
+    const float4 xi4 = src[i];
+    const float3 xi = f3(xi4);
+    const float3 acc = correction_terms<LPP>(p, src, xi, xi4.w, [&](auto &&load, auto &&f) {
+        for_each_candidate<LPP, DEEP>(
+            p, cell_start, list, cnt, i, xi, sub, [&](unsigned int j) { return __ldg(src + j); }, f);
+        (void)load;
+    });
     if (!valid || sub != 0) return 0.0f;
     if (dp_out) dp_out[i] = make_float4(acc.x, acc.y, acc.z, 0.0f);
     float3 xn = solid_project(xi + acc, p);
@@ -922,7 +963,7 @@ __device__ __forceinline__ void correction_tail(const DevParams &lp, DevCtl *ctl
 /* PRE: m / rho_j comes from mrho (written once per particle by k_finalize,
  * the same correctly rounded quotient) instead of a division per pair, and
  * the pass leaves (|omega_i|, m / rho_i) in wm for vort_apply_body<true>. */
-template <bool NBR = true, bool PRE = false>
+template <bool NBR = true, bool PRE = false, bool DEEP = false>
 __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const unsigned int *__restrict__ cell_start,
                                                const float4 *__restrict__ pos, const float4 *__restrict__ vel,
                                                const float *__restrict__ dens, float4 *__restrict__ vel_out,
@@ -942,7 +983,7 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
     float3 nv = make_float3(0.f, 0.f, 0.f), nd = make_float3(0.f, 0.f, 0.f);
     /* branch-free pair terms: q and t clamp to zero outside h, and the self
      * pair (d = 0, v_ij = 0) adds only to the neighbour count */
-    for_each_candidate<1>(
+    for_each_candidate<1, DEEP>(
         p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return __ldg(pos + j); },
         [&](unsigned int j, const float4 &xj4) {
             const float3 d = xi - f3(xj4);
@@ -1020,7 +1061,7 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
  * v_i <- v_i + dt f. */
 /* PRE: (|omega_j|, m / rho_j) from wm (one 8-byte gather per pair, no
  * division or square root; the same values xsph_vort_body<.., true> wrote). */
-template <bool PRE = false>
+template <bool PRE = false, bool DEEP = false>
 __device__ __forceinline__ void vort_apply_body(const DevParams &p, int i, const unsigned int *__restrict__ cell_start,
                                                 const float4 *__restrict__ pos, const float4 *__restrict__ vort,
                                                 const float *__restrict__ dens, const float4 *__restrict__ vel_in,
@@ -1033,7 +1074,7 @@ __device__ __forceinline__ void vort_apply_body(const DevParams &p, int i, const
         const float3 wi = f3(vort[i]);
         const float wmi = sqrtf(dot3(wi, wi));
         float3 eta = make_float3(0.f, 0.f, 0.f);
-        for_each_candidate<1>(
+        for_each_candidate<1, DEEP>(
             p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return __ldg(pos + j); },
             [&](unsigned int j, const float4 &xj4) {
                 const float3 d = xi - f3(xj4);
