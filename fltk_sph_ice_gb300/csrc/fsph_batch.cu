@@ -50,12 +50,29 @@ struct BatchArgs {
     int ntiles;
 };
 
-/* The tile's scene constants into shared memory (every thread calls it). */
-__device__ __forceinline__ BTile tile_begin(const BatchArgs &b, int t, DevParams &s_p) {
+/* The tiles of a block are consecutive (mostly of one scene, neighbours in
+ * space): tile_first / tile_last, and tile_begin for each, which every thread
+ * calls.  It reads the scene's constants into shared memory when the scene
+ * changes, all threads a word each.  Strided over the grid, every tile was of
+ * another scene and one thread copied its constants between two barriers.  The
+ * barrier per tile stays: it keeps a block's warps on neighbouring slots. */
+__device__ __forceinline__ int tile_first(const BatchArgs &b) {
+    return (int)((long long)b.ntiles * blockIdx.x / gridDim.x);
+}
+__device__ __forceinline__ int tile_last(const BatchArgs &b) {
+    return (int)((long long)b.ntiles * (blockIdx.x + 1) / gridDim.x);
+}
+__device__ __forceinline__ BTile tile_begin(const BatchArgs &b, int t, DevParams &s_p, int &scene) {
+    static_assert(sizeof(DevParams) % 4 == 0, "copied word by word");
     const BTile tl = b.tiles[t];
     __syncthreads(); /* the previous tile is done with s_p */
-    if (threadIdx.x == 0) s_p = b.scenes[tl.scene];
-    __syncthreads();
+    if (tl.scene != scene) {
+        scene = tl.scene;
+        const unsigned int *src = reinterpret_cast<const unsigned int *>(b.scenes + scene);
+        unsigned int *dst = reinterpret_cast<unsigned int *>(&s_p);
+        for (int k = threadIdx.x; k < (int)(sizeof(DevParams) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
+        __syncthreads();
+    }
     return tl;
 }
 
@@ -65,8 +82,8 @@ __global__ void __launch_bounds__(BLOCK) kb_predict_hash(BatchArgs b, const floa
                                                          unsigned int *__restrict__ key, unsigned int *__restrict__ rank,
                                                          unsigned int *__restrict__ count) {
     __shared__ DevParams s_p;
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
             predict_body(p, tl.start + threadIdx.x, pos, vel, nullptr, ppos_out, key, rank, count, nullptr, nullptr);
@@ -80,8 +97,8 @@ __global__ void __launch_bounds__(BLOCK) kb_hash_parity(BatchArgs b, const float
                                                         unsigned int *__restrict__ count) {
     __shared__ DevParams s_p;
     const float4 *x4 = ctl->parity ? ppos1 : ppos0;
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count) {
             const int i = tl.start + threadIdx.x;
@@ -99,8 +116,8 @@ __global__ void __launch_bounds__(kListBlock) kb_build_list(BatchArgs b, const u
                                                             unsigned char *__restrict__ cnt) {
     __shared__ DevParams s_p;
     __shared__ PairTile s_tile[kListBlock / 32];
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         for (int o = 0; o < tl.count; o += kListBlock) {
             const int at = o + (int)threadIdx.x;
@@ -124,8 +141,8 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK)
     float4 *pp = par ? ppos1 : ppos0;
     float e1 = 0.f, e2 = 0.f, em = 0.f;
     const int li = threadIdx.x / LPP, sub = threadIdx.x % LPP;
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         const bool valid = li < tl.count;
         const int i = tl.start + (valid ? li : 0);
@@ -156,8 +173,8 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK) kb_correctio
     float4 *__restrict__ dst = par ? ppos0 : ppos1;
     float worst = 0.f;
     const int li = threadIdx.x / LPP, sub = threadIdx.x % LPP;
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         const bool valid = li < tl.count;
         const int i = tl.start + (valid ? li : 0);
@@ -167,15 +184,31 @@ __global__ void __launch_bounds__(BLOCK, FSPH_PASS_THREADS / BLOCK) kb_correctio
     correction_tail(lp, ctl, part, worst, par, hif, hif2, use_graph);
 }
 
-/* m / rho_i of every particle with its scene's mass, for the XSPH and
- * vorticity passes (FSPH_POST_PRE) */
+/* v = (x* - x) / dt, x = x* (rx_sph_pbd.cpp:464-471), id / attr back to the
+ * home buffers, and m / rho with the scene's mass for the XSPH and vorticity
+ * passes: one pass over the particles where k_finalize and a tiled m / rho pass
+ * took 51 and 58 us. */
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) kb_mrho(BatchArgs b, const float *__restrict__ dens,
-                                                 float *__restrict__ mrho) {
-    __shared__ DevParams s_p;
+__global__ void __launch_bounds__(BLOCK) kb_finalize(BatchArgs b, float inv_dt, const float4 *__restrict__ pos_b,
+                                                     const float4 *ppos0, const float4 *ppos1, const DevCtl *ctl,
+                                                     const unsigned int *__restrict__ id_b,
+                                                     const unsigned int *__restrict__ attr_b,
+                                                     float4 *__restrict__ pos_a, float4 *__restrict__ vel_a,
+                                                     unsigned int *__restrict__ id_a,
+                                                     unsigned int *__restrict__ attr_a,
+                                                     const float *__restrict__ dens, float *__restrict__ mrho) {
+    const float4 *pp = ctl->parity ? ppos1 : ppos0;
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
-        if ((int)threadIdx.x < tl.count) mrho[tl.start + threadIdx.x] = s_p.mass / dens[tl.start + threadIdx.x];
+        const BTile tl = b.tiles[t];
+        if ((int)threadIdx.x >= tl.count) continue;
+        const int i = tl.start + (int)threadIdx.x;
+        mrho[i] = __ldg(&b.scenes[tl.scene].mass) / dens[i];
+        const float3 xs = f3(pp[i]), x = f3(pos_b[i]);
+        const float3 v = inv_dt * (xs - x);
+        pos_a[i] = make_float4(xs.x, xs.y, xs.z, 0.0f);
+        vel_a[i] = make_float4(v.x, v.y, v.z, 0.0f);
+        id_a[i] = id_b[i];
+        attr_a[i] = attr_b[i];
     }
 }
 
@@ -189,8 +222,8 @@ __global__ void __launch_bounds__(BLOCK) kb_xsph_vort(BatchArgs b, const unsigne
                                                       const float *__restrict__ mrho, float2 *__restrict__ wm) {
     __shared__ DevParams s_p;
     const FeatureOut fo{};
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
             xsph_vort_body<false, FSPH_POST_PRE != 0>(p, tl.start + threadIdx.x, cell_start, pos, vel, dens, vel_out,
@@ -207,8 +240,8 @@ __global__ void __launch_bounds__(BLOCK) kb_vort_apply(BatchArgs b, const unsign
                                                        const unsigned char *__restrict__ cnt,
                                                       const float2 *__restrict__ wm) {
     __shared__ DevParams s_p;
-    for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-        const BTile tl = tile_begin(b, t, s_p);
+    for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
+        const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
             vort_apply_body<FSPH_POST_PRE != 0>(p, tl.start + threadIdx.x, cell_start, pos, vort, dens, vel_in,
@@ -216,35 +249,65 @@ __global__ void __launch_bounds__(BLOCK) kb_vort_apply(BatchArgs b, const unsign
     }
 }
 
-/* Per-scene density errors of the last lambda pass, one block per scene,
- * fixed-order: err[3 s + 0..2] = one-sided mean, two-sided mean, max. */
-__global__ void __launch_bounds__(256) kb_scene_errors(const int *__restrict__ offs, const DevParams *__restrict__ scenes,
-                                                       const float *__restrict__ dens, float *__restrict__ err) {
-    __shared__ double s1[8], s2[8];
-    __shared__ float sm[8];
-    const int s = blockIdx.x;
-    const int a = offs[s], e = offs[s + 1];
-    const float inv = scenes[s].inv_rest_dens;
+/* Density errors of the last lambda pass: the partial sums of each tile (one
+ * warp a tile, sums of floats with their rounding errors kept, so as exact as
+ * doubles: FP64 runs at 2 lanes a clock and SM), then one warp per scene adds
+ * its tiles' in order: err[3 s + 0..2] = one-sided mean, two-sided mean, max.
+ * One block a scene over its particles in double took 156 us, the largest
+ * scene's block alone at the end. */
+struct TileErr {
+    double s1, s2;
+    float mx, pad;
+};
+__device__ __forceinline__ void exact_add(float2 &s, float v) { /* s.x + s.y += v */
+    const float t = __fadd_rn(s.x, v), bb = __fsub_rn(t, s.x);
+    s.y = __fadd_rn(s.y, __fadd_rn(__fsub_rn(s.x, __fsub_rn(t, bb)), __fsub_rn(v, bb)));
+    s.x = t;
+}
+__global__ void __launch_bounds__(256) kb_tile_errors(BatchArgs b, const float *__restrict__ dens,
+                                                      TileErr *__restrict__ part) {
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= b.ntiles) return;
+    const BTile tl = b.tiles[t];
+    const float inv = __ldg(&b.scenes[tl.scene].inv_rest_dens);
+    float2 e1 = make_float2(0.f, 0.f), e2 = e1;
+    float m = 0.f;
+    for (int k = lane; k < tl.count; k += 32) {
+        const float C = dens[tl.start + k] * inv - 1.0f;
+        exact_add(e1, C > 0.0f ? C : 0.0f);
+        exact_add(e2, fabsf(C));
+        m = fmaxf(m, fabsf(C));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const float2 f1 = make_float2(__shfl_xor_sync(0xffffffffu, e1.x, o), __shfl_xor_sync(0xffffffffu, e1.y, o));
+        const float2 f2 = make_float2(__shfl_xor_sync(0xffffffffu, e2.x, o), __shfl_xor_sync(0xffffffffu, e2.y, o));
+        exact_add(e1, f1.x);
+        e1.y = __fadd_rn(e1.y, f1.y);
+        exact_add(e2, f2.x);
+        e2.y = __fadd_rn(e2.y, f2.y);
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
+    if (lane == 0) part[t] = TileErr{(double)e1.x + (double)e1.y, (double)e2.x + (double)e2.y, m, 0.f};
+}
+__global__ void __launch_bounds__(128) kb_scene_errors(int nscenes, const int *__restrict__ offs,
+                                                       const int *__restrict__ tile0, const TileErr *__restrict__ part,
+                                                       float *__restrict__ err) {
+    const int s = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (s >= nscenes) return;
     double e1 = 0.0, e2 = 0.0;
     float m = 0.f;
-    for (int i = a + (int)threadIdx.x; i < e; i += blockDim.x) {
-        const float C = dens[i] * inv - 1.0f;
-        e1 += C > 0.0f ? C : 0.0f;
-        e2 += fabsf(C);
-        m = fmaxf(m, fabsf(C));
+    for (int t = tile0[s] + lane; t < tile0[s + 1]; t += 32) {
+        e1 += part[t].s1;
+        e2 += part[t].s2;
+        m = fmaxf(m, part[t].mx);
     }
     for (int o = 16; o > 0; o >>= 1) {
         e1 += __shfl_xor_sync(0xffffffffu, e1, o);
         e2 += __shfl_xor_sync(0xffffffffu, e2, o);
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { s1[warp] = e1; s2[warp] = e2; sm[warp] = m; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        e1 = 0.0; e2 = 0.0; m = 0.f;
-        for (int w = 0; w < 8; ++w) { e1 += s1[w]; e2 += s2[w]; m = fmaxf(m, sm[w]); }
-        const double n = (double)(e > a ? e - a : 1);
+    if (lane == 0) {
+        const double n = (double)(offs[s + 1] > offs[s] ? offs[s + 1] - offs[s] : 1);
         err[3 * s + 0] = (float)(e1 / n);
         err[3 * s + 1] = (float)(e2 / n);
         err[3 * s + 2] = m;
@@ -285,8 +348,7 @@ struct BLaunch {
 void blaunch_predict_hash(const BLaunch &L, const float4 *pos, const float4 *vel, float4 *ppos_out,
                           unsigned int *key, unsigned int *rank, unsigned int *count, cudaStream_t s) {
     FSPH_BLOCK_SWITCH(L.block, {
-        auto k = kb_predict_hash<B_>;
-        k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, pos, vel, ppos_out, key, rank, count);
+        kb_predict_hash<B_><<<std::max(L.full.ntiles, 1), B_, 0, s>>>(L.full, pos, vel, ppos_out, key, rank, count);
     })
 }
 void blaunch_hash_parity(const BLaunch &L, const float4 *p0, const float4 *p1, const DevCtl *ctl, unsigned int *key,
@@ -323,14 +385,19 @@ unsigned int blaunch_correction(const BLaunch &L, const DevParams &lp, const uns
     }))
     return g;
 }
+void blaunch_finalize(const BLaunch &L, float inv_dt, const float4 *pos_b, const float4 *p0, const float4 *p1,
+                      const DevCtl *ctl, const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a,
+                      float4 *vel_a, unsigned int *id_a, unsigned int *attr_a, const float *dens, float *mrho,
+                      cudaStream_t s) {
+    FSPH_BLOCK_SWITCH(L.block, {
+        kb_finalize<B_><<<std::max(L.full.ntiles, 1), B_, 0, s>>>(L.full, inv_dt, pos_b, p0, p1, ctl, id_b, attr_b, pos_a, vel_a,
+                                                     id_a, attr_a, dens, mrho);
+    })
+}
 void blaunch_xsph_vort(const BLaunch &L, const unsigned int *cell_start, const float4 *pos, const float4 *vel,
                        const float *dens, float4 *vel_out, float4 *vort, const NbrLists &nl, cudaStream_t s,
                        float *mrho, float2 *wm) {
     FSPH_BLOCK_SWITCH(L.block, {
-        if (FSPH_POST_PRE) {
-            auto km = kb_mrho<B_>;
-            km<<<persistent_grid(km, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, dens, mrho);
-        }
         auto k = kb_xsph_vort<B_>;
         k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, cell_start, pos, vel, dens, vel_out, vort,
                                                                        nl.list, nl.cnt, mrho, wm);
@@ -377,6 +444,8 @@ struct fsph_batch {
     DevParams *d_scenes = nullptr;
     int *d_offs = nullptr;
     BTile *d_tiles_full = nullptr, *d_tiles_cons = nullptr;
+    int *d_tile0 = nullptr;       /* first full tile of each scene, nscenes + 1 */
+    TileErr *d_tile_err = nullptr;
     int nt_full = 0, nt_cons = 0, cap_tiles_full = 0, cap_tiles_cons = 0;
     DevCtl *ctl = nullptr, *ctl_host = nullptr;
     unsigned int *flag = nullptr; /* input-validation flag, pinned host memory */
@@ -439,6 +508,7 @@ void bfree(fsph_batch *b) {
     cudaFree(b->nl.list); cudaFree(b->nl.cnt); cudaFree(b->nl.cellb);
     cudaFree(b->count); cudaFree(b->cell_start); cudaFree(b->block_sums);
     cudaFree(b->d_scenes); cudaFree(b->d_offs); cudaFree(b->d_tiles_full); cudaFree(b->d_tiles_cons);
+    cudaFree(b->d_tile0); cudaFree(b->d_tile_err);
     cudaFree(b->ctl); cudaFree(b->epart); cudaFree(b->dpart); cudaFree(b->d_err);
     if (b->ctl_host) cudaFreeHost(b->ctl_host);
     if (b->flag) cudaFreeHost(b->flag);
@@ -486,8 +556,12 @@ int apply_config(fsph_batch *b, const fsph_batch_config &cfg, float dt) {
     FB_CUDA(b, cudaMemcpyAsync(b->d_scenes, h.data(), h.size() * sizeof(DevParams), cudaMemcpyHostToDevice, b->stream));
     std::vector<BTile> tf = make_tiles(b, cfg.block), tc = make_tiles(b, cfg.block / cfg.lanes);
     if ((int)tf.size() > b->cap_tiles_full) {
-        cudaFree(b->d_tiles_full);
+        cudaFree(b->d_tiles_full); cudaFree(b->d_tile_err);
+        b->d_tiles_full = nullptr;
+        b->d_tile_err = nullptr;
+        b->cap_tiles_full = 0;
         FB_TRY(balloc(b, &b->d_tiles_full, tf.size()));
+        FB_TRY(balloc(b, &b->d_tile_err, tf.size()));
         b->cap_tiles_full = (int)tf.size();
     }
     if ((int)tc.size() > b->cap_tiles_cons) {
@@ -495,6 +569,10 @@ int apply_config(fsph_batch *b, const fsph_batch_config &cfg, float dt) {
         FB_TRY(balloc(b, &b->d_tiles_cons, tc.size()));
         b->cap_tiles_cons = (int)tc.size();
     }
+    std::vector<int> first(b->nscenes + 1, 0);
+    for (const BTile &t : tf) ++first[t.scene + 1];
+    for (int k = 0; k < b->nscenes; ++k) first[k + 1] += first[k];
+    FB_CUDA(b, cudaMemcpyAsync(b->d_tile0, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     FB_CUDA(b, cudaMemcpyAsync(b->d_tiles_full, tf.data(), tf.size() * sizeof(BTile), cudaMemcpyHostToDevice, b->stream));
     FB_CUDA(b, cudaMemcpyAsync(b->d_tiles_cons, tc.data(), tc.size() * sizeof(BTile), cudaMemcpyHostToDevice, b->stream));
     b->nt_full = (int)tf.size();
@@ -576,11 +654,13 @@ void benqueue_pre(fsph_batch *b, const BLaunch &L, cudaStream_t s) {
 }
 
 void benqueue_post(fsph_batch *b, const BLaunch &L, const DevParams &lp, cudaStream_t s) {
-    launch_finalize(lp, b->pos[1], b->ppos[0], b->ppos[1], b->ctl, b->id[1], b->attr[1], b->pos[0], b->vel[0],
-                    b->id[0], b->attr[0], nullptr, nullptr, s);
+    blaunch_finalize(L, lp.inv_dt, b->pos[1], b->ppos[0], b->ppos[1], b->ctl, b->id[1], b->attr[1], b->pos[0],
+                     b->vel[0], b->id[0], b->attr[0], b->dens, b->mrho, s);
     blaunch_xsph_vort(L, b->cell_start, b->pos[0], b->vel[0], b->dens, b->vel[1], b->vort, b->nl, s, b->mrho, b->wm);
     blaunch_vort_apply(L, b->cell_start, b->pos[0], b->vort, b->dens, b->vel[1], b->vel[0], b->nl, s, b->wm);
-    kb_scene_errors<<<b->nscenes, 256, 0, s>>>(b->d_offs, b->d_scenes, b->dens, b->d_err);
+    kb_tile_errors<<<blocks_for(std::max(b->nt_full, 1), 8), 256, 0, s>>>(L.full, b->dens, b->d_tile_err);
+    kb_scene_errors<<<blocks_for(b->nscenes, 4), 128, 0, s>>>(b->nscenes, b->d_offs, b->d_tile0, b->d_tile_err,
+                                                             b->d_err);
 }
 
 int badd_conditional(fsph_batch *b, cudaGraph_t g, const cudaGraphNode_t *deps, size_t ndeps,
@@ -781,7 +861,7 @@ int fsph_batch_create(const fsph_params *params, const int *counts, int nscenes,
     A(&b->mrho, n); A(&b->wm, n);
     A(&b->key, n); A(&b->rank, n); A(&b->perm, n);
     A(&b->nl.list, n * kListMax); A(&b->nl.cnt, n); A(&b->nl.cellb, n);
-    A(&b->d_scenes, (size_t)nscenes); A(&b->d_offs, (size_t)nscenes + 1); A(&b->d_err, 3 * (size_t)nscenes);
+    A(&b->d_scenes, (size_t)nscenes); A(&b->d_offs, (size_t)nscenes + 1); A(&b->d_tile0, (size_t)nscenes + 1); A(&b->d_err, 3 * (size_t)nscenes);
     A(&b->ctl, 1);
     if (st != FSPH_OK) return bail(st);
     if (cudaMallocHost((void **)&b->ctl_host, sizeof(DevCtl)) != cudaSuccess) return bail(FSPH_OOM);
