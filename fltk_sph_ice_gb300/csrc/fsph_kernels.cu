@@ -662,56 +662,78 @@ void launch_boundary_lambda(const DevParams &p, const unsigned int *cell_start, 
  * the force pass's per-neighbour factors ride in the .w words of the sorted
  * copies: pos.w = p / rho^2, vel.w = 1 / rho.  Only .w words are written, so
  * the x, y, z the other threads read stay as they are. */
-__global__ void __launch_bounds__(kBlock) k_sph_density(DevParams p, const unsigned int *__restrict__ cell_start,
-                                                        float4 *pos, float4 *vel, float *__restrict__ dens,
-                                                        float *__restrict__ pres, ListEntry *__restrict__ list,
-                                                        unsigned char *__restrict__ cnt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    const float3 xi = f3(pos[i]);
-    const int3 c = cell_of(xi, p);
-    float acc = 0.0f;
-    int k = 0;
-    bool ovf = false;
-    ListEntry last = (ListEntry)i;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy) {
-            unsigned int s, e;
-            row_range(cell_start, c, dy, dz, p, s, e);
-            /* four candidates' loads in flight before their tests */
-            for (unsigned int j0 = s; j0 < e; j0 += 4) {
-                float4 xc[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) xc[u] = __ldg(pos + min(j0 + u, e - 1));
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (j0 + u >= e) break;
-                    const float3 d = xi - f3(xc[u]);
-                    const float r2 = dot3(d, d);
-                    if (r2 < p.h2) {
-                        const float q = p.h2 - r2;
-                        acc += q * q * q;
-                    }
-                    if (list && r2 < p.rl2) {
-                        last = (ListEntry)(j0 + u);
-                        if (k < kListMax) list[list_at(k, i, p.n)] = last;
-                        ++k;
-                    }
-                }
-            }
-        }
-    if (list) {
-        ovf = k > kListMax;
-        if (!ovf) /* pad the last group (k >= 1: the slot itself is always listed) */
-            for (int t = k; (t & 3) != 0; ++t) list[list_at(t, i, p.n)] = last;
-        cnt[i] = ovf ? kListOverflow : (unsigned char)k;
-    }
+__device__ __forceinline__ void sph_density_out(const DevParams &p, int i, float acc, float4 *pos, float4 *vel,
+                                                float *__restrict__ dens, float *__restrict__ pres) {
     const float rho = p.mass * p.aw * acc;
     const float prs = p.gas_k * (rho - p.rest_dens);
     dens[i] = rho;
     pres[i] = prs;
     reinterpret_cast<float *>(pos + i)[3] = prs / (rho * rho);
     reinterpret_cast<float *>(vel + i)[3] = 1.0f / rho;
+}
+/* A warp for 32 consecutive slots: its candidates from the tile
+ * (warp_candidates), each evaluated from a gathered position, four at a time,
+ * and listed; where they do not fit the tile, a thread's own walk.  A thread
+ * testing all its candidates was bound by issue and took 205 us at 1,030,301
+ * slots and 64.6 at 262,144, this form 171 and 59.5. */
+__global__ void __launch_bounds__(kListBlock) k_sph_density(DevParams p, const unsigned int *__restrict__ cell_start,
+                                                            float4 *pos, float4 *vel, float *__restrict__ dens,
+                                                            float *__restrict__ pres, ListEntry *__restrict__ list,
+                                                            unsigned char *__restrict__ cnt) {
+    __shared__ PairTile s_tile[kListBlock / 32];
+    PairTile &t = s_tile[threadIdx.x >> 5];
+    const int i = blockIdx.x * kListBlock + threadIdx.x;
+    const bool valid = i < p.n;
+    const float3 xi = valid ? f3(pos[i]) : make_float3(0.f, 0.f, 0.f);
+    const int3 c = cell_of(xi, p);
+    float acc[4] = {}; /* four partial sums: their error is no larger than that of the lanes' */
+    auto add = [&](float &sum, const float4 &xj) {
+        const float3 d = xi - f3(xj);
+        const float r2 = dot3(d, d);
+        if (r2 < p.h2) {
+            const float q = p.h2 - r2;
+            sum += q * q * q;
+        }
+        return r2;
+    };
+    warp_candidates(
+        p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.rl2, t,
+        [&](bool found, int count, TileWalk &walk) {
+            if (found) {
+                for (int k = 0; k < count; k += 4) {
+                    unsigned int v[4];
+                    float4 xj[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = walk.next(); /* the last group is padded with its last entry */
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) xj[u] = pos[v[u]];
+                    if (list && k < kListMax)
+                        reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
+                            make_uint4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (k + u < count) add(acc[u], xj[u]);
+                }
+            } else {
+                unsigned int last = (unsigned int)i;
+                count = 0;
+                for (int dz = -1; dz <= 1; ++dz)
+                    for (int dy = -1; dy <= 1; ++dy) {
+                        unsigned int s, e;
+                        row_range(cell_start, c, dy, dz, p, s, e);
+                        for (unsigned int j = s; j < e; ++j) {
+                            if (!(add(acc[0], pos[j]) < p.rl2)) continue;
+                            last = j;
+                            if (list && count < kListMax) list[list_at(count, i, p.n)] = last;
+                            ++count;
+                        }
+                    }
+                if (list && count <= kListMax) /* pad the last group (the slot itself is always listed) */
+                    for (int k = count; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = last;
+            }
+            if (list) cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
+            sph_density_out(p, i, (acc[0] + acc[1]) + (acc[2] + acc[3]), pos, vel, dens, pres);
+        });
 }
 
 /* k_sph_density with LPP lanes per particle, so that small scenes still
@@ -772,12 +794,7 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
             for (int u = k; (u & 3) != 0; ++u) list[list_at(u, i, p.n)] = (ListEntry)last;
         cnt[i] = ovf ? kListOverflow : (unsigned char)k;
     }
-    const float rho = p.mass * p.aw * acc;
-    const float prs = p.gas_k * (rho - p.rest_dens);
-    dens[i] = rho;
-    pres[i] = prs;
-    reinterpret_cast<float *>(pos + i)[3] = prs / (rho * rho);
-    reinterpret_cast<float *>(vel + i)[3] = 1.0f / rho;
+    sph_density_out(p, i, acc, pos, vel, dens, pres);
 }
 
 /* a_i = -sum_j m (p_i/rho_i^2 + p_j/rho_j^2) grad W_ij + mu sum_j m (v_j - v_i)
@@ -860,8 +877,8 @@ __device__ inline bool ref_neighbor(float3 xi, float3 xj, float h2) {
 /* Neighbour counts of a warp's 32 consecutive slots, in particle order
  * (cnt_p[id]), and the neighbours themselves in the list storage (up to
  * kListMax a slot; cnt = kListOverflow past that) for k_nb_rows: the search,
- * from the warp's tile (tile_masks, a hair wider than the radius), is done
- * once.  total: the sum over all slots. */
+ * from the warp's tile (warp_candidates, a hair wider than the radius), is
+ * done once.  total: the sum over all slots. */
 __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsigned int *__restrict__ cell_start,
                                                          const float4 *__restrict__ pos,
                                                          const unsigned int *__restrict__ id,
@@ -875,32 +892,28 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
     const bool valid = i < p.n;
     const float3 xi = valid ? f3(__ldg(pos + i)) : make_float3(0.f, 0.f, 0.f);
     const int3 c = cell_of(xi, p);
-    int found;
-    unsigned int some;
-    const bool ok = tile_masks(p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
-                               found, some);
     unsigned int k = 0;
-    if (valid) {
-        auto meet = [&](unsigned int j) {
-            if (ref_neighbor(xi, f3(__ldg(pos + j)), p.h2)) {
-                if (k < (unsigned int)kListMax) list[list_at((int)k, i, p.n)] = j;
-                ++k;
-            }
-        };
-        if (!ok) {
-            for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy) {
-                    unsigned int s, e;
-                    row_range(cell_start, c, dy, dz, p, s, e);
-                    for (unsigned int j = s; j < e; ++j) meet(j);
-                }
-        } else {
-            TileWalk walk(t, some);
-            for (int f = 0; f < found; ++f) meet(walk.next());
-        }
-        cnt_p[id[i]] = k;
-        cnt[i] = k > (unsigned int)kListMax ? kListOverflow : (unsigned char)k;
-    }
+    warp_candidates(p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
+                    [&](bool found, int count, TileWalk &walk) {
+                        auto meet = [&](unsigned int j) {
+                            if (ref_neighbor(xi, f3(__ldg(pos + j)), p.h2)) {
+                                if (k < (unsigned int)kListMax) list[list_at((int)k, i, p.n)] = j;
+                                ++k;
+                            }
+                        };
+                        if (found) {
+                            for (int f = 0; f < count; ++f) meet(walk.next());
+                        } else {
+                            for (int dz = -1; dz <= 1; ++dz)
+                                for (int dy = -1; dy <= 1; ++dy) {
+                                    unsigned int s, e;
+                                    row_range(cell_start, c, dy, dz, p, s, e);
+                                    for (unsigned int j = s; j < e; ++j) meet(j);
+                                }
+                        }
+                        cnt_p[id[i]] = k;
+                        cnt[i] = k > (unsigned int)kListMax ? kListOverflow : (unsigned char)k;
+                    });
     unsigned long long sum = k;
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total, sum);
@@ -1406,20 +1419,6 @@ void launch_vort_apply(const DevParams &p, const unsigned int *cell_start, const
     k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, pos, vort, dens, vel_in, vel_out,
                                                p.use_lists ? nl.list : nullptr, nl.cnt, wm);
 }
-static int lanes_to_fill(int n, int most);
-int sph_force_lanes(int n) { return lanes_to_fill(n, 8); }
-void launch_sph_density(const DevParams &p, const unsigned int *cell_start, float4 *pos, float4 *vel, float *dens,
-                        float *pres, const NbrLists &nl, cudaStream_t s) {
-    ListEntry *l = p.use_lists ? nl.list : nullptr;
-    const int lanes = FSPH_SPH_DENSITY_LANES ? sph_force_lanes(p.n) : 1;
-    const unsigned int g = blocks_for((long long)p.n * lanes);
-    switch (lanes) {
-    case 1: k_sph_density<<<g, kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt); break;
-    case 2: k_sph_density_lanes<2><<<g, kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt); break;
-    case 4: k_sph_density_lanes<4><<<g, kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt); break;
-    default: k_sph_density_lanes<8><<<g, kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt); break;
-    }
-}
 /* lanes per particle (a power of two, at most `most`): enough that the launch
  * holds about as many threads as the GPU keeps resident (1536 per SM) */
 static int lanes_to_fill(int n, int most) {
@@ -1432,6 +1431,25 @@ static int lanes_to_fill(int n, int most) {
     int lanes = 1;
     while (lanes < most && (long long)n * lanes < (long long)resident) lanes *= 2;
     return lanes;
+}
+static int sph_force_lanes(int n) { return lanes_to_fill(n, 8); }
+/* The density pass takes a warp's tile from here on, lanes of a particle's own
+ * candidates below, where a warp for 32 slots leaves SMs without work: at
+ * 15,625 slots the tile takes 22.5 us and 16 lanes 14.7, at 32,768 the tile and
+ * 8 lanes 22.7 each, at 64,000 29.1 and (4 lanes) 51.3.  With at most 8 lanes the
+ * pass took 16.4 us at 4,096 slots, with 32 it takes 8.2. */
+constexpr int kSphTileMin = 1 << 15;
+void launch_sph_density(const DevParams &p, const unsigned int *cell_start, float4 *pos, float4 *vel, float *dens,
+                        float *pres, const NbrLists &nl, cudaStream_t s) {
+    ListEntry *l = p.use_lists ? nl.list : nullptr;
+    if (p.n >= kSphTileMin) {
+        k_sph_density<<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
+        return;
+    }
+    const int lanes = lanes_to_fill(p.n, 32);
+    auto k = lanes >= 32 ? k_sph_density_lanes<32> : lanes >= 16 ? k_sph_density_lanes<16> : k_sph_density_lanes<8>;
+    const int lpp = std::max(lanes, 8);
+    k<<<blocks_for((long long)p.n * lpp), kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
 }
 void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,
                         float *dens, float *lambda, cudaStream_t s) {

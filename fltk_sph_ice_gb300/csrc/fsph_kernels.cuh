@@ -22,7 +22,7 @@ constexpr int kPassBlock = FSPH_PASS_BLOCK;
  * and a correction pass together: 31.0 -> 22.6 us at 6,912, 33.0 -> 27.7 at
  * 32,000, 43.1 -> 42.0 at 131,072, 71.4 -> 81.6 at 294,912 */
 constexpr int kDeepBlock = 64, kDeepMinB = 12, kDeepMax = 65536;
-constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 9.2 KB each */
+constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 8.7 KB each */
 constexpr int kBlockMax = 512;  /* largest block of the batched persistent kernels */
 constexpr int kScanTile = 4096; /* cells per block of the first scan phase */
 constexpr unsigned int kScanSum = 2048; /* tiles up to which the scan runs in two phases */
@@ -156,7 +156,6 @@ void launch_sph_density(const DevParams &p, const unsigned int *cell_start, floa
 /* acceleration from the lists and .w factors of launch_sph_density */
 void launch_sph_force(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vel,
                       float4 *acc, const NbrLists &nl, cudaStream_t s);
-int sph_force_lanes(int n);
 void launch_sph_integrate(const DevParams &p, const float4 *pos_b, const float4 *vel_b, const float4 *acc,
                           const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a, float4 *vel_a,
                           unsigned int *id_a, unsigned int *attr_a, cudaStream_t s);

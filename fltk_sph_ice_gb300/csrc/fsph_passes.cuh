@@ -310,27 +310,32 @@ __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const
 }
 
 /* The candidates of the 32 consecutive slots of a warp, searched together on
- * the tensor cores.  The slots lie in a run of three or four cells along x, so
- * in each of the nine rows of cells their candidates are one range of slots,
- * about 1.9 times what a lane's own three cells hold.  The warp takes 32 of
- * them at a time and computes all 32 x 32 values r^2 / rr^2 - 1 as products of
- * 16 terms (mma.m16n8k16): with coordinates relative to the warp, in units of
- * the radius and split into two halves of 11 bits each, r^2 = |xi|^2 + |xj|^2 -
- * 2 xi.xj needs the three products of the halves (their last, 2^-22, left out),
- * the two norms (split too) and the constant.  The error of a value is below
- * 1e-4 (coordinates of at most 5 in a run of six cells, sums of 16 terms below
- * 50), and the constant is 1 + 2^-12: every slot within the radius is found,
- * and one in some thousands that lies a hair beyond it, which a pass evaluates
- * to zero.  The signs shift into masks, eight candidates of four slots a lane,
- * which two shuffles turn into 32 candidates of one slot.
- * About 95 instructions for 32 x 32 tests.  Tested two at a time in packed
- * single precision they took 170 and the build 266 us at 1 M particles, a
- * thread walking its own cells 291 us, both bound by instruction issue; this
- * form takes 184 us, 18 instead of 33 us at 6,912 particles, and a batch step
- * went from 5,397 to 5,117 us. */
+ * the tensor cores.  The slots lie in a run of a few cells along x, so in each
+ * of the nine rows of cells their candidates are one range of slots, about 1.9
+ * times what a lane's own three cells hold.  The warp takes 32 of them at a
+ * time and computes all 32 x 32 values r^2 / rr^2 - 1 as products of 16 terms
+ * (mma.m16n8k16): with coordinates relative to the warp, in units of the radius
+ * and split into two halves of 11 bits each, r^2 = |xi|^2 + |xj|^2 - 2 xi.xj
+ * needs the three products of the halves (the last, 2^-22, left out), the two
+ * norms (split too) and the constant:
+ *
+ *   candidate  xh yh zh nh   xl yl zl nl   xh yh zh nh    1  1   1   1
+ *   slot      -2xh   ..  1  -2xh   ..  1  -2xl   ..  0   nh nl  -1  -2^-12
+ *
+ * The error of a value is below 1e-4 (coordinates of at most 6, sums of 16
+ * terms below 80) and the constant is 1 + 2^-12: every slot within the radius is
+ * found, and one in some thousands that lies a hair beyond it, which a pass
+ * evaluates to zero.  The signs shift into masks, eight candidates of four slots
+ * a lane, which two shuffles turn into 32 candidates of one slot.
+ * Tested two at a time in packed single precision 32 x 32 candidates took 170
+ * instructions and the list build 266 us at 1 M particles, a thread walking its
+ * own cells 291 us, both bound by instruction issue; this form takes 174 us, and
+ * 16 instead of 33 at 6,912 particles.  Without the walk over the
+ * masks and the rows' stores it takes 125, without the matrix instructions too 93:
+ * reading, converting and staging the candidates is what is left. */
 constexpr int kTileWords = 32; /* masks of a warp's candidates: 32 x 32 slots */
 struct __align__(16) PairTile {
-    uint4 k0[32], k1[32];               /* operand rows: the first and last eight of the 16 terms */
+    uint4 row[32];                      /* operand rows, eight terms each */
     unsigned int mask[kTileWords][32];  /* [w][lane], bit 31 - k: candidate k of word w is within the radius */
     unsigned int slot[kTileWords][32];  /* [w][k]: the candidates' slots */
 };
@@ -339,7 +344,29 @@ __device__ __forceinline__ unsigned int half_pair(float lo, float hi) {
     const __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const unsigned int *>(&v);
 }
-__device__ __forceinline__ float half_round(float v) { return __half2float(__float2half_rn(v)); }
+__device__ __forceinline__ float2 pair_floats(unsigned int v) {
+    return __half22float2(*reinterpret_cast<const __half2 *>(&v));
+}
+/* a point's terms: (xh, yh), (zh, nh) and the lower halves (xl, yl), (zl, nl) */
+struct PairTerms {
+    unsigned int h0, h1, l0, l1;
+    float nn;
+};
+__device__ __forceinline__ PairTerms pair_terms(float x, float y, float z) {
+    PairTerms t;
+    t.nn = x * x + y * y + z * z;
+    t.h0 = half_pair(x, y);
+    t.h1 = half_pair(z, t.nn);
+    const float2 a = pair_floats(t.h0), b = pair_floats(t.h1);
+    t.l0 = half_pair(x - a.x, y - a.y);
+    t.l1 = half_pair(z - b.x, t.nn - b.y);
+    return t;
+}
+/* both halves times -2 (exact) */
+__device__ __forceinline__ unsigned int times_m2(unsigned int v) {
+    const __half2 r = __hmul2(*reinterpret_cast<const __half2 *>(&v), __float2half2_rn(-2.0f));
+    return *reinterpret_cast<const unsigned int *>(&r);
+}
 __device__ __forceinline__ void load_matrices(unsigned int (&r)[4], const uint4 *row) {
     const unsigned int at = (unsigned int)__cvta_generic_to_shared(row);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -364,157 +391,184 @@ __device__ __forceinline__ void test_tile(unsigned int &m0, unsigned int &m1, un
     m1 = sign_in(sign_in(m1, d2), d3);
 }
 
-/* Fills t with the masks of the warp's slots (position xi, build cell `cell`,
- * cells ascending over the lanes; valid = false for padding lanes, after the
- * valid ones) against x4, within sqrt(r2max).  The candidates of one lane are
- * in ascending slot order.  count: how many this lane's slot has, some: bit
- * 31 - w set when word w holds any.  Returns false, for every lane of the
- * warp, when the candidates do not fit or a coordinate is out of the operands'
- * range (a particle far outside the box, or not a number).  Lanes in different
- * rows of cells, or more than six cells apart (a run that wraps, sparse fluid),
- * take turns: a row's range then never reaches the next row, and no slot is met
- * twice. */
-__device__ __forceinline__ bool tile_masks(const DevParams &p, const unsigned int *__restrict__ cell_start,
-                                           const float4 *__restrict__ x4, float3 xi, unsigned int cell, bool valid,
-                                           float r2max, PairTile &t, int &count, unsigned int &some) {
-    const int lane = threadIdx.x & 31;
-    const unsigned int row = (cell - p.cell_off) / (unsigned int)p.gx;
-    const float inv = rsqrtf(r2max);
-    /* operand B: candidate 8 q + 2 s + b is column 2 q + b of step s; the rows are
-     * stored so that neither the stores nor the loads of eight rows collide */
-    uint4 *const st0 = t.k0 + 8 * (lane >> 3) + 2 * ((lane >> 3) ^ ((lane >> 1) & 3)) + (lane & 1);
-    uint4 *const st1 = t.k1 + (st0 - t.k0);
-    const int lrow = 8 * ((lane & 7) >> 1) + 2 * (((lane & 7) >> 1) ^ (lane >> 3)) + (lane & 1);
-    const unsigned int pick1 = (lane & 2) ? 0x3726u : 0x5140u, pick2 = (lane & 1) ? 0x6273u : 0x0415u;
-    const int own = (lane >> 2) + 8 * (lane & 3); /* the slot whose 32 candidates this lane ends up with */
-    int cnt = 0;
-    unsigned int any = 0u;
-    bool bad = false;
-    unsigned int todo = __ballot_sync(0xffffffffu, valid);
-    int w = 0;
-    while (todo) {
-        const int lead = __ffs((int)todo) - 1;
-        const unsigned int lead_row = __shfl_sync(0xffffffffu, row, lead);
-        const unsigned int first = __shfl_sync(0xffffffffu, cell, lead);
-        const bool mine = (todo >> lane & 1u) && row == lead_row && cell - first <= 5u;
-        const unsigned int grp = __ballot_sync(0xffffffffu, mine);
-        const int tail = 31 - __clz((int)grp);
-        const unsigned int last = __shfl_sync(0xffffffffu, cell, tail);
-        todo &= ~grp;
-        const float ox = 0.5f * (__shfl_sync(0xffffffffu, xi.x, lead) + __shfl_sync(0xffffffffu, xi.x, tail));
-        const float oy = __shfl_sync(0xffffffffu, xi.y, lead), oz = __shfl_sync(0xffffffffu, xi.z, lead);
-        /* lane r < 9: row r's cells first - 1 .. last + 1 hold the slots from s on; the
-         * rows' candidates are numbered through, row r's from `from` on */
-        unsigned int s = 0u, len = 0u;
-        if (lane < 9) {
-            const int o = ((lane / 3 - 1) * p.gy + (lane % 3 - 1)) * p.gx;
-            const unsigned int a = (unsigned int)((int)first + o), b = (unsigned int)((int)last + o);
-            if (cell_row_ok(p, a) && cell_row_ok(p, b)) {
-                s = __ldg(cell_start + (a - 1u));
-                len = bounded(p, __ldg(cell_start + (b + 2u)), (unsigned int)p.n + 1u, kBoundSlot) - s;
-            }
-        }
-        unsigned int from = len;
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-            const unsigned int v = __shfl_up_sync(0xffffffffu, from, o);
-            if (lane >= o) from += v;
-        }
-        const unsigned int total = __shfl_sync(0xffffffffu, from, 8);
-        from -= len; /* lane 9 and on: the total */
-        const unsigned int shift = s - from;
-        if (total > (unsigned int)(kTileWords - w) * 32u) return false;
-        /* operand A: the warp's own slots */
-        __syncwarp(); /* the last operands of the group before have been read */
-        {
-            const float x = mine ? (xi.x - ox) * inv : 0.0f, y = mine ? (xi.y - oy) * inv : 0.0f,
-                        z = mine ? (xi.z - oz) * inv : 0.0f;
-            bad |= !(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= 8.0f) || !(x + y + z == x + y + z);
-            const float xh = half_round(x), yh = half_round(y), zh = half_round(z);
-            const float xl = half_round(x - xh), yl = half_round(y - yh), zl = half_round(z - zh);
-            const float nn = x * x + y * y + z * z, nh = half_round(nn);
-            t.k0[lane] = make_uint4(half_pair(-2.f * xh, -2.f * yh), half_pair(-2.f * zh, -2.f * xh),
-                                    half_pair(-2.f * yh, -2.f * zh), half_pair(-2.f * xl, -2.f * yl));
-            t.k1[lane] = make_uint4(half_pair(-2.f * zl, nh), half_pair(nn - nh, 1.0f), half_pair(1.0f, -1.0f),
-                                    half_pair(-0x1p-12f, 0.0f));
-        }
-        __syncwarp();
-        unsigned int a0[4], a1[4]; /* rows 0-7, 8-15, 16-23, 24-31; terms 0-7 and 8-15 */
-        load_matrices(a0, t.k0 + lane);
-        load_matrices(a1, t.k1 + lane);
-        int r = 0;
-#pragma unroll 1
-        for (unsigned int q0 = 0u; q0 < total; q0 += 32u, ++w) {
-            const unsigned int q = q0 + (unsigned int)lane;
-            unsigned int j = q + __shfl_sync(0xffffffffu, shift, r);
-            for (;;) { /* the rows that these 32 candidates reach into */
-                const unsigned int next = __shfl_sync(0xffffffffu, from, r + 1);
-                if (next >= q0 + 32u || r == 8) break;
-                ++r;
-                const unsigned int sh = __shfl_sync(0xffffffffu, shift, r);
-                if (q >= next) j = q + sh;
-            }
-            float x = 30.0f, y = 30.0f, z = 30.0f; /* past the last candidate: far away */
-            if (q < total) {
-                const float4 c = __ldg(x4 + j);
-                x = (c.x - ox) * inv;
-                y = (c.y - oy) * inv;
-                z = (c.z - oz) * inv;
-                bad |= !(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= 8.0f) || !(x + y + z == x + y + z);
-            }
-            const float xh = half_round(x), yh = half_round(y), zh = half_round(z);
-            const float nn = x * x + y * y + z * z, nh = half_round(nn);
-            const unsigned int xy = half_pair(xh, yh);
-            __syncwarp(); /* the operands of the last word have been read */
-            *st0 = make_uint4(xy, half_pair(zh, x - xh), half_pair(y - yh, z - zh), xy);
-            *st1 = make_uint4(half_pair(zh, 1.0f), half_pair(1.0f, nh), half_pair(nn - nh, 1.0f),
-                              half_pair(1.0f, 0.0f));
-            t.slot[w][lane] = j;
-            __syncwarp();
-            unsigned int b0[4], b1[4];
-            load_matrices(b0, t.k0 + lrow);
-            load_matrices(b1, t.k1 + lrow);
-            unsigned int m0 = 0u, m1 = 0u, m2 = 0u, m3 = 0u;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                test_tile(m0, m1, a0[0], a0[1], a1[0], a1[1], b0[k], b1[k]);
-                test_tile(m2, m3, a0[2], a0[3], a1[2], a1[3], b0[k], b1[k]);
-            }
-            /* byte k of lane c: candidates 8c .. 8c + 7 of slot g + 8k; the quad's four
-             * lanes exchange bytes until lane c has all of slot g + 8c */
-            unsigned int m = __byte_perm(__byte_perm(m0, m1, 0x0040), __byte_perm(m2, m3, 0x0040), 0x5410);
-            m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 2), pick1);
-            m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 1), pick2);
-            if (!(grp >> own & 1u)) m = 0u;
-            t.mask[w][own] = m;
-            cnt += __popc(m);
-            if (m) any |= 0x80000000u >> w;
-        }
-    }
-    __syncwarp();
-    const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
-    count = __shfl_sync(0xffffffffu, cnt, holder);
-    some = __shfl_sync(0xffffffffu, any, holder);
-    return !__any_sync(0xffffffffu, bad);
-}
-
-/* One lane's candidates of a tile, ascending: next() is called `count` times. */
+/* One lane's candidates of a tile, ascending.  next() gives the `left`-th from the
+ * end; called again after the last it keeps giving that one.  Selects instead of
+ * branches: at almost every call some lane of a warp opens its next word. */
 struct TileWalk {
     const PairTile &t;
     unsigned int some, m = 0u;
-    int w = 0;
-    __device__ __forceinline__ TileWalk(const PairTile &tile, unsigned int words) : t(tile), some(words) {}
+    int w = 0, left;
+    unsigned int last = 0u;
+    __device__ __forceinline__ TileWalk(const PairTile &tile, unsigned int words, int count)
+        : t(tile), some(words), left(count) {}
     __device__ __forceinline__ unsigned int next() {
-        if (m == 0u) {
-            w = __clz((int)some);
-            some ^= 0x80000000u >> w;
-            m = t.mask[w][threadIdx.x & 31];
-        }
-        const int b = __clz((int)m);
-        m ^= 0x80000000u >> b;
-        return t.slot[w][b];
+        const bool open = m == 0u;
+        const int wn = __clz((int)some) & 31;
+        const unsigned int mn = t.mask[wn][threadIdx.x & 31];
+        w = open ? wn : w;
+        m = open ? mn : m;
+        some = open ? some & ~(0x80000000u >> wn) : some;
+        const int b = __clz((int)m) & 31;
+        m &= ~(0x80000000u >> b);
+        const unsigned int j = t.slot[w][b];
+        last = left > 0 ? j : last;
+        --left;
+        return last;
     }
 };
+
+/* Calls emit(found, count, walk) once for each valid lane: found: the lane's
+ * `count` candidates against x4 within sqrt(r2max) come from walk, ascending;
+ * else they have to be looked for without the tile (more than fit it, or a
+ * coordinate out of the operands' range: a particle far outside the box, or not
+ * a number).  xi, cell: the lane's position and build cell, cells ascending over
+ * the lanes, padding lanes (valid = false) after the valid ones; every lane of
+ * the warp calls it.  Lanes in different rows of cells, or more than eight cells
+ * apart (a run that wraps, sparse fluid), take turns: a row's range then never
+ * reaches the next row, and no slot is met twice.  As many turns as fit the tile
+ * are emitted together. */
+template <class Emit>
+__device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
+                                                const float4 *__restrict__ x4, float3 xi, unsigned int cell,
+                                                bool valid, float r2max, PairTile &t, Emit &&emit) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int row = (cell - p.cell_off) / (unsigned int)p.gx;
+    const float inv = rsqrtf(r2max);
+    /* candidate 8 q + 2 s + b is column 2 q + b of step s; the rows are stored so
+     * that neither the stores nor the loads of eight rows collide */
+    uint4 *const st = t.row + 8 * (lane >> 3) + 2 * ((lane >> 3) ^ ((lane >> 1) & 3)) + (lane & 1);
+    const uint4 *const ld = t.row + 8 * ((lane & 7) >> 1) + 2 * (((lane & 7) >> 1) ^ (lane >> 3)) + (lane & 1);
+    const unsigned int pick1 = (lane & 2) ? 0x3726u : 0x5140u, pick2 = (lane & 1) ? 0x6273u : 0x0415u;
+    const unsigned int ones = 0x3c003c00u; /* (1, 1) */
+    const bool upper = (lane & 2) != 0;    /* terms 12-15 of a candidate are ones, 8-11 its terms 0-3 again */
+    const int own = (lane >> 2) + 8 * (lane & 3); /* the slot whose 32 candidates this lane ends up with */
+    unsigned int todo = __ballot_sync(0xffffffffu, valid);
+    while (todo) {
+        int cnt = 0, w = 0;
+        unsigned int any = 0u, done = 0u, over = 0u;
+        bool bad = false;
+        do { /* turns, until the tile is full */
+            const int lead = __ffs((int)todo) - 1;
+            const unsigned int lead_row = __shfl_sync(0xffffffffu, row, lead);
+            const unsigned int first = __shfl_sync(0xffffffffu, cell, lead);
+            const bool mine = (todo >> lane & 1u) && row == lead_row && cell - first <= 7u;
+            const unsigned int grp = __ballot_sync(0xffffffffu, mine);
+            const int tail = 31 - __clz((int)grp);
+            const unsigned int last = __shfl_sync(0xffffffffu, cell, tail);
+            /* lane r < 9: row r's cells first - 1 .. last + 1 hold the slots from s on; the
+             * rows' candidates are numbered through, row r's from `from` on */
+            unsigned int s = 0u, len = 0u;
+            if (lane < 9) {
+                const int o = ((lane / 3 - 1) * p.gy + (lane % 3 - 1)) * p.gx;
+                const unsigned int a = (unsigned int)((int)first + o), b = (unsigned int)((int)last + o);
+                if (cell_row_ok(p, a) && cell_row_ok(p, b)) {
+                    s = __ldg(cell_start + (a - 1u));
+                    len = bounded(p, __ldg(cell_start + (b + 2u)), (unsigned int)p.n + 1u, kBoundSlot) - s;
+                }
+            }
+            unsigned int from = len;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const unsigned int v = __shfl_up_sync(0xffffffffu, from, o);
+                if (lane >= o) from += v;
+            }
+            const unsigned int total = __shfl_sync(0xffffffffu, from, 8);
+            from -= len; /* lane 9 and on: the total */
+            const unsigned int shift = s - from;
+            if (total > (unsigned int)(kTileWords - w) * 32u) {
+                if (w) break; /* after what the tile holds now */
+                over = grp;   /* never fits */
+                done |= grp;
+                todo &= ~grp;
+                break;
+            }
+            done |= grp;
+            todo &= ~grp;
+            const float ox = 0.5f * (__shfl_sync(0xffffffffu, xi.x, lead) + __shfl_sync(0xffffffffu, xi.x, tail));
+            const float oy = __shfl_sync(0xffffffffu, xi.y, lead), oz = __shfl_sync(0xffffffffu, xi.z, lead);
+            unsigned int a0[4], a1[4]; /* the slots' terms: rows 0-7, 8-15, 16-23, 24-31; terms 0-7 and 8-15 */
+            {
+                const PairTerms v = mine ? pair_terms((xi.x - ox) * inv, (xi.y - oy) * inv, (xi.z - oz) * inv)
+                                         : PairTerms{0u, 0u, 0u, 0u, 0.0f};
+                bad |= !(v.nn <= 64.0f);
+                const unsigned int h0 = times_m2(v.h0), h1 = times_m2(v.h1), l0 = times_m2(v.l0), l1 = times_m2(v.l1);
+                const unsigned int z1 = (h1 & 0xffffu) | (ones & 0xffff0000u); /* (-2 zh, 1) */
+                __syncwarp(); /* the last operands of the turn before have been read */
+                t.row[lane] = make_uint4(h0, z1, h0, z1);
+                __syncwarp();
+                load_matrices(a0, t.row + lane);
+                __syncwarp();
+                t.row[lane] = make_uint4(l0, l1 & 0xffffu, __byte_perm(v.h1, v.l1, 0x7632),
+                                         half_pair(-1.0f, -0x1p-12f));
+                __syncwarp();
+                load_matrices(a1, t.row + lane);
+            }
+            const bool keep = (grp >> own & 1u) != 0u;
+            int r = 0;
+            /* this lane's candidate of the word from q0 on, its position on the way */
+            auto fetch = [&](unsigned int q0, unsigned int &j) {
+                const unsigned int q = q0 + (unsigned int)lane;
+                j = q + __shfl_sync(0xffffffffu, shift, r);
+                for (;;) { /* the rows that these 32 candidates reach into */
+                    const unsigned int next = __shfl_sync(0xffffffffu, from, r + 1);
+                    if (next >= q0 + 32u || r == 8) break;
+                    ++r;
+                    const unsigned int sh = __shfl_sync(0xffffffffu, shift, r);
+                    if (q >= next) j = q + sh;
+                }
+                /* past the last candidate: some slot's position, not used */
+                return __ldg(x4 + min(q < total ? j : j - (q - total + 1u), (unsigned int)p.n - 1u));
+            };
+            unsigned int jn;
+            float4 cn = fetch(0u, jn);
+#pragma unroll 1
+            for (unsigned int q0 = 0u; q0 < total; q0 += 32u, ++w) {
+                const unsigned int q = q0 + (unsigned int)lane, j = jn;
+                const float4 c = cn;
+                if (q0 + 32u < total) cn = fetch(q0 + 32u, jn);
+                PairTerms v{0x4f804f80u, 0x4f804f80u, 0u, 0u, 0.0f}; /* past the last candidate: 30 30 30, far away */
+                if (q < total) {
+                    v = pair_terms((c.x - ox) * inv, (c.y - oy) * inv, (c.z - oz) * inv);
+                } else {
+                    v.h1 = half_pair(30.0f, 2700.0f);
+                }
+                bad |= !(v.nn <= 64.0f);
+                __syncwarp(); /* the operands of the last word have been read */
+                *st = make_uint4(v.h0, v.h1, v.l0, v.l1);
+                t.slot[w][lane] = j;
+                __syncwarp();
+                unsigned int b[4];
+                load_matrices(b, ld);
+                unsigned int m0 = 0u, m1 = 0u, m2 = 0u, m3 = 0u;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const unsigned int b1 = upper ? ones : b[k];
+                    test_tile(m0, m1, a0[0], a0[1], a1[0], a1[1], b[k], b1);
+                    test_tile(m2, m3, a0[2], a0[3], a1[2], a1[3], b[k], b1);
+                }
+                /* byte k of lane c: candidates 8c .. 8c + 7 of slot g + 8k; the quad's four
+                 * lanes exchange bytes until lane c has all of slot g + 8c */
+                unsigned int m = __byte_perm(__byte_perm(m0, m1, 0x0040), __byte_perm(m2, m3, 0x0040), 0x5410);
+                m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 2), pick1);
+                m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 1), pick2);
+                if (!keep) m = 0u;
+                t.mask[w][own] = m;
+                cnt += __popc(m);
+                if (m) any |= 0x80000000u >> w;
+            }
+        } while (todo);
+        __syncwarp();
+        const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
+        const int count = __shfl_sync(0xffffffffu, cnt, holder);
+        const unsigned int some = __shfl_sync(0xffffffffu, any, holder);
+        const bool found = !over && !__any_sync(0xffffffffu, bad);
+        if (done >> lane & 1u) {
+            TileWalk walk(t, some, count);
+            emit(found, count, walk);
+        }
+        __syncwarp(); /* the tile is free again */
+    }
+}
 
 /* The lists of a warp's 32 consecutive slots (i ascending over the lanes,
  * padding lanes last).  The entries leave four at a time, one 16-byte store
@@ -526,28 +580,21 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
                                                 unsigned char *__restrict__ cnt, PairTile &t) {
     const float3 xi = valid ? f3(__ldg(xb + i)) : make_float3(0.f, 0.f, 0.f);
     const unsigned int cell = valid ? __ldg(cellb + i) : 0u;
-    int count;
-    unsigned int some;
-    const bool ok = tile_masks(p, cell_start, xb, xi, cell, valid, p.rl2, t, count, some);
-    if (!valid) return;
-    if (!ok) {
-        build_list_body(p, i, cell_start, xb, cell, list, cnt);
-        return;
-    }
-    TileWalk walk(t, some);
-    unsigned int last = 0u;
-    const int most = min(count, kListMax);
-    for (int k = 0; k < most; k += 4) {
-        unsigned int v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) { /* the last group is padded with its last entry */
-            if (k + u < most) last = walk.next();
-            v[u] = last;
+    warp_candidates(p, cell_start, xb, xi, cell, valid, p.rl2, t, [&](bool found, int count, TileWalk &walk) {
+        if (!found) {
+            build_list_body(p, i, cell_start, xb, cell, list, cnt);
+            return;
         }
-        reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
-            make_uint4(v[0], v[1], v[2], v[3]);
-    }
-    cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
+        const int most = min(count, kListMax);
+        for (int k = 0; k < most; k += 4) {
+            unsigned int v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = walk.next(); /* the last group is padded with its last entry */
+            reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
+                make_uint4(v[0], v[1], v[2], v[3]);
+        }
+        cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
+    });
 }
 
 /* ---------------- constraint iterations ---------------- */
