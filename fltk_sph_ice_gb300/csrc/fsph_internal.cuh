@@ -185,7 +185,7 @@ struct DevCtl {
     unsigned int mlp_err;       /* 1 when a tcgen05 inference gave up waiting on an MMA */
     float err1, err2, errmax;   /* errors of the last lambda pass */
     unsigned int bounds_bits;   /* FSPH_DEBUG_BOUNDS builds: the index checks that failed (kBound*) */
-    unsigned int grab, grab2;   /* FSPH_DYN_CHUNKS: chunks handed out on demand (lambda, correction pass) */
+    unsigned int grab;          /* chunks of the lambda pass handed out on demand */
     unsigned int loops;         /* launches of the one-kernel constraint loop in this step */
     unsigned int wait_err;      /* 1 when that loop gave up waiting for its blocks */
 };
@@ -196,6 +196,7 @@ struct LoopCtl {
     unsigned long long e1[3], e2[3]; /* error sums in units of 2^-32 */
     unsigned int em[3], disp[3];     /* largest |C| and |x* - xb|^2 (float bits) */
     unsigned int nan[3];             /* a density (of this iteration) or a position (of the one before) is not a number */
+    unsigned int grab[3], grab2[3];  /* slots handed out on demand (lambda, correction) */
     unsigned int arrived, left;      /* the grid barrier's and the last block's counters */
 };
 

@@ -405,7 +405,12 @@ __global__ void k_pbf_visc(DevParams p, const unsigned int *__restrict__ cell_st
 /* lambda pass: density, C, sum |grad C|^2 (with the k = i term), lambda
  * into x*.w, block partial errors; the last block reduces the errors in a
  * fixed order, advances the iteration counter and decides whether the
- * device-side loop continues. */
+ * device-side loop continues.
+ * As many blocks as are resident; each warp takes chunks of 32 slots, the first
+ * and all but the last whole round in turn, the rest on demand.  At 1 M particles
+ * 92 us as a plain grid, 82 round-robin, 78 with the leftovers on demand, 74 with
+ * one more round (81 with every chunk: the counter contends; that form took 30.6
+ * us at 221,184 particles, where there is one round, and takes 22.8 now). */
 template <bool KAHAN, bool DEEP>
 __global__ void __launch_bounds__(DEEP ? kDeepBlock : kPassBlock, DEEP ? kDeepMinB : FSPH_PASS_MINB) k_lambda(DevParams p, const unsigned int *__restrict__ cell_start,
                                                    float4 *ppos0, float4 *ppos1, float *__restrict__ dens,
@@ -415,16 +420,14 @@ __global__ void __launch_bounds__(DEEP ? kDeepBlock : kPassBlock, DEEP ? kDeepMi
                                                    const unsigned char *__restrict__ cnt) {
     const unsigned int par = *((volatile unsigned int *)&ctl->parity);
     float4 *pp = par ? ppos1 : ppos0;
-    /* persistent warps: whole round-robin rounds, then the leftover chunks
-     * on demand (DEEP: one chunk a warp, in order); the error sums are fixed
-     * point, exact in any order */
+    /* DEEP: one chunk a warp, in order */
     unsigned long long q1 = 0ull, q2 = 0ull;
     float em = 0.f;
     const int lane = threadIdx.x & 31, warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5), nchunks = (p.n + 31) >> 5;
-    const int stat = DEEP ? nchunks : max(nchunks / nw - FSPH_DYN_EXTRA, 0) * nw;
-    for (int c = DEEP ? warp : first_chunk(warp, stat, &ctl->grab, lane); c < nchunks;
-         c = DEEP ? nchunks : next_chunk(c, nw, stat, &ctl->grab, lane)) {
+    const int stat = max(nchunks / nw - 1, 1) * nw;
+    for (int c = warp; c < nchunks;
+         c = DEEP || stat >= nchunks ? nchunks : next_chunk(c, nw, stat, &ctl->grab, lane)) {
         const int i = c * 32 + lane;
         if (i < p.n) {
             const float C = lambda_body<1, KAHAN, DEEP>(p, cell_start, pp, dens, ctl, list, cnt, i, 0, true);

@@ -102,11 +102,11 @@ void launch_pbf_visc(const DevParams &p, const unsigned int *cell_start, const f
 void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1, float *dens,
                    DevCtl *ctl, ErrPartial *part, unsigned long long while_handle, int use_graph,
                    const NbrLists &nl, cudaStream_t s);
-/* The whole constraint loop of a small scene in one cooperative kernel
- * (fsph_loop.cu): iterations until the loop ends or a grid rebuild is due, then
- * the three conditions are set (post: the third exists).  loop_fits: p.n is at
- * most kLoopMax, lists are on, there is no boundary (its lambda is a kernel of
- * its own between the passes) and every block is resident at once. */
+/* The whole constraint loop in one cooperative kernel (fsph_loop.cu): iterations
+ * until the loop ends or a grid rebuild is due, then the three conditions are set
+ * (post: the third exists).  loop_fits: lists are on, there is no boundary (its
+ * lambda is a kernel of its own between the passes) and every block is resident at
+ * once.  Up to kLoopMax particles each has a thread of its own. */
 constexpr int kLoopMax = 65536;
 bool loop_fits(const DevParams &p);
 cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,

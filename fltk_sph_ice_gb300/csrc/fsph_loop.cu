@@ -1,18 +1,27 @@
 /*
- * fsph_loop.cu -- the constraint iterations of a small PBF scene in one
- * cooperative kernel.
+ * fsph_loop.cu -- the constraint iterations of a PBF step in one cooperative
+ * kernel, in two forms.
  *
  * A scene of up to kLoopMax particles leaves most of the GPU idle in a lambda
  * or correction launch: what an iteration costs is the chain of dependent
  * accesses of each launch (the loop state, the counts, list group after list
  * group and the positions behind each, the block partials and their last
- * block) and the launches themselves.  Here one launch keeps every particle on
+ * block) and the launches themselves.  k_pbf_loop keeps every particle on
  * its own thread for all iterations: its position and lambda stay in
  * registers, its list in shared memory (16-bit slots), so a pass is one round
  * of gathers, up to sixteen in flight, and a barrier over the grid.  Measured,
- * an iteration of 6,912 particles takes 12 us instead of 23.5 (31 before the
- * passes had their form for few warps), of 32,000 13.5 instead of 27.3; the
- * whole step of 6,912 (10 iterations, results read back) 360 -> 272 us.
+ * an iteration of 6,912 particles takes 12.3 us instead of 23.5 (31 before the
+ * passes had their form for few warps), of 32,000 13.3 instead of 27.3.
+ *
+ * From there on a launch of its own still costs each pass about 8 us (launch, a
+ * first round of loads with nothing to hide it, the last block's reduction).
+ * k_pbf_sweep runs the same passes from the lists in memory, over the slots
+ * that fit the GPU's threads at once and then the rest, with a barrier between
+ * them.  Measured, an iteration takes, in us, launches / sweep: 69,632
+ * particles 29.8 / 21.4, 131,072 35.8 / 24.9, 221,184 46.3 / 35.0, 262,144
+ * 55.7 / 49.6, 524,288 88.1 / 78.9, 1,048,576 148.7 / 137.5, 8,192,000 1010 /
+ * 998.  What bounds the passes is in fsph_passes.cuh: the L1 wavefronts of the
+ * gathers.
  *
  * The pair terms, their order and the order-free error sums are those of
  * k_lambda and k_correction (fsph_passes.cuh): the results are the same bit
@@ -28,9 +37,10 @@ namespace fsph {
 
 namespace {
 
-/* polls before a block gives the barrier up (about a second; a co-resident
- * grid needs a few) */
-constexpr unsigned int kLoopPolls = 1u << 21;
+/* polls before a block gives the barrier up: about two seconds, and as much
+ * again for each 65,536 particles (a co-resident grid needs a few; a scene that
+ * has collapsed into one cell may take long over a pass) */
+constexpr unsigned long long kLoopPolls = 1ull << 21;
 
 /* The grid barrier in two halves, so that what need not be done before the
  * other blocks go on is done while waiting for them.  Writes of the block
@@ -44,12 +54,17 @@ __device__ __forceinline__ void grid_arrive(LoopCtl *lc) {
         atomicAdd(&lc->arrived, 1u);
     }
 }
-__device__ __forceinline__ bool grid_wait(LoopCtl *lc, unsigned int want, int &s_ok) {
+__device__ __forceinline__ bool grid_wait(const DevParams &p, LoopCtl *lc, unsigned int want, int &s_ok) {
     if (threadIdx.x == 0) {
-        unsigned int seen = 0u, polls = 0u;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&lc->arrived) : "memory");
-        } while (seen < want && ++polls < kLoopPolls);
+        unsigned long long polls = kLoopPolls * (1ull + ((unsigned int)p.n >> 16));
+        unsigned int seen;
+        while (true) {
+            /* relaxed, and with a pause: an acquire would empty the SM's L1 at every
+             * poll, under the blocks that are still in their pass */
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&lc->arrived) : "memory");
+            if (seen >= want || --polls == 0ull) break;
+            __nanosleep(64);
+        }
         __threadfence();
         s_ok = seen >= want ? 1 : 0;
     }
@@ -96,6 +111,65 @@ __device__ __forceinline__ void for_each_kept(const DevParams &p, const unsigned
     }
 }
 
+/* One block's state of a launch, the same in every block (thread 0 decides for
+ * the block from sums that nobody writes any more). */
+struct LoopState {
+    unsigned int par, iter, cont, rebuild, at;
+    float md;
+};
+/* the next iteration's sums: last read before the barrier that ended the iteration
+ * before, next written after this one's first */
+__device__ __forceinline__ void loop_clear(LoopCtl *lc, unsigned int nx) {
+    lc->e1[nx] = lc->e2[nx] = 0ull;
+    lc->em[nx] = lc->disp[nx] = lc->nan[nx] = lc->grab[nx] = lc->grab2[nx] = 0u;
+}
+__device__ __forceinline__ void loop_add(LoopCtl *lc, unsigned int at, unsigned long long q1, unsigned long long q2,
+                                         float qm, float disp2) {
+    atomicAdd(&lc->e1[at], q1);
+    atomicAdd(&lc->e2[at], q2);
+    atomicMax(&lc->em[at], __float_as_uint(qm)); /* |C| >= 0: the bits order as the values */
+    atomicMax(&lc->disp[at], __float_as_uint(disp2));
+}
+/* continue (cont) and rebuild first (rebuild) after the iteration that s.iter
+ * counts up to; true: another iteration follows in this launch */
+__device__ __forceinline__ bool loop_decide(const DevParams &p, const LoopCtl *lc, LoopState &s) {
+    const unsigned long long e = __ldcg(p.error_mode ? &lc->e2[s.at] : &lc->e1[s.at]);
+    s.md = __uint_as_float(__ldcg(&lc->disp[s.at]));
+    const unsigned int bad = __ldcg(&lc->nan[s.at]);
+    const int it = (int)s.iter + 1, minit = p.min_iter > 1 ? p.min_iter : 1;
+    s.cont = it < p.max_iter && !bad;
+    if (s.cont && it >= minit) /* the mean in double, as lambda_tail_fix (two slow divisions: only when it decides) */
+        s.cont = !((float)((double)e * 0x1p-32 / (double)p.n) <= p.eta);
+    s.rebuild = (s.md > p.skin2 || !(s.md == s.md)) ? 1u : 0u;
+    return s.cont && !s.rebuild;
+}
+/* thread 0 of each block, last: the last block out leaves the step's loop state,
+ * and the counters for another launch */
+__device__ __forceinline__ void loop_leave(const DevParams &p, DevCtl *ctl, LoopCtl *lc, const LoopState &s, bool ok,
+                                           cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif,
+                                           cudaGraphConditionalHandle hif2, int post) {
+    if (!ok) ctl->wait_err = 1u;
+    __threadfence();
+    if (atomicAdd(&lc->left, 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    ctl->err1 = (float)((double)__ldcg(&lc->e1[s.at]) * 0x1p-32 / (double)p.n);
+    ctl->err2 = (float)((double)__ldcg(&lc->e2[s.at]) * 0x1p-32 / (double)p.n);
+    ctl->errmax = __uint_as_float(__ldcg(&lc->em[s.at]));
+    ctl->iter = s.iter;
+    ctl->done = s.cont ? 0u : 1u;
+    ctl->disp2_bits = __float_as_uint(s.md);
+    ctl->rebuild = s.rebuild;
+    ctl->parity = s.par;
+    ctl->loops += 1u;
+    lc->arrived = 0u;
+    lc->left = 0u;
+    for (unsigned int k = 0; k < 3u; ++k) loop_clear(lc, k);
+    const unsigned int cont = __ldcg(&ctl->wait_err) ? 0u : s.cont; /* a wait ran out: the step ends and reports it */
+    cudaGraphSetConditional(hwhile, cont);
+    cudaGraphSetConditional(hif, cont & s.rebuild);
+    if (post) cudaGraphSetConditional(hif2, s.rebuild);
+}
+
 template <bool KAHAN, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
     k_pbf_loop(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
@@ -108,13 +182,13 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
     __shared__ int s_ok, s_go;
     const int i = blockIdx.x * BLOCK + (int)threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool valid = i < p.n;
-    unsigned int par = *((volatile unsigned int *)&ctl->parity), iter = *((volatile unsigned int *)&ctl->iter);
+    LoopState st{*((volatile unsigned int *)&ctl->parity), *((volatile unsigned int *)&ctl->iter), 1u, 0u, 0u, 0.f};
     unsigned int *kept = s_kept + threadIdx.x;
     float3 xi = make_float3(0.f, 0.f, 0.f), xbi = xi;
     int k = 0;
     if (valid) {
         k = (int)cnt[i];
-        xi = f3((par ? ppos1 : ppos0)[i]);
+        xi = f3((st.par ? ppos1 : ppos0)[i]);
         xbi = f3(xb[i]);
         if (k != (int)kListOverflow) {
             const uint4 *lg = reinterpret_cast<const uint4 *>(list) + i;
@@ -129,19 +203,14 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
         }
     }
     const unsigned int nb = gridDim.x;
-    unsigned int want = 0u, cont = 1u, rebuild = 0u, at = 0u;
-    float md = 0.f, rho = 0.f;
+    unsigned int want = 0u;
+    float rho = 0.f;
     bool ok = true;
     while (true) {
-        float4 *pp = par ? ppos1 : ppos0, *dst = par ? ppos0 : ppos1;
-        const unsigned int nx = at == 2u ? 0u : at + 1u;
+        float4 *pp = st.par ? ppos1 : ppos0, *dst = st.par ? ppos0 : ppos1;
+        const unsigned int at = st.at, nx = at == 2u ? 0u : at + 1u;
+        if (blockIdx.x == 0 && threadIdx.x == 0) loop_clear(lc, nx);
         /* lambda of every particle, its error terms */
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            /* the next iteration's sums: last read before the barrier that ended the
-             * iteration before, next written after this one's first */
-            lc->e1[nx] = lc->e2[nx] = 0ull;
-            lc->em[nx] = lc->disp[nx] = lc->nan[nx] = 0u;
-        }
         float li = 0.f;
         unsigned long long q1 = 0ull, q2 = 0ull;
         float qm = 0.f;
@@ -165,7 +234,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
         qm = warp_max(qm);
         if (lane == 0) { s_e1[warp] = q1; s_e2[warp] = q2; s_em[warp] = qm; }
         want += nb;
-        if (!(ok = grid_wait(lc, want, s_ok))) break;
+        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
         /* corrections from every particle's lambda */
         float disp2 = 0.f;
         if (valid) {
@@ -192,59 +261,139 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
                 qm = fmaxf(qm, s_em[w]);
                 disp2 = fmaxf(disp2, s_d[w]);
             }
-            atomicAdd(&lc->e1[at], q1);
-            atomicAdd(&lc->e2[at], q2);
-            atomicMax(&lc->em[at], __float_as_uint(qm)); /* |C| >= 0: the bits order as the values */
-            atomicMax(&lc->disp[at], __float_as_uint(disp2));
+            loop_add(lc, at, q1, q2, qm, disp2);
         }
         grid_arrive(lc);
         want += nb;
-        if (!(ok = grid_wait(lc, want, s_ok))) break;
-        /* the loop's decisions, from the same numbers in every block (the sums and
-         * flags of this iteration, which nobody writes any more) */
-        if (threadIdx.x == 0) {
-            const unsigned long long e = __ldcg(p.error_mode ? &lc->e2[at] : &lc->e1[at]);
-            md = __uint_as_float(__ldcg(&lc->disp[at]));
-            const unsigned int bad = __ldcg(&lc->nan[at]);
-            const int it = (int)iter + 1, minit = p.min_iter > 1 ? p.min_iter : 1;
-            cont = it < p.max_iter && !bad;
-            if (cont && it >= minit) /* the mean in double, as lambda_tail_fix (two slow divisions: only when it decides) */
-                cont = !((float)((double)e * 0x1p-32 / (double)p.n) <= p.eta);
-            rebuild = (md > p.skin2 || !(md == md)) ? 1u : 0u;
-            s_go = cont && !rebuild;
-        }
+        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        if (threadIdx.x == 0) s_go = loop_decide(p, lc, st);
         __syncthreads();
-        ++iter;
-        par ^= 1u;
+        ++st.iter;
+        st.par ^= 1u;
         if (!s_go) break;
-        at = nx;
+        st.at = nx;
     }
     if (valid) dens[i] = rho;
-    if (threadIdx.x != 0) return;
-    if (!ok) ctl->wait_err = 1u;
-    __threadfence();
-    if (atomicAdd(&lc->left, 1u) != nb - 1u) return;
-    /* the last block out: the step's loop state, and the counters for another launch */
-    __threadfence();
-    ctl->err1 = (float)((double)__ldcg(&lc->e1[at]) * 0x1p-32 / (double)p.n);
-    ctl->err2 = (float)((double)__ldcg(&lc->e2[at]) * 0x1p-32 / (double)p.n);
-    ctl->errmax = __uint_as_float(__ldcg(&lc->em[at]));
-    ctl->iter = iter;
-    ctl->done = cont ? 0u : 1u;
-    ctl->disp2_bits = __float_as_uint(md);
-    ctl->rebuild = rebuild;
-    ctl->parity = par;
-    ctl->loops += 1u;
-    lc->arrived = 0u;
-    lc->left = 0u;
-    for (int s = 0; s < 3; ++s) {
-        lc->e1[s] = lc->e2[s] = 0ull;
-        lc->em[s] = lc->disp[s] = lc->nan[s] = 0u;
+    if (threadIdx.x == 0) loop_leave(p, ctl, lc, st, ok, hwhile, hif, hif2, post);
+}
+
+/* The same loop from the lists in memory, for scenes that do not fit k_pbf_loop:
+ * two blocks per SM of as many warps as there are chunks of 32 slots for, at most
+ * 24 (40 registers a thread).  A warp takes whole rounds in turn and the last two
+ * on demand, as k_lambda does.  Two large blocks, because each block's arrival and
+ * polls cost the barrier: an iteration at 1,048,576 particles took 150.4 us in
+ * blocks of 256, 142.4 of 512 and 138.2 of 768 (137.3 with the pause between
+ * polls), and with the same 768 threads at 131,072 particles, where 171 blocks
+ * leave the SMs uneven, 33.9 instead of 24.9. */
+constexpr int kSweepBlock = 768;
+template <bool KAHAN>
+__global__ void __launch_bounds__(kSweepBlock, 2)
+    k_pbf_sweep(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
+                float *__restrict__ dens, const float4 *__restrict__ xb, DevCtl *ctl, LoopCtl *lc,
+                cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hif2,
+                int post, const ListEntry *__restrict__ list, const unsigned char *__restrict__ cnt) {
+    __shared__ unsigned long long s_e1[kSweepBlock / 32], s_e2[kSweepBlock / 32];
+    __shared__ float s_em[kSweepBlock / 32], s_d[kSweepBlock / 32];
+    __shared__ int s_ok, s_go;
+    __shared__ LoopState st;
+    const int lane = threadIdx.x & 31, nchunks = (p.n + 31) >> 5;
+    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
+    const int stat = max(nchunks / nw - 1, 1) * nw;
+    if (threadIdx.x == 0)
+        st = LoopState{*((volatile unsigned int *)&ctl->parity), *((volatile unsigned int *)&ctl->iter), 1u, 0u, 0u, 0.f};
+    __syncthreads();
+    unsigned int want = 0u;
+    bool ok = true;
+    while (true) {
+        {
+            float4 *pp = st.par ? ppos1 : ppos0;
+            const unsigned int at = st.at;
+            if (blockIdx.x == 0 && threadIdx.x == 0) loop_clear(lc, at == 2u ? 0u : at + 1u);
+            unsigned long long q1 = 0ull, q2 = 0ull;
+            float qm = 0.f;
+            for (int c = warp; c < nchunks;
+                 c = stat >= nchunks ? nchunks : next_chunk(c, nw, stat, &lc->grab[at], lane)) {
+                const int i = c * 32 + lane;
+                if (i < p.n) {
+                    const float3 xi = f3(pp[i]);
+                    float rho, li;
+                    const float C = lambda_terms<1, KAHAN>(
+                        p, pp, xi,
+                        [&](auto &&load, auto &&f) {
+                            for_each_candidate<1>(p, cell_start, list, cnt, i, xi, 0, load, f);
+                        },
+                        rho, li);
+                    reinterpret_cast<float *>(pp + i)[3] = li;
+                    dens[i] = rho;
+                    if (!(rho == rho)) {
+                        ctl->nan_flag = 1u;
+                        lc->nan[at] = 1u;
+                    }
+                    q1 += err_fix(C > 0.0f ? C : 0.0f);
+                    q2 += err_fix(fabsf(C));
+                    qm = fmaxf(qm, fabsf(C));
+                }
+            }
+            q1 = warp_sum_u64(q1);
+            q2 = warp_sum_u64(q2);
+            qm = warp_max(qm);
+            if (lane == 0) { s_e1[threadIdx.x >> 5] = q1; s_e2[threadIdx.x >> 5] = q2; s_em[threadIdx.x >> 5] = qm; }
+        }
+        grid_arrive(lc);
+        want += gridDim.x;
+        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        {
+            const float4 *src = st.par ? ppos1 : ppos0;
+            float4 *dst = st.par ? ppos0 : ppos1;
+            const unsigned int at = st.at;
+            float disp2 = 0.f;
+            for (int c = warp; c < nchunks;
+                 c = stat >= nchunks ? nchunks : next_chunk(c, nw, stat, &lc->grab2[at], lane)) {
+                const int i = c * 32 + lane;
+                if (i < p.n) {
+                    const float4 xi4 = src[i];
+                    const float3 xi = f3(xi4);
+                    const float3 dp = correction_terms<1>(p, src, xi, xi4.w, [&](auto &&load, auto &&f) {
+                        for_each_candidate<1>(p, cell_start, list, cnt, i, xi, 0, load, f);
+                    });
+                    const float3 xn = solid_project(xi + dp, p);
+                    dst[i] = make_float4(xn.x, xn.y, xn.z, 0.0f);
+                    if (!(xn.x == xn.x && xn.y == xn.y && xn.z == xn.z)) {
+                        ctl->nan_flag = 1u;
+                        lc->nan[at == 2u ? 0u : at + 1u] = 1u; /* stops the loop at the next errors, as k_lambda does */
+                    }
+                    const float3 dd = xn - f3(xb[i]);
+                    disp2 = fmaxf(disp2, dot3(dd, dd));
+                }
+            }
+            disp2 = warp_max(disp2);
+            if (lane == 0) s_d[threadIdx.x >> 5] = disp2;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long q1 = 0ull, q2 = 0ull;
+            float qm = 0.f, disp2 = 0.f;
+            for (unsigned int w = 0; w < blockDim.x >> 5; ++w) {
+                q1 += s_e1[w];
+                q2 += s_e2[w];
+                qm = fmaxf(qm, s_em[w]);
+                disp2 = fmaxf(disp2, s_d[w]);
+            }
+            loop_add(lc, st.at, q1, q2, qm, disp2);
+        }
+        grid_arrive(lc);
+        want += gridDim.x;
+        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        if (threadIdx.x == 0) {
+            s_go = loop_decide(p, lc, st);
+            ++st.iter;
+            st.par ^= 1u;
+            if (s_go) st.at = st.at == 2u ? 0u : st.at + 1u;
+        }
+        __syncthreads();
+        if (!s_go) break;
     }
-    if (__ldcg(&ctl->wait_err)) cont = 0u; /* a wait ran out: the step ends and reports it */
-    cudaGraphSetConditional(hwhile, cont);
-    cudaGraphSetConditional(hif, cont & rebuild);
-    if (post) cudaGraphSetConditional(hif2, rebuild);
+    if (threadIdx.x == 0) loop_leave(p, ctl, lc, st, ok, hwhile, hif, hif2, post);
 }
 
 typedef void (*LoopKernel)(DevParams, const unsigned int *, float4 *, float4 *, float *, const float4 *, DevCtl *,
@@ -266,39 +415,47 @@ LoopShape loop_shape(const DevParams &p, int sms) {
     const bool kahan = p.compensated != 0;
     if (p.n <= 2 * sms * 64) return LoopShape{loop_kernel<64>(kahan), 64};
     if (p.n <= 2 * sms * 128) return LoopShape{loop_kernel<128>(kahan), 128};
-    return LoopShape{loop_kernel<256>(kahan), 256};
+    if (p.n <= kLoopMax) return LoopShape{loop_kernel<256>(kahan), 256};
+    /* two blocks per SM, as many warps in each as there are chunks for */
+    const int warps = blocks_for(p.n, 2 * sms * 32);
+    return LoopShape{kahan ? k_pbf_sweep<true> : k_pbf_sweep<false>, std::min(32 * warps, kSweepBlock)};
 }
 
 }  // namespace
 
-bool loop_fits(const DevParams &p) {
-    if (p.n <= 0 || p.n > kLoopMax || !p.use_lists || p.nb) return false;
+/* the launch's blocks, every one resident at once; 0: it cannot be launched so */
+static unsigned int loop_blocks(const DevParams &p, LoopShape &sh) {
     int dev = 0, sms = 0, coop = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
-        return false;
-    const LoopShape sh = loop_shape(p, sms);
+        return 0u;
+    sh = loop_shape(p, sms);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)sh.kernel, sh.block, 0) != cudaSuccess)
-        return false;
-    return (long long)per * sms * sh.block >= (long long)p.n; /* every block resident at once */
+        return 0u;
+    const unsigned int all = blocks_for(p.n, sh.block), room = (unsigned int)(per * sms);
+    if (p.n > kLoopMax) return std::min(all, std::min(room, 2u * (unsigned int)sms));
+    return all <= room ? all : 0u;
+}
+
+bool loop_fits(const DevParams &p) {
+    LoopShape sh;
+    return p.n > 0 && p.use_lists && !p.nb && loop_blocks(p, sh) > 0u;
 }
 
 cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                             float *dens, const float4 *xb, DevCtl *ctl, LoopCtl *lc, unsigned long long while_handle,
                             unsigned long long if_handle, unsigned long long if_handle2, int post, const NbrLists &nl,
                             cudaStream_t s) {
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const LoopShape sh = loop_shape(p, sms);
+    LoopShape sh;
+    const unsigned int blocks = loop_blocks(p, sh);
+    if (!blocks) return cudaErrorCooperativeLaunchTooLarge;
     DevParams q = p;
     cudaGraphConditionalHandle hw = while_handle, h1 = if_handle, h2 = if_handle2;
     const ListEntry *list = nl.list;
     const unsigned char *cnt = nl.cnt;
     void *args[] = {&q, &cell_start, &ppos0, &ppos1, &dens, &xb, &ctl, &lc, &hw, &h1, &h2, &post, &list, &cnt};
-    return cudaLaunchCooperativeKernel((const void *)sh.kernel, dim3(blocks_for(p.n, sh.block)), dim3(sh.block), args,
-                                       0, s);
+    return cudaLaunchCooperativeKernel((const void *)sh.kernel, dim3(blocks), dim3(sh.block), args, 0, s);
 }
 
 }  // namespace fsph

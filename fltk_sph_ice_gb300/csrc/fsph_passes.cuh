@@ -47,40 +47,6 @@ constexpr int kBatch = FSPH_KBATCH;
 #ifndef FSPH_FOLD
 #define FSPH_FOLD 1
 #endif
-/* FSPH_PERSIST_LAMBDA / FSPH_PERSIST_CORRECTION 1: that single-scene
- * constraint pass runs as many blocks as are resident on the GPU, each warp
- * taking 32-slot chunks round-robin (FSPH_PERSIST sets both).  Measured on
- * the 1M double dam break: lambda 92 -> 82 us with identical results, so on
- * by default; the correction pass gets slower (90 -> 95 us, warm step 2.855
- * -> 2.917 ms), so off. */
-#ifdef FSPH_PERSIST
-#define FSPH_PERSIST_LAMBDA FSPH_PERSIST
-#define FSPH_PERSIST_CORRECTION FSPH_PERSIST
-#endif
-/* FSPH_DYN_CHUNKS 1 (default): the persistent passes take their last
- * chunks on demand (an atomic counter per pass) instead of round-robin, so
- * warps that finish early take the leftovers; the lambda pass then sums its
- * errors in 64-bit fixed point (units of 2^-32), which is exact and so
- * independent of which warp ran which chunk.  FSPH_DYN_EXTRA whole rounds
- * join the leftovers in the on-demand pool.  Measured on the 1M double dam
- * break (same positions bit for bit): lambda 78.1 -> 75.6 us with the
- * leftovers alone, 73.7 us with one more round (default), 75 / 76 us with
- * two / three, 81 us with every chunk on demand (the counter contends);
- * the correction pass made persistent this way got slower (86 -> 92 us) and
- * stays a plain grid. */
-#ifndef FSPH_DYN_CHUNKS
-#define FSPH_DYN_CHUNKS 1
-#endif
-#ifndef FSPH_DYN_EXTRA
-#define FSPH_DYN_EXTRA 1
-#endif
-#ifndef FSPH_PERSIST_LAMBDA
-#define FSPH_PERSIST_LAMBDA 1
-#endif
-#ifndef FSPH_PERSIST_CORRECTION
-#define FSPH_PERSIST_CORRECTION 0
-#endif
-
 /* Neighbour-list loads do not allocate in L1 (ld.global.nc.L1::no_allocate):
  * a pass streams ≈ 160 B of list per particle once, while the gathered
  * positions (16 B per particle, each read ≈ 40 times per pass) keep L1 to
@@ -769,17 +735,13 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-/* the next chunk of a persistent pass: round-robin while whole rounds last,
- * then on demand from the pass's counter (warp-uniform) */
+/* The next 32 slots of a persistent pass (warp-uniform): round-robin while whole
+ * rounds last (stat), the rest on demand, so that warps that finish early take the
+ * leftovers; the error sums are fixed point (units of 2^-32), exact and so
+ * independent of which warp ran which chunk. */
 __device__ __forceinline__ int next_chunk(int c, int nw, int stat, unsigned int *ctr, int lane) {
     c += nw;
     if (c < stat) return c;
-    unsigned int v = 0u;
-    if (lane == 0) v = atomicAdd(ctr, 1u);
-    return stat + (int)__shfl_sync(0xffffffffu, v, 0);
-}
-__device__ __forceinline__ int first_chunk(int w, int stat, unsigned int *ctr, int lane) {
-    if (w < stat) return w;
     unsigned int v = 0u;
     if (lane == 0) v = atomicAdd(ctr, 1u);
     return stat + (int)__shfl_sync(0xffffffffu, v, 0);
@@ -988,7 +950,6 @@ __device__ __forceinline__ void correction_tail(const DevParams &lp, DevCtl *ctl
         ctl->rebuild = rb;
         ctl->parity = 1u - par;
         ctl->ticket2 = 0u;
-        ctl->grab2 = 0u;
         if (use_graph & 1) {
             unsigned int more = ctl->done ? 0u : 1u;
             cudaGraphSetConditional(hif, rb & more);

@@ -1,8 +1,7 @@
-"""The one-kernel constraint loop of small PBF scenes (a graph step without a
-boundary, up to 65,536 particles) against the host-driven loop of separate
-passes (use_graph = 0): the same positions, velocities, densities, iteration
-counts, errors and grid builds bit for bit, at block edges and on both sides of
-every size at which the launch shape changes."""
+"""The one-kernel constraint loop (a graph step without a boundary) against the
+host-driven loop of separate passes (use_graph = 0): the same positions,
+velocities, densities, iteration counts, errors and grid builds bit for bit, at
+block edges and on both sides of every size at which the launch shape changes."""
 import threading
 
 import numpy as np
@@ -108,3 +107,27 @@ def test_contexts_step_side_by_side(gpu):
         t.join()
     for g in got:
         assert g[0] == want[0] and all(np.array_equal(a, b) for a, b in zip(g[1], want[1]))
+
+
+@pytest.mark.parametrize("n", [69632, 155649, 233473, 300007, 500001])
+def test_swept_scenes(gpu, n):
+    """More particles than the loop keeps on threads of their own: less than one
+    round of the resident warps, one and a little, more, a ragged last chunk."""
+    p, x, v = _state(n, n)
+    p.eta, p.min_iter, p.max_iter, p.error_mode = 0.0, 2, 4, abi.ERR_TWO_SIDED
+    assert [r[0] for r in _same(p, x, v)] == [4, 4]
+
+
+@pytest.mark.parametrize("kahan", [0, 1])
+def test_swept_scene_with_rebuilds_and_overflowed_lists(gpu, kahan):
+    p, x, v = _state(80000, 9, squeeze=0.72)
+    p.eta, p.min_iter, p.max_iter, p.cell_skin, p.compensated_density = 0.0, 2, 12, 0.03, kahan
+    rec = _same(p, x, v, 3)
+    assert max(r[1] for r in rec) > 2
+
+
+@pytest.mark.parametrize("mode", [abi.ERR_ONE_SIDED, abi.ERR_TWO_SIDED])
+def test_swept_scene_stops_at_its_tolerance(gpu, mode):
+    p, x, v = _state(90000, 5)
+    p.error_mode, p.min_iter, p.max_iter, p.eta = mode, 2, 60, 5e-3 if mode == abi.ERR_ONE_SIDED else 5e-2
+    _same(p, x, v, 2)
