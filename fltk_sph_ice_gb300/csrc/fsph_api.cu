@@ -77,8 +77,7 @@ struct fsph_ctx {
     BufSet set[2];
     float4 *ppos[2] = {nullptr, nullptr};
     float4 *xb = nullptr, *acc = nullptr, *vort = nullptr;
-    float *mrho = nullptr;  /* m / rho per particle, for the XSPH and vorticity passes */
-    float2 *wm = nullptr;   /* (|omega|, m / rho) per particle, from the XSPH pass to the vorticity pass */
+    float *mag = nullptr;   /* |omega| per particle, from the XSPH pass to the vorticity pass */
     float *dens = nullptr, *pres = nullptr;
     unsigned int *key = nullptr, *rank = nullptr, *perm = nullptr;
     NbrLists nl;
@@ -309,9 +308,8 @@ void free_particles(fsph_ctx *c) {
     c->xpred = c->dstep = c->dwarm = c->tmp4 = nullptr;
     c->feat = nullptr;
     c->xb = c->acc = c->vort = nullptr;
-    cudaFree(c->mrho); cudaFree(c->wm);
-    c->mrho = nullptr;
-    c->wm = nullptr;
+    cudaFree(c->mag);
+    c->mag = nullptr;
     c->dens = c->pres = nullptr;
     c->key = c->rank = c->perm = nullptr;
     c->epart = nullptr;
@@ -580,7 +578,7 @@ int alloc_particles(fsph_ctx *c, int cap) {
         FSPH_TRY(dalloc(c, &c->ppos[k], n));
     }
     FSPH_TRY(dalloc(c, &c->xb, n)); FSPH_TRY(dalloc(c, &c->acc, n)); FSPH_TRY(dalloc(c, &c->vort, n));
-    FSPH_TRY(dalloc(c, &c->mrho, n)); FSPH_TRY(dalloc(c, &c->wm, n));
+    FSPH_TRY(dalloc(c, &c->mag, n));
     FSPH_TRY(dalloc(c, &c->dens, n)); FSPH_TRY(dalloc(c, &c->pres, n));
     FSPH_TRY(dalloc(c, &c->key, n)); FSPH_TRY(dalloc(c, &c->rank, n)); FSPH_TRY(dalloc(c, &c->perm, n));
     FSPH_TRY(dalloc(c, &c->res_id, n));
@@ -768,10 +766,12 @@ int enqueue_pbf_pre(fsph_ctx *c, const DevParams &p, cudaStream_t s) {
 
 void enqueue_pbf_post(fsph_ctx *c, const DevParams &p, int it, cudaStream_t s) {
     const bool ws = pbf_warm_active(c);
-    const bool ext = pbf_finalize_ext(c), pre = ext && FSPH_POST_PRE;
+    const bool ext = pbf_finalize_ext(c);
+    /* the build positions are not read again before the next build: their place
+     * takes x* with m / rho, for the passes below */
     launch_finalize(p, c->set[it].pos, c->ppos[0], c->ppos[1], c->ctl, c->set[it].id, c->set[it].attr,
                     c->set[0].pos, c->set[0].vel, c->set[0].id, c->set[0].attr, ws ? c->xpred : nullptr,
-                    ws ? c->dstep : nullptr, s, c->dens, pre ? c->mrho : nullptr);
+                    ws ? c->dstep : nullptr, s, c->dens, ext ? c->xb : nullptr);
     if (ext) {
         FeatureOut fo;
         if (ws) {
@@ -783,10 +783,8 @@ void enqueue_pbf_post(fsph_ctx *c, const DevParams &p, int it, cudaStream_t s) {
             fo.ctl = c->ctl;
             fo.valid = c->warm_valid;
         }
-        launch_xsph_vort(p, c->cell_start, c->set[0].pos, c->set[0].vel, c->dens, c->set[1].vel, c->vort, fo, c->nl,
-                         s, pre ? c->mrho : nullptr, pre ? c->wm : nullptr);
-        launch_vort_apply(p, c->cell_start, c->set[0].pos, c->vort, c->dens, c->set[1].vel, c->set[0].vel, c->nl, s,
-                          pre ? c->wm : nullptr);
+        launch_xsph_vort(p, c->cell_start, c->xb, c->set[0].vel, c->dens, c->set[1].vel, c->vort, fo, c->nl, s, c->mag);
+        launch_vort_apply(p, c->cell_start, c->xb, c->vort, c->dens, c->set[1].vel, c->set[0].vel, c->nl, s, c->mag);
     }
 }
 

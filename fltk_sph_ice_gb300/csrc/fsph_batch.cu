@@ -196,16 +196,16 @@ __global__ void __launch_bounds__(BLOCK) kb_finalize(BatchArgs b, float inv_dt, 
                                                      float4 *__restrict__ pos_a, float4 *__restrict__ vel_a,
                                                      unsigned int *__restrict__ id_a,
                                                      unsigned int *__restrict__ attr_a,
-                                                     const float *__restrict__ dens, float *__restrict__ mrho) {
+                                                     const float *__restrict__ dens, float4 *__restrict__ xm) {
     const float4 *pp = ctl->parity ? ppos1 : ppos0;
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const BTile tl = b.tiles[t];
         if ((int)threadIdx.x >= tl.count) continue;
         const int i = tl.start + (int)threadIdx.x;
-        mrho[i] = __ldg(&b.scenes[tl.scene].mass) / dens[i];
         const float3 xs = f3(pp[i]), x = f3(pos_b[i]);
         const float3 v = inv_dt * (xs - x);
         pos_a[i] = make_float4(xs.x, xs.y, xs.z, 0.0f);
+        xm[i] = make_float4(xs.x, xs.y, xs.z, __ldg(&b.scenes[tl.scene].mass) / dens[i]);
         vel_a[i] = make_float4(v.x, v.y, v.z, 0.0f);
         id_a[i] = id_b[i];
         attr_a[i] = attr_b[i];
@@ -219,15 +219,15 @@ __global__ void __launch_bounds__(BLOCK) kb_xsph_vort(BatchArgs b, const unsigne
                                                       float4 *__restrict__ vort,
                                                       const ListEntry *__restrict__ list,
                                                       const unsigned char *__restrict__ cnt,
-                                                      const float *__restrict__ mrho, float2 *__restrict__ wm) {
+                                                      float *__restrict__ mag) {
     __shared__ DevParams s_p;
     const FeatureOut fo{};
     for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
         const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
-            xsph_vort_body<false, FSPH_POST_PRE != 0>(p, tl.start + threadIdx.x, cell_start, pos, vel, dens, vel_out,
-                                                      vort, fo, list, cnt, mrho, wm);
+            xsph_vort_body<false, false, true>(p, tl.start + threadIdx.x, cell_start, pos, vel, dens, vel_out,
+                                                      vort, fo, list, cnt, mag);
     }
 }
 
@@ -238,14 +238,14 @@ __global__ void __launch_bounds__(BLOCK) kb_vort_apply(BatchArgs b, const unsign
                                                        const float4 *__restrict__ vel_in, float4 *__restrict__ vel_out,
                                                        const ListEntry *__restrict__ list,
                                                        const unsigned char *__restrict__ cnt,
-                                                      const float2 *__restrict__ wm) {
+                                                      const float *__restrict__ mag) {
     __shared__ DevParams s_p;
     for (int t = tile_first(b), e = tile_last(b), scene = -1; t < e; ++t) {
         const BTile tl = tile_begin(b, t, s_p, scene);
         const DevParams p = s_p;
         if ((int)threadIdx.x < tl.count)
-            vort_apply_body<FSPH_POST_PRE != 0>(p, tl.start + threadIdx.x, cell_start, pos, vort, dens, vel_in,
-                                                vel_out, list, cnt, wm);
+            vort_apply_body<true>(p, tl.start + threadIdx.x, cell_start, pos, vort, dens, vel_in,
+                                                vel_out, list, cnt, mag);
     }
 }
 
@@ -387,29 +387,29 @@ unsigned int blaunch_correction(const BLaunch &L, const DevParams &lp, const uns
 }
 void blaunch_finalize(const BLaunch &L, float inv_dt, const float4 *pos_b, const float4 *p0, const float4 *p1,
                       const DevCtl *ctl, const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a,
-                      float4 *vel_a, unsigned int *id_a, unsigned int *attr_a, const float *dens, float *mrho,
+                      float4 *vel_a, unsigned int *id_a, unsigned int *attr_a, const float *dens, float4 *xm,
                       cudaStream_t s) {
     FSPH_BLOCK_SWITCH(L.block, {
         kb_finalize<B_><<<std::max(L.full.ntiles, 1), B_, 0, s>>>(L.full, inv_dt, pos_b, p0, p1, ctl, id_b, attr_b, pos_a, vel_a,
-                                                     id_a, attr_a, dens, mrho);
+                                                     id_a, attr_a, dens, xm);
     })
 }
 void blaunch_xsph_vort(const BLaunch &L, const unsigned int *cell_start, const float4 *pos, const float4 *vel,
                        const float *dens, float4 *vel_out, float4 *vort, const NbrLists &nl, cudaStream_t s,
-                       float *mrho, float2 *wm) {
+                       float *mag) {
     FSPH_BLOCK_SWITCH(L.block, {
         auto k = kb_xsph_vort<B_>;
         k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, cell_start, pos, vel, dens, vel_out, vort,
-                                                                       nl.list, nl.cnt, mrho, wm);
+                                                                       nl.list, nl.cnt, mag);
     })
 }
 void blaunch_vort_apply(const BLaunch &L, const unsigned int *cell_start, const float4 *pos, const float4 *vort,
                         const float *dens, const float4 *vel_in, float4 *vel_out, const NbrLists &nl, cudaStream_t s,
-                        const float2 *wm) {
+                        const float *mag) {
     FSPH_BLOCK_SWITCH(L.block, {
         auto k = kb_vort_apply<B_>;
         k<<<persistent_grid(k, B_, L.full.ntiles, L.sms), B_, 0, s>>>(L.full, cell_start, pos, vort, dens, vel_in,
-                                                                       vel_out, nl.list, nl.cnt, wm);
+                                                                       vel_out, nl.list, nl.cnt, mag);
     })
 }
 
@@ -433,8 +433,7 @@ struct fsph_batch {
     float4 *ppos[2] = {nullptr, nullptr};
     float4 *xb = nullptr, *vort = nullptr, *tmp4 = nullptr;
     float *dens = nullptr, *tdens = nullptr;
-    float *mrho = nullptr;  /* m / rho per particle (XSPH and vorticity passes) */
-    float2 *wm = nullptr;   /* (|omega|, m / rho) per particle */
+    float *mag = nullptr;   /* |omega| per particle */
     unsigned int *key = nullptr, *rank = nullptr, *perm = nullptr;
     NbrLists nl;
     /* grid */
@@ -503,7 +502,7 @@ void bfree(fsph_batch *b) {
         cudaFree(b->pos[k]); cudaFree(b->vel[k]); cudaFree(b->id[k]); cudaFree(b->attr[k]); cudaFree(b->ppos[k]);
     }
     cudaFree(b->xb); cudaFree(b->vort); cudaFree(b->tmp4); cudaFree(b->dens); cudaFree(b->tdens);
-    cudaFree(b->mrho); cudaFree(b->wm);
+    cudaFree(b->mag);
     cudaFree(b->key); cudaFree(b->rank); cudaFree(b->perm);
     cudaFree(b->nl.list); cudaFree(b->nl.cnt); cudaFree(b->nl.cellb);
     cudaFree(b->count); cudaFree(b->cell_start); cudaFree(b->block_sums);
@@ -655,9 +654,10 @@ void benqueue_pre(fsph_batch *b, const BLaunch &L, cudaStream_t s) {
 
 void benqueue_post(fsph_batch *b, const BLaunch &L, const DevParams &lp, cudaStream_t s) {
     blaunch_finalize(L, lp.inv_dt, b->pos[1], b->ppos[0], b->ppos[1], b->ctl, b->id[1], b->attr[1], b->pos[0],
-                     b->vel[0], b->id[0], b->attr[0], b->dens, b->mrho, s);
-    blaunch_xsph_vort(L, b->cell_start, b->pos[0], b->vel[0], b->dens, b->vel[1], b->vort, b->nl, s, b->mrho, b->wm);
-    blaunch_vort_apply(L, b->cell_start, b->pos[0], b->vort, b->dens, b->vel[1], b->vel[0], b->nl, s, b->wm);
+                     b->vel[0], b->id[0], b->attr[0], b->dens, b->xb, s);
+    /* the build positions are not read again before the next build: x* with m / rho takes their place */
+    blaunch_xsph_vort(L, b->cell_start, b->xb, b->vel[0], b->dens, b->vel[1], b->vort, b->nl, s, b->mag);
+    blaunch_vort_apply(L, b->cell_start, b->xb, b->vort, b->dens, b->vel[1], b->vel[0], b->nl, s, b->mag);
     kb_tile_errors<<<blocks_for(std::max(b->nt_full, 1), 8), 256, 0, s>>>(L.full, b->dens, b->d_tile_err);
     kb_scene_errors<<<blocks_for(b->nscenes, 4), 128, 0, s>>>(b->nscenes, b->d_offs, b->d_tile0, b->d_tile_err,
                                                              b->d_err);
@@ -858,7 +858,7 @@ int fsph_batch_create(const fsph_params *params, const int *counts, int nscenes,
         A(&b->pos[k], n); A(&b->vel[k], n); A(&b->id[k], n); A(&b->attr[k], n); A(&b->ppos[k], n);
     }
     A(&b->xb, n); A(&b->vort, n); A(&b->tmp4, n); A(&b->dens, n); A(&b->tdens, n);
-    A(&b->mrho, n); A(&b->wm, n);
+    A(&b->mag, n);
     A(&b->key, n); A(&b->rank, n); A(&b->perm, n);
     A(&b->nl.list, n * kListMax); A(&b->nl.cnt, n); A(&b->nl.cellb, n);
     A(&b->d_scenes, (size_t)nscenes); A(&b->d_offs, (size_t)nscenes + 1); A(&b->d_tile0, (size_t)nscenes + 1); A(&b->d_err, 3 * (size_t)nscenes);

@@ -218,15 +218,6 @@ __device__ inline float3 operator+(float3 a, float3 b) { return make_float3(a.x 
 __device__ inline float3 operator*(float s, float3 a) { return make_float3(s * a.x, s * a.y, s * a.z); }
 __device__ inline float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 
-/* FSPH_POST_PRE 1 (default): m / rho is computed once per particle before
- * the XSPH pass (k_finalize, kb_mrho) and the XSPH pass hands (|omega|,
- * m / rho) to the vorticity pass, so neither divides nor takes a square
- * root per pair (0: per pair; the results are the same bit for bit).
- * Measured on the 1M double dam break: warm step 2.790 -> 2.714 ms, plain
- * step 9.758 -> 9.683 ms, positions bit-identical. */
-#ifndef FSPH_POST_PRE
-#define FSPH_POST_PRE 1
-#endif
 /* 1 / sqrt(max(r2, 1e-20)) for the pair loops.  FSPH_RSQRT_FTZ 1 (default)
  * issues rsqrt.approx.ftz.f32: the argument is clamped to a normal number
  * and the result is normal, so the flush-to-zero form, which skips the

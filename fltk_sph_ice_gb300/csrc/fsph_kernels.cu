@@ -499,15 +499,15 @@ __global__ void k_finalize(DevParams p, const float4 *__restrict__ pos_b, const 
                            const unsigned int *__restrict__ attr_b, float4 *__restrict__ pos_a,
                            float4 *__restrict__ vel_a, unsigned int *__restrict__ id_a,
                            unsigned int *__restrict__ attr_a, const float4 *__restrict__ xpred,
-                           float4 *__restrict__ dstep, const float *__restrict__ dens, float *__restrict__ mrho) {
+                           float4 *__restrict__ dstep, const float *__restrict__ dens, float4 *__restrict__ xm) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    if (mrho) mrho[i] = p.mass / dens[i]; /* m / rho_i for the XSPH and vorticity passes */
     const float4 *pp = ctl->parity ? ppos1 : ppos0;
     float3 xs = f3(pp[i]);
     float3 x = f3(pos_b[i]);
     float3 v = p.inv_dt * (xs - x);
     pos_a[i] = make_float4(xs.x, xs.y, xs.z, 0.0f);
+    if (xm) xm[i] = make_float4(xs.x, xs.y, xs.z, p.mass / dens[i]); /* what the XSPH and vorticity passes gather */
     vel_a[i] = make_float4(v.x, v.y, v.z, 0.0f);
     id_a[i] = id_b[i];
     attr_a[i] = attr_b[i];
@@ -520,23 +520,23 @@ __global__ void k_finalize(DevParams p, const float4 *__restrict__ pos_b, const 
 
 /* omega_i = sum_j (v_j - v_i) x grad_j W_ij (grad_j = -grad_i), and the
  * XSPH update v_i + c sum_j (m / rho_j)(v_j - v_i) W_ij. */
-template <bool NBR, bool PRE, bool DEEP>
-__global__ void __launch_bounds__(DEEP ? kDeepBlock : kBlock) k_xsph_vort(DevParams p, const unsigned int *__restrict__ cell_start,
+template <bool FEAT, bool NBR, bool PRE, bool DEEP>
+__global__ void __launch_bounds__(DEEP ? kDeepBlock : kPostBlock) k_xsph_vort(DevParams p, const unsigned int *__restrict__ cell_start,
                                                       const float4 *__restrict__ pos, const float4 *__restrict__ vel,
                                                       const float *__restrict__ dens, float4 *__restrict__ vel_out,
                                                       float4 *__restrict__ vort, FeatureOut fo,
                                                       const ListEntry *__restrict__ list,
                                                       const unsigned char *__restrict__ cnt,
-                                                      const float *__restrict__ mrho, float2 *__restrict__ wm) {
+                                                      float *__restrict__ mag) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    xsph_vort_body<NBR, PRE, DEEP>(p, i, cell_start, pos, vel, dens, vel_out, vort, fo, list, cnt, mrho, wm);
+    xsph_vort_body<FEAT, NBR, PRE, DEEP>(p, i, cell_start, pos, vel, dens, vel_out, vort, fo, list, cnt, mag);
 }
 
 /* eta_i = sum_j (m / rho_j)(|w_j| - |w_i|) grad_i W_ij; f = eps (eta/|eta|) x w_i;
  * v_i <- v_i + dt f. */
 template <bool PRE, bool DEEP>
-__global__ void __launch_bounds__(DEEP ? kDeepBlock : kBlock) k_vort_apply(DevParams p, const unsigned int *__restrict__ cell_start,
+__global__ void __launch_bounds__(DEEP ? kDeepBlock : kPostBlock) k_vort_apply(DevParams p, const unsigned int *__restrict__ cell_start,
                                                        const float4 *__restrict__ pos,
                                                        const float4 *__restrict__ vort,
                                                        const float *__restrict__ dens,
@@ -544,10 +544,10 @@ __global__ void __launch_bounds__(DEEP ? kDeepBlock : kBlock) k_vort_apply(DevPa
                                                        float4 *__restrict__ vel_out,
                                                        const ListEntry *__restrict__ list,
                                                        const unsigned char *__restrict__ cnt,
-                                                      const float2 *__restrict__ wm) {
+                                                      const float *__restrict__ mag) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
-    vort_apply_body<PRE, DEEP>(p, i, cell_start, pos, vort, dens, vel_in, vel_out, list, cnt, wm);
+    vort_apply_body<PRE, DEEP>(p, i, cell_start, pos, vort, dens, vel_in, vel_out, list, cnt, mag);
 }
 
 /* ======================================================================== */
@@ -807,9 +807,6 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
  * Branch-free pair terms: t = max(h - r, 0) is 0 at and beyond h, and at
  * r = 0 too (h - 0 * rsqrt(0) is NaN, which fmaxf maps to 0), so the self
  * pair and coincident particles add nothing, as the reference skips them. */
-struct PosVel {
-    float4 x, v;
-};
 template <int LPP>
 __global__ void __launch_bounds__(kBlock) k_sph_force(DevParams p, const unsigned int *__restrict__ cell_start,
                                                       const float4 *__restrict__ pos, const float4 *__restrict__ vel,
@@ -1396,31 +1393,31 @@ void launch_correction(const DevParams &p, const unsigned int *cell_start, float
 void launch_finalize(const DevParams &p, const float4 *pos_b, const float4 *ppos0, const float4 *ppos1,
                      const DevCtl *ctl, const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a,
                      float4 *vel_a, unsigned int *id_a, unsigned int *attr_a, const float4 *xpred, float4 *dstep,
-                     cudaStream_t s, const float *dens, float *mrho) {
+                     cudaStream_t s, const float *dens, float4 *xm) {
     k_finalize<<<blocks_for(p.n), kBlock, 0, s>>>(p, pos_b, ppos0, ppos1, ctl, id_b, attr_b, pos_a, vel_a, id_a,
-                                                  attr_a, xpred, dstep, dens, mrho);
+                                                  attr_a, xpred, dstep, dens, xm);
 }
 void launch_xsph_vort(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vel,
                       const float *dens, float4 *vel_out, float4 *vort, const FeatureOut &fo, const NbrLists &nl,
-                      cudaStream_t s, const float *mrho, float2 *wm) {
+                      cudaStream_t s, float *mag) {
     /* the neighbour means cost a gather per pair: only when they are used */
-    const bool nbr = fo.feat && fo.nbr, pre = mrho && wm, deep = deep_pass(p);
-    auto k = nbr ? (pre ? (deep ? k_xsph_vort<true, true, true> : k_xsph_vort<true, true, false>)
-                        : k_xsph_vort<true, false, false>)
-                 : (pre ? (deep ? k_xsph_vort<false, true, true> : k_xsph_vort<false, true, false>)
-                        : k_xsph_vort<false, false, false>);
-    const int block = deep && pre ? kDeepBlock : kBlock;
+    const bool deep = mag && deep_pass(p), nbr = fo.nbr != 0;
+    auto k = !mag      ? k_xsph_vort<false, false, false, false>
+             : fo.feat ? (deep ? (nbr ? k_xsph_vort<true, true, true, true> : k_xsph_vort<true, false, true, true>)
+                               : (nbr ? k_xsph_vort<true, true, true, false> : k_xsph_vort<true, false, true, false>))
+                       : (deep ? k_xsph_vort<false, false, true, true> : k_xsph_vort<false, false, true, false>);
+    const int block = deep ? kDeepBlock : kPostBlock;
     k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, pos, vel, dens, vel_out, vort, fo,
-                                               p.use_lists ? nl.list : nullptr, nl.cnt, mrho, wm);
+                                               p.use_lists ? nl.list : nullptr, nl.cnt, mag);
 }
 void launch_vort_apply(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vort,
                        const float *dens, const float4 *vel_in, float4 *vel_out, const NbrLists &nl, cudaStream_t s,
-                       const float2 *wm) {
-    const bool deep = wm && deep_pass(p);
-    auto k = deep ? k_vort_apply<true, true> : wm ? k_vort_apply<true, false> : k_vort_apply<false, false>;
-    const int block = deep ? kDeepBlock : kBlock;
+                       const float *mag) {
+    const bool deep = mag && deep_pass(p);
+    auto k = deep ? k_vort_apply<true, true> : mag ? k_vort_apply<true, false> : k_vort_apply<false, false>;
+    const int block = deep ? kDeepBlock : kPostBlock;
     k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, pos, vort, dens, vel_in, vel_out,
-                                               p.use_lists ? nl.list : nullptr, nl.cnt, wm);
+                                               p.use_lists ? nl.list : nullptr, nl.cnt, mag);
 }
 /* lanes per particle (a power of two, at most `most`): enough that the launch
  * holds about as many threads as the GPU keeps resident (1536 per SM) */

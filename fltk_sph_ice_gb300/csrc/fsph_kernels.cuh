@@ -22,6 +22,11 @@ constexpr int kPassBlock = FSPH_PASS_BLOCK;
  * and a correction pass together: 31.0 -> 22.6 us at 6,912, 33.0 -> 27.7 at
  * 32,000, 43.1 -> 42.0 at 131,072, 71.4 -> 81.6 at 294,912 */
 constexpr int kDeepBlock = 64, kDeepMinB = 12, kDeepMax = 65536;
+/* The XSPH and vorticity passes of larger scenes: a step of 1 M particles with two
+ * iterations took 852 us in blocks of 128, 857 of 256, 865 of 512, 878 with eight
+ * candidates in flight; with registers for five or six blocks of 256 per SM 867
+ * and 914. */
+constexpr int kPostBlock = 128;
 constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 8.7 KB each */
 constexpr int kBlockMax = 512;  /* largest block of the batched persistent kernels */
 constexpr int kScanTile = 4096; /* cells per block of the first scan phase */
@@ -123,17 +128,17 @@ void launch_correction(const DevParams &p, const unsigned int *cell_start, float
 void launch_finalize(const DevParams &p, const float4 *pos_b, const float4 *ppos0, const float4 *ppos1,
                      const DevCtl *ctl, const unsigned int *id_b, const unsigned int *attr_b, float4 *pos_a,
                      float4 *vel_a, unsigned int *id_a, unsigned int *attr_a, const float4 *xpred, float4 *dstep,
-                     cudaStream_t s, const float *dens = nullptr, float *mrho = nullptr);
-/* XSPH + vorticity (omega) pass; with fo.feat also the warm-start features.
- * With mrho (m / rho per particle, from launch_finalize) and wm the pass
- * reads m / rho_j instead of dividing per pair and leaves (|omega|, m / rho)
- * in wm, which launch_vort_apply then gathers in place of vort and dens. */
+                     cudaStream_t s, const float *dens = nullptr, float4 *xm = nullptr);
+/* XSPH + vorticity (omega) pass; with fo.feat (and mag) also the warm-start
+ * features.  With mag, pos is launch_finalize's xm: the pass takes m / rho_j from
+ * pos[j].w instead of dividing per pair and leaves |omega| in mag, which
+ * launch_vort_apply then gathers with xm in place of vort and dens. */
 void launch_xsph_vort(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vel,
                       const float *dens, float4 *vel_out, float4 *vort, const FeatureOut &fo, const NbrLists &nl,
-                      cudaStream_t s, const float *mrho = nullptr, float2 *wm = nullptr);
+                      cudaStream_t s, float *mag = nullptr);
 void launch_vort_apply(const DevParams &p, const unsigned int *cell_start, const float4 *pos, const float4 *vort,
                        const float *dens, const float4 *vel_in, float4 *vel_out, const NbrLists &nl, cudaStream_t s,
-                       const float2 *wm = nullptr);
+                       const float *mag = nullptr);
 
 /* ---- static boundary particles (p.bpos / p.bcell / p.bnear of the sorted boundary) ---- */
 /* bscale[b] = rho0 psi_b / m with psi_b = m / sum_b' m W(r_bb') (rx_sph_pbd.cpp:1061-1090) */

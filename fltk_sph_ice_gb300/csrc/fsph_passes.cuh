@@ -968,18 +968,26 @@ __device__ __forceinline__ void correction_tail(const DevParams &lp, DevCtl *ctl
  * eps = 1e-4 then drives the flow unstable).  The XSPH update
  * v_i + c sum_j (m / rho_j)(v_j - v_i) W_ij, and (fo.feat) the warm-start
  * features of the particle. */
-/* PRE: m / rho_j comes from mrho (written once per particle by k_finalize,
- * the same correctly rounded quotient) instead of a division per pair, and
- * the pass leaves (|omega_i|, m / rho_i) in wm for vort_apply_body<true>. */
-template <bool NBR = true, bool PRE = false, bool DEEP = false>
+/* PRE: pos[j].w is m / rho_j (written once per particle by k_finalize, the
+ * same correctly rounded quotient), and the pass leaves |omega_i| in mag for
+ * vort_apply_body<true>; else a division per pair.  FEAT: the features are
+ * wanted, NBR: with the neighbour means.
+ * Both passes are bound as the constraint passes are, by the L1 wavefronts of
+ * their gathers (78 % and 68 % of the unit's peak while active at 262,144
+ * particles with m / rho in an array of its own and the features' sums always
+ * kept): two gathers a pair here and one and a 4-byte one there, all of a
+ * group's in flight before its first pair.  262,144 particles 37.0 -> 32.5 us
+ * and 31.9 -> 26.8, 16.8 M particles 1656 -> 1554 and 1188 -> 1056. */
+struct PosVel {
+    float4 x, v;
+};
+template <bool FEAT, bool NBR, bool PRE, bool DEEP = false>
 __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const unsigned int *__restrict__ cell_start,
                                                const float4 *__restrict__ pos, const float4 *__restrict__ vel,
                                                const float *__restrict__ dens, float4 *__restrict__ vel_out,
                                                float4 *__restrict__ vort, const FeatureOut &fo,
                                                const ListEntry *__restrict__ list,
-                                               const unsigned char *__restrict__ cnt,
-                                               const float *__restrict__ mrho_in = nullptr,
-                                               float2 *__restrict__ wm = nullptr) {
+                                               const unsigned char *__restrict__ cnt, float *__restrict__ mag) {
     const float3 xi = f3(pos[i]), vi = f3(vel[i]);
     float3 om = make_float3(0.f, 0.f, 0.f), xs = make_float3(0.f, 0.f, 0.f);
     float3 off = make_float3(0.f, 0.f, 0.f), cg = make_float3(0.f, 0.f, 0.f);
@@ -992,23 +1000,23 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
     /* branch-free pair terms: q and t clamp to zero outside h, and the self
      * pair (d = 0, v_ij = 0) adds only to the neighbour count */
     for_each_candidate<1, DEEP>(
-        p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return __ldg(pos + j); },
-        [&](unsigned int j, const float4 &xj4) {
-            const float3 d = xi - f3(xj4);
+        p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return PosVel{__ldg(pos + j), __ldg(vel + j)}; },
+        [&](unsigned int j, const PosVel &b) {
+            const float3 d = xi - f3(b.x);
             const float r2 = dot3(d, d);
-            const float inside = r2 < p.h2 ? 1.0f : 0.0f;
             const float q = fmaxf(p.h2 - r2, 0.0f);
             const float inv_r = pair_rsqrt(r2);
             const float t = fmaxf(p.h - r2 * inv_r, 0.0f);
             const float g = p.ag * t * t * inv_r;
-            const float3 vij = f3(__ldg(vel + j)) - vi;
+            const float3 vij = f3(b.v) - vi;
             const float rhoj = (NBR || !PRE) ? __ldg(dens + j) : 0.0f;
-            const float mrho = PRE ? __ldg(mrho_in + j) : p.mass / rhoj;
+            const float mrho = PRE ? b.x.w : p.mass / rhoj;
             om = om + cross3(vij, (-g * mrho) * d);
             xs = xs + (p.aw * q * q * q * mrho) * vij;
-            cntf += inside;
-            off = off - inside * d;
-            if (fo.feat) {
+            if (FEAT) {
+                const float inside = r2 < p.h2 ? 1.0f : 0.0f;
+                cntf += inside;
+                off = off - inside * d;
                 /* the pair at the next step's prediction x + dt v (gravity cancels
                  * in relative positions): poly6 and its spiky gradient there */
                 const float3 ds = d - p.dt * vij;
@@ -1027,12 +1035,12 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
                 }
             }
         });
-    cntf = fmaxf(cntf, 1.0f);
     float3 vn = vi + p.xsph_c * xs;
     vel_out[i] = make_float4(vn.x, vn.y, vn.z, 0.0f);
     vort[i] = make_float4(om.x, om.y, om.z, 0.0f);
-    if (PRE) wm[i] = make_float2(sqrtf(dot3(om, om)), mrho_in[i]);
-    if (fo.feat) {
+    if (PRE) mag[i] = sqrtf(dot3(om, om));
+    if (FEAT) {
+        cntf = fmaxf(cntf, 1.0f);
         /* warm-start features at the end of the step (dimensionless; see kFeatures) */
         const float inv_h = 1.0f / p.h;
         const float4 *pl = fo.ctl->parity ? fo.ppos0 : fo.ppos1; /* buffer of the last lambda pass */
@@ -1067,33 +1075,37 @@ __device__ __forceinline__ void xsph_vort_body(const DevParams &p, int i, const 
 
 /* eta_i = sum_j (m / rho_j)(|w_j| - |w_i|) grad_i W_ij; f = eps (eta/|eta|) x w_i;
  * v_i <- v_i + dt f. */
-/* PRE: (|omega_j|, m / rho_j) from wm (one 8-byte gather per pair, no
- * division or square root; the same values xsph_vort_body<.., true> wrote). */
+/* PRE: |omega_j| from mag (what xsph_vort_body wrote) and m / rho_j from
+ * pos[j].w, so neither a division nor a square root per pair. */
 template <bool PRE = false, bool DEEP = false>
 __device__ __forceinline__ void vort_apply_body(const DevParams &p, int i, const unsigned int *__restrict__ cell_start,
                                                 const float4 *__restrict__ pos, const float4 *__restrict__ vort,
                                                 const float *__restrict__ dens, const float4 *__restrict__ vel_in,
                                                 float4 *__restrict__ vel_out, const ListEntry *__restrict__ list,
                                                 const unsigned char *__restrict__ cnt,
-                                               const float2 *__restrict__ wm = nullptr) {
+                                                const float *__restrict__ mag) {
     float4 v4 = vel_in[i];
     if (p.vort_eps != 0.0f) {
         const float3 xi = f3(pos[i]);
         const float3 wi = f3(vort[i]);
         const float wmi = sqrtf(dot3(wi, wi));
         float3 eta = make_float3(0.f, 0.f, 0.f);
+        struct PosMag {
+            float4 x;
+            float w;
+        };
         for_each_candidate<1, DEEP>(
-            p, cell_start, list, cnt, i, xi, 0, [&](unsigned int j) { return __ldg(pos + j); },
-            [&](unsigned int j, const float4 &xj4) {
-                const float3 d = xi - f3(xj4);
+            p, cell_start, list, cnt, i, xi, 0,
+            [&](unsigned int j) { return PosMag{__ldg(pos + j), PRE ? __ldg(mag + j) : 0.0f}; },
+            [&](unsigned int j, const PosMag &b) {
+                const float3 d = xi - f3(b.x);
                 const float r2 = dot3(d, d);
                 const float inv_r = pair_rsqrt(r2);
                 const float t = fmaxf(p.h - r2 * inv_r, 0.0f);
                 const float g = p.ag * t * t * inv_r;
                 float k;
                 if (PRE) {
-                    const float2 b = __ldg(wm + j); /* (|omega_j|, m / rho_j) */
-                    k = b.y * (b.x - wmi) * g;
+                    k = b.x.w * (b.w - wmi) * g;
                 } else {
                     const float3 wj = f3(__ldg(vort + j));
                     k = p.mass / __ldg(dens + j) * (sqrtf(dot3(wj, wj)) - wmi) * g;
