@@ -75,10 +75,18 @@ __global__ void k_mlp_pack(const float *__restrict__ b, MlpDev *__restrict__ d) 
     if (threadIdx.x == 0) d->out_scale = b[kBScale];
 }
 
+/* 16 bytes a load and, at 128 threads, all of a thread's in flight: word by word
+ * the copy was a chain of loads at the head of every launch.  sm is 16-byte
+ * aligned; the struct's size, which saved states record, is not a multiple of 16. */
 __device__ __forceinline__ void copy_model(MlpDev &sm, const MlpDev *__restrict__ gm) {
-    const unsigned *src = reinterpret_cast<const unsigned *>(gm);
-    unsigned *dst = reinterpret_cast<unsigned *>(&sm);
-    for (int k = threadIdx.x; k < (int)(sizeof(MlpDev) / 4); k += blockDim.x) dst[k] = src[k];
+    constexpr int kVec = (int)(sizeof(MlpDev) / 16), kWords = (int)(sizeof(MlpDev) / 4);
+    const uint4 *src = reinterpret_cast<const uint4 *>(gm);
+    uint4 *dst = reinterpret_cast<uint4 *>(&sm);
+#pragma unroll 14
+    for (int k = threadIdx.x; k < kVec; k += blockDim.x) dst[k] = __ldg(src + k);
+    if (4 * kVec + (int)threadIdx.x < kWords)
+        reinterpret_cast<unsigned *>(&sm)[4 * kVec + threadIdx.x] =
+            reinterpret_cast<const unsigned *>(gm)[4 * kVec + threadIdx.x];
 }
 
 /* Forward pass of one warp's 16 rows starting at base.  Leaves the ReLU'd
@@ -86,34 +94,53 @@ __device__ __forceinline__ void copy_model(MlpDev &sm, const MlpDev *__restrict_
  * 2c, 2c+1; columns >= 3 are padding).  Rows >= n read zero features. */
 struct Fwd {
     float h1[8][4], h2[8][4], o[4];
-    unsigned ax[kIn / 16][4];
-    /* normalised inputs of this thread, per 16-column k tile kt:
-     * (g, 16kt+2c..+1), (g+8, ..), (g, 16kt+2c+8..+9), (g+8, ..) */
-    float xn[kIn / 2];
 };
+
+/* The inputs of one thread, rows g and g+8 (past the last row: zero), per
+ * 16-column k tile kt: columns 16kt+2c..+1 and 16kt+2c+8..+9. */
+template <int KT>
+__device__ __forceinline__ void mlp_load(const float *__restrict__ x, int n, int base, int g, int c, float (&v)[KT][8]) {
+    const int r0 = base + g, r1 = base + g + 8;
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int col = 16 * kt + 2 * c + (q & 1) + 8 * (q >> 1);
+            v[kt][q] = r0 < n ? __ldg(x + (size_t)r0 * kIn + col) : 0.0f;
+            v[kt][4 + q] = r1 < n ? __ldg(x + (size_t)r1 * kIn + col) : 0.0f;
+        }
+}
+/* ... normalised, as operands */
+template <int KT>
+__device__ __forceinline__ void mlp_inputs(const MlpDev &sm, const float (&v)[KT][8], int n, int base, int g, int c,
+                                           unsigned (&ax)[KT][4]) {
+    const int r0 = base + g, r1 = base + g + 8;
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) {
+        float xn[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int col = 16 * kt + 2 * c + (q & 1) + 8 * (q >> 1);
+            xn[q] = r0 < n ? (v[kt][q] - sm.mu[col]) * sm.isig[col] : 0.0f;         /* row g   */
+            xn[4 + q] = r1 < n ? (v[kt][4 + q] - sm.mu[col]) * sm.isig[col] : 0.0f; /* row g+8 */
+        }
+        ax[kt][0] = pack2(xn[0], xn[1]);
+        ax[kt][1] = pack2(xn[4], xn[5]);
+        ax[kt][2] = pack2(xn[2], xn[3]);
+        ax[kt][3] = pack2(xn[6], xn[7]);
+    }
+}
 
 /* KT: the 16-wide input tiles read (inputs past them contribute nothing:
  * a network that gives them no weight runs with KT = 1) */
 template <int KT = kIn / 16>
 __device__ __forceinline__ void mlp_forward(const MlpDev &sm, const float *__restrict__ x, int n, int base, int g,
                                             int c, Fwd &F) {
-    const int r0 = base + g, r1 = base + g + 8;
-#pragma unroll
-    for (int kt = 0; kt < KT; ++kt) {
-        const int cols[4] = {16 * kt + 2 * c, 16 * kt + 2 * c + 1, 16 * kt + 2 * c + 8, 16 * kt + 2 * c + 9};
-        float *xn = F.xn + 8 * kt;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int col = cols[q];
-            const float v0 = r0 < n ? __ldg(x + (size_t)r0 * kIn + col) : 0.0f;
-            const float v1 = r1 < n ? __ldg(x + (size_t)r1 * kIn + col) : 0.0f;
-            xn[q] = r0 < n ? (v0 - sm.mu[col]) * sm.isig[col] : 0.0f;       /* row g   */
-            xn[4 + q] = r1 < n ? (v1 - sm.mu[col]) * sm.isig[col] : 0.0f;   /* row g+8 */
-        }
-        F.ax[kt][0] = pack2(xn[0], xn[1]);
-        F.ax[kt][1] = pack2(xn[4], xn[5]);
-        F.ax[kt][2] = pack2(xn[2], xn[3]);
-        F.ax[kt][3] = pack2(xn[6], xn[7]);
+    unsigned ax[KT][4];
+    {
+        float v[KT][8];
+        mlp_load<KT>(x, n, base, g, c, v);
+        mlp_inputs<KT>(sm, v, n, base, g, c, ax);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -122,7 +149,7 @@ __device__ __forceinline__ void mlp_forward(const MlpDev &sm, const float *__res
 #pragma unroll
         for (int kt = 0; kt < KT; ++kt) {
             const __nv_bfloat16 *w = sm.w1t + (8 * j + g) * kS1 + 16 * kt + 2 * c;
-            mma16816(F.h1[j], F.ax[kt], ld32(w), ld32(w + 8));
+            mma16816(F.h1[j], ax[kt], ld32(w), ld32(w + 8));
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) F.h1[j][e] = fmaxf(F.h1[j][e], 0.0f);
@@ -212,7 +239,73 @@ int mlp_grad_blocks(int n) {
     return chunks < 304 ? (chunks > 0 ? chunks : 1) : 304;
 }
 
-__global__ void __launch_bounds__(128) k_mlp_grad(const MlpDev *__restrict__ gm, const float *__restrict__ x,
+__device__ __forceinline__ unsigned smem_at(const __nv_bfloat16 *p) { return (unsigned)__cvta_generic_to_shared(p); }
+/* four 8 x 8 matrices, lane 8m + r gives row r of matrix m */
+__device__ __forceinline__ void load_m4(unsigned (&v)[4], const __nv_bfloat16 *row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(smem_at(row))
+                 : "memory");
+}
+/* two, from the rows of lanes 0-15 */
+__device__ __forceinline__ void load_m2(unsigned &v0, unsigned &v1, const __nv_bfloat16 *row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];"
+                 : "=r"(v0), "=r"(v1)
+                 : "r"(smem_at(row))
+                 : "memory");
+}
+/* the same, to memory and transposed */
+__device__ __forceinline__ void store_t4(__nv_bfloat16 *row, const unsigned (&v)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_at(row)),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ void store_t2(__nv_bfloat16 *row, unsigned v0, unsigned v1) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x2.trans.shared.b16 [%0], {%1, %2};" ::"r"(smem_at(row)), "r"(v0), "r"(v1)
+                 : "memory");
+}
+/* acc += a (16 x 64) times eight columns whose 64 weights each lie in a row; row:
+ * this lane's for k = 0 .. 31 */
+__device__ __forceinline__ void mma_row64(float (&acc)[4], const unsigned (&a)[4][4], const __nv_bfloat16 *row) {
+#pragma unroll
+    for (int s = 0; s < 4; s += 2) {
+        unsigned v[4];
+        load_m4(v, row + 16 * s);
+        mma16816(acc, a[s], v[0], v[1]);
+        mma16816(acc, a[s + 1], v[2], v[3]);
+    }
+}
+/* tiles 2s and 2s + 1 as the next product's operand, and the bits of what passes */
+__device__ __forceinline__ void relu_pack(float (&h)[2][4], int s, unsigned (&a)[4], unsigned &on) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            h[u][e] = fmaxf(h[u][e], 0.0f);
+            if (h[u][e] > 0.0f) on |= 1u << (4 * (2 * s + u) + e);
+        }
+        a[2 * u] = pack2(h[u][0], h[u][1]);
+        a[2 * u + 1] = pack2(h[u][2], h[u][3]);
+    }
+}
+__device__ __forceinline__ void mask_pack(float (&d)[2][4], int s, unsigned on, unsigned (&a)[4]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[u][e] = (on >> (4 * (2 * s + u) + e) & 1u) ? d[u][e] : 0.f;
+        a[2 * u] = pack2(d[u][0], d[u][1]);
+        a[2 * u + 1] = pack2(d[u][2], d[u][3]);
+    }
+}
+
+/* What bounds it is latency: 8 warps per SM (216 registers, which hold the sums of
+ * the weight gradients), each a chain of small products, 15 % of the issue slots
+ * used.  So the loads from memory leave early (the model 16 bytes at a time, the
+ * next chunk's inputs before this one's weight products, the targets before the
+ * layers), and operands move as 8 x 8 matrices.  65,536 rows: 27.6 -> 23.0 us; with
+ * three blocks per SM (168 registers, 456 partial gradients to add) the call took
+ * 54 us instead of 49. */
+__global__ void __launch_bounds__(128, 2) k_mlp_grad(const MlpDev *__restrict__ gm, const float *__restrict__ x,
                                                   const float *__restrict__ t, int n, float *__restrict__ part,
                                                   float *__restrict__ loss_part) {
     extern __shared__ __align__(16) unsigned char dsm[];
@@ -224,9 +317,15 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const MlpDev *__restrict__ gm,
     __nv_bfloat16 *sd2 = sd1 + kHid * kSS;
     __nv_bfloat16 *sdy = sd2 + kHid * kSS;
     __shared__ float s_loss[4];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, c = lane & 3;
+    float xv[kIn / 16][8]; /* the next chunk's inputs, on the way during the products of this one */
+    mlp_load<kIn / 16>(x, n, (int)blockIdx.x * kChunk + w * 16, g, c, xv);
     copy_model(sm, gm);
     __syncthreads();
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, c = lane & 3;
+    const int row8 = lane & 7, mat = lane >> 3; /* the row of the 8 x 8 matrix that this lane addresses */
+    const int st_at = (8 * (mat >> 1) + row8) * kSS + 16 * w + 8 * (mat & 1); /* features down, this warp's samples */
+    const int a_at = (8 * (mat & 1) + row8) * kSS + 8 * (mat >> 1); /* a left operand's four matrices */
+    const int b_at = (8 * (mat >> 1) + row8) * kSS + 8 * (mat & 1); /* two right operands' */
     const float inv_scale = sm.out_scale != 0.0f ? 1.0f / sm.out_scale : 0.0f;
     const float gscale = 2.0f / (float)n;
     float acc2[8][4], acc3[4], acc1[kIn / 16][2][4];
@@ -241,7 +340,7 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const MlpDev *__restrict__ gm,
      * products read anyway: products with a matrix of ones (all 16 rows alike),
      * warp w for columns 16w .. 16w + 15 (they had been summed by 64 threads over
      * the 64 staged samples while the other threads waited).  With the reduction
-     * below, a gradient over 65,536 rows went from 92 to 44 us. */
+     * below, a gradient over 65,536 rows went from 92 to 44 us, and to 41 with the loads of this kernel moved ahead. */
     float accb1[2][4], accb2[2][4], accb3[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int jj = 0; jj < 2; ++jj) {
@@ -254,132 +353,119 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const MlpDev *__restrict__ gm,
     const int nchunks = (n + kChunk - 1) / kChunk;
     for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         const int base = ch * kChunk + w * 16;
-        const int sl0 = w * 16 + g, sl1 = sl0 + 8; /* sample columns in the staging */
         const int r0 = base + g, r1 = base + g + 8;
-        Fwd F;
-        mlp_forward(sm, x, n, base, g, c, F);
-        /* stage x~, h1, h2 transposed */
+        /* forward; x~, h1 and h2 go to the staging transposed as they are made */
+        unsigned ax[kIn / 16][4], a[4][4];
+        mlp_inputs<kIn / 16>(sm, xv, n, base, g, c, ax);
+        /* the targets are needed after three layers */
+        const bool in0 = 2 * c < kOut, in1 = 2 * c + 1 < kOut;
+        const float t00 = (r0 < n && in0) ? __ldg(t + 3 * (size_t)r0 + 2 * c) * inv_scale : 0.f;
+        const float t01 = (r0 < n && in1) ? __ldg(t + 3 * (size_t)r0 + 2 * c + 1) * inv_scale : 0.f;
+        const float t10 = (r1 < n && in0) ? __ldg(t + 3 * (size_t)r1 + 2 * c) * inv_scale : 0.f;
+        const float t11 = (r1 < n && in1) ? __ldg(t + 3 * (size_t)r1 + 2 * c + 1) * inv_scale : 0.f;
 #pragma unroll
-        for (int kt = 0; kt < kIn / 16; ++kt) {
-            const int cols[4] = {16 * kt + 2 * c, 16 * kt + 2 * c + 1, 16 * kt + 2 * c + 8, 16 * kt + 2 * c + 9};
+        for (int kt = 0; kt < kIn / 16; ++kt) store_t4(sx + 16 * kt * kSS + st_at, ax[kt]);
+        unsigned on1 = 0u, on2 = 0u; /* bit 4j + e: element e of tile j is positive */
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                sx[cols[q] * kSS + sl0] = __float2bfloat16(F.xn[8 * kt + q]);
-                sx[cols[q] * kSS + sl1] = __float2bfloat16(F.xn[8 * kt + 4 + q]);
+        for (int s = 0; s < 4; ++s) {
+            float h[2][4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = 2 * s + u;
+                const float b0v = sm.b1[8 * j + 2 * c], b1v = sm.b1[8 * j + 2 * c + 1];
+                h[u][0] = b0v; h[u][1] = b1v; h[u][2] = b0v; h[u][3] = b1v;
+                unsigned wv[4];
+                load_m4(wv, sm.w1t + 8 * j * kS1 + row8 * kS1 + 8 * mat);
+                mma16816(h[u], ax[0], wv[0], wv[1]);
+                mma16816(h[u], ax[1], wv[2], wv[3]);
             }
+            relu_pack(h, s, a[s], on1);
+            store_t4(sh1 + 16 * s * kSS + st_at, a[s]);
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int f0 = 8 * j + 2 * c;
-            sh1[f0 * kSS + sl0] = __float2bfloat16(F.h1[j][0]);
-            sh1[(f0 + 1) * kSS + sl0] = __float2bfloat16(F.h1[j][1]);
-            sh1[f0 * kSS + sl1] = __float2bfloat16(F.h1[j][2]);
-            sh1[(f0 + 1) * kSS + sl1] = __float2bfloat16(F.h1[j][3]);
-            sh2[f0 * kSS + sl0] = __float2bfloat16(F.h2[j][0]);
-            sh2[(f0 + 1) * kSS + sl0] = __float2bfloat16(F.h2[j][1]);
-            sh2[f0 * kSS + sl1] = __float2bfloat16(F.h2[j][2]);
-            sh2[(f0 + 1) * kSS + sl1] = __float2bfloat16(F.h2[j][3]);
-        }
-        /* dL/dy = 2 (y - t / out_scale) / n for the 3 real outputs of real rows */
-        float dy[4];
         {
-            const int c0 = 2 * c, c1 = 2 * c + 1;
-            float t00 = (r0 < n && c0 < kOut) ? __ldg(t + 3 * (size_t)r0 + c0) * inv_scale : 0.f;
-            float t01 = (r0 < n && c1 < kOut) ? __ldg(t + 3 * (size_t)r0 + c1) * inv_scale : 0.f;
-            float t10 = (r1 < n && c0 < kOut) ? __ldg(t + 3 * (size_t)r1 + c0) * inv_scale : 0.f;
-            float t11 = (r1 < n && c1 < kOut) ? __ldg(t + 3 * (size_t)r1 + c1) * inv_scale : 0.f;
-            float e00 = (r0 < n && c0 < kOut) ? F.o[0] - t00 : 0.f;
-            float e01 = (r0 < n && c1 < kOut) ? F.o[1] - t01 : 0.f;
-            float e10 = (r1 < n && c0 < kOut) ? F.o[2] - t10 : 0.f;
-            float e11 = (r1 < n && c1 < kOut) ? F.o[3] - t11 : 0.f;
-            loss += e00 * e00 + e01 * e01 + e10 * e10 + e11 * e11;
-            dy[0] = gscale * e00; dy[1] = gscale * e01; dy[2] = gscale * e10; dy[3] = gscale * e11;
-            sdy[c0 * kSS + sl0] = __float2bfloat16(dy[0]);
-            sdy[c1 * kSS + sl0] = __float2bfloat16(dy[1]);
-            sdy[c0 * kSS + sl1] = __float2bfloat16(dy[2]);
-            sdy[c1 * kSS + sl1] = __float2bfloat16(dy[3]);
-        }
-        /* dH2 = (dY W3^T) * relu'(H2); dY padded to K = 16 */
-        unsigned ady[4] = {pack2(dy[0], dy[1]), pack2(dy[2], dy[3]), 0u, 0u};
-        float d2[8][4];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            d2[j][0] = d2[j][1] = d2[j][2] = d2[j][3] = 0.f;
-            const __nv_bfloat16 *wp = sm.w3 + (8 * j + g) * kS3 + 2 * c;
-            mma16816(d2[j], ady, ld32(wp), ld32(wp + 8));
-#pragma unroll
-            for (int e = 0; e < 4; ++e) d2[j][e] = F.h2[j][e] > 0.f ? d2[j][e] : 0.f;
-            const int f0 = 8 * j + 2 * c;
-            sd2[f0 * kSS + sl0] = __float2bfloat16(d2[j][0]);
-            sd2[(f0 + 1) * kSS + sl0] = __float2bfloat16(d2[j][1]);
-            sd2[f0 * kSS + sl1] = __float2bfloat16(d2[j][2]);
-            sd2[(f0 + 1) * kSS + sl1] = __float2bfloat16(d2[j][3]);
-        }
-        /* dH1 = (dH2 W2^T) * relu'(H1) */
-        {
-            unsigned a[4][4];
+            unsigned a2[4][4];
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
-                a[s][0] = pack2(d2[2 * s][0], d2[2 * s][1]);
-                a[s][1] = pack2(d2[2 * s][2], d2[2 * s][3]);
-                a[s][2] = pack2(d2[2 * s + 1][0], d2[2 * s + 1][1]);
-                a[s][3] = pack2(d2[2 * s + 1][2], d2[2 * s + 1][3]);
-            }
+                float h[2][4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float d1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const __nv_bfloat16 *wp = sm.w2 + (8 * j + g) * kS2 + 16 * s + 2 * c;
-                    mma16816(d1, a[s], ld32(wp), ld32(wp + 8));
+                for (int u = 0; u < 2; ++u) {
+                    const int j = 2 * s + u;
+                    const float b0v = sm.b2[8 * j + 2 * c], b1v = sm.b2[8 * j + 2 * c + 1];
+                    h[u][0] = b0v; h[u][1] = b1v; h[u][2] = b0v; h[u][3] = b1v;
+                    mma_row64(h[u], a, sm.w2t + (8 * j + row8) * kS2 + 8 * mat);
                 }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) d1[e] = F.h1[j][e] > 0.f ? d1[e] : 0.f;
-                const int f0 = 8 * j + 2 * c;
-                sd1[f0 * kSS + sl0] = __float2bfloat16(d1[0]);
-                sd1[(f0 + 1) * kSS + sl0] = __float2bfloat16(d1[1]);
-                sd1[f0 * kSS + sl1] = __float2bfloat16(d1[2]);
-                sd1[(f0 + 1) * kSS + sl1] = __float2bfloat16(d1[3]);
+                relu_pack(h, s, a2[s], on2);
+                store_t4(sh2 + 16 * s * kSS + st_at, a2[s]);
             }
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) a[s][e] = a2[s][e];
         }
+        float o[4] = {sm.b3[2 * c], sm.b3[2 * c + 1], sm.b3[2 * c], sm.b3[2 * c + 1]};
+        mma_row64(o, a, sm.w3t + row8 * kS2 + 8 * mat);
+        /* dL/dy = 2 (y - t / out_scale) / n for the 3 real outputs of real rows */
+        unsigned ady[4] = {0u, 0u, 0u, 0u}; /* padded to K = 16 */
+        {
+            const float e00 = (r0 < n && in0) ? o[0] - t00 : 0.f;
+            const float e01 = (r0 < n && in1) ? o[1] - t01 : 0.f;
+            const float e10 = (r1 < n && in0) ? o[2] - t10 : 0.f;
+            const float e11 = (r1 < n && in1) ? o[3] - t11 : 0.f;
+            loss += e00 * e00 + e01 * e01 + e10 * e10 + e11 * e11;
+            ady[0] = pack2(gscale * e00, gscale * e01);
+            ady[1] = pack2(gscale * e10, gscale * e11);
+            store_t2(sdy + row8 * kSS + w * 16 + 8 * (mat & 1), ady[0], ady[1]);
+        }
+        /* dH2 = (dY W3^T) * relu'(H2) */
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            unsigned wv[4];
+            load_m4(wv, sm.w3 + (16 * s + 8 * (mat >> 1) + row8) * kS3 + 8 * (mat & 1));
+            float d[2][4] = {};
+            mma16816(d[0], ady, wv[0], wv[1]);
+            mma16816(d[1], ady, wv[2], wv[3]);
+            mask_pack(d, s, on2, a[s]);
+            store_t4(sd2 + 16 * s * kSS + st_at, a[s]);
+        }
+        /* dH1 = (dH2 W2^T) * relu'(H1) */
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            float d[2][4] = {};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) mma_row64(d[u], a, sm.w2 + (8 * (2 * s + u) + row8) * kS2 + 8 * mat);
+            unsigned v[4];
+            mask_pack(d, s, on1, v);
+            store_t4(sd1 + 16 * s * kSS + st_at, v);
+        }
+        mlp_load<kIn / 16>(x, n, (ch + (int)gridDim.x < nchunks ? ch + (int)gridDim.x : ch) * kChunk + w * 16, g, c, xv);
         __syncthreads();
         /* weight gradients of the chunk: K = the 64 samples, 4 k-steps.
          * warp w owns dW2 rows 16w..16w+15, dW3 rows 16w.., dW1 columns 16w.. */
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-            const int k0 = 16 * ks + 2 * c;
-            unsigned ah1[4] = {ld32(sh1 + (16 * w + g) * kSS + k0), ld32(sh1 + (16 * w + g + 8) * kSS + k0),
-                               ld32(sh1 + (16 * w + g) * kSS + k0 + 8), ld32(sh1 + (16 * w + g + 8) * kSS + k0 + 8)};
+            unsigned ah[4], bv[4];
+            load_m4(ah, sh1 + 16 * w * kSS + a_at + 16 * ks);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const __nv_bfloat16 *bp = sd2 + (8 * j + g) * kSS + k0;
-                mma16816(acc2[j], ah1, ld32(bp), ld32(bp + 8));
+            for (int j = 0; j < 8; j += 2) {
+                load_m4(bv, sd2 + 8 * j * kSS + b_at + 16 * ks);
+                mma16816(acc2[j], ah, bv[0], bv[1]);
+                mma16816(acc2[j + 1], ah, bv[2], bv[3]);
             }
-            unsigned ah2[4] = {ld32(sh2 + (16 * w + g) * kSS + k0), ld32(sh2 + (16 * w + g + 8) * kSS + k0),
-                               ld32(sh2 + (16 * w + g) * kSS + k0 + 8), ld32(sh2 + (16 * w + g + 8) * kSS + k0 + 8)};
-            {
-                const __nv_bfloat16 *bp = sdy + g * kSS + k0;
-                const unsigned b0 = ld32(bp), b1 = ld32(bp + 8);
-                mma16816(acc3, ah2, b0, b1);
-                mma16816(accb3, ones, b0, b1);
-            }
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {
-                const __nv_bfloat16 *b2 = sd2 + (8 * (2 * w + jj) + g) * kSS + k0;
-                mma16816(accb2[jj], ones, ld32(b2), ld32(b2 + 8));
-                const __nv_bfloat16 *b1 = sd1 + (8 * (2 * w + jj) + g) * kSS + k0;
-                mma16816(accb1[jj], ones, ld32(b1), ld32(b1 + 8));
-            }
+            load_m4(ah, sh2 + 16 * w * kSS + a_at + 16 * ks);
+            load_m2(bv[0], bv[1], sdy + row8 * kSS + 8 * (mat & 1) + 16 * ks);
+            mma16816(acc3, ah, bv[0], bv[1]);
+            mma16816(accb3, ones, bv[0], bv[1]);
+            load_m4(bv, sd2 + 16 * w * kSS + b_at + 16 * ks);
+            mma16816(accb2[0], ones, bv[0], bv[1]);
+            mma16816(accb2[1], ones, bv[2], bv[3]);
+            load_m4(bv, sd1 + 16 * w * kSS + b_at + 16 * ks);
+            mma16816(accb1[0], ones, bv[0], bv[1]);
+            mma16816(accb1[1], ones, bv[2], bv[3]);
 #pragma unroll
             for (int mt = 0; mt < kIn / 16; ++mt) {
-                const __nv_bfloat16 *xr = sx + 16 * mt * kSS;
-                unsigned axx[4] = {ld32(xr + g * kSS + k0), ld32(xr + (g + 8) * kSS + k0),
-                                   ld32(xr + g * kSS + k0 + 8), ld32(xr + (g + 8) * kSS + k0 + 8)};
-#pragma unroll
-                for (int jj = 0; jj < 2; ++jj) {
-                    const __nv_bfloat16 *bp = sd1 + (8 * (2 * w + jj) + g) * kSS + k0;
-                    mma16816(acc1[mt][jj], axx, ld32(bp), ld32(bp + 8));
-                }
+                load_m4(ah, sx + 16 * mt * kSS + a_at + 16 * ks);
+                mma16816(acc1[mt][0], ah, bv[0], bv[1]);
+                mma16816(acc1[mt][1], ah, bv[2], bv[3]);
             }
         }
         __syncthreads();
