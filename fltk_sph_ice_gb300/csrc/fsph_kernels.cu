@@ -78,41 +78,81 @@ __device__ __forceinline__ unsigned int block_scan(unsigned int v, unsigned int 
     return warp_tot[warp] + incl - v;
 }
 
-/* Scan phase 1: each 1024-thread block scans kScanTile = 4096 counts, four a
- * thread in one 16-byte load (count and out are 16-byte aligned arrays), and
- * zeroes them.  A table of one tile ends here: the block also writes the
- * grand total to out[ncells]. */
-__global__ void __launch_bounds__(1024) k_scan_local(unsigned int *__restrict__ count,
-                                                     unsigned int *__restrict__ out,
-                                                     unsigned int *__restrict__ block_sums, unsigned int ncells) {
+/* Scan phase 1: a block scans kScanTile = 4096 counts and zeroes them; a thread
+ * takes four 16-byte words 4 KB apart (count and out are 16-byte aligned arrays),
+ * all in flight, and the 32 runs of 128 cells meet in one warp.  A table of one
+ * tile ends here: the block also writes the grand total to out[ncells].  With 1024
+ * threads of one word each, two blocks per SM waited at their barriers with
+ * nothing in flight: 32.5 M cells 281 -> 111 us, 280,000 8.1 -> 4.1 (phase 3,
+ * changed the same way, 38 -> 33 and 4.1 -> 3.3). */
+__global__ void __launch_bounds__(kScanBlock) k_scan_local(unsigned int *__restrict__ count,
+                                                           unsigned int *__restrict__ out,
+                                                           unsigned int *__restrict__ block_sums,
+                                                           unsigned int ncells) {
+    __shared__ unsigned int run_tot[32], s_total;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned int base = blockIdx.x * kScanTile + threadIdx.x * 4;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    const bool whole = base + 4 <= ncells;
-    if (whole) {
-        v = *reinterpret_cast<const uint4 *>(count + base);
-        *reinterpret_cast<uint4 *>(count + base) = make_uint4(0u, 0u, 0u, 0u);
-    } else {
-        unsigned int t[4] = {0u, 0u, 0u, 0u};
-        for (int k = 0; k < 4; ++k)
-            if (base + k < ncells) {
-                t[k] = count[base + k];
-                count[base + k] = 0u;
-            }
-        v = make_uint4(t[0], t[1], t[2], t[3]);
+    uint4 v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const unsigned int at = base + r * (kScanBlock * 4);
+        v[r] = make_uint4(0u, 0u, 0u, 0u);
+        if (at + 4 <= ncells) {
+            v[r] = *reinterpret_cast<const uint4 *>(count + at);
+        } else if (at < ncells) {
+            v[r].x = count[at];
+            if (at + 1 < ncells) v[r].y = count[at + 1];
+            if (at + 2 < ncells) v[r].z = count[at + 2];
+        }
     }
-    unsigned int total;
-    const unsigned int run = block_scan(v.x + v.y + v.z + v.w, total);
-    const uint4 r = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
-    if (whole) {
-        *reinterpret_cast<uint4 *>(out + base) = r;
-    } else {
-        const unsigned int t[4] = {r.x, r.y, r.z, r.w};
-        for (int k = 0; k < 4; ++k)
-            if (base + k < ncells) out[base + k] = t[k];
+    unsigned int before[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const unsigned int at = base + r * (kScanBlock * 4);
+        if (at + 4 <= ncells) {
+            *reinterpret_cast<uint4 *>(count + at) = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+            for (unsigned int k = at; k < ncells; ++k) count[k] = 0u;
+        }
+        const unsigned int own = v[r].x + v[r].y + v[r].z + v[r].w;
+        unsigned int incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        before[r] = incl - own;
+        if (lane == 31) run_tot[r * (kScanBlock / 32) + warp] = incl;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned int own = run_tot[lane];
+        unsigned int incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        run_tot[lane] = incl - own;
+        if (lane == 31) s_total = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const unsigned int at = base + r * (kScanBlock * 4);
+        const unsigned int run = run_tot[r * (kScanBlock / 32) + warp] + before[r];
+        const uint4 e = make_uint4(run, run + v[r].x, run + v[r].x + v[r].y, run + v[r].x + v[r].y + v[r].z);
+        if (at + 4 <= ncells) {
+            *reinterpret_cast<uint4 *>(out + at) = e;
+        } else if (at < ncells) {
+            out[at] = e.x;
+            if (at + 1 < ncells) out[at + 1] = e.y;
+            if (at + 2 < ncells) out[at + 2] = e.z;
+        }
     }
     if (threadIdx.x == 0) {
-        block_sums[blockIdx.x] = total;
-        if (gridDim.x == 1) out[ncells] = total;
+        block_sums[blockIdx.x] = s_total;
+        if (gridDim.x == 1) out[ncells] = s_total;
     }
 }
 
@@ -139,25 +179,38 @@ __global__ void __launch_bounds__(1024) k_scan_top(unsigned int *__restrict__ bl
  * still the tiles' own (no phase 2 has run), so the block sums the b totals
  * before it; the last block writes the grand total. */
 template <bool SUM>
-__global__ void __launch_bounds__(1024) k_scan_add(unsigned int *__restrict__ out,
-                                                   const unsigned int *__restrict__ block_sums, unsigned int ncells) {
-    unsigned int add;
+__global__ void __launch_bounds__(kScanBlock) k_scan_add(unsigned int *__restrict__ out,
+                                                         const unsigned int *__restrict__ block_sums,
+                                                         unsigned int ncells) {
+    __shared__ unsigned int s_sum[kScanBlock / 32];
+    const unsigned int base = blockIdx.x * kScanTile + threadIdx.x * 4;
+    uint4 v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const unsigned int at = base + r * (kScanBlock * 4);
+        if (at + 4 <= ncells) v[r] = *reinterpret_cast<const uint4 *>(out + at);
+    }
+    unsigned int add = 0u;
     if (SUM) {
-        unsigned int t = 0;
-        for (unsigned int k = threadIdx.x; k < blockIdx.x; k += 1024u) t += block_sums[k];
-        block_scan(t, add);
+        unsigned int t = 0u;
+        for (unsigned int k = threadIdx.x; k < blockIdx.x; k += kScanBlock) t += block_sums[k];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = t;
+        __syncthreads();
+        for (int w = 0; w < kScanBlock / 32; ++w) add += s_sum[w];
         if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) out[ncells] = add + block_sums[blockIdx.x];
     } else {
         add = block_sums[blockIdx.x];
     }
-    const unsigned int base = blockIdx.x * kScanTile + threadIdx.x * 4;
-    if (base + 4 <= ncells) {
-        uint4 v = *reinterpret_cast<const uint4 *>(out + base);
-        v.x += add; v.y += add; v.z += add; v.w += add;
-        *reinterpret_cast<uint4 *>(out + base) = v;
-    } else {
-        for (int k = 0; k < 4; ++k)
-            if (base + k < ncells) out[base + k] += add;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const unsigned int at = base + r * (kScanBlock * 4);
+        if (at + 4 <= ncells) {
+            v[r].x += add; v[r].y += add; v[r].z += add; v[r].w += add;
+            *reinterpret_cast<uint4 *>(out + at) = v[r];
+        } else {
+            for (unsigned int k = at; k < ncells; ++k) out[k] += add;
+        }
     }
 }
 
@@ -1271,17 +1324,17 @@ void launch_hash(const DevParams &p, const float4 *x, unsigned int *key, unsigne
 void launch_scan(unsigned int *count, unsigned int *cell_start, unsigned int *block_sums, unsigned int ncells,
                  cudaStream_t s) {
     const unsigned int nb = scan_blocks(ncells);
-    k_scan_local<<<nb, 1024, 0, s>>>(count, cell_start, block_sums, ncells);
+    k_scan_local<<<nb, kScanBlock, 0, s>>>(count, cell_start, block_sums, ncells);
     if (nb == 1) return;
     /* Up to kScanSum tiles every block of the last phase sums the totals before
-     * it itself (at most kScanSum / 1024 loads a thread) instead of a phase of
+     * it itself (at most kScanSum / kScanBlock loads a thread) instead of a phase of
      * one block between the two: a launch less, about 4 us of each grid build.
      * Past it those loads (nb^2 / 2 words in all) cost more than the launch. */
     if (nb <= kScanSum) {
-        k_scan_add<true><<<nb, 1024, 0, s>>>(cell_start, block_sums, ncells);
+        k_scan_add<true><<<nb, kScanBlock, 0, s>>>(cell_start, block_sums, ncells);
     } else {
         k_scan_top<<<1, 1024, 0, s>>>(block_sums, nb, cell_start, ncells);
-        k_scan_add<false><<<nb, 1024, 0, s>>>(cell_start, block_sums, ncells);
+        k_scan_add<false><<<nb, kScanBlock, 0, s>>>(cell_start, block_sums, ncells);
     }
 }
 bool launch_small_grid(const DevParams &p, unsigned int ncells, const float4 *x4, float4 *x_out, unsigned int *order,
