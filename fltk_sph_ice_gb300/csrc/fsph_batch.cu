@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kListBlock) kb_build_list(BatchArgs b, const u
         const DevParams p = s_p;
         for (int o = 0; o < tl.count; o += kListBlock) {
             const int at = o + (int)threadIdx.x;
-            build_list_warp(p, tl.start + at, at < tl.count, cell_start, xb, cellb, list, cnt,
+            build_list_warp<1>(p, tl.start + at, at < tl.count, cell_start, xb, cellb, list, cnt,
                             s_tile[threadIdx.x >> 5]);
         }
     }

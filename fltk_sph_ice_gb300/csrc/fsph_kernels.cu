@@ -378,15 +378,15 @@ __global__ void k_rebuild_copy(int n, DevCtl *ctl, const float4 *__restrict__ t_
 /* neighbour lists                                                          */
 /* ======================================================================== */
 
-/* The lists of every slot, a warp for 32 consecutive ones (build_list_warp). */
-__global__ void __launch_bounds__(kListBlock) k_build_list(DevParams p, const unsigned int *__restrict__ cell_start,
-                                                           const float4 *__restrict__ xb,
-                                                           const unsigned int *__restrict__ cellb,
-                                                           ListEntry *__restrict__ list,
-                                                           unsigned char *__restrict__ cnt) {
-    __shared__ PairTile s_tile[kListBlock / 32];
-    const int i = blockIdx.x * kListBlock + threadIdx.x;
-    build_list_warp(p, i, i < p.n, cell_start, xb, cellb, list, cnt, s_tile[threadIdx.x >> 5]);
+/* The lists of every slot, W warps for 32 consecutive ones (build_list_warp). */
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
+    k_build_list(DevParams p, const unsigned int *__restrict__ cell_start, const float4 *__restrict__ xb,
+                 const unsigned int *__restrict__ cellb, ListEntry *__restrict__ list,
+                 unsigned char *__restrict__ cnt) {
+    __shared__ PairTileOf<W> s_tile[W == 1 ? kListBlock / 32 : 1];
+    const int i = W == 1 ? blockIdx.x * kListBlock + threadIdx.x : blockIdx.x * 32 + (threadIdx.x & 31);
+    build_list_warp<W>(p, i, i < p.n, cell_start, xb, cellb, list, cnt, s_tile[W == 1 ? threadIdx.x >> 5 : 0]);
 }
 
 /* ======================================================================== */
@@ -708,6 +708,31 @@ void launch_boundary_lambda(const DevParams &p, const unsigned int *cell_start, 
     k_boundary_lambda<<<blocks_for(p.nb), kBlock, 0, s>>>(p, cell_start, ppos0, ppos1, ctl, bstat, blam);
 }
 
+/* Sums and products of two floats without their rounding errors: the result
+ * and its error (Knuth; Dekker; the product's error from one fused operation),
+ * with no contraction by the compiler. */
+struct Split {
+    float h, l; /* the value is h + l */
+};
+__device__ __forceinline__ Split two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    return Split{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
+__device__ __forceinline__ Split two_diff(float a, float b) { return two_sum(a, -b); }
+__device__ __forceinline__ Split two_prod(float a, float b) {
+    const float q = __fmul_rn(a, b);
+    return Split{q, __fmaf_rn(a, b, -q)};
+}
+/* h + l with the error of the sum kept (|h| >= |l| or h = 0) */
+__device__ __forceinline__ Split renorm(float h, float l) {
+    const float s = __fadd_rn(h, l);
+    return Split{s, __fsub_rn(l, __fsub_rn(s, h))};
+}
+__device__ __forceinline__ Split split_of(double v) {
+    const float h = (float)v;
+    return Split{h, (float)(v - (double)h)};
+}
+
 /* ======================================================================== */
 /* WCSPH                                                                    */
 /* ======================================================================== */
@@ -728,35 +753,45 @@ __device__ __forceinline__ void sph_density_out(const DevParams &p, int i, float
     reinterpret_cast<float *>(pos + i)[3] = prs / (rho * rho);
     reinterpret_cast<float *>(vel + i)[3] = 1.0f / rho;
 }
-/* A warp for 32 consecutive slots: its candidates from the tile
+/* W warps for 32 consecutive slots: their candidates from the tile
  * (warp_candidates), each evaluated from a gathered position, four at a time,
  * and listed; where they do not fit the tile, a thread's own walk.  A thread
  * testing all its candidates was bound by issue and took 205 us at 1,030,301
  * slots and 64.6 at 262,144, this form 171 and 59.5. */
-__global__ void __launch_bounds__(kListBlock) k_sph_density(DevParams p, const unsigned int *__restrict__ cell_start,
-                                                            float4 *pos, float4 *vel, float *__restrict__ dens,
-                                                            float *__restrict__ pres, ListEntry *__restrict__ list,
-                                                            unsigned char *__restrict__ cnt) {
-    __shared__ PairTile s_tile[kListBlock / 32];
-    PairTile &t = s_tile[threadIdx.x >> 5];
-    const int i = blockIdx.x * kListBlock + threadIdx.x;
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
+    k_sph_density(DevParams p, const unsigned int *__restrict__ cell_start, float4 *pos, float4 *vel,
+                  float *__restrict__ dens, float *__restrict__ pres, ListEntry *__restrict__ list,
+                  unsigned char *__restrict__ cnt) {
+    __shared__ PairTileOf<W> s_tile[W == 1 ? kListBlock / 32 : 1];
+    const int i = W == 1 ? blockIdx.x * kListBlock + threadIdx.x : blockIdx.x * 32 + (threadIdx.x & 31);
     const bool valid = i < p.n;
     const float3 xi = valid ? f3(pos[i]) : make_float3(0.f, 0.f, 0.f);
     const int3 c = cell_of(xi, p);
-    float acc[4] = {}; /* four partial sums: their error is no larger than that of the lanes' */
-    auto add = [&](float &sum, const float4 &xj) {
+    /* W = 1: four partial sums, whose error is no larger than that of the lanes'; a
+     * warp of several holds whole rows of cells, of very different weight, and keeps
+     * its sum's error beside it */
+    float acc[4] = {};
+    auto add = [&](int u, const float4 &xj) {
         const float3 d = xi - f3(xj);
         const float r2 = dot3(d, d);
         if (r2 < p.h2) {
             const float q = p.h2 - r2;
-            sum += q * q * q;
+            if (W == 1) {
+                acc[u] += q * q * q;
+            } else {
+                const float y = q * q * q - acc[1], s = acc[0] + y;
+                acc[1] = (s - acc[0]) - y;
+                acc[0] = s;
+            }
         }
         return r2;
     };
     warp_candidates(
-        p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.rl2, t,
-        [&](bool found, int count, TileWalk &walk) {
+        p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.rl2, s_tile[W == 1 ? threadIdx.x >> 5 : 0],
+        [&](bool found, int first, int count, int total, TileWalk<W> &walk) {
             if (found) {
+                unsigned int last = 0u;
                 for (int k = 0; k < count; k += 4) {
                     unsigned int v[4];
                     float4 xj[4];
@@ -764,12 +799,24 @@ __global__ void __launch_bounds__(kListBlock) k_sph_density(DevParams p, const u
                     for (int u = 0; u < 4; ++u) v[u] = walk.next(); /* the last group is padded with its last entry */
 #pragma unroll
                     for (int u = 0; u < 4; ++u) xj[u] = pos[v[u]];
-                    if (list && k < kListMax)
-                        reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
-                            make_uint4(v[0], v[1], v[2], v[3]);
+                    if (W == 1) {
+                        if (list && k < kListMax)
+                            reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
+                                make_uint4(v[0], v[1], v[2], v[3]);
+                    } else if (list) {
+                        last = v[3];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (k + u < count && first + k + u < kListMax) list[list_at(first + k + u, i, p.n)] = v[u];
+                    }
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        if (k + u < count) add(acc[u], xj[u]);
+                        if (k + u < count) add(u, xj[u]);
+                }
+                if (W > 1) {
+                    if (list && count && first + count == total && total < kListMax)
+                        for (int k = total; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = last;
+                    count = total;
                 }
             } else {
                 unsigned int last = (unsigned int)i;
@@ -779,7 +826,7 @@ __global__ void __launch_bounds__(kListBlock) k_sph_density(DevParams p, const u
                         unsigned int s, e;
                         row_range(cell_start, c, dy, dz, p, s, e);
                         for (unsigned int j = s; j < e; ++j) {
-                            if (!(add(acc[0], pos[j]) < p.rl2)) continue;
+                            if (!(add(0, pos[j]) < p.rl2)) continue;
                             last = j;
                             if (list && count < kListMax) list[list_at(count, i, p.n)] = last;
                             ++count;
@@ -788,9 +835,19 @@ __global__ void __launch_bounds__(kListBlock) k_sph_density(DevParams p, const u
                 if (list && count <= kListMax) /* pad the last group (the slot itself is always listed) */
                     for (int k = count; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = last;
             }
-            if (list) cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
-            sph_density_out(p, i, (acc[0] + acc[1]) + (acc[2] + acc[3]), pos, vel, dens, pres);
+            if (list && (W == 1 || threadIdx.x < 32u)) cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
+            if (W == 1) sph_density_out(p, i, (acc[0] + acc[1]) + (acc[2] + acc[3]), pos, vel, dens, pres);
         });
+    if (W > 1) {
+        __shared__ double s_sum[W][32];
+        s_sum[threadIdx.x >> 5][threadIdx.x & 31] = (double)acc[0] - (double)acc[1];
+        __syncthreads();
+        if (threadIdx.x >= 32u || !valid) return;
+        double sum = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) sum += s_sum[w][threadIdx.x];
+        sph_density_out(p, i, (float)sum, pos, vel, dens, pres);
+    }
 }
 
 /* k_sph_density with LPP lanes per particle, so that small scenes still
@@ -843,7 +900,17 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
                 }
             }
         }
-    acc = group_sum<LPP>(acc);
+    /* the lanes' sums, each addition's error kept: LPP = 16 or 32 lanes add more
+     * often than the 8 that were the most before */
+    float err = 0.0f;
+#pragma unroll
+    for (int o = LPP / 2; o > 0; o >>= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, acc, o);
+        const Split t = two_sum(acc, other);
+        err += __shfl_xor_sync(0xffffffffu, err, o) + t.l;
+        acc = t.h;
+    }
+    acc += err;
     if (!valid || sub != 0) return;
     if (list) {
         const bool ovf = k > kListMax;
@@ -948,7 +1015,7 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
     const int3 c = cell_of(xi, p);
     unsigned int k = 0;
     warp_candidates(p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
-                    [&](bool found, int count, TileWalk &walk) {
+                    [&](bool found, int, int count, int, TileWalk<1> &walk) {
                         auto meet = [&](unsigned int j) {
                             if (ref_neighbor(xi, f3(__ldg(pos + j)), p.h2)) {
                                 if (k < (unsigned int)kListMax) list[list_at((int)k, i, p.n)] = j;
@@ -1116,31 +1183,6 @@ __global__ void k_gather_rows(int n, const unsigned int *__restrict__ perm, cons
 /* ======================================================================== */
 /* density on a lattice (for meshing)                                       */
 /* ======================================================================== */
-
-/* Sums and products of two floats without their rounding errors: the result
- * and its error (Knuth; Dekker; the product's error from one fused operation),
- * with no contraction by the compiler. */
-struct Split {
-    float h, l; /* the value is h + l */
-};
-__device__ __forceinline__ Split two_sum(float a, float b) {
-    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-    return Split{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
-__device__ __forceinline__ Split two_diff(float a, float b) { return two_sum(a, -b); }
-__device__ __forceinline__ Split two_prod(float a, float b) {
-    const float q = __fmul_rn(a, b);
-    return Split{q, __fmaf_rn(a, b, -q)};
-}
-/* h + l with the error of the sum kept (|h| >= |l| or h = 0) */
-__device__ __forceinline__ Split renorm(float h, float l) {
-    const float s = __fadd_rn(h, l);
-    return Split{s, __fsub_rn(l, __fsub_rn(s, h))};
-}
-__device__ __forceinline__ Split split_of(double v) {
-    const float h = (float)v;
-    return Split{h, (float)(v - (double)h)};
-}
 
 /* The density field at the nodes of an nx x ny x nz lattice (i fastest),
  * node (i, j, k) at minp + (i, j, k) d: 0 outside [lo, hi], else
@@ -1434,10 +1476,17 @@ void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *p
                                                         (cudaGraphConditionalHandle)while_handle, use_graph,
                                                         p.use_lists ? nl.list : nullptr, nl.cnt);
 }
+/* The list build: four warps / one warp for 32 slots take, in us, 10.3 / 16.4 at
+ * 6,912 slots, 12.3 / 15.8 at 16,384, 16.5 / 20.5 at 32,000, 19.5 / 17.2 at 42,592,
+ * 23.0 / 18.5 at 62,500 (two 18.5 at 32,000, eight 20.5). */
+constexpr int kListSplitMax = 1 << 15;
 void launch_build_list(const DevParams &p, const unsigned int *cell_start, const float4 *xb, const NbrLists &nl,
                        cudaStream_t s) {
     if (!p.use_lists) return;
-    k_build_list<<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, xb, nl.cellb, nl.list, nl.cnt);
+    if (p.n <= kListSplitMax)
+        k_build_list<4><<<blocks_for(p.n, 32), 128, 0, s>>>(p, cell_start, xb, nl.cellb, nl.list, nl.cnt);
+    else
+        k_build_list<1><<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, xb, nl.cellb, nl.list, nl.cnt);
 }
 void launch_correction(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                        const float4 *xb, DevCtl *ctl, float *part, unsigned long long if_handle,
@@ -1494,17 +1543,21 @@ static int lanes_to_fill(int n, int most) {
     return lanes;
 }
 static int sph_force_lanes(int n) { return lanes_to_fill(n, 8); }
-/* The density pass takes a warp's tile from here on, lanes of a particle's own
- * candidates below, where a warp for 32 slots leaves SMs without work: at
- * 15,625 slots the tile takes 22.5 us and 16 lanes 14.7, at 32,768 the tile and
- * 8 lanes 22.7 each, at 64,000 29.1 and (4 lanes) 51.3.  With at most 8 lanes the
- * pass took 16.4 us at 4,096 slots, with 32 it takes 8.2. */
-constexpr int kSphTileMin = 1 << 15;
+/* The density pass by size, us at 8,000 / 15,625 / 32,768 / 64,000 / 125,000 /
+ * 262,144 slots: lanes of a particle's own candidates (up to 32) 10.9 / 16.3 /
+ * 22.7 / 51.3 / - / -, four warps for the tile of 32 slots 14.4 / 14.3 / 16.4 /
+ * 28.2 / 45.5 / 84.5, one warp 20.5 / 22.5 / 22.8 / 28.8 / 36.9 / 59.6; at 4,096
+ * the lanes take 8.7 (16.4 when they were at most eight). */
+constexpr int kSphTileMin = 12288, kSphSplitMax = 1 << 16;
 void launch_sph_density(const DevParams &p, const unsigned int *cell_start, float4 *pos, float4 *vel, float *dens,
                         float *pres, const NbrLists &nl, cudaStream_t s) {
     ListEntry *l = p.use_lists ? nl.list : nullptr;
+    if (p.n > kSphSplitMax) {
+        k_sph_density<1><<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
+        return;
+    }
     if (p.n >= kSphTileMin) {
-        k_sph_density<<<blocks_for(p.n, kListBlock), kListBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
+        k_sph_density<4><<<blocks_for(p.n, 32), 128, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
         return;
     }
     const int lanes = lanes_to_fill(p.n, 32);

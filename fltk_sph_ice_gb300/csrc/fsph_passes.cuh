@@ -300,11 +300,14 @@ __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const
  * masks and the rows' stores it takes 125, without the matrix instructions too 93:
  * reading, converting and staging the candidates is what is left. */
 constexpr int kTileWords = 32; /* masks of a warp's candidates: 32 x 32 slots */
-struct __align__(16) PairTile {
-    uint4 row[32];                      /* operand rows, eight terms each */
+template <int W> /* the warps that share it */
+struct __align__(16) PairTileOf {
+    uint4 row[W][32];                   /* operand rows, eight terms each */
     unsigned int mask[kTileWords][32];  /* [w][lane], bit 31 - k: candidate k of word w is within the radius */
     unsigned int slot[kTileWords][32];  /* [w][k]: the candidates' slots */
+    int cnt[W][32];                     /* what each warp found for a lane's slot (W > 1) */
 };
+using PairTile = PairTileOf<1>;
 
 __device__ __forceinline__ unsigned int half_pair(float lo, float hi) {
     const __half2 v = __floats2half2_rn(lo, hi);
@@ -360,12 +363,13 @@ __device__ __forceinline__ void test_tile(unsigned int &m0, unsigned int &m1, un
 /* One lane's candidates of a tile, ascending.  next() gives the `left`-th from the
  * end; called again after the last it keeps giving that one.  Selects instead of
  * branches: at almost every call some lane of a warp opens its next word. */
+template <int W>
 struct TileWalk {
-    const PairTile &t;
+    const PairTileOf<W> &t;
     unsigned int some, m = 0u;
     int w = 0, left;
     unsigned int last = 0u;
-    __device__ __forceinline__ TileWalk(const PairTile &tile, unsigned int words, int count)
+    __device__ __forceinline__ TileWalk(const PairTileOf<W> &tile, unsigned int words, int count)
         : t(tile), some(words), left(count) {}
     __device__ __forceinline__ unsigned int next() {
         const bool open = m == 0u;
@@ -383,27 +387,33 @@ struct TileWalk {
     }
 };
 
-/* Calls emit(found, count, walk) once for each valid lane: found: the lane's
- * `count` candidates against x4 within sqrt(r2max) come from walk, ascending;
- * else they have to be looked for without the tile (more than fit it, or a
+/* Calls emit(found, first, count, total, walk) once for each valid lane: found:
+ * the lane's `count` candidates against x4 within sqrt(r2max) come from walk,
+ * ascending; else they have to be looked for without the tile (more than fit it, or a
  * coordinate out of the operands' range: a particle far outside the box, or not
  * a number).  xi, cell: the lane's position and build cell, cells ascending over
  * the lanes, padding lanes (valid = false) after the valid ones; every lane of
  * the warp calls it.  Lanes in different rows of cells, or more than eight cells
  * apart (a run that wraps, sparse fluid), take turns: a row's range then never
  * reaches the next row, and no slot is met twice.  As many turns as fit the tile
- * are emitted together. */
-template <class Emit>
+ * are emitted together.
+ * W > 1: the W warps of a block share the same 32 slots (a lane's slot is the same
+ * in each) and the tile.  Each takes a W-th of every turn's words and emits what
+ * it found there: `count` of the lane's `total`, from the `first` on; what is not
+ * found is warp 0's alone.  A warp's twenty words in a row, latency bound, are the
+ * pass of a small scene: 16 us at 6,912 slots with one warp, 10 with four. */
+template <int W, class Emit>
 __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                                 const float4 *__restrict__ x4, float3 xi, unsigned int cell,
-                                                bool valid, float r2max, PairTile &t, Emit &&emit) {
-    const int lane = threadIdx.x & 31;
+                                                bool valid, float r2max, PairTileOf<W> &t, Emit &&emit) {
+    const int lane = threadIdx.x & 31, wid = W > 1 ? (int)(threadIdx.x >> 5) : 0;
+    uint4 *const rows = t.row[wid];
     const unsigned int row = (cell - p.cell_off) / (unsigned int)p.gx;
     const float inv = rsqrtf(r2max);
     /* candidate 8 q + 2 s + b is column 2 q + b of step s; the rows are stored so
      * that neither the stores nor the loads of eight rows collide */
-    uint4 *const st = t.row + 8 * (lane >> 3) + 2 * ((lane >> 3) ^ ((lane >> 1) & 3)) + (lane & 1);
-    const uint4 *const ld = t.row + 8 * ((lane & 7) >> 1) + 2 * (((lane & 7) >> 1) ^ (lane >> 3)) + (lane & 1);
+    uint4 *const st = rows + 8 * (lane >> 3) + 2 * ((lane >> 3) ^ ((lane >> 1) & 3)) + (lane & 1);
+    const uint4 *const ld = rows + 8 * ((lane & 7) >> 1) + 2 * (((lane & 7) >> 1) ^ (lane >> 3)) + (lane & 1);
     const unsigned int pick1 = (lane & 2) ? 0x3726u : 0x5140u, pick2 = (lane & 1) ? 0x6273u : 0x0415u;
     const unsigned int ones = 0x3c003c00u; /* (1, 1) */
     const bool upper = (lane & 2) != 0;    /* terms 12-15 of a candidate are ones, 8-11 its terms 0-3 again */
@@ -460,14 +470,14 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 const unsigned int h0 = times_m2(v.h0), h1 = times_m2(v.h1), l0 = times_m2(v.l0), l1 = times_m2(v.l1);
                 const unsigned int z1 = (h1 & 0xffffu) | (ones & 0xffff0000u); /* (-2 zh, 1) */
                 __syncwarp(); /* the last operands of the turn before have been read */
-                t.row[lane] = make_uint4(h0, z1, h0, z1);
+                rows[lane] = make_uint4(h0, z1, h0, z1);
                 __syncwarp();
-                load_matrices(a0, t.row + lane);
+                load_matrices(a0, rows + lane);
                 __syncwarp();
-                t.row[lane] = make_uint4(l0, l1 & 0xffffu, __byte_perm(v.h1, v.l1, 0x7632),
+                rows[lane] = make_uint4(l0, l1 & 0xffffu, __byte_perm(v.h1, v.l1, 0x7632),
                                          half_pair(-1.0f, -0x1p-12f));
                 __syncwarp();
-                load_matrices(a1, t.row + lane);
+                load_matrices(a1, rows + lane);
             }
             const bool keep = (grp >> own & 1u) != 0u;
             int r = 0;
@@ -485,13 +495,19 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 /* past the last candidate: some slot's position, not used */
                 return __ldg(x4 + min(q < total ? j : j - (q - total + 1u), (unsigned int)p.n - 1u));
             };
+            /* this warp's words */
+            const unsigned int words = (total + 31u) >> 5;
+            const unsigned int begin = W > 1 ? words * wid / W * 32u : 0u;
+            const unsigned int end = W > 1 ? min(total, words * (wid + 1) / W * 32u) : total;
             unsigned int jn;
-            float4 cn = fetch(0u, jn);
+            float4 cn;
+            if (W == 1 || begin < end) cn = fetch(begin, jn);
 #pragma unroll 1
-            for (unsigned int q0 = 0u; q0 < total; q0 += 32u, ++w) {
+            for (unsigned int q0 = begin; q0 < end; q0 += 32u, w += W == 1 ? 1 : 0) {
+                const int at = W == 1 ? w : w + (int)(q0 >> 5);
                 const unsigned int q = q0 + (unsigned int)lane, j = jn;
                 const float4 c = cn;
-                if (q0 + 32u < total) cn = fetch(q0 + 32u, jn);
+                if (q0 + 32u < end) cn = fetch(q0 + 32u, jn);
                 PairTerms v{0x4f804f80u, 0x4f804f80u, 0u, 0u, 0.0f}; /* past the last candidate: 30 30 30, far away */
                 if (q < total) {
                     v = pair_terms((c.x - ox) * inv, (c.y - oy) * inv, (c.z - oz) * inv);
@@ -501,7 +517,7 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 bad |= !(v.nn <= 64.0f);
                 __syncwarp(); /* the operands of the last word have been read */
                 *st = make_uint4(v.h0, v.h1, v.l0, v.l1);
-                t.slot[w][lane] = j;
+                t.slot[at][lane] = j;
                 __syncwarp();
                 unsigned int b[4];
                 load_matrices(b, ld);
@@ -518,48 +534,81 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 2), pick1);
                 m = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 1), pick2);
                 if (!keep) m = 0u;
-                t.mask[w][own] = m;
+                t.mask[at][own] = m;
                 cnt += __popc(m);
-                if (m) any |= 0x80000000u >> w;
+                if (m) any |= 0x80000000u >> at;
             }
+            if (W > 1) w += (int)words;
         } while (todo);
-        __syncwarp();
         const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
         const int count = __shfl_sync(0xffffffffu, cnt, holder);
         const unsigned int some = __shfl_sync(0xffffffffu, any, holder);
-        const bool found = !over && !__any_sync(0xffffffffu, bad);
-        if (done >> lane & 1u) {
-            TileWalk walk(t, some, count);
-            emit(found, count, walk);
+        int first = 0, all = count;
+        bool found = !over;
+        if (W > 1) {
+            t.cnt[wid][lane] = count;
+            found = !__syncthreads_or(bad) && found;
+            all = 0;
+#pragma unroll
+            for (int v = 0; v < W; ++v) {
+                const int n = t.cnt[v][lane];
+                if (v < wid) first += n;
+                all += n;
+            }
+        } else {
+            found = !__any_sync(0xffffffffu, bad) && found;
+            __syncwarp();
         }
-        __syncwarp(); /* the tile is free again */
+        if ((done >> lane & 1u) && (found || wid == 0)) {
+            TileWalk<W> walk(t, some, count);
+            emit(found, first, count, all, walk);
+        }
+        /* the tile is free again */
+        if (W > 1)
+            __syncthreads();
+        else
+            __syncwarp();
     }
 }
 
 /* The lists of a warp's 32 consecutive slots (i ascending over the lanes,
  * padding lanes last).  The entries leave four at a time, one 16-byte store
- * per lane and 512 consecutive bytes per warp. */
+ * per lane and 512 consecutive bytes per warp; with W > 1 warps for the slots
+ * one by one. */
+template <int W>
 __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool valid,
                                                 const unsigned int *__restrict__ cell_start,
                                                 const float4 *__restrict__ xb,
                                                 const unsigned int *__restrict__ cellb, ListEntry *__restrict__ list,
-                                                unsigned char *__restrict__ cnt, PairTile &t) {
+                                                unsigned char *__restrict__ cnt, PairTileOf<W> &t) {
     const float3 xi = valid ? f3(__ldg(xb + i)) : make_float3(0.f, 0.f, 0.f);
     const unsigned int cell = valid ? __ldg(cellb + i) : 0u;
-    warp_candidates(p, cell_start, xb, xi, cell, valid, p.rl2, t, [&](bool found, int count, TileWalk &walk) {
+    warp_candidates(p, cell_start, xb, xi, cell, valid, p.rl2, t,
+                    [&](bool found, int first, int count, int total, TileWalk<W> &walk) {
         if (!found) {
             build_list_body(p, i, cell_start, xb, cell, list, cnt);
             return;
         }
-        const int most = min(count, kListMax);
-        for (int k = 0; k < most; k += 4) {
-            unsigned int v[4];
+        if (W == 1) {
+            const int most = min(count, kListMax);
+            for (int k = 0; k < most; k += 4) {
+                unsigned int v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = walk.next(); /* the last group is padded with its last entry */
-            reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
-                make_uint4(v[0], v[1], v[2], v[3]);
+                for (int u = 0; u < 4; ++u) v[u] = walk.next(); /* the last group is padded with its last entry */
+                reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
+                    make_uint4(v[0], v[1], v[2], v[3]);
+            }
+        } else {
+            unsigned int v = 0u;
+            const int most = min(first + count, kListMax);
+            for (int k = first; k < most; ++k) {
+                v = walk.next();
+                list[list_at(k, i, p.n)] = v;
+            }
+            if (count && first + count == total && total < kListMax) /* pad the last group */
+                for (int k = total; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = v;
         }
-        cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
+        if (W == 1 || threadIdx.x < 32u) cnt[i] = total > kListMax ? kListOverflow : (unsigned char)total;
     });
 }
 

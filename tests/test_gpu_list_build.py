@@ -37,7 +37,7 @@ def _scene(kind, n, seed):
 
 
 @pytest.mark.parametrize("kind", ["sparse", "thin", "flat", "clumped", "dense"])
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 161, 2500])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 161, 2500, 32768, 32801])
 def test_lists_step_as_the_cell_walk(gpu, kind, n):
     p, x = _scene(kind, n, n)
     got = []

@@ -1,4 +1,4 @@
-"""The WCSPH density pass on both sides of the size where it changes form, with
+"""The WCSPH density pass on both sides of the sizes where it changes form, with
 full and ragged warps, sparse fluid (a warp's slots in many cells) and clumps
 (more neighbours than a list or a tile holds): density, and the forces of the
 lists that the pass leaves, against 64 bits."""
@@ -36,7 +36,7 @@ def _scene(kind, n):
 
 
 @pytest.mark.parametrize("kind", ["lattice", "sparse", "clumped"])
-@pytest.mark.parametrize("n", [1, 33, 5000, 9000, 32767, 32768, 32801])
+@pytest.mark.parametrize("n", [1, 33, 5000, 9000, 12287, 12288, 32767, 32801, 65536, 65537])
 def test_density_and_forces_against_64_bits(gpu, kind, n):
     """A density term (h^2 - r^2)^3 <= h^6 is rounded fewer than 20 times at its
     full size, a sum of k terms k times at most; a force term is rounded fewer
