@@ -48,3 +48,28 @@ def test_lattices_against_64_bits(gpu, n, h):
     top = _field(x[:, :3].astype(np.float64), (1, 1, 1), x[60, :3].astype(float), d, float(p.h), float(p.mass), lo,
                  hi).max()
     assert np.abs(got - want).max() <= 8.4e-6 * max(want.max(), 0.1 * top)
+
+
+@pytest.mark.parametrize("d", [0.11, 0.5, 1.0, 1.3, 1.4, 2.2])
+def test_spacings_on_both_sides_of_the_shared_bricks(gpu, d):
+    """Nodes from far denser than the particles to ones that share no neighbour:
+    the bricks' common set (in several goes where they are large) and the lanes'
+    own walks."""
+    h = 0.0457
+    rng = np.random.default_rng(int(100 * d))
+    m = 14
+    s = 0.5 * h
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    x = np.zeros((m ** 3, 4), np.float32)
+    x[:, :3] = (g + 0.8) * s + rng.uniform(-0.3, 0.3, (m ** 3, 3)) * s
+    box = [(m + 2) * s] * 3
+    p = scenes.pbf_params(h, [0.0] * 3, box, m ** 3, particle_radius=0.25 * h)
+    p.mass = scenes.lattice_mass(h, s)
+    ps = rxPBDSPH(p)
+    ps.Set(x)
+    n = [min(int(b / (d * h)), 22) for b in box]
+    got = ps.CalImplicitField(n, [0.1 * h] * 3, [d * h] * 3)
+    ps.close()
+    lo, hi = [-0.005 * b for b in box], [b + 0.005 * b for b in box]
+    want = _field(x[:, :3].astype(np.float64), n, [0.1 * h] * 3, [d * h] * 3, float(p.h), float(p.mass), lo, hi)
+    assert np.abs(got - want).max() <= 8.4e-6 * want.max()
