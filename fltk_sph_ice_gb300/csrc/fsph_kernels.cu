@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(DEEP ? kDeepBlock : kPassBlock, DEEP ? kDeepMi
  * allocation-free entry point, which keeps no lists.  One thread a particle
  * leaves 8 blocks and a serial walk of 290 candidates at 4,096 particles (47 us);
  * with 32 lanes a row of cells is one coalesced step.  The whole call went from
- * 84 to 36 us at 4,096 particles.  The sums are the lanes' partial sums, as in
+ * 84 to 36 us at 4,096 particles (21 with the grid built by one block).  The sums are the lanes' partial sums, as in
  * the batched passes with several lanes. */
 template <int LPP>
 __global__ void __launch_bounds__(kBlock) k_lambda_walk(DevParams p, const unsigned int *__restrict__ cell_start,
@@ -865,7 +865,7 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
     const int sub = t % LPP, lane = threadIdx.x & 31;
     const bool valid = t / LPP < p.n;
     const int i = valid ? t / LPP : p.n - 1; /* padding groups walk a real slot and write nothing */
-    const unsigned int gmask = ((1u << LPP) - 1u) << (lane & ~(LPP - 1));
+    const unsigned int gmask = (0xffffffffu >> (32 - LPP)) << (lane & ~(LPP - 1));
     const float3 xi = f3(pos[i]);
     const int3 c = cell_of(xi, p);
     float acc = 0.0f;

@@ -27,7 +27,7 @@ constexpr int kDeepBlock = 64, kDeepMinB = 12, kDeepMax = 65536;
  * candidates in flight; with registers for five or six blocks of 256 per SM 867
  * and 914. */
 constexpr int kPostBlock = 128;
-constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 8.7 KB each */
+constexpr int kListBlock = 128; /* threads per block of the list build: four warps with a tile of 8.8 KB each */
 constexpr int kBlockMax = 512;  /* largest block of the batched persistent kernels */
 constexpr int kScanTile = 4096, kScanBlock = 256; /* cells and threads per block of the first scan phase */
 constexpr unsigned int kScanSum = 2048; /* tiles up to which the scan runs in two phases */
