@@ -8,9 +8,9 @@
  * group and the positions behind each, the block partials and their last
  * block) and the launches themselves.  k_pbf_loop keeps every particle on
  * its own thread for all iterations: its position and lambda stay in
- * registers, its list in shared memory (16-bit slots), so a pass is one round
- * of gathers, up to sixteen in flight, and a barrier over the grid.  Measured,
- * an iteration of 6,912 particles takes 12.3 us instead of 23.5 (31 before the
+ * registers, its list in shared memory (16-bit slots), so a pass is a few rounds
+ * of gathers and a barrier over the grid.  Measured,
+ * an iteration of 6,912 particles takes 10.7 us instead of 23.5 (31 before the
  * passes had their form for few warps), of 32,000 13.3 instead of 27.3.
  *
  * From there on a launch of its own still costs each pass about 8 us (launch, a
@@ -73,8 +73,14 @@ __device__ __forceinline__ bool grid_wait(const DevParams &p, LoopCtl *lc, unsig
 }
 
 /* One particle's candidates from its list in shared memory (two 16-bit slots a
- * word, word w of a thread at [w * BLOCK]), the next eight gathers in flight while
- * eight are evaluated; an overflowed list walks the cells. */
+ * word, word w of a thread at [w * BLOCK]); an overflowed list walks the cells.
+ * Blocks of 64 threads are up to two per SM, with registers to spare and no other
+ * warp to hide a load: 24 gathers leave together, two rounds for most particles.
+ * In larger blocks the next eight are in flight while eight are evaluated.  An
+ * iteration of 6,912 particles takes 12.3 us by eights, 11.5 with 16 together, 10.7
+ * with 24, 12.3 with 28, 14.0 with 40; 32,000 particles (blocks of 128) 13.6 by
+ * eights and 14.2 with 24. */
+constexpr int kTogether = 24;
 template <int BLOCK, class Load, class F>
 __device__ __forceinline__ void for_each_kept(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                               const unsigned int *kept, int k, int i, float3 xi, Load &&load, F &&f) {
@@ -95,6 +101,20 @@ __device__ __forceinline__ void for_each_kept(const DevParams &p, const unsigned
         for (int u = 0; u < 8; ++u) xj[u] = load(j[u]);
     };
     if (k == 0) return;
+    if (BLOCK == 64) {
+        for (int t0 = 0; t0 < k; t0 += kTogether) {
+            unsigned int v[kTogether / 2];
+            float4 xj[kTogether];
+#pragma unroll
+            for (int u = 0; u < kTogether / 2; ++u) v[u] = kept[min((t0 >> 1) + u, (k - 1) >> 1) * BLOCK];
+#pragma unroll
+            for (int u = 0; u < kTogether; ++u) xj[u] = load(u & 1 ? v[u / 2] >> 16 : v[u / 2] & 0xffffu);
+#pragma unroll
+            for (int u = 0; u < kTogether; ++u)
+                if (t0 + u < k) f(u & 1 ? v[u / 2] >> 16 : v[u / 2] & 0xffffu, xj[u]);
+        }
+        return;
+    }
     float4 xa[8], xb[8];
     unsigned int ja[8], jb[8];
     fetch(0, xa, ja);
@@ -171,7 +191,7 @@ __device__ __forceinline__ void loop_leave(const DevParams &p, DevCtl *ctl, Loop
 }
 
 template <bool KAHAN, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
+__global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
     k_pbf_loop(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
                float *__restrict__ dens, const float4 *__restrict__ xb, DevCtl *ctl, LoopCtl *lc,
                cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hif2,
