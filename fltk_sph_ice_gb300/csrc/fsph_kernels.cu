@@ -1558,11 +1558,14 @@ static unsigned int resident_blocks(const void *kernel) {
 
 /* the passes' shape by size (kDeepMax in fsph_kernels.cuh) */
 static bool deep_pass(const DevParams &p) { return p.n <= kDeepMax && p.use_lists; }
+static bool deep_constraint(const DevParams &p) {
+    return p.n <= (p.nb ? kDeepMaxBoundary : kDeepMax) && p.use_lists;
+}
 
 void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1, float *dens,
                    DevCtl *ctl, ErrPartial *part, unsigned long long while_handle, int use_graph,
                    const NbrLists &nl, cudaStream_t s) {
-    const bool deep = deep_pass(p);
+    const bool deep = deep_constraint(p);
     auto k = deep ? (p.compensated ? k_lambda<true, true> : k_lambda<false, true>)
                   : (p.compensated ? k_lambda<true, false> : k_lambda<false, false>);
     const unsigned int blocks = deep ? blocks_for(p.n, kDeepBlock)
@@ -1587,7 +1590,7 @@ void launch_correction(const DevParams &p, const unsigned int *cell_start, float
                        const float4 *xb, DevCtl *ctl, float *part, unsigned long long if_handle,
                        unsigned long long if_handle2, int use_graph, float4 *dp_out, const NbrLists &nl,
                        cudaStream_t s) {
-    const bool deep = deep_pass(p);
+    const bool deep = deep_constraint(p);
     auto k = deep ? k_correction<true> : k_correction<false>;
     const int block = deep ? kDeepBlock : kPassBlock;
     k<<<blocks_for(p.n, block), block, 0, s>>>(p, cell_start, ppos0, ppos1, xb, ctl, part,

@@ -22,6 +22,13 @@ constexpr int kPassBlock = FSPH_PASS_BLOCK;
  * and a correction pass together: 31.0 -> 22.6 us at 6,912, 33.0 -> 27.7 at
  * 32,000, 43.1 -> 42.0 at 131,072, 71.4 -> 81.6 at 294,912 */
 constexpr int kDeepBlock = 64, kDeepMinB = 12, kDeepMax = 65536;
+/* Beside a boundary a pass waits for the few warps at its shell, and which form is
+ * the faster depends on where they land: steps with a shell took, deep / plain, in
+ * us, 948 / 1,044 at 13,824 particles, 1,332 / 1,244 at 46,656, 1,070 / 1,245 and
+ * (10 iterations) 1,591 / 1,812 at 54,872, 851 / 777 and 1,366 / 1,110 at 59,319,
+ * 1,097 / 1,185 and (10 iterations) 1,922 / 1,737 at 64,000.  The line lies where
+ * the plain form begins to be mostly the faster. */
+constexpr int kDeepMaxBoundary = 57344;
 /* The XSPH and vorticity passes of larger scenes: a step of 1 M particles with two
  * iterations took 852 us in blocks of 128, 857 of 256, 865 of 512, 878 with eight
  * candidates in flight; with registers for five or six blocks of 256 per SM 867

@@ -27,11 +27,13 @@ def _state(n, seed, squeeze=1.0, jitter=0.03):
     return p, x, v
 
 
-def _run(p, x, v, steps, graph):
+def _run(p, x, v, steps, graph, boundary=None):
     q = abi.FsphParams.from_buffer_copy(p)
     q.use_graph = graph
     ps = rxPBDSPH(q)
     ps.Set(x, v)
+    if boundary is not None:
+        ps.SetBoundary(boundary)
     rec = []
     for _ in range(steps):
         ps.Update(0.0016)
@@ -131,3 +133,22 @@ def test_swept_scene_stops_at_its_tolerance(gpu, mode):
     p, x, v = _state(90000, 5)
     p.error_mode, p.min_iter, p.max_iter, p.eta = mode, 2, 60, 5e-3 if mode == abi.ERR_ONE_SIDED else 5e-2
     _same(p, x, v, 2)
+
+
+def test_boundary_passes_on_both_sides_of_their_change_of_form(gpu):
+    """57,344 particles beside a shell, and the same with one more far away, which
+    takes the other form of the constraint passes: the same bits for all the rest."""
+    n = 57344
+    p, x, v = _state(n, 4)
+    far = np.zeros((1, 4), np.float32)
+    far[0, :3] = np.array(list(p.box_max)[:3]) - H
+    p.eta, p.min_iter, p.max_iter = 0.0, 2, 3
+    mid = 0.5 * (x[:, :3].min(0) + x[:, :3].max(0)) - 0.05
+    b = scenes.box_surface([float(c) for c in mid], 0.1, 0.3 * H)
+    got = []
+    for y, w in ((x, v), (np.concatenate([x, far]), np.concatenate([v, 0 * far]))):
+        q = abi.FsphParams.from_buffer_copy(p)
+        q.max_particles = len(y)
+        got.append(_run(q, y, w, 2, 1, b)[1])
+    for s, t in zip(*got):
+        assert np.array_equal(s[:n], t[:n])
