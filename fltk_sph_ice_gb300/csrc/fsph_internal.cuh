@@ -191,7 +191,7 @@ struct DevCtl {
 };
 
 /* State of the one-kernel constraint loop (fsph_loop.cu) between its blocks;
- * all zero outside a launch.  Iteration t of a launch uses the sums t % 3. */
+ * all zero outside a step.  Iteration t of a launch uses the sums t % 3. */
 struct LoopCtl {
     unsigned long long e1[3], e2[3]; /* error sums in units of 2^-32 */
     unsigned int em[3], disp[3];     /* largest |C| and |x* - xb|^2 (float bits) */

@@ -62,11 +62,11 @@ __device__ __forceinline__ bool grid_wait(const DevParams &p, LoopCtl *lc, unsig
             /* relaxed, and with a pause: an acquire would empty the SM's L1 at every
              * poll, under the blocks that are still in their pass */
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&lc->arrived) : "memory");
-            if (seen >= want || --polls == 0ull) break;
+            if ((int)(seen - want) >= 0 || --polls == 0ull) break; /* the counter may wrap */
             __nanosleep(64);
         }
         __threadfence();
-        s_ok = seen >= want ? 1 : 0;
+        s_ok = (int)(seen - want) >= 0 ? 1 : 0;
     }
     __syncthreads();
     return s_ok != 0;
@@ -185,6 +185,9 @@ __device__ __forceinline__ void loop_leave(const DevParams &p, DevCtl *ctl, Loop
     lc->left = 0u;
     for (unsigned int k = 0; k < 3u; ++k) loop_clear(lc, k);
     const unsigned int cont = __ldcg(&ctl->wait_err) ? 0u : s.cont; /* a wait ran out: the step ends and reports it */
+    /* a correction that was not a number also asks for a rebuild: the launch after
+     * it stops at its first errors, as k_lambda does */
+    if (cont && __ldcg(&ctl->nan_flag)) lc->nan[0] = 1u;
     cudaGraphSetConditional(hwhile, cont);
     cudaGraphSetConditional(hif, cont & s.rebuild);
     if (post) cudaGraphSetConditional(hif2, s.rebuild);
