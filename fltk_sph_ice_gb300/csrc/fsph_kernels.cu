@@ -498,9 +498,10 @@ __global__ void __launch_bounds__(DEEP ? kDeepBlock : kPassBlock, DEEP ? kDeepMi
  * allocation-free entry point, which keeps no lists.  One thread a particle
  * leaves 8 blocks and a serial walk of 290 candidates at 4,096 particles (47 us);
  * with 32 lanes a row of cells is one coalesced step.  The whole call went from
- * 84 to 36 us at 4,096 particles (21 with the grid built by one block).  The sums are the lanes' partial sums, as in
- * the batched passes with several lanes. */
-template <int LPP>
+ * 84 to 36 us at 4,096 particles (21 with the grid built by one block).  The sums
+ * are the lanes' partial sums, as in the batched passes with several lanes; KAHAN:
+ * each compensated, and added with the errors of the additions. */
+template <int LPP, bool KAHAN>
 __global__ void __launch_bounds__(kBlock) k_lambda_walk(DevParams p, const unsigned int *__restrict__ cell_start,
                                                         const float4 *__restrict__ x,
                                                         const unsigned int *__restrict__ order,
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(kBlock) k_lambda_walk(DevParams p, const unsig
     const int i = valid ? t / LPP : p.n - 1; /* padding lanes run a real slot and write nothing */
     const float3 xi = f3(__ldg(x + i));
     float rho, lam;
-    lambda_terms<LPP, false>(
+    lambda_terms<LPP, KAHAN>(
         p, x, xi,
         [&](auto &&load, auto &&f) {
             for_each_candidate<LPP>(p, cell_start, nullptr, nullptr, i, xi, sub, load, f);
@@ -708,16 +709,7 @@ void launch_boundary_lambda(const DevParams &p, const unsigned int *cell_start, 
     k_boundary_lambda<<<blocks_for(p.nb), kBlock, 0, s>>>(p, cell_start, ppos0, ppos1, ctl, bstat, blam);
 }
 
-/* Sums and products of two floats without their rounding errors: the result
- * and its error (Knuth; Dekker; the product's error from one fused operation),
- * with no contraction by the compiler. */
-struct Split {
-    float h, l; /* the value is h + l */
-};
-__device__ __forceinline__ Split two_sum(float a, float b) {
-    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-    return Split{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
+/* the rest of the arithmetic of split floats (Split, two_sum: fsph_passes.cuh) */
 __device__ __forceinline__ Split two_diff(float a, float b) { return two_sum(a, -b); }
 __device__ __forceinline__ Split two_prod(float a, float b) {
     const float q = __fmul_rn(a, b);
@@ -1666,8 +1658,14 @@ void launch_sph_density(const DevParams &p, const unsigned int *cell_start, floa
 void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,
                         float *dens, float *lambda, cudaStream_t s) {
     const int lanes = lanes_to_fill(p.n, 32);
-    auto k = lanes >= 32 ? k_lambda_walk<32> : lanes >= 16 ? k_lambda_walk<16> : lanes >= 8 ? k_lambda_walk<8>
-                                                                                        : k_lambda_walk<4>;
+    auto k = p.compensated ? (lanes >= 32   ? k_lambda_walk<32, true>
+                              : lanes >= 16 ? k_lambda_walk<16, true>
+                              : lanes >= 8  ? k_lambda_walk<8, true>
+                                            : k_lambda_walk<4, true>)
+                           : (lanes >= 32   ? k_lambda_walk<32, false>
+                              : lanes >= 16 ? k_lambda_walk<16, false>
+                              : lanes >= 8  ? k_lambda_walk<8, false>
+                                            : k_lambda_walk<4, false>);
     const int lpp = lanes >= 4 ? lanes : 4;
     k<<<blocks_for((long long)p.n * lpp), kBlock, 0, s>>>(p, cell_start, x, order, dens, lambda);
 }

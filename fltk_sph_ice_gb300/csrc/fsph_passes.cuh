@@ -205,6 +205,29 @@ __device__ __forceinline__ float group_sum(float v) {
     return v;
 }
 
+/* Sums and products of two floats without their rounding errors: the result
+ * and its error (Knuth; Dekker; the product's error from one fused operation),
+ * with no contraction by the compiler. */
+struct Split {
+    float h, l; /* the value is h + l */
+};
+__device__ __forceinline__ Split two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    return Split{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
+/* group_sum of v + e, e the part of each lane's sum that v has lost: every lane
+ * gets the same value (each addition is the same seen from either side) */
+template <int LPP>
+__device__ __forceinline__ float group_sum_split(float v, float e) {
+#pragma unroll
+    for (int o = LPP / 2; o > 0; o >>= 1) {
+        const Split t = two_sum(v, __shfl_xor_sync(0xffffffffu, v, o));
+        e = __fadd_rn(__fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, o)), t.l);
+        v = t.h;
+    }
+    return __fadd_rn(v, e);
+}
+
 /* ---------------- grid build ---------------- */
 
 /* x* = walls(x + dt (v + dt a)), a = gravity when acc == NULL, then the
@@ -655,7 +678,7 @@ __device__ __forceinline__ float lambda_terms(const DevParams &p, const float4 *
             sd += g * g * r2;
         });
     if (LPP > 1) {
-        wsum = group_sum<LPP>(wsum);
+        wsum = KAHAN ? group_sum_split<LPP>(wsum, -wc) : group_sum<LPP>(wsum);
         sd = group_sum<LPP>(sd);
         gs.x = group_sum<LPP>(gs.x);
         gs.y = group_sum<LPP>(gs.y);
