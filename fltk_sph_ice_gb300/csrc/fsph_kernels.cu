@@ -1482,11 +1482,8 @@ bool launch_small_grid(const DevParams &p, unsigned int ncells, const float4 *x4
     constexpr size_t most = 200 * 1024;
     const size_t bytes = ((size_t)ncells + 1 + (size_t)p.n) * sizeof(unsigned int);
     if (p.n > kSmallGrid || bytes > most) return false;
-    static const bool ok = [] { /* once, thread-safely */
-        return cudaFuncSetAttribute(k_small_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) ==
-               cudaSuccess;
-    }();
-    if (!ok) return false;
+    static PerDevice limit;
+    if (!raise_shared_limit(limit, (const void *)k_small_grid, most)) return false;
     k_small_grid<<<1, 1024, bytes, s>>>(p, ncells, x4, x_out, order, cell_start);
     return true;
 }

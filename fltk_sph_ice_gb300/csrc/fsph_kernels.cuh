@@ -5,8 +5,25 @@
  */
 #pragma once
 #include "fsph_internal.cuh"
+#include "fsph_per_device.h"
 
 namespace fsph {
+
+/* raises a kernel's dynamic shared-memory limit on the current device, once for
+ * each (done: the kernel's own); false, with no error left pending, when it cannot */
+inline bool raise_shared_limit(PerDevice &done, const void *kernel, size_t bytes) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return done.once(dev, [&] {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+            return true;
+        cudaGetLastError();
+        return false;
+    });
+}
 
 constexpr int kBlock = 256;
 /* threads per block of the two constraint passes (k_lambda, k_correction);

@@ -120,6 +120,9 @@ extern "C" int fsph_pbf_eval_lambda_noalloc(const fsph_params *params, const flo
         g.dst4[0] = x;
         launch_gather(n, o, g, nullptr, s);
     }
+    /* without its grid the pass would read the order of an earlier call, whose
+     * particles may lie past these outputs */
+    if (cudaGetLastError() != cudaSuccess) return FSPH_CUDA_ERROR;
     launch_lambda_walk(p, cell_start, x, rank, dens, lambda, s);
     if (cudaGetLastError() != cudaSuccess) return FSPH_CUDA_ERROR;
     return FSPH_OK;
