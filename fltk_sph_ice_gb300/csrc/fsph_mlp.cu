@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/fsph.h"
+#include "fsph_kernels.cuh"
 #include "fsph_mlp.cuh"
 
 namespace fsph {
@@ -581,11 +582,8 @@ void launch_mlp_forward3(const MlpDev *m, const float *x, int n, float *y, cudaS
 }
 void launch_mlp_grad(const MlpDev *m, const float *x, const float *t, int n, float *part, float *loss_part,
                      cudaStream_t s) {
-    static const bool attr = [] { /* set once, thread-safely */
-        cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem);
-        return true;
-    }();
-    (void)attr;
+    static PerDevice limit;
+    raise_shared_limit(limit, (const void *)k_mlp_grad, kGradSmem); /* without it the launch fails */
     k_mlp_grad<<<mlp_grad_blocks(n), 128, kGradSmem, s>>>(m, x, t, n, part, loss_part);
 }
 void launch_mlp_reduce(const float *part, const float *loss_part, int nblocks, int n, float *grad, float *loss,

@@ -20,3 +20,12 @@ def test_each_device_once(tmp_path):
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
+
+
+def test_no_limit_is_raised_once_a_process():
+    """Every kernel's limit goes through that record."""
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                n = f.read().count("cudaFuncSetAttribute(")
+            assert n == (1 if name == "fsph_kernels.cuh" else 0), name
