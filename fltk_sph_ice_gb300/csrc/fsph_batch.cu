@@ -250,9 +250,10 @@ __global__ void __launch_bounds__(BLOCK) kb_vort_apply(BatchArgs b, const unsign
 }
 
 /* Density errors of the last lambda pass: the partial sums of each tile (one
- * warp a tile, sums of floats with their rounding errors kept, so as exact as
- * doubles: FP64 runs at 2 lanes a clock and SM), then one warp per scene adds
- * its tiles' in order: err[3 s + 0..2] = one-sided mean, two-sided mean, max.
+ * warp a tile, sums of floats with their rounding errors kept, 48 bits, which
+ * hold a tile's sum to far below the float it ends in: FP64 runs at 2 lanes a
+ * clock and SM; a tile whose sum leaves the range of floats is summed again in
+ * doubles), then one warp per scene adds its tiles' in order: err[3 s + 0..2] = one-sided mean, two-sided mean, max.
  * One block a scene over its particles in double took 156 us, the largest
  * scene's block alone at the end. */
 struct TileErr {
@@ -287,7 +288,20 @@ __global__ void __launch_bounds__(256) kb_tile_errors(BatchArgs b, const float *
         e2.y = __fadd_rn(e2.y, f2.y);
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
-    if (lane == 0) part[t] = TileErr{(double)e1.x + (double)e1.y, (double)e2.x + (double)e2.y, m, 0.f};
+    double s1 = (double)e1.x + (double)e1.y, s2 = (double)e2.x + (double)e2.y;
+    if (__any_sync(0xffffffffu, !isfinite(s2))) { /* a sum past the largest float, infinite or not a number */
+        s1 = s2 = 0.0;
+        for (int k = lane; k < tl.count; k += 32) {
+            const float C = dens[tl.start + k] * inv - 1.0f;
+            s1 += C > 0.0f ? C : 0.0f;
+            s2 += fabsf(C);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        }
+    }
+    if (lane == 0) part[t] = TileErr{s1, s2, m, 0.f};
 }
 __global__ void __launch_bounds__(128) kb_scene_errors(int nscenes, const int *__restrict__ offs,
                                                        const int *__restrict__ tile0, const TileErr *__restrict__ part,
