@@ -735,7 +735,8 @@ __device__ __forceinline__ Split split_of(double v) {
  * (every slot within the list radius, here the cell width h (1 + 1e-3));
  * the force pass's per-neighbour factors ride in the .w words of the sorted
  * copies: pos.w = p / rho^2, vel.w = 1 / rho.  Only .w words are written, so
- * the x, y, z the other threads read stay as they are. */
+ * the x, y, z the other threads read stay as they are; they read them by plain
+ * loads (ld.global.nc is for what no thread of the launch writes beside). */
 __device__ __forceinline__ void sph_density_out(const DevParams &p, int i, float acc, float4 *pos, float4 *vel,
                                                 float *__restrict__ dens, float *__restrict__ pres) {
     const float rho = p.mass * p.aw * acc;
@@ -780,7 +781,8 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
         return r2;
     };
     warp_candidates(
-        p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.rl2, s_tile[W == 1 ? threadIdx.x >> 5 : 0],
+        p, cell_start, [&](unsigned int j) { return pos[j]; }, xi, valid ? cell_index(c, p) : 0u, valid, p.rl2,
+        s_tile[W == 1 ? threadIdx.x >> 5 : 0],
         [&](bool found, int first, int count, int total, TileWalk<W> &walk) {
             if (found) {
                 unsigned int last = 0u;
@@ -871,7 +873,7 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
                 const unsigned int j = j0 + (unsigned int)sub;
                 bool hit = false;
                 if (j < e) {
-                    const float3 d = xi - f3(__ldg(pos + j));
+                    const float3 d = xi - f3(pos[j]);
                     const float r2 = dot3(d, d);
                     if (r2 < p.h2) {
                         const float q = p.h2 - r2;
@@ -1006,7 +1008,8 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
     const float3 xi = valid ? f3(__ldg(pos + i)) : make_float3(0.f, 0.f, 0.f);
     const int3 c = cell_of(xi, p);
     unsigned int k = 0;
-    warp_candidates(p, cell_start, pos, xi, valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
+    warp_candidates(p, cell_start, [&](unsigned int j) { return __ldg(pos + j); }, xi,
+                    valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
                     [&](bool found, int, int count, int, TileWalk<1> &walk) {
                         auto meet = [&](unsigned int j) {
                             if (ref_neighbor(xi, f3(__ldg(pos + j)), p.h2)) {

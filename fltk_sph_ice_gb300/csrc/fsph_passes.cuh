@@ -411,10 +411,11 @@ struct TileWalk {
 };
 
 /* Calls emit(found, first, count, total, walk) once for each valid lane: found:
- * the lane's `count` candidates against x4 within sqrt(r2max) come from walk,
- * ascending; else they have to be looked for without the tile (more than fit it, or a
+ * the lane's `count` candidates within sqrt(r2max) come from walk, ascending;
+ * else they have to be looked for without the tile (more than fit it, or a
  * coordinate out of the operands' range: a particle far outside the box, or not
- * a number).  xi, cell: the lane's position and build cell, cells ascending over
+ * a number).  load(j): slot j's position, a plain load where the kernel writes
+ * beside it.  xi, cell: the lane's position and build cell, cells ascending over
  * the lanes, padding lanes (valid = false) after the valid ones; every lane of
  * the warp calls it.  Lanes in different rows of cells, or more than eight cells
  * apart (a run that wraps, sparse fluid), take turns: a row's range then never
@@ -425,10 +426,10 @@ struct TileWalk {
  * it found there: `count` of the lane's `total`, from the `first` on; what is not
  * found is warp 0's alone.  A warp's twenty words in a row, latency bound, are the
  * pass of a small scene: 16 us at 6,912 slots with one warp, 10 with four. */
-template <int W, class Emit>
+template <int W, class Load, class Emit>
 __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
-                                                const float4 *__restrict__ x4, float3 xi, unsigned int cell,
-                                                bool valid, float r2max, PairTileOf<W> &t, Emit &&emit) {
+                                                Load &&load, float3 xi, unsigned int cell, bool valid, float r2max,
+                                                PairTileOf<W> &t, Emit &&emit) {
     const int lane = threadIdx.x & 31, wid = W > 1 ? (int)(threadIdx.x >> 5) : 0;
     uint4 *const rows = t.row[wid];
     const unsigned int row = (cell - p.cell_off) / (unsigned int)p.gx;
@@ -516,7 +517,7 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                     if (q >= next) j = q + sh;
                 }
                 /* past the last candidate: some slot's position, not used */
-                return __ldg(x4 + min(q < total ? j : j - (q - total + 1u), (unsigned int)p.n - 1u));
+                return load(min(q < total ? j : j - (q - total + 1u), (unsigned int)p.n - 1u));
             };
             /* this warp's words */
             const unsigned int words = (total + 31u) >> 5;
@@ -606,7 +607,7 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
                                                 unsigned char *__restrict__ cnt, PairTileOf<W> &t) {
     const float3 xi = valid ? f3(__ldg(xb + i)) : make_float3(0.f, 0.f, 0.f);
     const unsigned int cell = valid ? __ldg(cellb + i) : 0u;
-    warp_candidates(p, cell_start, xb, xi, cell, valid, p.rl2, t,
+    warp_candidates(p, cell_start, [&](unsigned int j) { return __ldg(xb + j); }, xi, cell, valid, p.rl2, t,
                     [&](bool found, int first, int count, int total, TileWalk<W> &walk) {
         if (!found) {
             build_list_body(p, i, cell_start, xb, cell, list, cnt);
