@@ -156,7 +156,8 @@ EXPORTS = [
     "fsph_set_box_obstacle", "fsph_set_sphere_obstacle", "fsph_move_sphere_obstacle", "fsph_get_sphere_obstacle_pos",
     "fsph_clear_obstacles", "fsph_num_obstacles", "fsph_density_grid", "fsph_num_active", "fsph_add_delete_region",
     "fsph_clear_delete_regions", "fsph_add_inlet_line", "fsph_clear_inlets", "fsph_emit_inlets",
-    "fsph_set_step_log", "fsph_set_alloc_fault", "fsph_reference_cell_hash", "fsph_save_state", "fsph_load_state",
+    "fsph_set_step_log", "fsph_set_alloc_fault", "fsph_set_wait_limit", "fsph_reference_cell_hash", "fsph_save_state",
+    "fsph_load_state",
     "fsph_set_polygon_obstacle", "fsph_clear_polygon_obstacles", "fsph_num_polygon_triangles", "fsph_polygon_collide", "fsph_num_inlets",
     "fsph_mlp_create", "fsph_mlp_destroy", "fsph_mlp_set_blob", "fsph_mlp_get_blob", "fsph_mlp_last_error",
     "fsph_mlp_forward", "fsph_mlp_forward_tcgen05", "fsph_mlp_gradient", "fsph_mlp_train", "fsph_set_warm_start_model",
@@ -229,6 +230,7 @@ def _declare(L: ctypes.CDLL) -> ctypes.CDLL:
     L.fsph_load_state.argtypes = [c_void_p, ctypes.c_char_p]
     L.fsph_reference_cell_hash.argtypes = [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]
     L.fsph_set_alloc_fault.argtypes = [ctypes.c_longlong, ctypes.c_longlong]
+    L.fsph_set_wait_limit.argtypes = [c_void_p, ctypes.c_longlong]
     L.fsph_time_pass.argtypes = [c_void_p, c_int, c_int, P(c_float)]
     L.fsph_mlp_create.argtypes = [P(c_void_p)]
     L.fsph_mlp_destroy.argtypes = [c_void_p]
@@ -275,8 +277,8 @@ def _declare(L: ctypes.CDLL) -> ctypes.CDLL:
                  "fsph_move_sphere_obstacle", "fsph_get_sphere_obstacle_pos", "fsph_clear_obstacles",
                  "fsph_num_obstacles", "fsph_density_grid", "fsph_num_active", "fsph_add_delete_region",
                  "fsph_clear_delete_regions", "fsph_add_inlet_line", "fsph_clear_inlets", "fsph_emit_inlets",
-                 "fsph_set_step_log", "fsph_set_alloc_fault", "fsph_reference_cell_hash", "fsph_save_state",
-                 "fsph_load_state", "fsph_set_polygon_obstacle", "fsph_clear_polygon_obstacles",
+                 "fsph_set_step_log", "fsph_set_alloc_fault", "fsph_set_wait_limit", "fsph_reference_cell_hash",
+                 "fsph_save_state", "fsph_load_state", "fsph_set_polygon_obstacle", "fsph_clear_polygon_obstacles",
                  "fsph_num_polygon_triangles", "fsph_polygon_collide", "fsph_num_inlets"]:
         getattr(L, name).restype = c_int
     return L

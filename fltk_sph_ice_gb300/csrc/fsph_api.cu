@@ -88,6 +88,7 @@ struct fsph_ctx {
     DevCtl *ctl_host = nullptr;
     LoopCtl *loop = nullptr;           /* the one-kernel constraint loop's counters */
     bool loop_kernel = false;          /* the step graph runs it */
+    unsigned long long wait_polls = 0; /* of its grid barrier; 0: its own limit */
     unsigned int *flag = nullptr;      /* input-validation flag, pinned host memory */
     /* warm start */
     float4 *xpred = nullptr;           /* x* before the iterations, iteration order */
@@ -881,7 +882,7 @@ int build_pbf_graph(fsph_ctx *c, const DevParams &p) {
     cudaError_t le = cudaSuccess;
     if (c->loop_kernel) {
         le = launch_pbf_loop(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->xb, c->ctl, c->loop, hw, hrb, hrb2,
-                             ext ? 1 : 0, c->nl, c->s2);
+                             ext ? 1 : 0, c->wait_polls, c->nl, c->s2);
     } else {
         launch_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->ctl, c->epart, hw, 1, c->nl, c->s2);
         launch_boundary_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->ctl, c->b_stat, c->b_lam, c->s2);
@@ -1486,6 +1487,14 @@ int fsph_set_step_log(fsph_ctx *c, const char *path) {
     if (!path || !*path) return FSPH_OK;
     c->log = std::fopen(path, "a");
     if (!c->log) return fail(c, FSPH_INVALID_ARG, std::string("cannot open ") + path);
+    return FSPH_OK;
+}
+
+int fsph_set_wait_limit(fsph_ctx *c, long long polls) {
+    if (!c) return FSPH_INVALID_ARG;
+    if (polls < 0) return fail(c, FSPH_INVALID_ARG, "polls < 0");
+    c->wait_polls = (unsigned long long)polls;
+    c->graph_valid = false; /* the launch in it holds the limit */
     return FSPH_OK;
 }
 

@@ -135,13 +135,14 @@ void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *p
  * until the loop ends or a grid rebuild is due, then the three conditions are set
  * (post: the third exists).  loop_fits: lists are on, there is no boundary (its
  * lambda is a kernel of its own between the passes) and every block is resident at
- * once.  Up to kLoopMax particles each has a thread of its own. */
+ * once.  Up to kLoopMax particles each has a thread of its own.  polls: before a
+ * block gives a barrier up (0: the default). */
 constexpr int kLoopMax = 65536;
 bool loop_fits(const DevParams &p);
 cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                             float *dens, const float4 *xb, DevCtl *ctl, LoopCtl *lc, unsigned long long while_handle,
-                            unsigned long long if_handle, unsigned long long if_handle2, int post, const NbrLists &nl,
-                            cudaStream_t s);
+                            unsigned long long if_handle, unsigned long long if_handle2, int post,
+                            unsigned long long polls, const NbrLists &nl, cudaStream_t s);
 /* density and lambda of x (slot order) at order[slot], walking the cells */
 void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,
                         float *dens, float *lambda, cudaStream_t s);

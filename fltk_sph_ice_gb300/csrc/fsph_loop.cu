@@ -37,16 +37,16 @@ namespace fsph {
 
 namespace {
 
-/* polls before a block gives the barrier up: about two seconds, and as much
- * again for each 65,536 particles (a co-resident grid needs a few; a scene that
- * has collapsed into one cell may take long over a pass) */
+/* polls before a block gives the barrier up, where the caller sets no limit: about
+ * two seconds, and as much again for each 65,536 particles (a co-resident grid needs
+ * a few; a scene that has collapsed into one cell may take long over a pass) */
 constexpr unsigned long long kLoopPolls = 1ull << 21;
 
 /* The grid barrier in two halves, so that what need not be done before the
  * other blocks go on is done while waiting for them.  Writes of the block
  * before grid_arrive are visible to every block after its grid_wait(want),
  * want = the arrivals since the kernel began.  grid_wait is false, for every
- * thread of the block alike, when the wait ran out. */
+ * thread of the block alike, when `polls` polls did not see them all. */
 __device__ __forceinline__ void grid_arrive(LoopCtl *lc) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -54,9 +54,8 @@ __device__ __forceinline__ void grid_arrive(LoopCtl *lc) {
         atomicAdd(&lc->arrived, 1u);
     }
 }
-__device__ __forceinline__ bool grid_wait(const DevParams &p, LoopCtl *lc, unsigned int want, int &s_ok) {
+__device__ __forceinline__ bool grid_wait(LoopCtl *lc, unsigned int want, unsigned long long polls, int &s_ok) {
     if (threadIdx.x == 0) {
-        unsigned long long polls = kLoopPolls * (1ull + ((unsigned int)p.n >> 16));
         unsigned int seen;
         while (true) {
             /* relaxed, and with a pause: an acquire would empty the SM's L1 at every
@@ -198,7 +197,8 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
     k_pbf_loop(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
                float *__restrict__ dens, const float4 *__restrict__ xb, DevCtl *ctl, LoopCtl *lc,
                cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hif2,
-               int post, const ListEntry *__restrict__ list, const unsigned char *__restrict__ cnt) {
+               int post, unsigned long long polls, const ListEntry *__restrict__ list,
+               const unsigned char *__restrict__ cnt) {
     __shared__ unsigned int s_kept[(kListMax / 2) * BLOCK];
     __shared__ unsigned long long s_e1[BLOCK / 32], s_e2[BLOCK / 32];
     __shared__ float s_em[BLOCK / 32], s_d[BLOCK / 32];
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
         qm = warp_max(qm);
         if (lane == 0) { s_e1[warp] = q1; s_e2[warp] = q2; s_em[warp] = qm; }
         want += nb;
-        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        if (!(ok = grid_wait(lc, want, polls, s_ok))) break;
         /* corrections from every particle's lambda */
         float disp2 = 0.f;
         if (valid) {
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
         }
         grid_arrive(lc);
         want += nb;
-        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        if (!(ok = grid_wait(lc, want, polls, s_ok))) break;
         if (threadIdx.x == 0) s_go = loop_decide(p, lc, st);
         __syncthreads();
         ++st.iter;
@@ -314,7 +314,8 @@ __global__ void __launch_bounds__(kSweepBlock, 2)
     k_pbf_sweep(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
                 float *__restrict__ dens, const float4 *__restrict__ xb, DevCtl *ctl, LoopCtl *lc,
                 cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hif2,
-                int post, const ListEntry *__restrict__ list, const unsigned char *__restrict__ cnt) {
+                int post, unsigned long long polls, const ListEntry *__restrict__ list,
+                const unsigned char *__restrict__ cnt) {
     __shared__ unsigned long long s_e1[kSweepBlock / 32], s_e2[kSweepBlock / 32];
     __shared__ float s_em[kSweepBlock / 32], s_d[kSweepBlock / 32];
     __shared__ int s_ok, s_go;
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kSweepBlock, 2)
         }
         grid_arrive(lc);
         want += gridDim.x;
-        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        if (!(ok = grid_wait(lc, want, polls, s_ok))) break;
         {
             const float4 *src = st.par ? ppos1 : ppos0;
             float4 *dst = st.par ? ppos0 : ppos1;
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(kSweepBlock, 2)
         }
         grid_arrive(lc);
         want += gridDim.x;
-        if (!(ok = grid_wait(p, lc, want, s_ok))) break;
+        if (!(ok = grid_wait(lc, want, polls, s_ok))) break;
         if (threadIdx.x == 0) {
             s_go = loop_decide(p, lc, st);
             ++st.iter;
@@ -421,7 +422,8 @@ __global__ void __launch_bounds__(kSweepBlock, 2)
 
 typedef void (*LoopKernel)(DevParams, const unsigned int *, float4 *, float4 *, float *, const float4 *, DevCtl *,
                            LoopCtl *, cudaGraphConditionalHandle, cudaGraphConditionalHandle,
-                           cudaGraphConditionalHandle, int, const ListEntry *, const unsigned char *);
+                           cudaGraphConditionalHandle, int, unsigned long long, const ListEntry *,
+                           const unsigned char *);
 
 template <int BLOCK>
 LoopKernel loop_kernel(bool kahan) {
@@ -468,8 +470,8 @@ bool loop_fits(const DevParams &p) {
 
 cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                             float *dens, const float4 *xb, DevCtl *ctl, LoopCtl *lc, unsigned long long while_handle,
-                            unsigned long long if_handle, unsigned long long if_handle2, int post, const NbrLists &nl,
-                            cudaStream_t s) {
+                            unsigned long long if_handle, unsigned long long if_handle2, int post,
+                            unsigned long long polls, const NbrLists &nl, cudaStream_t s) {
     LoopShape sh;
     const unsigned int blocks = loop_blocks(p, sh);
     if (!blocks) return cudaErrorCooperativeLaunchTooLarge;
@@ -477,7 +479,8 @@ cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, 
     cudaGraphConditionalHandle hw = while_handle, h1 = if_handle, h2 = if_handle2;
     const ListEntry *list = nl.list;
     const unsigned char *cnt = nl.cnt;
-    void *args[] = {&q, &cell_start, &ppos0, &ppos1, &dens, &xb, &ctl, &lc, &hw, &h1, &h2, &post, &list, &cnt};
+    if (!polls) polls = kLoopPolls * (1ull + ((unsigned int)p.n >> 16));
+    void *args[] = {&q, &cell_start, &ppos0, &ppos1, &dens, &xb, &ctl, &lc, &hw, &h1, &h2, &post, &polls, &list, &cnt};
     return cudaLaunchCooperativeKernel((const void *)sh.kernel, dim3(blocks), dim3(sh.block), args, 0, s);
 }
 

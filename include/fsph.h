@@ -521,6 +521,13 @@ int fsph_set_step_log(fsph_ctx *ctx, const char *path);
  * calling cudaMalloc.  fsph_set_alloc_fault(-1, -1) switches it off.
  * No counterpart in the reference. */
 int fsph_set_alloc_fault(long long max_bytes, long long fail_at);
+/* How often a block of the one-kernel constraint loop looks for the others at a
+ * barrier before it gives up, for testing that path: the step then ends with
+ * FSPH_TIMEOUT, its particles are undefined (set them again), and the next step
+ * is as any other.  0: the library's own limit, about two seconds and more for
+ * larger scenes.  Steps whose passes are launches of their own have no such wait.
+ * No counterpart in the reference. */
+int fsph_set_wait_limit(fsph_ctx *ctx, long long polls);
 
 /* ---- measurement ---- */
 typedef enum fsph_pass {
