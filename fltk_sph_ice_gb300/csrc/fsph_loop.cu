@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
             }
             q1 = err_fix(C > 0.0f ? C : 0.0f);
             q2 = err_fix(fabsf(C));
-            qm = fabsf(C);
+            qm = fmaxf(qm, fabsf(C)); /* a C that is not a number is left out, as in k_lambda */
         }
         grid_arrive(lc);
         /* the error sums are needed only by the barrier after the corrections */
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
                 lc->nan[nx] = 1u; /* stops the loop at the next errors, as k_lambda does */
             }
             const float3 dd = xn - xbi;
-            disp2 = dot3(dd, dd);
+            disp2 = fmaxf(disp2, dot3(dd, dd));
             xi = xn;
         }
         disp2 = warp_max(disp2);

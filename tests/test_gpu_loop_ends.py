@@ -1,5 +1,5 @@
 """How the one-kernel constraint loop ends when it does not end at its tolerance
-(a barrier's wait that runs out), and that graph
+(a density that is not a number, a barrier's wait that runs out), and that graph
 steps without a boundary do run it."""
 import numpy as np
 import pytest
@@ -52,6 +52,28 @@ def test_iterations_are_no_launches(gpu, n, boundary):
         got.append(st.kernels)
         ps.close()
     assert got[1] - got[0] == (18 if boundary else 0)
+
+
+@pytest.mark.parametrize("n", FORMS)
+def test_a_density_that_is_not_a_number_stops_it(gpu, n):
+    """h = 1e-8: the kernel's coefficient is infinite and the terms underflow to
+    zero, so every density is not a number.  Both forms stop at the first
+    iteration, report it and leave the same arrays."""
+    p, x = _scene(n, 1e-8)
+    got = []
+    for graph in (1, 0):
+        ps = rxPBDSPH(_fixed(p, 5, graph))
+        ps.Set(x)
+        with pytest.raises(FsphError) as e:
+            ps.Update(1e-4)
+        assert e.value.status == abi.NAN_DETECTED
+        st = ps.last_stats
+        got.append(([st.iterations, st.grid_builds, st.density_error_max, st.density_error_one_sided], _arrays(ps)))
+        ps.close()
+    assert got[0][0][0] == 1
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1], got[1][1]):
+        np.testing.assert_array_equal(a, b)
 
 
 @pytest.mark.parametrize("n", FORMS)
