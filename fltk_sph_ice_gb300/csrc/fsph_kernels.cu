@@ -815,17 +815,14 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
             } else {
                 unsigned int last = (unsigned int)i;
                 count = 0;
-                for (int dz = -1; dz <= 1; ++dz)
-                    for (int dy = -1; dy <= 1; ++dy) {
-                        unsigned int s, e;
-                        row_range(cell_start, c, dy, dz, p, s, e);
-                        for (unsigned int j = s; j < e; ++j) {
-                            if (!(add(0, pos[j]) < p.rl2)) continue;
-                            last = j;
-                            if (list && count < kListMax) list[list_at(count, i, p.n)] = last;
-                            ++count;
-                        }
-                    }
+                walk_cells(
+                    p, cell_start, cell_index(c, p), [&](unsigned int j) { return pos[j]; },
+                    [&](unsigned int j, const float4 &xj) {
+                        if (!(add(0, xj) < p.rl2)) return;
+                        last = j;
+                        if (list && count < kListMax) list[list_at(count, i, p.n)] = last;
+                        ++count;
+                    });
                 if (list && count <= kListMax) /* pad the last group (the slot itself is always listed) */
                     for (int k = count; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = last;
             }
@@ -1011,21 +1008,20 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
     warp_candidates(p, cell_start, [&](unsigned int j) { return __ldg(pos + j); }, xi,
                     valid ? cell_index(c, p) : 0u, valid, p.h2 * (1.0f + 1e-4f), t,
                     [&](bool found, int, int count, int, TileWalk<1> &walk) {
-                        auto meet = [&](unsigned int j) {
-                            if (ref_neighbor(xi, f3(__ldg(pos + j)), p.h2)) {
+                        auto load = [&](unsigned int j) { return __ldg(pos + j); };
+                        auto meet = [&](unsigned int j, const float4 &xj) {
+                            if (ref_neighbor(xi, f3(xj), p.h2)) {
                                 if (k < (unsigned int)kListMax) list[list_at((int)k, i, p.n)] = j;
                                 ++k;
                             }
                         };
                         if (found) {
-                            for (int f = 0; f < count; ++f) meet(walk.next());
+                            for (int f = 0; f < count; ++f) {
+                                const unsigned int j = walk.next();
+                                meet(j, load(j));
+                            }
                         } else {
-                            for (int dz = -1; dz <= 1; ++dz)
-                                for (int dy = -1; dy <= 1; ++dy) {
-                                    unsigned int s, e;
-                                    row_range(cell_start, c, dy, dz, p, s, e);
-                                    for (unsigned int j = s; j < e; ++j) meet(j);
-                                }
+                            walk_cells(p, cell_start, cell_index(c, p), load, meet);
                         }
                         cnt_p[id[i]] = k;
                         cnt[i] = k > (unsigned int)kListMax ? kListOverflow : (unsigned char)k;

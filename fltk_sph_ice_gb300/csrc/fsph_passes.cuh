@@ -262,36 +262,54 @@ __device__ __forceinline__ void hash_body(const DevParams &p, int i, float3 x, u
     rank[i] = atomicAdd(count + c, 1u);
 }
 
+/* Calls f(j, load(j)) for every slot j of the 27 cells around `cell`, in ascending
+ * order: a thread's own search, for the slots of a warp that do not search
+ * together (warp_candidates).  Four positions and the bounds of three rows in
+ * flight. */
+template <class Load, class F>
+__device__ __forceinline__ void walk_cells(const DevParams &p, const unsigned int *__restrict__ cell_start,
+                                           unsigned int cell, Load &&load, F &&f) {
+#pragma unroll 1
+    for (int z = -1; z <= 1; ++z) {
+        unsigned int s[3], e[3];
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+            const unsigned int base = cell + (unsigned int)((z * p.gy + (y - 1)) * p.gx);
+            s[y] = e[y] = 0u;
+            if (!cell_row_ok(p, base)) continue;
+            s[y] = __ldg(cell_start + base - 1);
+            e[y] = bounded(p, __ldg(cell_start + base + 2), (unsigned int)p.n + 1u, kBoundSlot);
+        }
+#pragma unroll
+        for (int y = 0; y < 3; ++y)
+            for (unsigned int j0 = s[y]; j0 < e[y]; j0 += 4) {
+                float4 xc[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) xc[u] = load(min(j0 + u, e[y] - 1));
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (j0 + u < e[y]) f(j0 + u, xc[u]);
+            }
+    }
+}
+
 /* Every slot j within the list radius (= the cell width) of slot i at the
- * build positions xb, self included, in ascending order: one thread on its
- * own, for the slots of a warp whose candidates do not fit its tile. */
+ * build positions xb, self included, in ascending order: one thread on its own. */
 __device__ __forceinline__ void build_list_body(const DevParams &p, int i, const unsigned int *__restrict__ cell_start,
                                                 const float4 *__restrict__ xb, unsigned int cell,
                                                 ListEntry *__restrict__ list, unsigned char *__restrict__ cnt) {
     const float3 xi = f3(xb[i]);
     int k = 0;
     ListEntry last = 0;
-#pragma unroll 1
-    for (int r = 0; r < 9; ++r) {
-        const unsigned int base = cell + (unsigned int)(((r / 3 - 1) * p.gy + (r % 3 - 1)) * p.gx);
-        if (!cell_row_ok(p, base)) continue;
-        const unsigned int s = __ldg(cell_start + base - 1);
-        const unsigned int e = bounded(p, __ldg(cell_start + base + 2), (unsigned int)p.n + 1u, kBoundSlot);
-        for (unsigned int j0 = s; j0 < e; j0 += 4) { /* four loads in flight */
-            float4 xc[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) xc[u] = __ldg(xb + min(j0 + u, e - 1));
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float3 d = xi - f3(xc[u]);
-                if (j0 + u < e && dot3(d, d) < p.rl2) {
-                    last = j0 + u;
-                    if (k < kListMax) list[list_at(k, i, p.n)] = last;
-                    ++k;
-                }
-            }
-        }
-    }
+    walk_cells(
+        p, cell_start, cell, [&](unsigned int j) { return __ldg(xb + j); },
+        [&](unsigned int j, const float4 &xj) {
+            const float3 d = xi - f3(xj);
+            if (!(dot3(d, d) < p.rl2)) return;
+            last = j;
+            if (k < kListMax) list[list_at(k, i, p.n)] = last;
+            ++k;
+        });
     const bool overflow = k > kListMax;
     if (!overflow) /* pad the last group (k >= 1: the slot itself is always listed) */
         for (int t = k; (t & 3) != 0; ++t) list[list_at(t, i, p.n)] = last;
@@ -412,10 +430,10 @@ struct TileWalk {
 
 /* Calls emit(found, first, count, total, walk) once for each valid lane: found:
  * the lane's `count` candidates within sqrt(r2max) come from walk, ascending;
- * else they have to be looked for without the tile (more than fit it, or a
- * coordinate out of the operands' range: a particle far outside the box, or not
- * a number).  load(j): slot j's position, a plain load where the kernel writes
- * beside it.  xi, cell: the lane's position and build cell, cells ascending over
+ * else they have to be looked for without the tile (more than fit it, lanes far
+ * apart, or a coordinate out of the operands' range: a particle far outside the
+ * box, or not a number).  load(j): slot j's position, a plain load where the
+ * kernel writes beside it.  xi, cell: the lane's position and build cell, cells ascending over
  * the lanes, padding lanes (valid = false) after the valid ones; every lane of
  * the warp calls it.  Lanes in different rows of cells, or more than eight cells
  * apart (a run that wraps, sparse fluid), take turns: a row's range then never
@@ -425,7 +443,15 @@ struct TileWalk {
  * in each) and the tile.  Each takes a W-th of every turn's words and emits what
  * it found there: `count` of the lane's `total`, from the `first` on; what is not
  * found is warp 0's alone.  A warp's twenty words in a row, latency bound, are the
- * pass of a small scene: 16 us at 6,912 slots with one warp, 10 with four. */
+ * pass of a small scene: 16 us at 6,912 slots with one warp, 10 with four.
+ *
+ * In sparse fluid (spray) the lanes share few candidates and a warp takes up to 32
+ * turns: there each lane looks for its own, once the cells between the lanes, at
+ * most three a pair, are more than kTileApart (a lattice at rest has about 5).  The
+ * list build in us, own / tile, at 1 M particles at random with one in (0.8 h)^3 129
+ * / 128, h^3 123 / 143, (1.2 h)^3 96 / 145, (2 h)^3 56 / 252; with four warps, 30,000
+ * particles, (0.8 h)^3 17 / 13, h^3 17 / 19, (1.2 h)^3 13 / 34, (2 h)^3 8 / 34. */
+constexpr int kTileApart = 24, kTileApartSplit = 36; /* one warp, several */
 template <int W, class Load, class Emit>
 __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
                                                 Load &&load, float3 xi, unsigned int cell, bool valid, float r2max,
@@ -442,6 +468,16 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
     const unsigned int ones = 0x3c003c00u; /* (1, 1) */
     const bool upper = (lane & 2) != 0;    /* terms 12-15 of a candidate are ones, 8-11 its terms 0-3 again */
     const int own = (lane >> 2) + 8 * (lane & 3); /* the slot whose 32 candidates this lane ends up with */
+    /* lanes too far apart to share candidates look for their own */
+    const unsigned int prev = __shfl_up_sync(0xffffffffu, cell, 1);
+    if (__reduce_add_sync(0xffffffffu, valid && lane > 0 ? min(cell - prev, 3u) : 0u) >
+        (unsigned int)(W == 1 ? kTileApart : kTileApartSplit)) {
+        if (valid && wid == 0) {
+            TileWalk<W> walk(t, 0u, 0);
+            emit(false, 0, 0, 0, walk);
+        }
+        return;
+    }
     unsigned int todo = __ballot_sync(0xffffffffu, valid);
     while (todo) {
         int cnt = 0, w = 0;
