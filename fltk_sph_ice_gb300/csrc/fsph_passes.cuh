@@ -449,8 +449,9 @@ struct TileWalk {
  * turns: there each lane looks for its own, once the cells between the lanes, at
  * most three a pair, are more than kTileApart (a lattice at rest has about 5).  The
  * list build in us, own / tile, at 1 M particles at random with one in (0.8 h)^3 129
- * / 128, h^3 123 / 143, (1.2 h)^3 96 / 145, (2 h)^3 56 / 252; with four warps, 30,000
- * particles, (0.8 h)^3 17 / 13, h^3 17 / 19, (1.2 h)^3 13 / 34, (2 h)^3 8 / 34. */
+ * / 128, h^3 125 / 143, (1.2 h)^3 100 / 145, (2 h)^3 58 / 252; with four warps, 30,000
+ * particles, (0.8 h)^3 17 / 13, h^3 17 / 19, (1.2 h)^3 15 / 34, (2 h)^3 9 / 34.  At
+ * rest the choice costs the batched build 815 -> 853 us, the others nothing. */
 constexpr int kTileApart = 24, kTileApartSplit = 36; /* one warp, several */
 template <int W, class Load, class Emit>
 __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
@@ -470,20 +471,18 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
     const int own = (lane >> 2) + 8 * (lane & 3); /* the slot whose 32 candidates this lane ends up with */
     /* lanes too far apart to share candidates look for their own */
     const unsigned int prev = __shfl_up_sync(0xffffffffu, cell, 1);
-    if (__reduce_add_sync(0xffffffffu, valid && lane > 0 ? min(cell - prev, 3u) : 0u) >
-        (unsigned int)(W == 1 ? kTileApart : kTileApartSplit)) {
-        if (valid && wid == 0) {
-            TileWalk<W> walk(t, 0u, 0);
-            emit(false, 0, 0, 0, walk);
-        }
-        return;
-    }
+    const bool apart = __reduce_add_sync(0xffffffffu, valid && lane > 0 ? min(cell - prev, 3u) : 0u) >
+                       (unsigned int)(W == 1 ? kTileApart : kTileApartSplit);
     unsigned int todo = __ballot_sync(0xffffffffu, valid);
     while (todo) {
         int cnt = 0, w = 0;
         unsigned int any = 0u, done = 0u, over = 0u;
         bool bad = false;
-        do { /* turns, until the tile is full */
+        if (apart) {
+            over = done = todo;
+            todo = 0u;
+        }
+        while (todo) { /* turns, until the tile is full */
             const int lead = __ffs((int)todo) - 1;
             const unsigned int lead_row = __shfl_sync(0xffffffffu, row, lead);
             const unsigned int first = __shfl_sync(0xffffffffu, cell, lead);
@@ -599,7 +598,7 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 if (m) any |= 0x80000000u >> at;
             }
             if (W > 1) w += (int)words;
-        } while (todo);
+        }
         const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
         const int count = __shfl_sync(0xffffffffu, cnt, holder);
         const unsigned int some = __shfl_sync(0xffffffffu, any, holder);
