@@ -841,22 +841,17 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
     }
 }
 
-/* k_sph_density with LPP lanes per particle, so that small scenes still
- * fill the GPU: the lanes of a group take the candidates of each row in
- * turn (lane s the s-th of every LPP consecutive ones), and each LPP-wide
- * chunk's hits are ranked by a ballot inside the group, so the list holds
- * the same slots in the same order as one thread's walk.  The density is
- * the group's sum of the lanes' partial sums (same terms, other order). */
-template <int LPP>
+/* The same with a warp per particle, for scenes that would leave the GPU idle: its
+ * lanes take the candidates of each row side by side and a ballot ranks the hits,
+ * so the list holds the same slots in the same order.  The density is the sum of
+ * the lanes' partial sums (same terms, other order), the errors of their additions
+ * kept. */
 __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const unsigned int *__restrict__ cell_start,
                                                               float4 *pos, float4 *vel, float *__restrict__ dens,
                                                               float *__restrict__ pres, ListEntry *__restrict__ list,
                                                               unsigned char *__restrict__ cnt) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int sub = t % LPP, lane = threadIdx.x & 31;
-    const bool valid = t / LPP < p.n;
-    const int i = valid ? t / LPP : p.n - 1; /* padding groups walk a real slot and write nothing */
-    const unsigned int gmask = (0xffffffffu >> (32 - LPP)) << (lane & ~(LPP - 1));
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (i >= p.n) return;
     const float3 xi = f3(pos[i]);
     const int3 c = cell_of(xi, p);
     float acc = 0.0f;
@@ -866,8 +861,8 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
         for (int dy = -1; dy <= 1; ++dy) {
             unsigned int s, e;
             row_range(cell_start, c, dy, dz, p, s, e);
-            for (unsigned int j0 = s; j0 < e; j0 += LPP) { /* the same trip count for the whole group */
-                const unsigned int j = j0 + (unsigned int)sub;
+            for (unsigned int j0 = s; j0 < e; j0 += 32) {
+                const unsigned int j = j0 + (unsigned int)lane;
                 bool hit = false;
                 if (j < e) {
                     const float3 d = xi - f3(pos[j]);
@@ -879,30 +874,20 @@ __global__ void __launch_bounds__(kBlock) k_sph_density_lanes(DevParams p, const
                     hit = r2 < p.rl2;
                 }
                 if (list) {
-                    const unsigned int m = __ballot_sync(gmask, hit) & gmask;
+                    const unsigned int m = __ballot_sync(0xffffffffu, hit);
                     if (m) {
                         if (hit) {
                             const int at = k + __popc(m & ((1u << lane) - 1u));
                             if (at < kListMax) list[list_at(at, i, p.n)] = (ListEntry)j;
                         }
-                        last = __shfl_sync(gmask, j, 31 - __clz(m));
+                        last = j0 + (unsigned int)(31 - __clz((int)m));
                         k += __popc(m);
                     }
                 }
             }
         }
-    /* the lanes' sums, each addition's error kept: LPP = 16 or 32 lanes add more
-     * often than the 8 that were the most before */
-    float err = 0.0f;
-#pragma unroll
-    for (int o = LPP / 2; o > 0; o >>= 1) {
-        const float other = __shfl_xor_sync(0xffffffffu, acc, o);
-        const Split t = two_sum(acc, other);
-        err += __shfl_xor_sync(0xffffffffu, err, o) + t.l;
-        acc = t.h;
-    }
-    acc += err;
-    if (!valid || sub != 0) return;
+    acc = group_sum_split<32>(acc, 0.0f);
+    if (lane != 0) return;
     if (list) {
         const bool ovf = k > kListMax;
         if (!ovf) /* pad the last group (k >= 1: the slot itself is always listed) */
@@ -1630,10 +1615,10 @@ static int lanes_to_fill(int n, int most) {
 }
 static int sph_force_lanes(int n) { return lanes_to_fill(n, 8); }
 /* The density pass by size, us at 8,000 / 15,625 / 32,768 / 64,000 / 125,000 /
- * 262,144 slots: lanes of a particle's own candidates (up to 32) 10.9 / 16.3 /
- * 22.7 / 51.3 / - / -, four warps for the tile of 32 slots 14.4 / 14.3 / 16.4 /
- * 28.2 / 45.5 / 84.5, one warp 20.5 / 22.5 / 22.8 / 28.8 / 36.9 / 59.6; at 4,096
- * the lanes take 8.7 (16.4 when they were at most eight). */
+ * 262,144 slots: a warp a particle 10.9 / 16.3 / 22.7 / 51.3 / - / -, four warps
+ * for the tile of 32 slots 14.4 / 14.3 / 16.4 / 28.2 / 45.5 / 84.5, one warp 20.5 /
+ * 22.5 / 22.8 / 28.8 / 36.9 / 59.6; at 4,096 a warp a particle takes 8.7 (eight
+ * lanes 16.4). */
 constexpr int kSphTileMin = 12288, kSphSplitMax = 1 << 16;
 void launch_sph_density(const DevParams &p, const unsigned int *cell_start, float4 *pos, float4 *vel, float *dens,
                         float *pres, const NbrLists &nl, cudaStream_t s) {
@@ -1646,10 +1631,7 @@ void launch_sph_density(const DevParams &p, const unsigned int *cell_start, floa
         k_sph_density<4><<<blocks_for(p.n, 32), 128, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
         return;
     }
-    const int lanes = lanes_to_fill(p.n, 32);
-    auto k = lanes >= 32 ? k_sph_density_lanes<32> : lanes >= 16 ? k_sph_density_lanes<16> : k_sph_density_lanes<8>;
-    const int lpp = std::max(lanes, 8);
-    k<<<blocks_for((long long)p.n * lpp), kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
+    k_sph_density_lanes<<<blocks_for((long long)p.n * 32), kBlock, 0, s>>>(p, cell_start, pos, vel, dens, pres, l, nl.cnt);
 }
 void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,
                         float *dens, float *lambda, cudaStream_t s) {
