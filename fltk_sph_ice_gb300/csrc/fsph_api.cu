@@ -1377,7 +1377,7 @@ int fsph_set_array(fsph_ctx *c, int type, const void *data, int start, int count
             FSPH_CUDA(c, cudaMemcpyAsync(c->tmp4, data, (size_t)count * 16, k, s));
             launch_check_finite(count, c->tmp4, nullptr, c->flag, s);
         }
-            FSPH_TRY(check_launch(c));
+        FSPH_TRY(check_launch(c));
         FSPH_CUDA(c, cudaStreamSynchronize(s));
         if (*c->flag) return fail(c, FSPH_NAN_DETECTED, "non-finite position or velocity");
         float4 *dst = type == FSPH_POSITION ? c->set[0].pos : c->set[0].vel;
@@ -1472,7 +1472,8 @@ int fsph_step(fsph_ctx *c, float dt, void *stream, fsph_step_stats *stats) {
             std::fflush(c->log);
         }
         if (stats->status == FSPH_NAN_DETECTED) return fail(c, FSPH_NAN_DETECTED, "NaN in density or position");
-        if (stats->status == FSPH_TIMEOUT) return fail(c, FSPH_TIMEOUT, c->ctl_host->wait_err ? "constraint loop: a grid barrier's wait ran out"
+        if (stats->status == FSPH_TIMEOUT)
+            return fail(c, FSPH_TIMEOUT, c->ctl_host->wait_err ? "constraint loop: a grid barrier's wait ran out"
                                                                : "warm-start inference: an MMA wait ran out");
         if (stats->bounds_bits)
             return fail(c, FSPH_CUDA_ERROR, "debug bounds check: an index out of range (bits " +
@@ -1672,7 +1673,7 @@ int fsph_neighbors_ex(fsph_ctx *c, const float *pos4, int n, float radius, int w
                                      where == FSPH_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
         *c->flag = 0u;
         launch_check_finite(n, c->tmp4, nullptr, c->flag, s);
-            FSPH_CUDA(c, cudaStreamSynchronize(s));
+        FSPH_CUDA(c, cudaStreamSynchronize(s));
         if (*c->flag) return fail(c, FSPH_NAN_DETECTED, "non-finite position");
         launch_iota(n, c->set[1].attr, s);
         x = c->tmp4;
