@@ -314,10 +314,14 @@ def run_leg(ctx, warm: bool, blob):
                     "not_converged_steps": unconv, "status": "FSPH_NOT_CONVERGED" if unconv else "FSPH_OK"}
 
 
+# its columns; k_pbf_sweep's figures are one iteration's
+PROFILE_COLUMNS = {"k_lambda": 0, "k_correction": 1, "k_pbf_sweep": 2}
+LOOP_MAX = 65536  # particles up to which the loop kernel keeps each on a thread of its own
 TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "k_lambda_k_correction_pbf_double_dam_break_1M.md")
 # the sources of the constraint-pass kernels: a profile's figures hold for the
 # kernels built from exactly these files
 KERNEL_SOURCES = ("fltk_sph_ice_gb300/csrc/fsph_passes.cuh", "fltk_sph_ice_gb300/csrc/fsph_kernels.cu",
+                  "fltk_sph_ice_gb300/csrc/fsph_loop.cu",
                   "fltk_sph_ice_gb300/csrc/fsph_kernels.cuh", "fltk_sph_ice_gb300/csrc/fsph_internal.cuh")
 
 
@@ -360,8 +364,8 @@ def ncu_traffic(kname: str):
         for line in f:
             if line.startswith("| **traffic per launch**"):
                 mb = [float(x) for x in re.findall(r"([0-9.]+) MB", line)]
-                col = {"k_lambda": 0, "k_correction": 1}.get(kname)
-                if col is not None and len(mb) >= 2:
+                col = PROFILE_COLUMNS.get(kname)
+                if col is not None and len(mb) > col:
                     return mb[col] * 1e6
     return None
 
@@ -377,8 +381,8 @@ def ncu_warp_instructions(kname: str):
         for line in f:
             if line.startswith("| warp instructions"):
                 m = [float(x) for x in re.findall(r"([0-9.]+) M", line)]
-                col = {"k_lambda": 0, "k_correction": 1}.get(kname)
-                if col is not None and len(m) >= 2:
+                col = PROFILE_COLUMNS.get(kname)
+                if col is not None and len(m) > col:
                     return m[col] * 1e6
     return None
 
@@ -395,8 +399,8 @@ def ncu_l1tex(kname: str):
         for line in f:
             if line.startswith("| **L1TEX throughput"):
                 m = [float(x) for x in re.findall(r"([0-9.]+) %", line)]
-                col = {"k_lambda": 0, "k_correction": 1}.get(kname)
-                if col is not None and len(m) >= 2:
+                col = PROFILE_COLUMNS.get(kname)
+                if col is not None and len(m) > col:
                     return {"pct_of_peak_active": m[col], "source": "ncu l1tex__throughput"}
     return None
 
@@ -423,16 +427,27 @@ def issue_bound(kname: str, launch_ms: float):
         return None
 
 
-def roofline_of(L, abi, ps, n, mean_iters):
-    t_lam, t_cor, t_grid, t_list = (ctypes.c_float(0) for _ in range(4))
+def roofline_of(L, abi, ps, n, mean_iters, loop=True):
+    """The dominant kernel.  loop: graph steps, whose iterations run inside one
+    kernel (both passes, 60 bytes a particle; launch_ms and traffic are one
+    iteration's); else, and beside a boundary, the passes are launches and the
+    longer one is reported.  lambda_ms and correction_ms are those launches'."""
+    t_lam, t_cor, t_grid, t_list, t_loop = (ctypes.c_float(0) for _ in range(5))
     L.fsph_time_pass(ps.handle, abi.PASS_LAMBDA, 20, ctypes.byref(t_lam))
     L.fsph_time_pass(ps.handle, abi.PASS_CORRECTION, 20, ctypes.byref(t_cor))
     L.fsph_time_pass(ps.handle, abi.PASS_GRID, 10, ctypes.byref(t_grid))
     L.fsph_time_pass(ps.handle, abi.PASS_LIST, 10, ctypes.byref(t_list))
-    if t_cor.value >= t_lam.value:
-        kname, kms, kbytes = "k_correction", t_cor.value, BYTES_CORRECTION * n
+    loop_st = L.fsph_time_pass(ps.handle, abi.PASS_LOOP, 20, ctypes.byref(t_loop))
+    loop = loop and loop_st == abi.OK
+    if loop:
+        kname = "k_pbf_loop" if n <= LOOP_MAX else "k_pbf_sweep"
+        kms, kbytes, iter_ms = t_loop.value, (BYTES_LAMBDA + BYTES_CORRECTION) * n, t_loop.value
     else:
-        kname, kms, kbytes = "k_lambda", t_lam.value, BYTES_LAMBDA * n
+        iter_ms = t_lam.value + t_cor.value
+        if t_cor.value >= t_lam.value:
+            kname, kms, kbytes = "k_correction", t_cor.value, BYTES_CORRECTION * n
+        else:
+            kname, kms, kbytes = "k_lambda", t_lam.value, BYTES_LAMBDA * n
     peak, peak_kind = measured_peaks()
     achieved = kbytes / (kms / 1000.0) / 1e9
     traffic = ncu_traffic(kname)
@@ -441,9 +456,9 @@ def roofline_of(L, abi, ps, n, mean_iters):
            else f"none: the committed profile was captured from other kernel sources than these ({digest})")
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "traffic_source": src, "kernel": kname, "launch_ms": kms, "peak_kind": peak_kind,
-            "lambda_ms": t_lam.value, "correction_ms": t_cor.value, "grid_build_ms": t_grid.value,
-            "list_build_ms": t_list.value, "issue": issue_bound(kname, kms), "l1tex": ncu_l1tex(kname),
-            "passes_ms_per_step": mean_iters * (t_lam.value + t_cor.value)}
+            "iteration_ms": iter_ms, "lambda_ms": t_lam.value, "correction_ms": t_cor.value,
+            "grid_build_ms": t_grid.value, "list_build_ms": t_list.value, "issue": issue_bound(kname, kms),
+            "l1tex": ncu_l1tex(kname), "passes_ms_per_step": mean_iters * iter_ms}
 
 
 # compulsory HBM bytes per particle-step of a PBF step with I constraint
@@ -551,7 +566,7 @@ def gpu_arm(args):
         ps, sc, warm = run_leg(ctx, True, blob)
     clocks = clk.summary()
     n = sc.n
-    roofline = roofline_of(L, abi, ps, n, warm["mean_iterations"])
+    roofline = roofline_of(L, abi, ps, n, warm["mean_iterations"], not args.eager)
     # the passes above advanced the state; a fresh warm-start context for e2e
     ps.close()
     e2e = None
@@ -578,9 +593,9 @@ def gpu_arm(args):
 
     # kernel launches of the timed warm-start steps, counted by the library from the step graph's
     # kernel nodes, the executed iterations and the grid rebuilds (eager mode does not count them:
-    # MLP, predict+hash, 3 scan, scatter, cell sort, gather, list build, 2 per iteration, finalize,
+    # MLP, predict+hash, 2 scan, scatter, gather, list build, 2 per iteration, finalize,
     # XSPH/vorticity/features, vorticity apply, without rebuilds)
-    gpu_launches = warm["kernels"] or int(args.steps * (12 + 2 * warm["mean_iterations"]))
+    gpu_launches = warm["kernels"] or int(args.steps * (10 + 2 * warm["mean_iterations"]))
     if rank == 0:
         cfg = {"workload": WORKLOAD, "particles": n, "block": list(BLOCK), "dt": sc.dt, "eta_one_sided": 1e-3,
                "constraint": "unilateral (clamped C >= 0)", "method": method_of(meta),
@@ -689,7 +704,7 @@ def config_arm(args):
     value, tot_s = replica_rate(sc.n, args.steps, tot_s, dist)
     peak, peak_kind = measured_peaks()
     if pbf:
-        roof = roofline_of(L, abi, ps, sc.n, 4.0)
+        roof = roofline_of(L, abi, ps, sc.n, 4.0, not args.eager)
         roof["step"] = step_roofline(value, 4.0, float(np.mean(builds)))
     else:
         roof = sph_roofline(L, abi, ps, sc.n)

@@ -168,7 +168,7 @@ EXPORTS = [
 ]
 
 # fsph_pass
-PASS_LAMBDA, PASS_CORRECTION, PASS_GRID, PASS_LIST, PASS_SPH_DENSITY, PASS_SPH_FORCE = 0, 1, 2, 3, 4, 5
+PASS_LAMBDA, PASS_CORRECTION, PASS_GRID, PASS_LIST, PASS_SPH_DENSITY, PASS_SPH_FORCE, PASS_LOOP = 0, 1, 2, 3, 4, 5, 6
 
 _LIB = None
 

@@ -882,7 +882,7 @@ int build_pbf_graph(fsph_ctx *c, const DevParams &p) {
     cudaError_t le = cudaSuccess;
     if (c->loop_kernel) {
         le = launch_pbf_loop(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->xb, c->ctl, c->loop, hw, hrb, hrb2,
-                             ext ? 1 : 0, c->wait_polls, c->nl, c->s2);
+                             ext ? 3 : 1, c->wait_polls, c->nl, c->s2);
     } else {
         launch_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->ctl, c->epart, hw, 1, c->nl, c->s2);
         launch_boundary_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->ctl, c->b_stat, c->b_lam, c->s2);
@@ -2335,6 +2335,42 @@ int fsph_emit_inlets(fsph_ctx *c, int step, int *emitted) {
     return FSPH_OK;
 }
 
+namespace {
+/* one launch of the loop kernel that makes `reps` iterations, on lists already
+ * built: no tolerance and no rebuild ends it before */
+int time_loop(fsph_ctx *c, DevParams p, int reps, float *avg_ms) {
+    if (!loop_fits(p)) return fail(c, FSPH_UNSUPPORTED, "this scene's steps launch the passes one by one");
+    cudaStream_t s = c->stream;
+    p.min_iter = p.max_iter = reps;
+    p.eta = 0.0f;
+    p.skin2 = INFINITY;
+    cudaEvent_t e0, e1;
+    FSPH_CUDA(c, cudaEventCreate(&e0));
+    FSPH_CUDA(c, cudaEventCreate(&e1));
+    float ms = 0.0f;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) { /* the first warms up */
+        if (k) e = cudaMemsetAsync(c->ctl, 0, sizeof(DevCtl), s);
+        if (e == cudaSuccess) e = cudaEventRecord(e0, s);
+        if (e == cudaSuccess)
+            e = launch_pbf_loop(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->xb, c->ctl, c->loop, 0ull, 0ull,
+                                0ull, 0, c->wait_polls, c->nl, s);
+        if (e == cudaSuccess) e = cudaEventRecord(e1, s);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c->ctl_host, c->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    FSPH_CUDA(c, e);
+    if (c->ctl_host->wait_err) return fail(c, FSPH_TIMEOUT, "constraint loop: a grid barrier's wait ran out");
+    if (c->ctl_host->nan_flag || (int)c->ctl_host->iter != reps)
+        return fail(c, FSPH_NAN_DETECTED, "NaN in density or position");
+    *avg_ms = ms / (float)reps;
+    return FSPH_OK;
+}
+}  // namespace
+
 int fsph_time_pass(fsph_ctx *c, int pass, int reps, float *avg_ms) {
     if (!c || !avg_ms || reps <= 0) return FSPH_INVALID_ARG;
     FSPH_USABLE(c);
@@ -2377,6 +2413,7 @@ int fsph_time_pass(fsph_ctx *c, int pass, int reps, float *avg_ms) {
     /* the state after a step: x* = x in the home set, already cell-ordered */
     FSPH_TRY(build_on(c, p, c->set[0].pos));
     FSPH_CUDA(c, cudaMemsetAsync(c->ctl, 0, sizeof(DevCtl), s));
+    if (pass == FSPH_PASS_LOOP) return time_loop(c, p, reps, avg_ms);
     launch_lambda(p, c->cell_start, c->ppos[0], c->ppos[1], c->dens, c->ctl, c->epart, 0ull, 0, c->nl, s);
     cudaEvent_t e0, e1;
     FSPH_CUDA(c, cudaEventCreate(&e0));

@@ -133,7 +133,7 @@ void launch_lambda(const DevParams &p, const unsigned int *cell_start, float4 *p
                    const NbrLists &nl, cudaStream_t s);
 /* The whole constraint loop in one cooperative kernel (fsph_loop.cu): iterations
  * until the loop ends or a grid rebuild is due, then the three conditions are set
- * (post: the third exists).  loop_fits: lists are on, there is no boundary (its
+ * (use_graph: 1, with the third 3, outside a graph 0).  loop_fits: lists are on, there is no boundary (its
  * lambda is a kernel of its own between the passes) and every block is resident at
  * once.  Up to kLoopMax particles each has a thread of its own.  polls: before a
  * block gives a barrier up (0: the default). */
@@ -141,7 +141,7 @@ constexpr int kLoopMax = 65536;
 bool loop_fits(const DevParams &p);
 cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                             float *dens, const float4 *xb, DevCtl *ctl, LoopCtl *lc, unsigned long long while_handle,
-                            unsigned long long if_handle, unsigned long long if_handle2, int post,
+                            unsigned long long if_handle, unsigned long long if_handle2, int use_graph,
                             unsigned long long polls, const NbrLists &nl, cudaStream_t s);
 /* density and lambda of x (slot order) at order[slot], walking the cells */
 void launch_lambda_walk(const DevParams &p, const unsigned int *cell_start, const float4 *x, const unsigned int *order,

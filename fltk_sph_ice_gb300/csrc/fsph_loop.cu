@@ -166,7 +166,7 @@ __device__ __forceinline__ bool loop_decide(const DevParams &p, const LoopCtl *l
  * and the counters for another launch */
 __device__ __forceinline__ void loop_leave(const DevParams &p, DevCtl *ctl, LoopCtl *lc, const LoopState &s, bool ok,
                                            cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif,
-                                           cudaGraphConditionalHandle hif2, int post) {
+                                           cudaGraphConditionalHandle hif2, int use_graph) {
     if (!ok) ctl->wait_err = 1u;
     __threadfence();
     if (atomicAdd(&lc->left, 1u) != gridDim.x - 1u) return;
@@ -187,9 +187,11 @@ __device__ __forceinline__ void loop_leave(const DevParams &p, DevCtl *ctl, Loop
     /* a correction that was not a number also asks for a rebuild: the launch after
      * it stops at its first errors, as k_lambda does */
     if (cont && __ldcg(&ctl->nan_flag)) lc->nan[0] = 1u;
-    cudaGraphSetConditional(hwhile, cont);
-    cudaGraphSetConditional(hif, cont & s.rebuild);
-    if (post) cudaGraphSetConditional(hif2, s.rebuild);
+    if (use_graph & 1) {
+        cudaGraphSetConditional(hwhile, cont);
+        cudaGraphSetConditional(hif, cont & s.rebuild);
+        if (use_graph & 2) cudaGraphSetConditional(hif2, s.rebuild);
+    }
 }
 
 template <bool KAHAN, int BLOCK>
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
     k_pbf_loop(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
                float *__restrict__ dens, const float4 *__restrict__ xb, DevCtl *ctl, LoopCtl *lc,
                cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hif2,
-               int post, unsigned long long polls, const ListEntry *__restrict__ list,
+               int use_graph, unsigned long long polls, const ListEntry *__restrict__ list,
                const unsigned char *__restrict__ cnt) {
     __shared__ unsigned int s_kept[(kListMax / 2) * BLOCK];
     __shared__ unsigned long long s_e1[BLOCK / 32], s_e2[BLOCK / 32];
@@ -297,7 +299,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 64 ? 4 : 512 / BLOCK)
         st.at = nx;
     }
     if (valid) dens[i] = rho;
-    if (threadIdx.x == 0) loop_leave(p, ctl, lc, st, ok, hwhile, hif, hif2, post);
+    if (threadIdx.x == 0) loop_leave(p, ctl, lc, st, ok, hwhile, hif, hif2, use_graph);
 }
 
 /* The same loop from the lists in memory, for scenes that do not fit k_pbf_loop:
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(kSweepBlock, 2)
     k_pbf_sweep(DevParams p, const unsigned int *__restrict__ cell_start, float4 *ppos0, float4 *ppos1,
                 float *__restrict__ dens, const float4 *__restrict__ xb, DevCtl *ctl, LoopCtl *lc,
                 cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hif2,
-                int post, unsigned long long polls, const ListEntry *__restrict__ list,
+                int use_graph, unsigned long long polls, const ListEntry *__restrict__ list,
                 const unsigned char *__restrict__ cnt) {
     __shared__ unsigned long long s_e1[kSweepBlock / 32], s_e2[kSweepBlock / 32];
     __shared__ float s_em[kSweepBlock / 32], s_d[kSweepBlock / 32];
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(kSweepBlock, 2)
         __syncthreads();
         if (!s_go) break;
     }
-    if (threadIdx.x == 0) loop_leave(p, ctl, lc, st, ok, hwhile, hif, hif2, post);
+    if (threadIdx.x == 0) loop_leave(p, ctl, lc, st, ok, hwhile, hif, hif2, use_graph);
 }
 
 typedef void (*LoopKernel)(DevParams, const unsigned int *, float4 *, float4 *, float *, const float4 *, DevCtl *,
@@ -470,7 +472,7 @@ bool loop_fits(const DevParams &p) {
 
 cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, float4 *ppos0, float4 *ppos1,
                             float *dens, const float4 *xb, DevCtl *ctl, LoopCtl *lc, unsigned long long while_handle,
-                            unsigned long long if_handle, unsigned long long if_handle2, int post,
+                            unsigned long long if_handle, unsigned long long if_handle2, int use_graph,
                             unsigned long long polls, const NbrLists &nl, cudaStream_t s) {
     LoopShape sh;
     const unsigned int blocks = loop_blocks(p, sh);
@@ -480,7 +482,8 @@ cudaError_t launch_pbf_loop(const DevParams &p, const unsigned int *cell_start, 
     const ListEntry *list = nl.list;
     const unsigned char *cnt = nl.cnt;
     if (!polls) polls = kLoopPolls * (1ull + ((unsigned int)p.n >> 16));
-    void *args[] = {&q, &cell_start, &ppos0, &ppos1, &dens, &xb, &ctl, &lc, &hw, &h1, &h2, &post, &polls, &list, &cnt};
+    void *args[] = {&q, &cell_start, &ppos0, &ppos1, &dens, &xb, &ctl, &lc, &hw, &h1, &h2, &use_graph, &polls,
+                    &list, &cnt};
     return cudaLaunchCooperativeKernel((const void *)sh.kernel, dim3(blocks), dim3(sh.block), args, 0, s);
 }
 

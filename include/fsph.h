@@ -533,10 +533,13 @@ int fsph_set_wait_limit(fsph_ctx *ctx, long long polls);
 typedef enum fsph_pass {
     FSPH_PASS_LAMBDA = 0,      /* one lambda pass (density + constraint + error reduction) */
     FSPH_PASS_CORRECTION = 1,  /* one position-correction pass */
-    FSPH_PASS_GRID = 2,        /* one grid build (hash, scan, scatter, cell sort, reorder) */
+    FSPH_PASS_GRID = 2,        /* one grid build (hash, scan, scatter, reorder by rank) */
     FSPH_PASS_LIST = 3,        /* one neighbour-list build on the current grid */
     FSPH_PASS_SPH_DENSITY = 4, /* WCSPH: one density + pressure pass */
-    FSPH_PASS_SPH_FORCE = 5    /* WCSPH: one force (pressure + viscosity + gravity) pass */
+    FSPH_PASS_SPH_FORCE = 5,   /* WCSPH: one force (pressure + viscosity + gravity) pass */
+    FSPH_PASS_LOOP = 6         /* one iteration (both passes) inside the kernel that a graph step without a
+                                * boundary runs: the mean over one launch of `reps` iterations;
+                                * FSPH_UNSUPPORTED with a boundary or without lists */
 } fsph_pass;
 /* Time `reps` back-to-back launches of one pass of the current state (the
  * PBF passes on a PBF context, the WCSPH passes on a WCSPH one) with CUDA
