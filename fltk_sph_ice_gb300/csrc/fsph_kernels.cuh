@@ -40,11 +40,12 @@ constexpr int kPassBlock = FSPH_PASS_BLOCK;
  * 32,000, 43.1 -> 42.0 at 131,072, 71.4 -> 81.6 at 294,912 */
 constexpr int kDeepBlock = 64, kDeepMinB = 12, kDeepMax = 65536;
 /* Beside a boundary a pass waits for the few warps at its shell, and which form is
- * the faster depends on where they land: steps with a shell took, deep / plain, in
- * us, 948 / 1,044 at 13,824 particles, 1,332 / 1,244 at 46,656, 1,070 / 1,245 and
- * (10 iterations) 1,591 / 1,812 at 54,872, 851 / 777 and 1,366 / 1,110 at 59,319,
- * 1,097 / 1,185 and (10 iterations) 1,922 / 1,737 at 64,000.  The line lies where
- * the plain form begins to be mostly the faster. */
+ * the faster depends on where they land, which a particle count does not tell.
+ * Drops of 20^3 to 40^3 particles, 3 to 10 iterations, two skins, deep against
+ * plain: always the faster up to 13,824 (3 to 8 %), from 12 % faster to 12 % slower
+ * up to 54,872 (46,656 the slower, 1,301 against 1,171 us; 54,872 the faster, 988
+ * against 1,139), up to 22 % slower at 59,319 and from 6 % faster to 13 % slower at
+ * 64,000.  The line only keeps the worst of it out. */
 constexpr int kDeepMaxBoundary = 57344;
 /* The XSPH and vorticity passes of larger scenes: a step of 1 M particles with two
  * iterations took 852 us in blocks of 128, 857 of 256, 865 of 512, 878 with eight

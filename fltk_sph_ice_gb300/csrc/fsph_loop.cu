@@ -77,8 +77,11 @@ __device__ __forceinline__ bool grid_wait(LoopCtl *lc, unsigned int want, unsign
  * warp to hide a load: 24 gathers leave together, two rounds for most particles.
  * In larger blocks the next eight are in flight while eight are evaluated.  An
  * iteration of 6,912 particles takes 12.3 us by eights, 11.5 with 16 together, 10.7
- * with 24, 12.3 with 28, 14.0 with 40; 32,000 particles (blocks of 128) 13.6 by
- * eights and 14.2 with 24. */
+ * with 24, 12.3 with 28, 14.0 with 40, its lists of about 33 entries; with 37 (a
+ * stirred state) 13.5 by eights, 12.9 with 16, 13.1 with 24, 14.6 with 32, and so in
+ * proportion from 1,000 to 19,456 particles.  Past 64 entries the walks of the
+ * overflowed lists are what counts (55 us).  32,000 particles (blocks of 128) 13.6
+ * by eights and 14.2 with 24. */
 constexpr int kTogether = 24;
 template <int BLOCK, class Load, class F>
 __device__ __forceinline__ void for_each_kept(const DevParams &p, const unsigned int *__restrict__ cell_start,
