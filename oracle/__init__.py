@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes
 import os
 import subprocess
+import unittest
 
 import numpy as np
 
@@ -300,13 +301,18 @@ def ref_env_from_params(p, n: int) -> RefEnv:
     return e
 
 
+class ReferenceUnavailable(RuntimeError, unittest.SkipTest):
+    """The reference's code is not built on this host: a test that compares with
+    it is skipped, any other caller sees a RuntimeError."""
+
+
 class RefSolver:
     """The reference's rxPBDSPH (kind='pbf') or rxSPH (kind='sph'), CPU path."""
 
     def __init__(self, params, n: int, kind: str = "pbf"):
         self.L = ref_lib()
         if self.L is None:
-            raise RuntimeError("reference CPU code unavailable (oracle/_ref not built)")
+            raise ReferenceUnavailable("reference CPU code unavailable (oracle/_ref not built)")
         self.kind = kind
         self.n = int(n)
         self.env = ref_env_from_params(params, self.n)

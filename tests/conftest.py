@@ -15,6 +15,14 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (runs the sm_103a kernels)")
 
 
+def pytest_collection_modifyitems(items):
+    """Where the reference's code is not built, the tests that fail without it run
+    last: a run that stops at its first failure has then run all the others."""
+    import oracle
+    if oracle.ref_lib() is None:
+        items.sort(key=lambda it: "ref_available" in getattr(it, "fixturenames", ()))
+
+
 def cuda_device_count() -> int:
     for name in ("libcudart.so", "libcudart.so.13", "/usr/local/cuda/lib64/libcudart.so"):
         try:
