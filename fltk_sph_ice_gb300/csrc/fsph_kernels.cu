@@ -378,9 +378,13 @@ __global__ void k_rebuild_copy(int n, DevCtl *ctl, const float4 *__restrict__ t_
 /* neighbour lists                                                          */
 /* ======================================================================== */
 
+/* blocks per SM: seven of four warps (72 registers a thread), so that 32,768 slots
+ * are one round of the GPU (the WCSPH density took 19.8 us there with 80 registers,
+ * 16.8 with these); six of four tiles, what shared memory holds */
+constexpr int kSplitBlocks = 7, kTileBlocks = 6;
 /* The lists of every slot, W warps for 32 consecutive ones (build_list_warp). */
 template <int W>
-__global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
+__global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W, W == 1 ? kTileBlocks : kSplitBlocks)
     k_build_list(DevParams p, const unsigned int *__restrict__ cell_start, const float4 *__restrict__ xb,
                  const unsigned int *__restrict__ cellb, ListEntry *__restrict__ list,
                  unsigned char *__restrict__ cnt) {
@@ -752,7 +756,7 @@ __device__ __forceinline__ void sph_density_out(const DevParams &p, int i, float
  * testing all its candidates was bound by issue and took 205 us at 1,030,301
  * slots and 64.6 at 262,144, this form 171 and 59.5. */
 template <int W>
-__global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
+__global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W, W == 1 ? kTileBlocks : kSplitBlocks)
     k_sph_density(DevParams p, const unsigned int *__restrict__ cell_start, float4 *pos, float4 *vel,
                   float *__restrict__ dens, float *__restrict__ pres, ListEntry *__restrict__ list,
                   unsigned char *__restrict__ cnt) {
@@ -813,6 +817,10 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W)
                     count = total;
                 }
             } else {
+                if (W > 1) {
+                    acc[0] = acc[1] = 0.0f;
+                    if (threadIdx.x >= 32u) return;
+                }
                 unsigned int last = (unsigned int)i;
                 count = 0;
                 walk_cells(

@@ -428,10 +428,10 @@ struct TileWalk {
     }
 };
 
-/* Calls emit(found, first, count, total, walk) once for each valid lane: found:
+/* Calls emit(found, first, count, total, walk) for each valid lane: found:
  * the lane's `count` candidates within sqrt(r2max) come from walk, ascending;
- * else they have to be looked for without the tile (more than fit it, lanes far
- * apart, or a coordinate out of the operands' range: a particle far outside the
+ * else they have to be looked for without the tile (more than fit it, W = 1; lanes
+ * far apart; or a coordinate out of the operands' range: a particle far outside the
  * box, or not a number).  load(j): slot j's position, a plain load where the
  * kernel writes beside it.  xi, cell: the lane's position and build cell, cells ascending over
  * the lanes, padding lanes (valid = false) after the valid ones; every lane of
@@ -441,8 +441,11 @@ struct TileWalk {
  * are emitted together.
  * W > 1: the W warps of a block share the same 32 slots (a lane's slot is the same
  * in each) and the tile.  Each takes a W-th of every turn's words and emits what
- * it found there: `count` of the lane's `total`, from the `first` on; what is not
- * found is warp 0's alone.  A warp's twenty words in a row, latency bound, are the
+ * it found there: `count` of the lane's `total`, from the `first` on.  A turn that
+ * does not fit the tile goes through it in parts, each emitted with the total so
+ * far (a lane's own walk by one warp of the four took 178 us where the parts take
+ * 37: the density of a dam break of 32,768 particles after 400 steps, 71 neighbours
+ * on average).  found = false starts a lane again and is for warp 0 to act on.  A warp's twenty words in a row, latency bound, are the
  * pass of a small scene: 16 us at 6,912 slots with one warp, 10 with four.
  *
  * In sparse fluid (spray) the lanes share few candidates and a warp takes up to 32
@@ -474,9 +477,11 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
     const bool apart = __reduce_add_sync(0xffffffffu, valid && lane > 0 ? min(cell - prev, 3u) : 0u) >
                        (unsigned int)(W == 1 ? kTileApart : kTileApartSplit);
     unsigned int todo = __ballot_sync(0xffffffffu, valid);
+    unsigned int resume = 0u; /* W > 1: the word at which a turn in parts goes on */
+    int base = 0;             /* and what its earlier parts found for the lane */
     while (todo) {
         int cnt = 0, w = 0;
-        unsigned int any = 0u, done = 0u, over = 0u;
+        unsigned int any = 0u, done = 0u, over = 0u, part = 0u;
         bool bad = false;
         if (apart) {
             over = done = todo;
@@ -510,15 +515,25 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
             const unsigned int total = __shfl_sync(0xffffffffu, from, 8);
             from -= len; /* lane 9 and on: the total */
             const unsigned int shift = s - from;
-            if (total > (unsigned int)(kTileWords - w) * 32u) {
+            /* the words from lo on, n of them */
+            const unsigned int words = (total + 31u) >> 5, room = (unsigned int)(kTileWords - w), lo = resume;
+            unsigned int n = words - lo;
+            if (n > room) {
                 if (w) break; /* after what the tile holds now */
-                over = grp;   /* never fits */
+                if (W == 1) {
+                    over = grp; /* never fits */
+                    done |= grp;
+                    todo &= ~grp;
+                    break;
+                }
+                part = grp;
+                n = room;
+                resume = lo + room;
+            } else {
                 done |= grp;
                 todo &= ~grp;
-                break;
+                resume = 0u;
             }
-            done |= grp;
-            todo &= ~grp;
             const float ox = 0.5f * (__shfl_sync(0xffffffffu, xi.x, lead) + __shfl_sync(0xffffffffu, xi.x, tail));
             const float oy = __shfl_sync(0xffffffffu, xi.y, lead), oz = __shfl_sync(0xffffffffu, xi.z, lead);
             unsigned int a0[4], a1[4]; /* the slots' terms: rows 0-7, 8-15, 16-23, 24-31; terms 0-7 and 8-15 */
@@ -555,15 +570,14 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 return load(min(q < total ? j : j - (q - total + 1u), (unsigned int)p.n - 1u));
             };
             /* this warp's words */
-            const unsigned int words = (total + 31u) >> 5;
-            const unsigned int begin = W > 1 ? words * wid / W * 32u : 0u;
-            const unsigned int end = W > 1 ? min(total, words * (wid + 1) / W * 32u) : total;
+            const unsigned int begin = W > 1 ? (lo + n * wid / W) * 32u : 0u;
+            const unsigned int end = W > 1 ? min(total, (lo + n * (wid + 1) / W) * 32u) : total;
             unsigned int jn;
             float4 cn;
             if (W == 1 || begin < end) cn = fetch(begin, jn);
 #pragma unroll 1
             for (unsigned int q0 = begin; q0 < end; q0 += 32u, w += W == 1 ? 1 : 0) {
-                const int at = W == 1 ? w : w + (int)(q0 >> 5);
+                const int at = W == 1 ? w : w + (int)((q0 >> 5) - lo);
                 const unsigned int q = q0 + (unsigned int)lane, j = jn;
                 const float4 c = cn;
                 if (q0 + 32u < end) cn = fetch(q0 + 32u, jn);
@@ -597,7 +611,10 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 cnt += __popc(m);
                 if (m) any |= 0x80000000u >> at;
             }
-            if (W > 1) w += (int)words;
+            if (W > 1) {
+                w += (int)n;
+                if (part) break;
+            }
         }
         const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
         const int count = __shfl_sync(0xffffffffu, cnt, holder);
@@ -618,9 +635,15 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
             found = !__any_sync(0xffffffffu, bad) && found;
             __syncwarp();
         }
-        if ((done >> lane & 1u) && (found || wid == 0)) {
+        if (W > 1 && !found) { /* whatever its earlier parts gave, the lane starts again */
+            done |= part;
+            todo &= ~part;
+            part = resume = 0u;
+        }
+        if ((done | part) >> lane & 1u) {
             TileWalk<W> walk(t, some, count);
-            emit(found, first, count, all, walk);
+            emit(found, base + first, count, base + all, walk);
+            if (W > 1) base = (part >> lane & 1u) ? base + all : 0;
         }
         /* the tile is free again */
         if (W > 1)
@@ -645,7 +668,7 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
     warp_candidates(p, cell_start, [&](unsigned int j) { return __ldg(xb + j); }, xi, cell, valid, p.rl2, t,
                     [&](bool found, int first, int count, int total, TileWalk<W> &walk) {
         if (!found) {
-            build_list_body(p, i, cell_start, xb, cell, list, cnt);
+            if (W == 1 || threadIdx.x < 32u) build_list_body(p, i, cell_start, xb, cell, list, cnt);
             return;
         }
         if (W == 1) {
