@@ -752,9 +752,10 @@ __device__ __forceinline__ void sph_density_out(const DevParams &p, int i, float
 }
 /* W warps for 32 consecutive slots: their candidates from the tile
  * (warp_candidates), each evaluated from a gathered position, four at a time,
- * and listed; where they do not fit the tile, a thread's own walk.  A thread
+ * and listed; where the tile does not serve (spray), a thread's own walk.  A thread
  * testing all its candidates was bound by issue and took 205 us at 1,030,301
- * slots and 64.6 at 262,144, this form 171 and 59.5. */
+ * slots and 64.6 at 262,144, this form 171 and 59.5; in a collapsed dam (512,000
+ * slots, 106 neighbours on average) 380 and 291. */
 template <int W>
 __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W, W == 1 ? kTileBlocks : kSplitBlocks)
     k_sph_density(DevParams p, const unsigned int *__restrict__ cell_start, float4 *pos, float4 *vel,
@@ -797,7 +798,7 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W, W == 1 ? kTileBl
                     for (int u = 0; u < 4; ++u) v[u] = walk.next(); /* the last group is padded with its last entry */
 #pragma unroll
                     for (int u = 0; u < 4; ++u) xj[u] = pos[v[u]];
-                    if (W == 1) {
+                    if (W == 1 && first == 0) {
                         if (list && k < kListMax)
                             reinterpret_cast<uint4 *>(list)[(size_t)(k >> 2) * (size_t)p.n + (size_t)i] =
                                 make_uint4(v[0], v[1], v[2], v[3]);
@@ -811,16 +812,14 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W, W == 1 ? kTileBl
                     for (int u = 0; u < 4; ++u)
                         if (k + u < count) add(u, xj[u]);
                 }
-                if (W > 1) {
+                if (W > 1 || first > 0) {
                     if (list && count && first + count == total && total < kListMax)
                         for (int k = total; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = last;
                     count = total;
                 }
             } else {
-                if (W > 1) {
-                    acc[0] = acc[1] = 0.0f;
-                    if (threadIdx.x >= 32u) return;
-                }
+                acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+                if (W > 1 && threadIdx.x >= 32u) return;
                 unsigned int last = (unsigned int)i;
                 count = 0;
                 walk_cells(
@@ -835,9 +834,10 @@ __global__ void __launch_bounds__(W == 1 ? kListBlock : 32 * W, W == 1 ? kTileBl
                     for (int k = count; (k & 3) != 0; ++k) list[list_at(k, i, p.n)] = last;
             }
             if (list && (W == 1 || threadIdx.x < 32u)) cnt[i] = count > kListMax ? kListOverflow : (unsigned char)count;
-            if (W == 1) sph_density_out(p, i, (acc[0] + acc[1]) + (acc[2] + acc[3]), pos, vel, dens, pres);
         });
-    if (W > 1) {
+    if (W == 1) {
+        if (valid) sph_density_out(p, i, (acc[0] + acc[1]) + (acc[2] + acc[3]), pos, vel, dens, pres);
+    } else {
         __shared__ double s_sum[W][32];
         s_sum[threadIdx.x >> 5][threadIdx.x & 31] = (double)acc[0] - (double)acc[1];
         __syncthreads();
@@ -1008,6 +1008,7 @@ __global__ void __launch_bounds__(kListBlock) k_nb_count(DevParams p, const unsi
                                 ++k;
                             }
                         };
+                        if (!found) k = 0;
                         if (found) {
                             for (int f = 0; f < count; ++f) {
                                 const unsigned int j = walk.next();

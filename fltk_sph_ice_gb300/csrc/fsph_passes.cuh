@@ -428,25 +428,28 @@ struct TileWalk {
     }
 };
 
-/* Calls emit(found, first, count, total, walk) for each valid lane: found:
- * the lane's `count` candidates within sqrt(r2max) come from walk, ascending;
- * else they have to be looked for without the tile (more than fit it, W = 1; lanes
- * far apart; or a coordinate out of the operands' range: a particle far outside the
- * box, or not a number).  load(j): slot j's position, a plain load where the
- * kernel writes beside it.  xi, cell: the lane's position and build cell, cells ascending over
- * the lanes, padding lanes (valid = false) after the valid ones; every lane of
- * the warp calls it.  Lanes in different rows of cells, or more than eight cells
- * apart (a run that wraps, sparse fluid), take turns: a row's range then never
- * reaches the next row, and no slot is met twice.  As many turns as fit the tile
- * are emitted together.
+/* Calls emit(found, first, count, total, walk) for each valid lane: found: the
+ * lane's `count` candidates within sqrt(r2max) come from walk, ascending; else they
+ * have to be looked for without the tile (lanes far apart, or a coordinate out of the
+ * operands' range: a particle far outside the box, or not a number).  load(j): slot
+ * j's position, a plain load where the kernel writes beside it.  xi, cell: the lane's
+ * position and build cell, cells ascending over the lanes, padding lanes (valid =
+ * false) after the valid ones; every lane of the warp calls it.  Lanes in different
+ * rows of cells, or more than eight cells apart (a run that wraps), take turns: a
+ * row's range then never reaches the next row, and no slot is met twice.  As many
+ * turns as fit the tile are emitted together.
+ *
  * W > 1: the W warps of a block share the same 32 slots (a lane's slot is the same
- * in each) and the tile.  Each takes a W-th of every turn's words and emits what
- * it found there: `count` of the lane's `total`, from the `first` on.  A turn that
- * does not fit the tile goes through it in parts, each emitted with the total so
- * far (a lane's own walk by one warp of the four took 178 us where the parts take
- * 37: the density of a dam break of 32,768 particles after 400 steps, 71 neighbours
- * on average).  found = false starts a lane again and is for warp 0 to act on.  A warp's twenty words in a row, latency bound, are the
- * pass of a small scene: 16 us at 6,912 slots with one warp, 10 with four.
+ * in each) and the tile.  Each takes a W-th of every turn's words and emits what it
+ * found there: `count` of the lane's `total`, from the `first` on.  A warp's twenty
+ * words in a row, latency bound, are the pass of a small scene: 16 us at 6,912 slots
+ * with one warp, 10 with four.
+ *
+ * In compressed fluid a turn that does not fit the tile goes through it in parts, each
+ * emitted with the total so far; found = false then starts a lane again (for W > 1 it
+ * is for warp 0 to act on).  The lanes' own walks, which one warp of the four did,
+ * took 178 us where the parts take 37: the density of a collapsing dam of 32,768
+ * particles with 71 neighbours on average; of 512,000 with 106 444 and 291.
  *
  * In sparse fluid (spray) the lanes share few candidates and a warp takes up to 32
  * turns: there each lane looks for its own, once the cells between the lanes, at
@@ -454,7 +457,7 @@ struct TileWalk {
  * list build in us, own / tile, at 1 M particles at random with one in (0.8 h)^3 129
  * / 128, h^3 125 / 143, (1.2 h)^3 100 / 145, (2 h)^3 58 / 252; with four warps, 30,000
  * particles, (0.8 h)^3 17 / 13, h^3 17 / 19, (1.2 h)^3 15 / 34, (2 h)^3 9 / 34.  At
- * rest the choice costs the batched build 815 -> 853 us, the others nothing. */
+ * rest the choice costs the batched build 815 -> 850 us, the others nothing. */
 constexpr int kTileApart = 24, kTileApartSplit = 36; /* one warp, several */
 template <int W, class Load, class Emit>
 __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
@@ -477,14 +480,14 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
     const bool apart = __reduce_add_sync(0xffffffffu, valid && lane > 0 ? min(cell - prev, 3u) : 0u) >
                        (unsigned int)(W == 1 ? kTileApart : kTileApartSplit);
     unsigned int todo = __ballot_sync(0xffffffffu, valid);
-    unsigned int resume = 0u; /* W > 1: the word at which a turn in parts goes on */
-    int base = 0;             /* and what its earlier parts found for the lane */
+    unsigned int resume = 0u; /* the word at which a turn in parts goes on */
+    int base = 0;             /* what its earlier parts found for the lane */
     while (todo) {
         int cnt = 0, w = 0;
-        unsigned int any = 0u, done = 0u, over = 0u, part = 0u;
+        unsigned int any = 0u, done = 0u, part = 0u;
         bool bad = false;
         if (apart) {
-            over = done = todo;
+            done = todo;
             todo = 0u;
         }
         while (todo) { /* turns, until the tile is full */
@@ -520,12 +523,6 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
             unsigned int n = words - lo;
             if (n > room) {
                 if (w) break; /* after what the tile holds now */
-                if (W == 1) {
-                    over = grp; /* never fits */
-                    done |= grp;
-                    todo &= ~grp;
-                    break;
-                }
                 part = grp;
                 n = room;
                 resume = lo + room;
@@ -570,8 +567,7 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 return load(min(q < total ? j : j - (q - total + 1u), (unsigned int)p.n - 1u));
             };
             /* this warp's words */
-            const unsigned int begin = W > 1 ? (lo + n * wid / W) * 32u : 0u;
-            const unsigned int end = W > 1 ? min(total, (lo + n * (wid + 1) / W) * 32u) : total;
+            const unsigned int begin = (lo + n * wid / W) * 32u, end = min(total, (lo + n * (wid + 1) / W) * 32u);
             unsigned int jn;
             float4 cn;
             if (W == 1 || begin < end) cn = fetch(begin, jn);
@@ -611,16 +607,14 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
                 cnt += __popc(m);
                 if (m) any |= 0x80000000u >> at;
             }
-            if (W > 1) {
-                w += (int)n;
-                if (part) break;
-            }
+            if (W > 1) w += (int)n;
+            if (part) break;
         }
         const int holder = 4 * (lane & 7) + (lane >> 3); /* the lane that counted this lane's slot */
         const int count = __shfl_sync(0xffffffffu, cnt, holder);
         const unsigned int some = __shfl_sync(0xffffffffu, any, holder);
         int first = 0, all = count;
-        bool found = !over;
+        bool found = !apart;
         if (W > 1) {
             t.cnt[wid][lane] = count;
             found = !__syncthreads_or(bad) && found;
@@ -635,7 +629,7 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
             found = !__any_sync(0xffffffffu, bad) && found;
             __syncwarp();
         }
-        if (W > 1 && !found) { /* whatever its earlier parts gave, the lane starts again */
+        if (!found) { /* whatever its earlier parts gave, the lane starts again */
             done |= part;
             todo &= ~part;
             part = resume = 0u;
@@ -643,7 +637,7 @@ __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsign
         if ((done | part) >> lane & 1u) {
             TileWalk<W> walk(t, some, count);
             emit(found, base + first, count, base + all, walk);
-            if (W > 1) base = (part >> lane & 1u) ? base + all : 0;
+            base = (part >> lane & 1u) ? base + all : 0;
         }
         /* the tile is free again */
         if (W > 1)
@@ -671,7 +665,7 @@ __device__ __forceinline__ void build_list_warp(const DevParams &p, int i, bool 
             if (W == 1 || threadIdx.x < 32u) build_list_body(p, i, cell_start, xb, cell, list, cnt);
             return;
         }
-        if (W == 1) {
+        if (W == 1 && first == 0) {
             const int most = min(count, kListMax);
             for (int k = 0; k < most; k += 4) {
                 unsigned int v[4];
