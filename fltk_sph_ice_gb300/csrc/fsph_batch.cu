@@ -107,8 +107,10 @@ __global__ void __launch_bounds__(BLOCK) kb_hash_parity(BatchArgs b, const float
     }
 }
 
-/* the blocks are kListBlock threads whatever the tiles' size: each walks its
- * tile kListBlock slots at a time */
+/* The blocks are kListBlock threads whatever the tiles' size: each walks its tile
+ * kListBlock slots at a time.  A block a tile, handed out as SMs fall free: the
+ * tiles differ more than the constants' copy costs (a step of 256 scenes takes 4,591
+ * us so, 4,644 with four times the resident blocks, 4,765 with those alone). */
 __global__ void __launch_bounds__(kListBlock) kb_build_list(BatchArgs b, const unsigned int *__restrict__ cell_start,
                                                             const float4 *__restrict__ xb,
                                                             const unsigned int *__restrict__ cellb,
@@ -374,8 +376,8 @@ void blaunch_hash_parity(const BLaunch &L, const float4 *p0, const float4 *p1, c
 }
 void blaunch_build_list(const BLaunch &L, const unsigned int *cell_start, const float4 *xb, const NbrLists &nl,
                         cudaStream_t s) {
-    kb_build_list<<<persistent_grid(kb_build_list, kListBlock, L.full.ntiles, L.sms), kListBlock, 0, s>>>(
-        L.full, cell_start, xb, nl.cellb, nl.list, nl.cnt);
+    kb_build_list<<<std::max(L.full.ntiles, 1), kListBlock, 0, s>>>(L.full, cell_start, xb, nl.cellb, nl.list,
+                                                                    nl.cnt);
 }
 unsigned int blaunch_lambda(const BLaunch &L, const DevParams &lp, const unsigned int *cell_start, float4 *p0,
                             float4 *p1, float *dens, DevCtl *ctl, ErrPartial *part, unsigned long long hw,

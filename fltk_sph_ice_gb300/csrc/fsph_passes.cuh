@@ -456,8 +456,7 @@ struct TileWalk {
  * most three a pair, are more than kTileApart (a lattice at rest has about 5).  The
  * list build in us, own / tile, at 1 M particles at random with one in (0.8 h)^3 129
  * / 128, h^3 125 / 143, (1.2 h)^3 100 / 145, (2 h)^3 58 / 252; with four warps, 30,000
- * particles, (0.8 h)^3 17 / 13, h^3 17 / 19, (1.2 h)^3 15 / 34, (2 h)^3 9 / 34.  At
- * rest the choice costs the batched build 815 -> 850 us, the others nothing. */
+ * particles, (0.8 h)^3 17 / 13, h^3 17 / 19, (1.2 h)^3 15 / 34, (2 h)^3 9 / 34. */
 constexpr int kTileApart = 24, kTileApartSplit = 36; /* one warp, several */
 template <int W, class Load, class Emit>
 __device__ __forceinline__ void warp_candidates(const DevParams &p, const unsigned int *__restrict__ cell_start,
