@@ -353,7 +353,9 @@ int fsph_sph_eval_forces(fsph_ctx *ctx, const float *pos4, const float *vel4, in
  *   - pos4, dens and lambda are DEVICE pointers owned by the caller
  *     (n float4 in, n floats out each), in particle order.  No context is used,
  *     so static boundary particles (fsph_set_boundary) never enter: the
- *     results equal fsph_pbf_eval_lambda's only for a context without a boundary.
+ *     results agree with fsph_pbf_eval_lambda's (to the rounding of sums that
+ *     several lanes take, compensated or not as params asks) only for a context
+ *     without a boundary.
  *   - It allocates nothing: no cudaMalloc / cudaFree / allocating library call.
  *     Its working memory (grid tables, sorted copies) is one file-scope
  *     __device__ array that every GPU loading the library holds until exit.
